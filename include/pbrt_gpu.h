@@ -317,7 +317,7 @@ enum {
     PBRT_TRACE_PAIR_PERSISTENT = 1, /* binary pairs, persistent warps */
     PBRT_TRACE_WIDE = 2,            /* 4-wide nodes, one thread per ray */
     PBRT_TRACE_WIDE_PERSISTENT = 3, /* 4-wide nodes, persistent warps */
-    PBRT_TRACE_WIDE_SPECULATIVE = 4, /* 4-wide nodes, persistent warps, leaves tested in warp-wide rounds */
+    PBRT_TRACE_WIDE_SPECULATIVE = 4, /* the same walk as PBRT_TRACE_WIDE_PERSISTENT */
     PBRT_TRACE_PAIR_PACKET = 5       /* binary pairs, one thread per ray; a warp whose rays share their
                                         direction signs walks them together, node by node, each lane
                                         testing what its own walk tests (coherent rays) */
@@ -325,8 +325,9 @@ enum {
 typedef struct PbrtTraceConfig {
     int32_t kernel;         /* PBRT_TRACE_*: pbrtgpu_intersect / intersect_p batches */
     uint32_t refill;        /* persistent kernels: refill a warp when this many lanes idle */
-    uint32_t min_blocks;    /* 4-wide persistent kernel: 0, or 7 / 8 / 9 resident 128-thread
-                               blocks per SM requested (fewer registers per thread) */
+    uint32_t min_blocks;    /* 0, 7, 8 or 9: no effect on the walk, whose 64 registers per thread
+                               keep 8 128-thread blocks per SM resident; host-buffer calls
+                               are streamed with 0 only */
     int32_t render_kernel;  /* PBRT_TRACE_*: camera rays inside pbrtgpu_render; shadow
                                rays take the 4-wide kernel with a 4-wide choice, else
                                the binary one */

@@ -11,6 +11,8 @@
 // trace4.cuh), so results are the same bit for bit.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "batch.h"
 #include "kernels.h"
 #include "trace.cuh"
@@ -68,37 +70,12 @@ struct WorkSource {
 // every ray, or each job's own choice.
 enum { kClosest = 0, kAny = 1, kPerJob = 2 };
 
-template <bool WIDE, int S1, int S2>
-struct Walker;  // traversal state over one layout
-
-template <int SMAX, int OVF>
-struct Walker<true, SMAX, OVF> {
-    Traversal4<SMAX, OVF> T;
-    DevBVH4 bv;
-    __device__ __forceinline__ void bind(uint2* smem) { T.bind(smem, threadIdx.x, blockDim.x); }
-    __device__ __forceinline__ bool start(const RenderParams& P, const DRay& r) {
-        bv = P.bvh4;
-        return T.start(bv, r);
-    }
-    template <int MODE>
-    __device__ __forceinline__ bool step(const DRay& r, bool any) {
-        if (MODE == kClosest) return T.template step<false>(bv, r);
-        if (MODE == kAny) return T.template step<true>(bv, r);
-        return any ? T.template step<true>(bv, r) : T.template step<false>(bv, r);
-    }
-    __device__ __forceinline__ int failure() const { return T.overflow ? 6 : 0; }
-    __device__ __forceinline__ bool found() const { return T.found; }
-    __device__ __forceinline__ bool nan_hit() const { return T.nan_hit; }
-    __device__ __forceinline__ const TraceResult& res() const { return T.res; }
-};
-
 // INST = 1: the tree may hold instances (Traversal with INST).
 template <int STACK, int INST>
-struct Walker<false, STACK, INST> {
+struct Walker {
     Traversal<STACK, INST != 0> T;
     DevBVH bv;
     int st = 0;
-    __device__ __forceinline__ void bind(uint2*) {}
     __device__ __forceinline__ bool start(const RenderParams& P, const DRay& r) {
         bv = P.bvh;
         return T.start(bv, r);
@@ -117,9 +94,8 @@ struct Walker<false, STACK, INST> {
 
 // SHADOW = false: extend over the job rays; true: the shadow queue (any
 // hit, MODE = kAny).
-template <int BLOCK, bool SHADOW, bool WIDE, int S1, int S2, int MODE>
+template <int BLOCK, bool SHADOW, int S1, int S2, int MODE>
 __global__ void __launch_bounds__(BLOCK) kb_trace(BatchArgs A) {
-    extern __shared__ uint2 smem_stack[];
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t nj = A.hdr->n_jobs;
     const uint64_t n = SHADOW ? (uint64_t) * (volatile uint32_t*)(A.counters + kCtrShadowCount) : A.hdr->rays;
@@ -127,8 +103,7 @@ __global__ void __launch_bounds__(BLOCK) kb_trace(BatchArgs A) {
     const uint32_t refill = SHADOW ? A.refill_shadow : A.refill;
     WorkSource W;
     Cursor c{0, 1, 0};
-    Walker<WIDE, S1, S2> K;
-    K.bind(smem_stack);
+    Walker<S1, S2> K;
     DRay r;
     bool busy = false, any = MODE == kAny;
     uint32_t job = 0;
@@ -192,9 +167,14 @@ __global__ void __launch_bounds__(BLOCK) kb_trace(BatchArgs A) {
 // order, so the results equal kb_trace's (measured on GB300, the
 // 1024x1024x16 heightfield frame as one job: extend 3.47 -> 2.3 ms, shadow
 // 3.28 -> 2.3 ms, as with the single-render kernels).
+// WIDE: the 4-wide layout, S1 stack rows in shared memory, S2 overflow
+// entries; else the binary layout, S1 stack entries, S2 = 1 with instances.
 template <int BLOCK, bool SHADOW, bool WIDE, int S1, int S2, int MODE>
-__global__ void __launch_bounds__(BLOCK) kb_trace_flat(BatchArgs A) {
-    extern __shared__ uint2 smem_stack[];
+__global__ void __launch_bounds__(BLOCK, WIDE ? 1024 / BLOCK : 1) kb_trace_flat(BatchArgs A) {
+    using Closest = Walk4<BLOCK, WIDE ? S1 : 16, WIDE ? S2 : 64, false>;
+    using Any = Walk4<BLOCK, WIDE ? S1 : 16, WIDE ? S2 : 64, true>;
+    __shared__ typename std::conditional<WIDE, typename Closest::Shared, int>::type sh;
+    if constexpr (WIDE) sh.init();
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t nj = A.hdr->n_jobs;
     const uint64_t n = SHADOW ? (uint64_t) * (volatile uint32_t*)(A.counters + kCtrShadowCount) : A.hdr->rays;
@@ -222,48 +202,53 @@ __global__ void __launch_bounds__(BLOCK) kb_trace_flat(BatchArgs A) {
             }
             const JobRec& J = A.jobs[job];
             const bool any = MODE == kAny || (MODE == kPerJob && J.any != 0);
-            const DRay r = make_dray(__ldg(src), __ldg(src + 1));
-            TraceResult res;
-            int fail = 0;
-            bool nan = false, found;
-            if (WIDE) {
-                Traversal4<S1, S2> T;
-                T.bind(smem_stack, threadIdx.x, blockDim.x);
-                // by reference: the walk reads the tree's arrays from the job
-                // table (L1) instead of holding them in registers (80 -> 72,
-                // one more block per SM); the per-job mode keeps its copy
-                // (it spills without it)
-                const DevBVH4 bv_copy = MODE == kPerJob ? J.P.bvh4 : DevBVH4{};
-                const DevBVH4& bv = MODE == kPerJob ? bv_copy : J.P.bvh4;
-                if (T.start(bv, r)) {
-                    if (any) {
-                        while (T.template step<true>(bv, r)) {
-                        }
-                    } else {
-                        while (T.template step<false>(bv, r)) {
-                        }
-                    }
+            int* status = (int*)(J.P.counters + 2);
+            float4 hit = make_float4(0, 0, 0, 0);
+            bool found;
+            if constexpr (WIDE) {
+                // the walk reads the tree's arrays from the job table (L1)
+                // instead of holding them in registers
+                const DevBVH4& bv = J.P.bvh4;
+                typename Closest::Ovf ov;
+                auto walk = [&](auto& T, bool* exact) {
+                    T.bind(sh);
+                    const int st = T.start(bv, __ldg(src), __ldg(src + 1));
+                    if (st == kStartWalk) T.run(bv, sh, ov);
+                    if (T.spilled < 0) atomicMax(status, 6);
+                    *exact = st == kStartExact || T.give_up;
+                };
+                bool exact;
+                if (any) {
+                    Any T;
+                    walk(T, &exact);
+                    found = exact ? exact_any<S2 + 8, false>(bv.pair, src, status) : T.found();
+                } else {
+                    Closest T;
+                    walk(T, &exact);
+                    hit = exact ? exact_hit<S2 + 8, false>(bv.pair, src, status) : T.hit_record();
+                    found = false;
                 }
-                found = T.found;
-                nan = T.nan_hit;
-                res = T.res;
-                fail = T.overflow ? 6 : 0;
             } else {
                 const DevBVH& bv = J.P.bvh;  // from the job table, as above
+                const DRay r = make_dray(__ldg(src), __ldg(src + 1));
+                TraceResult res;
+                int fail = 0;
+                bool nan = false;
                 found = any ? traverse<S1, true, S2 != 0>(bv, r, &res, &fail)
                             : traverse<S1, false, S2 != 0>(bv, r, &res, &fail, &nan);
+                if (fail) atomicMax(status, fail);
+                hit = make_float4(__int_as_float(res.prim), res.t, res.b1, res.b2);
+                if (!any && nan) {  // rewritten by the replay stage
+                    hit = make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f);
+                    A.counters[kCtrReplay] = 1u;
+                }
             }
-            if (fail) atomicMax((int*)(J.P.counters + 2), fail);
-            if (SHADOW) {
+            if (SHADOW)
                 J.P.occluded[__ldg(A.q_slot + item)] = found ? 1 : 0;
-            } else if (any) {
+            else if (any)
                 J.occ[item] = found ? 1 : 0;
-            } else if (nan) {  // rewritten by the replay stage
-                J.hits[item] = make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f);
-                A.counters[kCtrReplay] = 1u;
-            } else {
-                J.hits[item] = make_float4(__int_as_float(res.prim), res.t, res.b1, res.b2);
-            }
+            else
+                J.hits[item] = hit;
         }
     }
 }
@@ -272,16 +257,19 @@ __global__ void __launch_bounds__(BLOCK) kb_trace_flat(BatchArgs A) {
 // walk (k_trace4_persistent): a lane keeps only its ray, its job and its
 // item, finds the job by a fresh binary search when it takes a ray, and
 // reads the job's tree from the job table at each step instead of holding
-// a copy, so the kernel fits the registers of 7 blocks of 128 per SM.
-// Idle lanes take new rays once `refill` of them are idle.  Each ray's walk
-// is the same as in the other stage kernels, so are the results.
+// a copy.  Idle lanes take new rays once `refill` of them are idle.  Each
+// ray's walk is the same as in the other stage kernels, so are the results.
 template <int BLOCK, bool SHADOW, int S1, int S2, int MODE>
-__global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs A) {
-    extern __shared__ uint2 smem_stack[];
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) kb_trace4_refill(BatchArgs A) {
+    // per job: every ray takes a closest-hit walk, which an any-hit job's
+    // rays leave at their first hit
+    using Walk = Walk4<BLOCK, S1, S2, MODE == kAny>;
+    __shared__ typename Walk::Shared sh;
+    sh.init();
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t nj = A.hdr->n_jobs;
     const uint32_t n =
-        SHADOW ? *(volatile uint32_t*)(A.counters + kCtrShadowCount) : (uint32_t)A.hdr->rays;  // < 2^32 (launch)
+        SHADOW ? *(volatile uint32_t*)(A.counters + kCtrShadowCount) : (uint32_t)A.hdr->rays;  // < 2^31 (batch limits)
     uint32_t* counter = A.counters + (SHADOW ? kCtrShadowWork : kCtrExtendWork);
     const uint32_t refill = SHADOW ? A.refill_shadow : A.refill;
     constexpr uint32_t kNone = 0xffffffffu;
@@ -289,23 +277,22 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs
     bool more = true;
     uint32_t job = kNone, item = 0;
     bool any = MODE == kAny;
-    DRay r;
-    Traversal4<S1, S2> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
-    auto finish = [&]() {
+    Walk T;
+    typename Walk::Ovf ov;
+    T.bind(sh);
+    auto finish = [&](bool exact) {
         const JobRec& J = A.jobs[job];
-        if (T.overflow) atomicMax((int*)(J.P.counters + 2), 6);
-        if (SHADOW) {
-            J.P.occluded[__ldg(A.q_slot + item)] = T.found ? 1 : 0;
-        } else if (any) {
-            J.occ[item] = T.found ? 1 : 0;
-        } else if (T.nan_hit) {  // rewritten by the replay stage
-            J.hits[item] = make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f);
-            A.counters[kCtrReplay] = 1u;
-        } else {
-            J.hits[item] = make_float4(__int_as_float(T.res.prim), T.res.t, T.res.b1, T.res.b2);
-        }
+        if (T.spilled < 0) atomicMax((int*)(J.P.counters + 2), 6);
+        if (exact) A.counters[SHADOW ? kCtrReplayShadow : kCtrReplay] = 1u;  // rewritten by the replay stage
+        const uint8_t found = exact ? kReplayOcc : (T.found() ? 1 : 0);
+        if (SHADOW)
+            J.P.occluded[__ldg(A.q_slot + item)] = found;
+        else if (any)
+            J.occ[item] = found;
+        else
+            J.hits[item] = exact ? make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f) : T.hit_record();
         job = kNone;
+        T.cur = kWalkDone;
     };
     for (;;) {
         const unsigned idle = __ballot_sync(kFull, job == kNone);
@@ -338,8 +325,8 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs
                         if (MODE == kPerJob) any = A.jobs[job].any != 0;
                         src = A.jobs[job].rays + 2 * (size_t)item;
                     }
-                    r = make_dray(__ldg(src), __ldg(src + 1));
-                    if (!T.start(A.jobs[job].P.bvh4, r)) finish();
+                    const int st = T.start(A.jobs[job].P.bvh4, __ldg(src), __ldg(src + 1));
+                    if (st != kStartWalk) finish(st == kStartExact);
                 }
             }
             next += nidle;
@@ -350,39 +337,39 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs
         }
         if (job != kNone) {
             const DevBVH4& bv = A.jobs[job].P.bvh4;
-            bool going;
-            if (MODE == kClosest)
-                going = T.template step<false>(bv, r);
-            else if (MODE == kAny)
-                going = T.template step<true>(bv, r);
-            else
-                going = any ? T.template step<true>(bv, r) : T.template step<false>(bv, r);
-            if (!going) finish();
+#pragma unroll
+            for (int k = 0; k < 3; ++k)  // visits per turn, as in k_trace4_persistent
+                if ((int32_t)T.cur >= 0) T.node(bv, ov);
+            if ((int32_t)T.cur < 0 && T.cur != kWalkDone) {
+                T.leaf(bv, sh, ov);
+                if (MODE == kPerJob && any && T.found()) T.stop();
+            }
+            if (T.cur == kWalkDone && !T.resume(ov)) finish(!any && T.give_up);
         }
     }
 }
 
-// The exact replay of the closest hits the extend stage marked (see
-// Traversal in trace.cuh): the binary walk with instances allowed; returns
+// The exact replay of what a traversal stage marked (see Traversal in
+// trace.cuh, and trace4.cuh): the binary walk with instances allowed; returns
 // at once when nothing was marked.
-template <int BLOCK>
+template <int BLOCK, bool SHADOW>
 __global__ void __launch_bounds__(BLOCK) kb_replay(BatchArgs A) {
-    if (*(const volatile uint32_t*)(A.counters + kCtrReplay) == 0u) return;
-    const uint64_t n = A.hdr->rays;
+    if (*(const volatile uint32_t*)(A.counters + (SHADOW ? kCtrReplayShadow : kCtrReplay)) == 0u) return;
+    const uint64_t n = SHADOW ? (uint64_t) * (volatile uint32_t*)(A.counters + kCtrShadowCount) : A.hdr->rays;
     const uint32_t nj = A.hdr->n_jobs;
     Cursor c{0, 1, 0};
     for (uint64_t g = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; g < n; g += (uint64_t)gridDim.x * BLOCK) {
-        const uint32_t j = locate(A.off_ray, nj, g, c);
+        const uint32_t j = SHADOW ? __ldg(A.q_job + g) : locate(A.off_ray, nj, g, c);
         const JobRec& J = A.jobs[j];
-        if (J.any) continue;
-        const uint64_t item = g - c.lo;
-        if (__float_as_int(J.hits[item].x) != kReplayMark) continue;
-        const DRay r = make_dray(__ldg(J.rays + 2 * item), __ldg(J.rays + 2 * item + 1));
-        TraceResult res;
-        int st = 0;
-        traverse<256, false, true, true>(J.P.bvh, r, &res, &st);
-        if (st) atomicMax((int*)(J.P.counters + 2), st);
-        J.hits[item] = make_float4(__int_as_float(res.prim), res.t, res.b1, res.b2);
+        int* status = (int*)(J.P.counters + 2);
+        const uint64_t item = SHADOW ? g : g - c.lo;
+        if (SHADOW || J.any) {
+            uint8_t* occ = SHADOW ? J.P.occluded + __ldg(A.q_slot + g) : J.occ + item;
+            const float4* ray = SHADOW ? reinterpret_cast<const float4*>(A.q_rays) + 2 * g : J.rays + 2 * item;
+            if (*occ == kReplayOcc) *occ = exact_any<256, true>(J.P.bvh, ray, status) ? 1 : 0;
+        } else if (__float_as_int(J.hits[item].x) == kReplayMark) {
+            J.hits[item] = exact_hit<256, true>(J.P.bvh, J.rays + 2 * item, status);
+        }
     }
 }
 
@@ -390,31 +377,31 @@ __global__ void __launch_bounds__(BLOCK) kb_replay(BatchArgs A) {
 template <int BLOCK, bool SHADOW, bool WIDE, int S1, int S2, int MODE, bool FLAT>
 cudaError_t go(const BatchArgs& A, int sms, cudaStream_t s) {
     static ShapeCache bps_cache;
-    const size_t smem = WIDE ? (size_t)S1 * sizeof(uint2) * BLOCK : 0;
     auto pick_kernel = [] {
         if constexpr (FLAT)
             return kb_trace_flat<BLOCK, SHADOW, WIDE, S1, S2, MODE>;
         else if constexpr (WIDE)
             return kb_trace4_refill<BLOCK, SHADOW, S1, S2, MODE>;
         else
-            return kb_trace<BLOCK, SHADOW, WIDE, S1, S2, MODE>;
+            return kb_trace<BLOCK, SHADOW, S1, S2, MODE>;
     };
     auto kernel = pick_kernel();
-    const int bps = resident_blocks(bps_cache, kernel, BLOCK, smem);
-    kernel<<<(unsigned)(sms * bps), BLOCK, smem, s>>>(A);
+    const int bps = resident_blocks(bps_cache, kernel, BLOCK, 0);
+    kernel<<<(unsigned)(sms * bps), BLOCK, 0, s>>>(A);
     return cudaGetLastError();
 }
 
+// The 4-wide kernels' shared stack has 16 rows (stack = 16) or 12 (stack = 8).
 template <int BLOCK, bool SHADOW, int MODE, bool FLAT>
 cudaError_t pick_layout(const BatchArgs& A, const BatchTuning& T, bool wide, bool inst, uint32_t cover, int sms,
                         cudaStream_t s) {
     if (inst) return go<BLOCK, SHADOW, false, 256, 1, MODE, FLAT>(A, sms, s);
     if (wide) {
         if (T.smax == 8)
-            return cover <= 64 ? go<BLOCK, SHADOW, true, 8, 56, MODE, FLAT>(A, sms, s)
-                               : go<BLOCK, SHADOW, true, 8, 248, MODE, FLAT>(A, sms, s);
-        return cover <= 64 ? go<BLOCK, SHADOW, true, 16, 48, MODE, FLAT>(A, sms, s)
-                           : go<BLOCK, SHADOW, true, 16, 240, MODE, FLAT>(A, sms, s);
+            return cover <= 64 ? go<BLOCK, SHADOW, true, 12, 64, MODE, FLAT>(A, sms, s)
+                               : go<BLOCK, SHADOW, true, 12, 256, MODE, FLAT>(A, sms, s);
+        return cover <= 64 ? go<BLOCK, SHADOW, true, 16, 64, MODE, FLAT>(A, sms, s)
+                           : go<BLOCK, SHADOW, true, 16, 256, MODE, FLAT>(A, sms, s);
     }
     return cover <= 64 ? go<BLOCK, SHADOW, false, 64, 0, MODE, FLAT>(A, sms, s)
                        : go<BLOCK, SHADOW, false, 256, 0, MODE, FLAT>(A, sms, s);
@@ -438,11 +425,12 @@ cudaError_t pick_block(const BatchArgs& A, const BatchTuning& T, bool shadow, bo
 
 }  // namespace
 
-cudaError_t launch_batch_replay(const BatchArgs& A, const BatchTuning& T, int sms, cudaStream_t s) {
+cudaError_t launch_batch_replay(const BatchArgs& A, const BatchTuning& T, bool shadow, int sms, cudaStream_t s) {
+    auto go = [&](auto kernel, int blocks) { kernel<<<(unsigned)(sms * blocks), T.block, 0, s>>>(A); };
     if (T.block == 256)
-        kb_replay<256><<<(unsigned)(sms * 2), 256, 0, s>>>(A);
+        shadow ? go(kb_replay<256, true>, 2) : go(kb_replay<256, false>, 2);
     else
-        kb_replay<128><<<(unsigned)(sms * 4), 128, 0, s>>>(A);
+        shadow ? go(kb_replay<128, true>, 4) : go(kb_replay<128, false>, 4);
     return cudaGetLastError();
 }
 

@@ -91,6 +91,42 @@ static int upload(T** dst, const std::vector<T>& src) {
     return cuda_status(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy");
 }
 
+// The 4-wide layout of a tree whose pairs are on the device; *out stays null
+// for a tree without one (or of one leaf).
+static int make_quads(const HostBVH& H, const NodePair* d_pairs, QuadNode** out) {
+    *out = nullptr;
+    if (!H.wide || H.n_quads == 0) return PBRT_OK;
+    uint32_t* quad_of = nullptr;
+    int st;
+    if ((st = cuda_status(cudaMalloc((void**)out, (size_t)H.n_quads * sizeof(QuadNode)), "cudaMalloc"))) return st;
+    if (!(st = upload(&quad_of, H.quad_of)) &&
+        !(st = cuda_status(launch_make_quads(d_pairs, quad_of, (uint32_t)H.pairs.size(), (uint32_t)H.ordered.size(),
+                                             *out, 0),
+                           "4-wide layout")))
+        st = cuda_status(cudaStreamSynchronize(0), "4-wide layout");
+    if (quad_of) cudaFree(quad_of);
+    return st;
+}
+
+// A tree's device record from its arrays.
+static DevBVH4 device_tree(const HostBVH& H, const NodePair* pairs, const QuadNode* quads, const LeafBox* boxes,
+                           const PrimRec* prims, const SphereRec* spheres, const DevBVH4* insts) {
+    DevBVH4 d{};
+    d.pair.pairs = pairs;
+    d.pair.prims = prims;
+    d.pair.spheres = spheres;
+    d.pair.root = H.root;
+    d.pair.has_spheres = H.has_spheres ? 1u : 0u;
+    d.pair.n_prims = (uint32_t)H.ordered.size();
+    d.pair.empty = H.nodes.empty() ? 1u : 0u;
+    d.pair.insts = insts;
+    d.nodes = quads;
+    d.boxes = boxes;
+    d.root_ref = H.quad_root;
+    d.reach = H.reach;
+    return d;
+}
+
 int bvh_upload(PbrtBVH* b) {
     std::lock_guard<std::mutex> lk(b->upload_mu);
     if (b->uploaded) return PBRT_OK;
@@ -99,54 +135,43 @@ int bvh_upload(PbrtBVH* b) {
     if ((st = upload(&b->d_pairs, b->host.pairs))) return st;
     if ((st = upload(&b->d_prims, b->host.recs))) return st;
     if ((st = upload(&b->d_spheres, b->host.spheres))) return st;
-    if ((st = upload(&b->d_nodes4, b->host.nodes4))) return st;
+    if ((st = upload(&b->d_leaf_boxes, b->host.leaf_boxes))) return st;
+    if ((st = make_quads(b->host, b->d_pairs, &b->d_quads))) return st;
     if ((st = cuda_status(cudaMalloc(&b->d_status, sizeof(int)), "cudaMalloc"))) return st;
     if ((st = cuda_status(cudaMemset(b->d_status, 0, sizeof(int)), "cudaMemset"))) return st;
-    // instance definitions: 4-wide layout, walked by instance_test
+    // instance definitions
     std::vector<DevBVH4> defs;
     for (const HostBVH& I : b->host.insts) {
-        Node4* nodes = nullptr;
+        NodePair* pairs = nullptr;
+        QuadNode* quads = nullptr;
+        LeafBox* boxes = nullptr;
         PrimRec* prims = nullptr;
         SphereRec* spheres = nullptr;
-        st = upload(&nodes, I.nodes4);
-        if (nodes) b->d_inst_bufs.push_back(nodes);
+        st = upload(&pairs, I.pairs);
+        if (pairs) b->d_inst_bufs.push_back(pairs);
+        if (!st) st = make_quads(I, pairs, &quads);
+        if (quads) b->d_inst_bufs.push_back(quads);
+        if (!st) st = upload(&boxes, I.leaf_boxes);
+        if (boxes) b->d_inst_bufs.push_back(boxes);
         if (!st) st = upload(&prims, I.recs);
         if (prims) b->d_inst_bufs.push_back(prims);
         if (!st) st = upload(&spheres, I.spheres);
         if (spheres) b->d_inst_bufs.push_back(spheres);
         if (st) return st;
-        DevBVH4 d{};
-        d.nodes = nodes;
-        d.prims = prims;
-        d.spheres = spheres;
-        d.root = I.root4;
-        d.empty = I.nodes.empty() ? 1u : 0u;
-        d.insts = nullptr;
-        defs.push_back(d);
+        defs.push_back(device_tree(I, pairs, quads, boxes, prims, spheres, nullptr));
     }
     b->inst_dev = defs;
     if ((st = upload(&b->d_insts, defs))) return st;
-    b->dev.insts = b->d_insts;
-    b->dev4.insts = b->d_insts;
-    b->dev.pairs = b->d_pairs;
-    b->dev.prims = b->d_prims;
-    b->dev.spheres = b->d_spheres;
-    b->dev.root = b->host.root;
-    b->dev.has_spheres = b->host.has_spheres ? 1u : 0u;
-    b->dev.n_prims = (uint32_t)b->host.recs.size();
-    b->dev.empty = b->host.nodes.empty() ? 1u : 0u;
-    b->dev4.nodes = b->d_nodes4;
-    b->dev4.prims = b->d_prims;
-    b->dev4.spheres = b->d_spheres;
-    b->dev4.root = b->host.root4;
-    b->dev4.empty = b->dev.empty;
+    b->dev4 = device_tree(b->host, b->d_pairs, b->d_quads, b->d_leaf_boxes, b->d_prims, b->d_spheres, b->d_insts);
+    b->dev = b->dev4.pair;
     b->uploaded = true;
     return PBRT_OK;
 }
 
-// The 4-wide layout when a compiled variant covers its stack bound.
+// The 4-wide layout when the tree has one and a compiled variant covers its
+// stack bound.
 const DevBVH4* wide_of(const PbrtBVH* b) {
-    return wide_stack_variant(b->host.stack4_bound) ? &b->dev4 : nullptr;
+    return b->host.wide && wide_stack_variant(b->host.stack4_bound) ? &b->dev4 : nullptr;
 }
 
 // Stream-ordered scratch for per-call temporaries (the ray permutation):
@@ -554,7 +579,8 @@ PbrtBVH::~PbrtBVH() {
     if (d_pairs) cudaFree(d_pairs);
     if (d_prims) cudaFree(d_prims);
     if (d_spheres) cudaFree(d_spheres);
-    if (d_nodes4) cudaFree(d_nodes4);
+    if (d_quads) cudaFree(d_quads);
+    if (d_leaf_boxes) cudaFree(d_leaf_boxes);
     if (d_status) cudaFree(d_status);
     stage_in.release();
     stage_out.release();
@@ -659,10 +685,13 @@ int pbrtgpu_bvh_num_primitives(const PbrtBVH* b, uint32_t* n) {
 int pbrtgpu_bvh_device_bytes(const PbrtBVH* b, uint64_t* bytes) {
     if (!b || !bytes) return set_error(PBRT_ERR_INVALID_ARGUMENT, "NULL argument");
     const HostBVH& H = b->host;
-    uint64_t n = H.pairs.size() * sizeof(NodePair) + H.recs.size() * sizeof(PrimRec) +
-                 H.spheres.size() * sizeof(SphereRec) + H.nodes4.size() * sizeof(Node4) + sizeof(int);
-    for (const HostBVH& I : H.insts)
-        n += I.nodes4.size() * sizeof(Node4) + I.recs.size() * sizeof(PrimRec) + I.spheres.size() * sizeof(SphereRec);
+    auto tree = [](const HostBVH& T) -> uint64_t {
+        return T.pairs.size() * sizeof(NodePair) + (T.wide ? (uint64_t)T.n_quads * sizeof(QuadNode) : 0) +
+               T.leaf_boxes.size() * sizeof(LeafBox) + T.recs.size() * sizeof(PrimRec) +
+               T.spheres.size() * sizeof(SphereRec);
+    };
+    uint64_t n = tree(H) + sizeof(int);
+    for (const HostBVH& I : H.insts) n += tree(I);
     n += H.insts.size() * sizeof(DevBVH4);
     *bytes = n;
     return PBRT_OK;

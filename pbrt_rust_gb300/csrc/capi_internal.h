@@ -43,7 +43,8 @@ struct PbrtBVH {
     pbrt::NodePair* d_pairs = nullptr;
     pbrt::PrimRec* d_prims = nullptr;
     pbrt::SphereRec* d_spheres = nullptr;
-    pbrt::Node4* d_nodes4 = nullptr;
+    pbrt::QuadNode* d_quads = nullptr;   // 4-wide layout (trees that have it)
+    pbrt::LeafBox* d_leaf_boxes = nullptr;
     pbrt::DevBVH4* d_insts = nullptr;    // per instance definition
     std::vector<void*> d_inst_bufs;      // the definitions' device arrays
     std::vector<pbrt::DevBVH4> inst_dev;  // host copy of d_insts

@@ -177,7 +177,7 @@ static int scene_upload(PbrtScene* S) {
         st = up(&sh, S->inst_shade[k]);
         if (sh) S->d_inst_bufs.push_back(sh);
         if (st) return st;
-        defs.push_back(InstShade{sh, S->bvh->inst_dev[k].spheres});
+        defs.push_back(InstShade{sh, S->bvh->inst_dev[k].pair.spheres});
     }
     if ((st = up(&S->d_inst_defs, defs))) return st;
     // the no-allocation render's scratch is set up with the scene, not in

@@ -425,24 +425,24 @@ static void fill_device_layout(HostBVH& H) {
         p.c[1] = rec(nd.offset);
     }
     if (m) H.root = rec(0);
-    H.recs.resize(H.ordered.size());
+    H.recs.resize(H.ordered.size() + 1);  // and the null record
+    std::memset(&H.recs.back(), 0, sizeof(PrimRec));
     for (size_t i = 0; i < H.ordered.size(); ++i) {
         const HostPrim& p = H.prims[H.ordered[i]];
         PrimRec& r = H.recs[i];
         std::memset(&r, 0, sizeof(r));
         uint32_t id = H.flat_id.empty() ? H.ordered[i] : H.flat_id[H.ordered[i]];
         if (p.kind == PBRT_SHAPE_TRIANGLE_MESH) {
-            V3 e1 = p.p2 - p.p1, e2 = p.p3 - p.p1;  // mesh.rs:45-46
             r.r0[0] = p.p1.x;
             r.r0[1] = p.p1.y;
             r.r0[2] = p.p1.z;
             std::memcpy(&r.r0[3], &id, 4);
-            r.r1[0] = e1.x;
-            r.r1[1] = e1.y;
-            r.r1[2] = e1.z;
-            r.r2[0] = e2.x;
-            r.r2[1] = e2.y;
-            r.r2[2] = e2.z;
+            r.r1[0] = p.p2.x;
+            r.r1[1] = p.p2.y;
+            r.r1[2] = p.p2.z;
+            r.r2[0] = p.p3.x;
+            r.r2[1] = p.p3.y;
+            r.r2[2] = p.p3.z;
         } else {
             uint32_t tagged = id | kSphereBit;
             uint32_t si = (uint32_t)p.sphere;
@@ -452,88 +452,78 @@ static void fill_device_layout(HostBVH& H) {
     }
 }
 
-// Collapse the binary tree two levels at a time (see layout.h: Node4) and
-// mark the last primitive of every leaf.
-static void fill_node4_layout(HostBVH& H) {
+// Where the 4-wide nodes start (two binary levels each, see layout.h:
+// QuadNode), the primitive flags of the 4-wide walk with the leaf boxes they
+// refer to, and whether the tree can have that layout at all.
+static void fill_quad_layout(HostBVH& H) {
     const size_t m = H.nodes.size();
-    H.nodes4.clear();
+    H.quad_of.assign(H.pairs.size(), kNoQuad);
+    H.leaf_boxes.clear();
+    H.n_quads = 0;
+    H.quad_root = 0;
     H.stack4_bound = 0;
+    H.reach = 0.0f;
+    auto set_flags = [&](size_t i, uint32_t f) {
+        uint32_t v;
+        std::memcpy(&v, &H.recs[i].r2[3], 4);
+        v |= f;
+        std::memcpy(&H.recs[i].r2[3], &v, 4);
+    };
+    set_flags(H.recs.size() - 1, kPrimLastBit);
+    H.wide = H.ordered.size() < 0x7ffffff0u && H.pairs.size() < (1u << kQuadAxisShift);
+    auto usable = [](float v) { return std::fabs(v) <= kWideReach; };  // false for NaN
+    auto usable3 = [&](V3 v) { return usable(v.x) && usable(v.y) && usable(v.z); };
     for (size_t k = 0; k < m; ++k) {
         const FlatNode& nd = H.nodes[k];
-        if (nd.leaf && nd.count > 0) {
-            uint32_t last = nd.offset + nd.count - 1;
-            uint32_t flag = kPrimLastBit;
-            std::memcpy(&H.recs[last].r2[3], &flag, 4);
+        if (!nd.leaf || nd.count == 0) continue;
+        H.wide = H.wide && usable3(nd.box.lo) && usable3(nd.box.hi);
+        for (uint32_t i = 0; i < nd.count; ++i) {
+            const HostPrim& p = H.prims[H.ordered[nd.offset + i]];
+            if (p.kind == PBRT_SHAPE_TRIANGLE_MESH)
+                H.wide = H.wide && usable3(p.p1) && usable3(p.p2) && usable3(p.p3);
         }
+        set_flags(nd.offset + nd.count - 1, kPrimLastBit);
+        const HostPrim& first = H.prims[H.ordered[nd.offset]];
+        if (nd.count == 1 && first.kind == PBRT_SHAPE_TRIANGLE_MESH) {
+            set_flags(nd.offset, kPrimOwnBox);
+            continue;
+        }
+        const bool entry = nd.count > 1 || H.spheres[first.sphere].kind == kQuadInstance;
+        if (H.leaf_boxes.size() >= (1u << (32u - kPrimBoxShift))) {
+            H.wide = false;
+            continue;
+        }
+        set_flags(nd.offset, (entry ? kPrimBoxEntry : kPrimHitBox) | ((uint32_t)H.leaf_boxes.size() << kPrimBoxShift));
+        const Box& b = nd.box;
+        H.leaf_boxes.push_back(LeafBox{{b.lo.x, b.lo.y, b.lo.z, 0.0f}, {b.hi.x, b.hi.y, b.hi.z, 0.0f}});
     }
+    for (const HostBVH& I : H.insts) H.wide = H.wide && I.wide;
     if (m == 0) return;
-    auto box_rec = [&](size_t k, ChildRec& c) {
-        const FlatNode& nd = H.nodes[k];
-        c.lo_x = nd.box.lo.x;
-        c.lo_y = nd.box.lo.y;
-        c.lo_z = nd.box.lo.z;
-        c.hi_x = nd.box.hi.x;
-        c.hi_y = nd.box.hi.y;
-        c.hi_z = nd.box.hi.z;
-    };
-    // index of the Node4 rooted at each binary inner node that starts one
-    std::vector<uint32_t> n4_of(m, kNode4Empty);
-    // pre-order walk: a binary inner node reached as a grandchild (or the
-    // root) starts a Node4
-    struct Item {
-        size_t k;
-        uint32_t pushes;  // stack entries the traversal may hold above it
-    };
-    std::vector<Item> todo{{0, 0}};
-    std::vector<size_t> order;
-    while (!todo.empty()) {
-        Item it = todo.back();
-        todo.pop_back();
-        const FlatNode& N = H.nodes[it.k];
-        if (N.leaf) continue;
-        n4_of[it.k] = (uint32_t)order.size();
-        order.push_back(it.k);
-        size_t L = it.k + 1, R = N.offset;
-        size_t kids[4] = {SIZE_MAX, SIZE_MAX, SIZE_MAX, SIZE_MAX};
-        if (H.nodes[L].leaf) kids[0] = L; else { kids[0] = L + 1; kids[1] = H.nodes[L].offset; }
-        if (H.nodes[R].leaf) kids[2] = R; else { kids[2] = R + 1; kids[3] = H.nodes[R].offset; }
-        uint32_t nk = 0;
-        for (size_t kk : kids) nk += kk != SIZE_MAX;
-        uint32_t here = it.pushes + nk - 1;
+    const Box& rb = H.nodes[0].box;
+    for (float v : {rb.lo.x, rb.lo.y, rb.lo.z, rb.hi.x, rb.hi.y, rb.hi.z}) H.reach = std::max(H.reach, 1.25f * std::fabs(v));
+    H.quad_root = H.nodes[0].leaf ? (kNode4Leaf | H.nodes[0].offset) : 0u;
+    if (H.nodes[0].leaf) return;
+    // pairs are numbered in pre-order, so a node's 4-wide start is decided
+    // before its grandchildren's
+    std::vector<uint32_t> deferred(H.pairs.size(), 0);  // entries the walk may hold above a start
+    std::vector<uint8_t> starts(H.pairs.size(), 0);      // split axis + 1 of a start
+    starts[0] = (uint8_t)(H.nodes[0].count + 1);
+    for (size_t p = 0; p < H.pairs.size(); ++p) {
+        if (!starts[p]) continue;
+        H.quad_of[p] = H.n_quads++ | ((uint32_t)(starts[p] - 1) << kQuadAxisShift);
+        uint32_t slots = 0;
+        for (const ChildRec& c : H.pairs[p].c) slots += (c.b & kLeafBit) ? 1u : 2u;
+        const uint32_t here = deferred[p] + slots - 1;
         H.stack4_bound = std::max(H.stack4_bound, here);
-        for (int s = 3; s >= 0; --s)
-            if (kids[s] != SIZE_MAX && !H.nodes[kids[s]].leaf) todo.push_back({kids[s], here});
-    }
-    H.nodes4.assign(order.size(), Node4{});
-    for (size_t i = 0; i < order.size(); ++i) {
-        size_t k = order[i];
-        const FlatNode& N = H.nodes[k];
-        size_t L = k + 1, R = N.offset;
-        size_t kids[4] = {SIZE_MAX, SIZE_MAX, SIZE_MAX, SIZE_MAX};
-        uint32_t axL = 0, axR = 0;
-        if (H.nodes[L].leaf) kids[0] = L; else { kids[0] = L + 1; kids[1] = H.nodes[L].offset; axL = H.nodes[L].count; }
-        if (H.nodes[R].leaf) kids[2] = R; else { kids[2] = R + 1; kids[3] = H.nodes[R].offset; axR = H.nodes[R].count; }
-        Node4& n4 = H.nodes4[i];
-        for (int s = 0; s < 4; ++s) {
-            ChildRec& c = n4.c[s];
-            if (kids[s] == SIZE_MAX) {
-                c.lo_x = c.lo_y = c.lo_z = FLT_MAX;
-                c.hi_x = c.hi_y = c.hi_z = -FLT_MAX;
-                c.a = kNode4Empty;
-            } else {
-                box_rec(kids[s], c);
-                const FlatNode& G = H.nodes[kids[s]];
-                c.a = G.leaf ? (kNode4Leaf | G.offset) : n4_of[kids[s]];
+        for (const ChildRec& c : H.pairs[p].c) {
+            if (c.b & kLeafBit) continue;
+            for (const ChildRec& g : H.pairs[c.a].c) {
+                if (g.b & kLeafBit) continue;
+                starts[g.a] = (uint8_t)(g.b + 1);
+                deferred[g.a] = here;
             }
-            c.b = 0;
         }
-        n4.c[0].b = N.count | (axL << 2) | (axR << 4);
     }
-    ChildRec r;
-    box_rec(0, r);
-    r.a = H.nodes[0].leaf ? (kNode4Leaf | H.nodes[0].offset) : 0u;
-    r.b = 0;
-    H.root4 = r;
 }
 
 int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_prims, const char* split_method,
@@ -556,7 +546,7 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
             *err = "instance definition without shapes";
             return PBRT_ERR_INVALID_ARGUMENT;
         }
-        if (H.insts[k].stack4_bound > 96) {  // kInstStack4 of the nested walk
+        if (H.insts[k].stack4_bound > 96) {  // kInstStack of the nested walk
             *err = "instance definition BVH too deep for the nested traversal stack (96 entries)";
             return PBRT_ERR_UNSUPPORTED;
         }
@@ -705,14 +695,14 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
                                                       : build_tree(H, max_prims, split, err);
     if (st) return st;
     fill_device_layout(H);
-    fill_node4_layout(H);
+    fill_quad_layout(H);
     if (!H.insts.empty()) {
         // the 4-wide walk enters a definition with two more entries (the
         // rest of the leaf, the exit word) on top of the scene's stack
         uint32_t inner = 0;
         for (const HostBVH& I : H.insts) inner = std::max(inner, I.stack4_bound);
         H.stack4_bound += 2 + inner;
-        if (H.recs.size() >= 0x7ffffffeu) {  // leaf words stay clear of the exit word
+        if (H.ordered.size() >= 0x7ffffffeu) {  // leaf words stay clear of the exit word
             *err = "too many primitives for a scene with instances";
             return PBRT_ERR_UNSUPPORTED;
         }

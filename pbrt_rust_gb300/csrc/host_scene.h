@@ -89,10 +89,19 @@ struct HostBVH {
     std::vector<NodePair> pairs;
     std::vector<PrimRec> recs;
     bool has_spheres = false;
-    // 4-wide layout (same tree, two binary levels per node)
-    ChildRec root4{};
-    std::vector<Node4> nodes4;
-    uint32_t stack4_bound = 0;  // most entries a 4-wide traversal can push
+    // 4-wide layout (layout.h: QuadNode; same tree, two binary levels per
+    // node), encoded on the device from the pairs: quad_of[pair] = index of
+    // the 4-wide node that starts at the pair's node | its split axis <<
+    // kQuadAxisShift, kNoQuad for the pairs in between
+    std::vector<uint32_t> quad_of;
+    uint32_t n_quads = 0;
+    uint32_t quad_root = 0;           // the root's child word
+    std::vector<LeafBox> leaf_boxes;  // leaf boxes the records' flags refer to
+    // the tree has the 4-wide layout: every coordinate is finite and at most
+    // kWideReach away from the origin
+    bool wide = false;
+    float reach = 0.0f;          // 5/4 of the largest coordinate of the root's box
+    uint32_t stack4_bound = 0;  // most entries a 4-wide traversal can defer
     // instance definitions: one BVH each, shared by all their instances
     std::vector<HostBVH> insts;
     // With instances, the id a hit reports: refined primitives numbered in
@@ -103,6 +112,10 @@ struct HostBVH {
     std::vector<uint32_t> flat_id;
     uint64_t n_flat = 0;
 };
+
+constexpr uint32_t kNoQuad = 0xffffffffu;
+constexpr uint32_t kQuadAxisShift = 30u;
+constexpr float kWideReach = 1.099511627776e12f;  // 2^40 (kRayReach in trace4.cuh)
 
 // Fully refine shapes, build and flatten the BVH, and fill the device
 // layout.  Returns a PbrtStatus; *err gets a message on failure.

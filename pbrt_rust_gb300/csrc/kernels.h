@@ -56,9 +56,10 @@ int trace_stack_for_depth(uint32_t depth);
 // `order` (a permutation of [0, n)) the kernels take ray order[j] as their
 // j-th ray; hits still land at each ray's own index.  `work` is the 4-wide
 // persistent kernel's chunk counter (see trace_chunk).  `replay` (closest
-// hit: required; a device word, zero at launch) flags that some ray's walk
-// accepted a NaN distance; a replay kernel queued after the traversal then
-// rewrites those rays' hits by the exact walk (see Traversal in trace.cuh).
+// hit: required; a device word, zero at launch) flags that some ray's binary
+// walk accepted a NaN distance; a replay kernel queued after such a traversal
+// then rewrites those rays' hits by the exact walk (see Traversal in
+// trace.cuh; the 4-wide kernels do so by themselves).
 // `in.ready` (streamed input; needs `work` and trace_streams()): the rays
 // arrive in pieces of 2^in.shift rays while the walk runs, in.ready[k] (zero
 // at launch) turning non-zero once piece k has landed; a piece that has not
@@ -78,6 +79,11 @@ cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays,
                          uint32_t wide_bound = 0, int kernel = -1, const uint32_t* order = nullptr,
                          uint32_t* work = nullptr, uint32_t* replay = nullptr, StreamIn in = {},
                          PbrtHit* host_hits = nullptr);
+// Encodes a tree's 4-wide layout (layout.h: QuadNode) on the device from its
+// binary one; quad_of, n_pairs and null_prim as in HostBVH.  d_quads holds
+// n_quads nodes.
+cudaError_t launch_make_quads(const NodePair* d_pairs, const uint32_t* d_quad_of, uint32_t n_pairs, uint32_t null_prim,
+                              QuadNode* d_quads, cudaStream_t s);
 // Whether the configured traversal of this tree can take streamed input
 // (the 4-wide persistent walk with its shared counter, rays in order).
 bool trace_streams(const DevBVH& bvh, const DevBVH4* wide, uint32_t wide_bound, uint32_t n);

@@ -37,29 +37,62 @@ static_assert(sizeof(NodePair) == 64, "node pair is 64 bytes");
 constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kCountMask = 0x7fffffffu;
 
-// 4-wide node collapsed from two levels of the reference's binary tree.
-// For a binary inner node N with children L (first) and R (second):
-//   slot 0/1 = L's first/second child (slot 0 = L itself if L is a leaf,
-//   slot 1 then empty), slot 2/3 = the same for R.
-// Child record words: a = kNode4Leaf | first primitive, or the index of
-// the child's own Node4, or kNode4Empty; b of slot 0 holds the node's
-// three binary split axes: axis(N) | axis(L) << 2 | axis(R) << 4.
-// The primitives of a leaf child end at the record that carries
-// kPrimLastBit (PrimRec r2[3]).
-struct alignas(128) Node4 {
-    ChildRec c[4];
+// 4-wide node, two levels of the reference's binary tree with the four
+// grandchildren's boxes on an 8-bit grid of the node's own extent.  For a
+// binary inner node N with children L (first) and R (second): slot 0/1 = L's
+// first/second child (slot 0 = L itself if L is a leaf, slot 1 then empty),
+// slot 2/3 = the same for R.
+//
+// Why 64 bytes: a divergent warp pays one L1 wavefront per lane and 32-byte
+// load, and with full-precision boxes (128 bytes, four loads) that pipe was
+// the limit once the box arithmetic had been cut (80 % busy on 2^20 rays
+// into 4096 random triangles).  Two loads halve it.
+//
+// Grid: plane code c (one byte) stands for the coordinate
+//   org + v(c) * scale,  v(c) = 128 + c for c < 128, 2 c for c >= 128
+// because v(c) is the float with bits 0x43000000 | c << 16: one byte permute
+// decodes a plane.  Lower planes are rounded down and upper planes up, so a
+// node's boxes contain the exact ones; the exact box of a leaf is tested when
+// one of its primitives is hit (trace4.cuh says why that gives the
+// reference's walk).
+//   sxy    scale of x as a float whose low 16 bits are the top half of the
+//          scale of y (a bfloat16)
+//   sz     scale of z
+//   order  3 bits per ray octant (bit i of the octant: the ray's direction is
+//          negative on axis i), at 3 * octant: bit 0 / 1 = L's / R's children
+//          swap places in the visit, bit 2 = L and R do
+//   lo/hi  one byte per slot
+//   ref    kNode4Leaf | first primitive, or the index of the child's own
+//          node; an empty slot refers to the leaf of the null primitive that
+//          ends the primitive array
+struct alignas(64) QuadNode {
+    float org_x, org_y, org_z;
+    uint32_t sxy;
+    float sz;
+    uint32_t order;
+    uint32_t lo_x, hi_x;
+    uint32_t lo_y, hi_y, lo_z, hi_z;
+    uint32_t ref[4];
 };
-static_assert(sizeof(Node4) == 128, "4-wide node is 128 bytes");
+static_assert(sizeof(QuadNode) == 64, "4-wide node is 64 bytes");
 constexpr uint32_t kNode4Leaf = 0x80000000u;
-constexpr uint32_t kNode4Empty = 0xffffffffu;
-constexpr uint32_t kPrimLastBit = 1u;
 
-// 48-byte primitive record in BVH (ordered) order.  Triangle: p1 and the
-// edges e1 = p2 - p1, e2 = p3 - p1, computed on the host with the same f32
-// subtraction the reference does per test (src/shape/mesh.rs:45-46).
-//   r0 = (p1.xyz, id)  id = refined input index | kSphereBit if a sphere
-//   r1 = (e1.xyz, sphere index bits for spheres)
-//   r2 = (e2.xyz, flags: kPrimLastBit on the last primitive of a leaf)
+// 48-byte primitive record in BVH (ordered) order; one null record (a
+// triangle of zeros that no ray hits) follows the last.  Triangle: its
+// vertices; the edges p2 - p1 and p3 - p1 are the f32 subtractions the
+// reference does per test (src/shape/mesh.rs:45-46).
+//   r0 = (p1.xyz, id)  id = refined input index | kSphereBit if analytic
+//   r1 = (p2.xyz, analytic record's index)
+//   r2 = (p3.xyz, flags)
+// Flags (4-wide walk): kPrimLastBit on the last primitive of a leaf; and, for
+// the exact box of the leaf,
+//   kPrimBoxEntry  first primitive of a leaf of several, or an instance: the
+//                  box in the table at flags >> kPrimBoxShift, tested before
+//                  the leaf's primitives
+//   kPrimOwnBox    a leaf of one triangle: the bounds of its vertices, tested
+//                  when the triangle is hit
+//   kPrimHitBox    a leaf of one analytic shape: the box in the table, tested
+//                  when the shape is hit
 struct alignas(16) PrimRec {
     float r0[4];
     float r1[4];
@@ -67,6 +100,16 @@ struct alignas(16) PrimRec {
 };
 static_assert(sizeof(PrimRec) == 48, "primitive record is 48 bytes");
 constexpr uint32_t kSphereBit = 0x80000000u;
+constexpr uint32_t kPrimLastBit = 1u;
+constexpr uint32_t kPrimBoxEntry = 2u;
+constexpr uint32_t kPrimOwnBox = 4u;
+constexpr uint32_t kPrimHitBox = 8u;
+constexpr uint32_t kPrimBoxShift = 4u;
+
+// A leaf's exact box in the table of leaf boxes.
+struct alignas(32) LeafBox {
+    float lo[4], hi[4];
+};
 
 // An analytic shape - sphere (src/shape/sphere.rs:16-25), disk
 // (src/shape/disk.rs:16-22) or cylinder (src/shape/cylinder.rs:16-23) -

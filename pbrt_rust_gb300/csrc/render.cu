@@ -71,20 +71,22 @@ __global__ void __launch_bounds__(128) k_shadow_packet(RenderParams P) {
     P.occluded[P.shadow_slot[q]] = occ ? 1 : 0;
 }
 
-template <int SMAX, int OVF, bool INST = false>
-__global__ void __launch_bounds__(128) k_shadow4(RenderParams P) {
-    extern __shared__ uint2 smem_stack[];
+template <int OVF, bool INST>
+__global__ void __launch_bounds__(128) k_shadow4(const __grid_constant__ RenderParams P) {
+    using Walk = Walk4<128, 16, OVF, true, INST>;
+    __shared__ typename Walk::Shared sh;
+    sh.init();
     uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= *(volatile uint32_t*)&P.counters[0]) return;
-    const float4* r4 = reinterpret_cast<const float4*>(P.shadow_rays);
-    DRay r = make_dray(r4[2 * (size_t)q], r4[2 * (size_t)q + 1]);
-    Traversal4<SMAX, OVF, INST> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
-    if (T.start(P.bvh4, r))
-        while (T.template step<true>(P.bvh4, r)) {
-        }
-    if (T.overflow) atomicMax((int*)&P.counters[2], 6);
-    P.occluded[P.shadow_slot[q]] = T.found ? 1 : 0;
+    const float4* ray = reinterpret_cast<const float4*>(P.shadow_rays) + 2 * (size_t)q;
+    int* status = (int*)&P.counters[2];
+    Walk T;
+    typename Walk::Ovf ov;
+    T.bind(sh);
+    const int st = T.start(P.bvh4, ray[0], ray[1]);
+    if (st == kStartWalk) T.run(P.bvh4, sh, ov);
+    if (T.spilled < 0) atomicMax(status, 6);
+    P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.give_up ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
 }
 
 // --------------------------------------------------------------- combine ---
@@ -187,7 +189,6 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         uint64_t max_shadow = P.n_samples * P.n_lights;
         if (max_shadow) {
-            const size_t smem = 16 * sizeof(uint2) * 128;
             // scenes with instances: the 4-wide walk with instances when a
             // variant covers its stack bound, else the binary one
             const bool inst = P.bvh.insts != nullptr;
@@ -195,9 +196,9 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             const bool wide_rk = rk == PBRT_TRACE_WIDE || rk == PBRT_TRACE_WIDE_PERSISTENT || rk == PBRT_TRACE_WIDE_SPECULATIVE;
             int wv = (P.has_wide && wide_rk && !inst) ? wide_stack_variant(P.wide_bound) : 0;
             if (iv == 64)
-                k_shadow4<16, 48, true><<<blocks_for(max_shadow, 128), 128, smem, s>>>(P);
+                k_shadow4<64, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (iv == 256)
-                k_shadow4<16, 240, true><<<blocks_for(max_shadow, 128), 128, smem, s>>>(P);
+                k_shadow4<256, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (inst && trace_stack_for_depth(P.depth) == 64)
                 k_shadow<64, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (inst)
@@ -207,9 +208,9 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             else if (rk == PBRT_TRACE_PAIR_PACKET)
                 k_shadow_packet<256><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (wv == 64)
-                k_shadow4<16, 48><<<blocks_for(max_shadow, 128), 128, smem, s>>>(P);
+                k_shadow4<64, false><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (wv == 256)
-                k_shadow4<16, 240><<<blocks_for(max_shadow, 128), 128, smem, s>>>(P);
+                k_shadow4<256, false><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (trace_stack_for_depth(P.depth) == 64)
                 k_shadow<64><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else

@@ -133,34 +133,32 @@ __global__ void __launch_bounds__(128) k_trace_persistent(const __grid_constant_
     if (st) atomicMax(status, st);
 }
 
+constexpr int kWalkBlock = 128;  // threads per block and stack rows of the 4-wide kernels
+constexpr int kWalkRows = 16;
+
 // 4-wide traversal, one thread per ray.
-template <int SMAX, int OVF, bool ANY>
-__global__ void __launch_bounds__(128) k_trace4(const __grid_constant__ DevBVH4 bvh, const float4* __restrict__ rays,
-                                                uint32_t n,
-                                                const uint32_t* __restrict__ order, float4* __restrict__ hits,
-                                                uint8_t* __restrict__ occ, int* __restrict__ status,
-                                                uint32_t* __restrict__ replay) {
-    extern __shared__ uint2 smem_stack[];
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int OVF, bool ANY>
+__global__ void __launch_bounds__(kWalkBlock) k_trace4(const __grid_constant__ DevBVH4 bvh,
+                                                       const float4* __restrict__ rays, uint32_t n,
+                                                       const uint32_t* __restrict__ order, float4* __restrict__ hits,
+                                                       uint8_t* __restrict__ occ, int* __restrict__ status) {
+    using Walk = Walk4<kWalkBlock, kWalkRows, OVF, ANY>;
+    __shared__ typename Walk::Shared sh;
+    sh.init();
+    uint32_t i = blockIdx.x * kWalkBlock + threadIdx.x;
     if (i >= n) return;
     if (order) i = __ldg(order + i);
-    DRay r = make_dray(__ldg(rays + 2 * (size_t)i), __ldg(rays + 2 * (size_t)i + 1));
-    Traversal4<SMAX, OVF> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
-    if (T.start(bvh, r))
-        while (T.template step<ANY>(bvh, r)) {
-        }
-    if (T.overflow) atomicMax(status, 6);
-    if (ANY) {
-        occ[i] = T.found ? 1 : 0;
-    } else {
-        if (T.nan_hit) {
-            hits[i] = make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f);
-            *replay = 1u;
-        } else {
-            hits[i] = make_float4(__int_as_float(T.res.prim), T.res.t, T.res.b1, T.res.b2);
-        }
-    }
+    const float4* ray = rays + 2 * (size_t)i;
+    Walk T;
+    typename Walk::Ovf ov;
+    T.bind(sh);
+    const int st = T.start(bvh, __ldg(ray), __ldg(ray + 1));
+    if (st == kStartWalk) T.run(bvh, sh, ov);
+    if (T.spilled < 0) atomicMax(status, 6);
+    if (ANY)
+        occ[i] = (st == kStartExact ? exact_any<OVF + 8, false>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
+    else
+        hits[i] = st == kStartExact || T.give_up ? exact_hit<OVF + 8, false>(bvh.pair, ray, status) : T.hit_record();
 }
 
 // A ray is read once: its lines go to L2 only, leaving L1 to the tree.
@@ -212,6 +210,12 @@ __device__ __noinline__ bool wait_piece(const uint32_t* ready, uint32_t k, uint3
 // through L2 (they are written while the kernel runs); a wait that runs out
 // sets PBRT_ERR_TIMEOUT and the warp drops its chunk.
 //
+// A turn of the loop hands out rays, makes kNodeSteps visits of inner nodes
+// and then tests the leaves that were reached: the votes and the leaf code,
+// which a few of the warp's lanes need at a time, are paid once per
+// kNodeSteps visits (one, two, three, four visits per turn: 586 / 501 / 480 /
+// 494 us for 2^22 incoherent rays into a terrain of a million triangles).
+//
 // HOSTOUT (closest hits, with `work`): `hits` is a device staging array and
 // `host_hits` the caller's pinned host memory mapped into the device's
 // address space.  Scattered 16-byte stores across NVLink-C2C run at a fifth
@@ -222,6 +226,7 @@ __device__ __noinline__ bool wait_piece(const uint32_t* ready, uint32_t k, uint3
 // chunk only when a slot is free (always the case once all its lanes are
 // idle).  The copies spread over the walk, sharing the link with the
 // streamed input.
+constexpr int kNodeSteps = 3;
 constexpr uint32_t kRingWords = 10 + 32;  // HOSTOUT: per warp, see k_trace4_persistent
 // HOSTOUT's copy of finished chunks (ring[9]: one bit per slot) from the
 // staging array to the host, one row of the warp's lanes at a time; out of
@@ -240,28 +245,33 @@ static __device__ __noinline__ void write_out_chunks(uint32_t* ring, const float
         for (uint32_t k = lane; k < cnt; k += 32u) host_hits[base + k] = __ldcg(hits + base + k);
     }
 }
-template <int SMAX, int OVF, bool ANY, int MINB, bool INST = false, bool HOSTOUT = false>
-__global__ void __launch_bounds__(128, MINB)
+template <int OVF, bool ANY, bool INST = false, bool HOSTOUT = false>
+__global__ void __launch_bounds__(kWalkBlock, INST ? 6 : 8)
     k_trace4_persistent(const __grid_constant__ DevBVH4 bvh, const float4* __restrict__ rays, uint32_t n,
                         const uint32_t* __restrict__ order,
                         float4* __restrict__ hits, uint8_t* __restrict__ occ, int* __restrict__ status,
                         uint32_t per_warp, uint32_t refill, uint32_t* __restrict__ work,
                         uint32_t* __restrict__ replay, const StreamIn in, float4* __restrict__ host_hits) {
     static_assert(!(HOSTOUT && ANY), "host write-out is for closest hits");
-    extern __shared__ uint2 smem_stack[];
+    using Walk = Walk4<kWalkBlock, kWalkRows, OVF, ANY, INST>;
+    __shared__ typename Walk::Shared sh;
+    __shared__ uint32_t rings[HOSTOUT ? kWalkBlock / 32 : 1][HOSTOUT ? kRingWords : 1];
+    sh.init();
     const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    // ray positions (32 bits suffice for the counter mode, n <= 0xF0000000)
-    using Pos = typename std::conditional<HOSTOUT, uint32_t, uint64_t>::type;
-    Pos next = work ? 0 : (Pos)(warp * per_warp);
-    Pos end = work ? 0 : (Pos)((warp * per_warp + per_warp < (uint64_t)n) ? warp * per_warp + per_warp : (uint64_t)n);
+    const uint32_t warp = (blockIdx.x * kWalkBlock + threadIdx.x) >> 5;
+    uint32_t next = 0, end = 0;
+    if (!work) {
+        const uint64_t lo = (uint64_t)warp * per_warp;
+        next = lo < n ? (uint32_t)lo : n;
+        end = lo + per_warp < n ? (uint32_t)lo + per_warp : n;
+    }
     bool more = work != nullptr;  // the shared counter may still hold rays
     const uint32_t kNone = 0xffffffffu;
     uint32_t ray = kNone;
     bool overflow = false;
-    DRay r;
-    Traversal4<SMAX, OVF, INST> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
+    Walk T;
+    typename Walk::Ovf ov;
+    T.bind(sh);
     // HOSTOUT: this warp's ring in shared memory: rays left in slot j at
     // ring[j], the slot's first ray at ring[4 + j], the slot of the chunk
     // being handed out at ring[8], the slots whose last ray finished (a bit
@@ -270,25 +280,12 @@ __global__ void __launch_bounds__(128, MINB)
     auto ring_of = [&]() -> uint32_t* {
         uint32_t tid;  // read afresh at each use: the address is not kept in a register across the walk
         asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
-        return reinterpret_cast<uint32_t*>(smem_stack + SMAX * blockDim.x) + (tid >> 5) * kRingWords;
+        return rings[tid >> 5];
     };
     if constexpr (HOSTOUT) {
         if (lane < 10) ring_of()[lane] = 0u;
         __syncwarp();
     }
-    auto put = [&](float4 h) {
-        // written once and not read here: streaming, except the staged hits
-        // that the write-out reads back
-        if constexpr (HOSTOUT)
-            hits[ray] = h;
-        else
-            __stcs(hits + ray, h);
-        if constexpr (HOSTOUT) {
-            uint32_t* ring = ring_of();
-            const uint32_t j = ring[10 + lane];
-            if (atomicSub(ring + j, 1u) == 1u) atomicOr(ring + 9, 1u << j);
-        }
-    };
     // HOSTOUT: the chunks whose last ray finished go out to the host.  Done
     // when the warp takes its next chunk (which needs a slot) and at the
     // end, not at every step of the walk.
@@ -298,6 +295,26 @@ __global__ void __launch_bounds__(128, MINB)
             uint32_t* ring = ring_of();
             if (ring[9]) write_out_chunks(ring, hits, host_hits, n, per_warp);
         }
+    };
+    // The lane's ray ends with what T found, or marked for the replay.
+    auto finish = [&](bool exact) {
+        if (T.spilled < 0) overflow = true;
+        if (exact) *replay = 1u;
+        if (ANY) {
+            occ[ray] = exact ? kReplayOcc : (T.found() ? 1 : 0);
+        } else {
+            const float4 h = exact ? make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f) : T.hit_record();
+            if constexpr (HOSTOUT) {
+                hits[ray] = h;
+                uint32_t* ring = ring_of();
+                const uint32_t j = ring[10 + lane];
+                if (atomicSub(ring + j, 1u) == 1u) atomicOr(ring + 9, 1u << j);
+            } else {
+                __stcs(hits + ray, h);  // written once and (but for marks) not read here
+            }
+        }
+        ray = kNone;
+        T.cur = kWalkDone;
     };
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, ray == kNone);
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(128, MINB)
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (base < n) {
                     next = base;
-                    end = (Pos)((uint64_t)base + per_warp < (uint64_t)n ? (uint64_t)base + per_warp : (uint64_t)n);
+                    end = n - base > per_warp ? base + per_warp : n;
                     if (in.ready) {  // streamed input: the chunk's rays must have landed
                         int ok = 1;
                         if (lane == 0)
@@ -333,7 +350,7 @@ __global__ void __launch_bounds__(128, MINB)
                         if (next < end) {
                             if (lane == 0) {
                                 uint32_t* ring = ring_of();
-                                ring[fs] = (uint32_t)(end - next);
+                                ring[fs] = end - next;
                                 ring[4 + fs] = base;
                                 ring[8] = (uint32_t)fs;
                             }
@@ -345,149 +362,43 @@ __global__ void __launch_bounds__(128, MINB)
                 }
             }
         }
-        const bool tail = !more && next + nidle >= end;
+        const bool tail = !more && end - next <= nidle;
         if (next < end && nidle >= (tail ? 1u : refill)) {
             if (ray == kNone) {
-                const Pos my = next + __popc(idle & ((1u << lane) - 1u));
-                if (my < end) {
-                    ray = order ? __ldg(order + my) : (uint32_t)my;
+                const uint32_t k = __popc(idle & ((1u << lane) - 1u));
+                if (k < end - next) {
+                    ray = order ? __ldg(order + next + k) : next + k;
                     if constexpr (HOSTOUT) {
                         uint32_t* ring = ring_of();
                         ring[10 + lane] = ring[8];
                     }
                     const float4* rp = rays + 2 * (size_t)ray;
-                    r = in.ready ? make_dray(__ldcg(rp), __ldcg(rp + 1)) : make_dray(ld_stream(rp), ld_stream(rp + 1));
-                    bool live = T.start(bvh, r);
-                    if (!live) {
-                        if (ANY)
-                            occ[ray] = 0;
-                        else
-                            put(make_float4(__int_as_float(-1), 0.0f, 0.0f, 0.0f));
-                        ray = kNone;
+                    float4 a, b;
+                    if (in.ready) {
+                        a = __ldcg(rp);
+                        b = __ldcg(rp + 1);
+                    } else {
+                        a = ld_stream(rp);
+                        b = ld_stream(rp + 1);
                     }
+                    const int st = T.start(bvh, a, b);
+                    if (st != kStartWalk) finish(st == kStartExact);
                 }
             }
-            next += nidle;
+            next += min(nidle, end - next);
         }
-        bool busy = ray != kNone;
-        if (!__any_sync(0xffffffffu, busy)) {
+        if (!__any_sync(0xffffffffu, ray != kNone)) {
             if (next >= end && !more) break;
             continue;
         }
-        if (busy && !T.template step<ANY>(bvh, r)) {
-            overflow |= T.overflow;
-            if (ANY) {
-                occ[ray] = T.found ? 1 : 0;
-            } else {
-                if (T.nan_hit) {
-                    put(make_float4(__int_as_float(kReplayMark), 0.0f, 0.0f, 0.0f));
-                    *replay = 1u;
-                } else {
-                    put(make_float4(__int_as_float(T.res.prim), T.res.t, T.res.b1, T.res.b2));
-                }
-            }
-            ray = kNone;
-        }
+        // an idle lane's `cur` is kWalkDone
+#pragma unroll
+        for (int k = 0; k < kNodeSteps; ++k)
+            if ((int32_t)T.cur >= 0) T.node(bvh, ov);
+        if ((int32_t)T.cur < 0 && T.cur != kWalkDone) T.leaf(bvh, sh, ov);
+        if (T.cur == kWalkDone && ray != kNone && !T.resume(ov)) finish(T.give_up);
     }
     write_out();
-    if (overflow) atomicMax(status, 6);
-}
-
-// 4-wide persistent traversal with postponed leaves.  A lane that reaches a
-// leaf keeps it aside and carries on down its stack; the warp tests the kept
-// leaves together once enough lanes are stuck behind a second leaf (or have
-// nothing else left), so the leaf code runs with many lanes instead of one
-// or two.  A kept leaf is always tested before the lane's next leaf, so
-// primitives are still tested in the reference's depth-first order; the
-// nodes a lane visits while a leaf is kept are tested against a maxt that
-// the kept leaf may still shrink, so some nodes the reference culls are
-// visited too - their primitives are all farther than the closest hit - and
-// the result, ties included, is the reference's.  Work comes from the
-// shared counter (chunks of per_warp rays) or from fixed per-warp ranges.
-template <int SMAX, int OVF, bool ANY>
-__global__ void __launch_bounds__(128)
-    k_trace4_spec(DevBVH4 bvh, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ order,
-                  float4* __restrict__ hits, uint8_t* __restrict__ occ, int* __restrict__ status, uint32_t per_warp,
-                  uint32_t refill, uint32_t* __restrict__ work) {
-    extern __shared__ uint2 smem_stack[];
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint64_t next = work ? 0 : warp * per_warp;
-    uint64_t end = work ? 0 : ((next + per_warp < (uint64_t)n) ? next + per_warp : (uint64_t)n);
-    bool more = work != nullptr;
-    const uint32_t kNone = 0xffffffffu;
-    uint32_t ray = kNone;
-    uint32_t kept = kNone;  // postponed leaf
-    bool live = false;      // `T.cur` holds the next node or leaf
-    bool overflow = false;
-    DRay r;
-    Traversal4<SMAX, OVF> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
-    auto finish = [&]() {
-        overflow |= T.overflow;
-        if (ANY)
-            occ[ray] = T.found ? 1 : 0;
-        else
-            hits[ray] = make_float4(__int_as_float(T.res.prim), T.res.t, T.res.b1, T.res.b2);
-        ray = kNone;
-        kept = kNone;
-        live = false;
-    };
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, ray == kNone);
-        const unsigned nidle = __popc(idle);
-        if (more && next >= end && nidle >= refill) {  // warp-uniform
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(work, per_warp);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base < n) {
-                next = base;
-                end = (uint64_t)base + per_warp < (uint64_t)n ? (uint64_t)base + per_warp : (uint64_t)n;
-            } else {
-                more = false;
-            }
-        }
-        const bool tail = !more && next + nidle >= end;
-        if (next < end && nidle >= (tail ? 1u : refill)) {
-            if (ray == kNone) {
-                const uint64_t my = next + __popc(idle & ((1u << lane) - 1u));
-                if (my < end) {
-                    ray = order ? __ldg(order + my) : (uint32_t)my;
-                    r = make_dray(__ldg(rays + 2 * (size_t)ray), __ldg(rays + 2 * (size_t)ray + 1));
-                    live = T.start(bvh, r);
-                    if (!live) finish();
-                }
-            }
-            next += nidle;
-        }
-        const bool busy = ray != kNone;
-        if (!__any_sync(0xffffffffu, busy)) {
-            if (next >= end && !more) break;
-            continue;
-        }
-        const bool at_leaf = busy && live && (T.cur & kNode4Leaf);
-        const bool blocked = busy && kept != kNone && (at_leaf || !live);
-        const unsigned nbusy = __popc(__ballot_sync(0xffffffffu, busy));
-        const unsigned nblocked = __popc(__ballot_sync(0xffffffffu, blocked));
-        const unsigned nkept = __popc(__ballot_sync(0xffffffffu, busy && kept != kNone));
-        if (nblocked && (4 * nblocked >= nbusy || nkept == nbusy)) {
-            // leaf round: every kept leaf is tested now
-            if (busy && kept != kNone) {
-                const bool stop = T.template leaf<ANY>(bvh, r, kept) == 1;
-                kept = kNone;
-                if (stop || T.overflow) finish();
-            }
-        } else if (busy && live && !blocked) {  // a blocked lane waits for the leaf round
-            if (at_leaf) {  // keep it, go on with the next stack entry
-                kept = T.cur;
-                live = T.pop();
-            } else {
-                live = T.template node<ANY>(bvh, r);
-                if (T.overflow) finish();
-            }
-        }
-        if (ray != kNone && !live && kept == kNone) finish();
-    }
     if (overflow) atomicMax(status, 6);
 }
 
@@ -541,63 +452,41 @@ static void read_variant() {
     }
 }
 
-// Rewrites the closest hits marked kReplayMark by the EXACT walk (see
-// Traversal in trace.cuh); returns at once when no ray of the launch was
-// marked, so a launch without NaN-distance hits pays one empty kernel.
-// `host_hits` (may be null): a second copy of the hits that the rewritten
-// ones also go to (the host memory of a write-out walk).
-template <int SMAX, int OVF, bool INST>
-__global__ void __launch_bounds__(128) k_replay4(const __grid_constant__ DevBVH4 bvh, const float4* __restrict__ rays,
-                                                 uint32_t n, float4* __restrict__ hits,
-                                                 const uint32_t* __restrict__ replay, int* __restrict__ status,
-                                                 float4* __restrict__ host_hits) {
-    extern __shared__ uint2 smem_stack[];
-    if (*(const volatile uint32_t*)replay == 0u) return;
-    Traversal4<SMAX, OVF, INST, true, true> T;
-    T.bind(smem_stack, threadIdx.x, blockDim.x);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (__float_as_int(hits[i].x) != kReplayMark) continue;
-        DRay r = make_dray(__ldg(rays + 2 * i), __ldg(rays + 2 * i + 1));
-        if (T.start(bvh, r)) {
-            while (T.template step<false>(bvh, r)) {
-            }
-        }
-        if (T.overflow) atomicMax(status, 6);
-        hits[i] = make_float4(__int_as_float(T.res.prim), T.res.t, T.res.b1, T.res.b2);
-        if (host_hits) host_hits[i] = hits[i];
-    }
-}
-
+// Rewrites what a traversal marked kReplayMark (closest hits) or kReplayOcc
+// (any hit) by the exact walk over the binary layout (see Traversal in
+// trace.cuh, and trace4.cuh for the rays that 4-wide walks mark); returns at
+// once when no ray of the launch was marked, so a launch without such rays
+// pays one empty kernel.  `host_hits` (may be null): a second copy of the
+// hits that the rewritten ones also go to (the host memory of a write-out
+// walk).
 template <int STACK, bool INST>
 __global__ void __launch_bounds__(128) k_replay2(const __grid_constant__ DevBVH bvh, const float4* __restrict__ rays,
-                                                 uint32_t n, float4* __restrict__ hits,
-                                                 const uint32_t* __restrict__ replay, int* __restrict__ status) {
+                                                 uint32_t n, float4* __restrict__ hits, uint8_t* __restrict__ occ,
+                                                 const uint32_t* __restrict__ replay, int* __restrict__ status,
+                                                 float4* __restrict__ host_hits) {
     if (*(const volatile uint32_t*)replay == 0u) return;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (__float_as_int(hits[i].x) != kReplayMark) continue;
-        DRay r = make_dray(__ldg(rays + 2 * i), __ldg(rays + 2 * i + 1));
-        TraceResult res;
-        int st = 0;
-        traverse<STACK, false, INST, true>(bvh, r, &res, &st);
-        if (st) atomicMax(status, st);
-        hits[i] = make_float4(__int_as_float(res.prim), res.t, res.b1, res.b2);
+        if (occ) {
+            if (occ[i] == kReplayOcc) occ[i] = exact_any<STACK, INST>(bvh, rays + 2 * i, status) ? 1 : 0;
+        } else if (__float_as_int(hits[i].x) == kReplayMark) {
+            hits[i] = exact_hit<STACK, INST>(bvh, rays + 2 * i, status);
+            if (host_hits) host_hits[i] = hits[i];
+        }
     }
 }
 
 // `host_hits` (closest hits, with `work`): the HOSTOUT walk, `h4` its
 // staging array.
-template <int SMAX, int OVF, bool ANY, int MINB, bool INST = false, bool HOSTOUT = false>
+template <int OVF, bool ANY, bool INST, bool HOSTOUT = false>
 static cudaError_t launch_wide_persistent(const DevBVH4& bvh, const float4* r4, uint32_t n, const uint32_t* order,
                                           float4* h4, uint8_t* occ, int* d_status, cudaStream_t stream,
-                                          uint32_t* work, uint32_t* replay, StreamIn in = {},
-                                          float4* host_hits = nullptr) {
-    const int block = 128;
-    // HOSTOUT: each warp's ring after the stacks
-    const size_t smem = (size_t)SMAX * sizeof(uint2) * block + (HOSTOUT ? (block / 32) * kRingWords * sizeof(uint32_t) : 0);
+                                          uint32_t* work, uint32_t* replay, StreamIn in, float4* host_hits) {
+    constexpr int warps_per_block = kWalkBlock / 32;
+    auto kernel = k_trace4_persistent<OVF, ANY, INST, HOSTOUT>;
     static ShapeCache bps_cache;
     const int sms = device_sms();
-    const int bps = resident_blocks(bps_cache, k_trace4_persistent<SMAX, OVF, ANY, MINB, INST, HOSTOUT>, block, smem);
-    uint64_t warps = (uint64_t)sms * bps * (block / 32);
+    const int bps = resident_blocks(bps_cache, kernel, kWalkBlock, 0);
+    uint64_t warps = (uint64_t)sms * bps * warps_per_block;
     uint32_t per_warp = (uint32_t)((n + warps - 1) / warps);
     if (per_warp < 32) per_warp = 32;
     if (work && g_chunk && n <= 0xF0000000u) {  // the counter cannot wrap past n
@@ -605,69 +494,42 @@ static cudaError_t launch_wide_persistent(const DevBVH4& bvh, const float4* r4, 
         // warps than chunks
         uint64_t chunks = (n + g_chunk - 1) / g_chunk;
         uint64_t w = chunks < warps ? chunks : warps;
-        unsigned grid = (unsigned)((w + (block / 32) - 1) / (block / 32));
-        k_trace4_persistent<SMAX, OVF, ANY, MINB, INST, HOSTOUT><<<grid, block, smem, stream>>>(
-            bvh, r4, n, order, h4, occ, d_status, g_chunk, g_refill, work, replay, in, host_hits);
+        unsigned grid = (unsigned)((w + warps_per_block - 1) / warps_per_block);
+        kernel<<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, h4, occ, d_status, g_chunk, g_refill, work, replay,
+                                                in, host_hits);
         return cudaGetLastError();
     }
     // fixed per-warp ranges would read rays out of order and have no chunks
     // to write out: no streamed input, no write-out
     if (in.ready || HOSTOUT) return cudaErrorInvalidValue;
-    uint64_t need_warps = (n + per_warp - 1) / per_warp;
-    unsigned grid = (unsigned)((need_warps + (block / 32) - 1) / (block / 32));
-    k_trace4_persistent<SMAX, OVF, ANY, MINB, INST, HOSTOUT><<<grid, block, smem, stream>>>(
-        bvh, r4, n, order, h4, occ, d_status, per_warp, g_refill, nullptr, replay, StreamIn{}, nullptr);
+    uint64_t need_warps = (n + (uint64_t)per_warp - 1) / per_warp;
+    unsigned grid = (unsigned)((need_warps + warps_per_block - 1) / warps_per_block);
+    kernel<<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, h4, occ, d_status, per_warp, g_refill, nullptr,
+                                            replay, StreamIn{}, nullptr);
     return cudaGetLastError();
 }
 
-template <int SMAX, int OVF, bool ANY>
-static cudaError_t launch_wide_spec(const DevBVH4& bvh, const float4* r4, uint32_t n, const uint32_t* order,
-                                    float4* h4, uint8_t* occ, int* d_status, cudaStream_t stream, uint32_t* work) {
-    const int block = 128;
-    const size_t smem = (size_t)SMAX * sizeof(uint2) * block;
-    static ShapeCache bps_cache;
-    const int sms = device_sms();
-    const int bps = resident_blocks(bps_cache, k_trace4_spec<SMAX, OVF, ANY>, block, smem);
-    const uint64_t warps = (uint64_t)sms * bps * (block / 32);
-    if (work && g_chunk && n <= 0xF0000000u) {
-        const uint64_t chunks = (n + g_chunk - 1) / g_chunk;
-        const uint64_t w = chunks < warps ? chunks : warps;
-        const unsigned grid = (unsigned)((w + (block / 32) - 1) / (block / 32));
-        k_trace4_spec<SMAX, OVF, ANY><<<grid, block, smem, stream>>>(bvh, r4, n, order, h4, occ, d_status, g_chunk,
-                                                                   g_refill, work);
-        return cudaGetLastError();
-    }
-    uint32_t per_warp = (uint32_t)((n + warps - 1) / warps);
-    if (per_warp < 32) per_warp = 32;
-    const uint64_t need_warps = (n + per_warp - 1) / per_warp;
-    const unsigned grid = (unsigned)((need_warps + (block / 32) - 1) / (block / 32));
-    k_trace4_spec<SMAX, OVF, ANY><<<grid, block, smem, stream>>>(bvh, r4, n, order, h4, occ, d_status, per_warp,
-                                                               g_refill, nullptr);
-    return cudaGetLastError();
-}
-
-template <int SMAX, int OVF, bool ANY>
+// The 4-wide kernel for a call: closest hits into h4 (occ null) or answers
+// into occ; persistent or one thread per ray (never with instances).
+template <int OVF>
 static cudaError_t launch_wide(const DevBVH4& bvh, const float4* r4, uint32_t n, const uint32_t* order, float4* h4,
                                uint8_t* occ, int* d_status, cudaStream_t stream, bool persistent, uint32_t* work,
-                               uint32_t* replay) {
-    const int block = 128;
-    const size_t smem = (size_t)SMAX * sizeof(uint2) * block;
-    if (!persistent) {
-        unsigned grid = (unsigned)((n + block - 1) / block);
-        k_trace4<SMAX, OVF, ANY><<<grid, block, smem, stream>>>(bvh, r4, n, order, h4, occ, d_status, replay);
-        return cudaGetLastError();
-    }
-    if (g_min_blocks == 7)
-        return launch_wide_persistent<SMAX, OVF, ANY, 7>(bvh, r4, n, order, h4, occ, d_status, stream, work,
-                                                         replay);
-    if (g_min_blocks == 8)
-        return launch_wide_persistent<SMAX, OVF, ANY, 8>(bvh, r4, n, order, h4, occ, d_status, stream, work,
-                                                         replay);
-    if (g_min_blocks == 9)
-        return launch_wide_persistent<SMAX, OVF, ANY, 9>(bvh, r4, n, order, h4, occ, d_status, stream, work,
-                                                         replay);
-    return launch_wide_persistent<SMAX, OVF, ANY, 0>(bvh, r4, n, order, h4, occ, d_status, stream, work,
-                                                         replay);
+                               uint32_t* replay, StreamIn in = {}, float4* host_hits = nullptr) {
+    auto pt = [&](auto launch) {
+        return launch(bvh, r4, n, order, h4, occ, d_status, stream, work, replay, in, host_hits);
+    };
+    if (bvh.pair.insts)
+        return host_hits ? pt(launch_wide_persistent<OVF, false, true, true>)
+               : occ     ? pt(launch_wide_persistent<OVF, true, true>)
+                         : pt(launch_wide_persistent<OVF, false, true>);
+    if (host_hits) return pt(launch_wide_persistent<OVF, false, false, true>);
+    if (persistent) return occ ? pt(launch_wide_persistent<OVF, true, false>) : pt(launch_wide_persistent<OVF, false, false>);
+    const unsigned grid = (unsigned)((n + (uint64_t)kWalkBlock - 1) / kWalkBlock);
+    if (occ)
+        k_trace4<OVF, true><<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, nullptr, occ, d_status);
+    else
+        k_trace4<OVF, false><<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, h4, nullptr, d_status);
+    return cudaGetLastError();
 }
 
 int set_trace_config(const PbrtTraceConfig& c) {
@@ -737,29 +599,30 @@ int trace_stack_for_depth(uint32_t depth) {
     return 0;
 }
 
+// *replays: the launch marks rays for the replay kernel (the binary kernels).
 static cudaError_t launch_main(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays, uint32_t n, PbrtHit* hits,
                                uint8_t* occluded, int* d_status, cudaStream_t stream, const DevBVH4* wide,
                                uint32_t wide_bound, int kernel, const uint32_t* order, uint32_t* work,
-                               uint32_t* replay) {
-    if (bvh.insts) {
-        // a scene with instances: the persistent walk with nested instance
-        // traversal (4-wide when a variant covers the stack bound),
-        // whatever the configured kernel
-        const float4* r4 = reinterpret_cast<const float4*>(rays);
-        float4* h4 = reinterpret_cast<float4*>(hits);
+                               uint32_t* replay, bool* replays) {
+    const int variant = kernel >= 0 ? kernel : g_kernel_variant;
+    // a scene with instances takes the persistent walk with nested instance
+    // traversal (4-wide when a variant covers the stack bound), whatever the
+    // configured kernel
+    const bool inst = bvh.insts != nullptr;
+    const int v = wide ? wide_stack_variant(wide_bound) : 0;
+    const float4* r4 = reinterpret_cast<const float4*>(rays);
+    float4* h4 = reinterpret_cast<float4*>(hits);
+    if (v && (inst || variant == kVariantWidePlain || variant == kVariantWidePersistent ||
+              variant == kVariantWideSpeculative)) {
+        const bool pt = inst || variant != kVariantWidePlain;
+        *replays = pt;
+        return v == 64 ? launch_wide<64>(*wide, r4, n, order, h4, occluded, d_status, stream, pt, work, replay)
+                       : launch_wide<256>(*wide, r4, n, order, h4, occluded, d_status, stream, pt, work, replay);
+    }
+    *replays = occluded == nullptr;
+    if (inst) {
         const int stack = trace_stack_for_depth(depth);
         const bool any = occluded != nullptr;
-        const int v = wide ? wide_stack_variant(wide_bound) : 0;
-        if (v == 64)
-            return any ? launch_wide_persistent<16, 48, true, 0, true>(*wide, r4, n, order, nullptr, occluded, d_status,
-                                                                       stream, work, replay)
-                       : launch_wide_persistent<16, 48, false, 0, true>(*wide, r4, n, order, h4, nullptr, d_status,
-                                                                        stream, work, replay);
-        if (v == 256)
-            return any ? launch_wide_persistent<16, 240, true, 0, true>(*wide, r4, n, order, nullptr, occluded,
-                                                                        d_status, stream, work, replay)
-                       : launch_wide_persistent<16, 240, false, 0, true>(*wide, r4, n, order, h4, nullptr, d_status,
-                                                                         stream, work, replay);
         if (stack == 64)
             return any ? launch_persistent<64, true, true>(bvh, r4, n, order, nullptr, occluded, d_status, stream, replay)
                        : launch_persistent<64, false, true>(bvh, r4, n, order, h4, nullptr, d_status, stream, replay);
@@ -768,35 +631,8 @@ static cudaError_t launch_main(const DevBVH& bvh, uint32_t depth, const PbrtRay*
                        : launch_persistent<256, false, true>(bvh, r4, n, order, h4, nullptr, d_status, stream, replay);
         return cudaErrorInvalidValue;
     }
-    const int variant = kernel >= 0 ? kernel : g_kernel_variant;
-    if (wide && variant == kVariantWideSpeculative) {
-        const float4* r4 = reinterpret_cast<const float4*>(rays);
-        float4* h4 = reinterpret_cast<float4*>(hits);
-        const bool any = occluded != nullptr;
-        const int v = wide_stack_variant(wide_bound);
-        if (v == 64)
-            return any ? launch_wide_spec<16, 48, true>(*wide, r4, n, order, nullptr, occluded, d_status, stream, work)
-                       : launch_wide_spec<16, 48, false>(*wide, r4, n, order, h4, nullptr, d_status, stream, work);
-        if (v == 256)
-            return any ? launch_wide_spec<16, 240, true>(*wide, r4, n, order, nullptr, occluded, d_status, stream, work)
-                       : launch_wide_spec<16, 240, false>(*wide, r4, n, order, h4, nullptr, d_status, stream, work);
-    }
-    if (wide && (variant == kVariantWidePlain || variant == kVariantWidePersistent)) {
-        const float4* r4 = reinterpret_cast<const float4*>(rays);
-        float4* h4 = reinterpret_cast<float4*>(hits);
-        const bool any = occluded != nullptr, pt = variant == kVariantWidePersistent;
-        int v = wide_stack_variant(wide_bound);
-        if (v == 64)
-            return any ? launch_wide<16, 48, true>(*wide, r4, n, order, nullptr, occluded, d_status, stream, pt, work, replay)
-                       : launch_wide<16, 48, false>(*wide, r4, n, order, h4, nullptr, d_status, stream, pt, work, replay);
-        if (v == 256)
-            return any ? launch_wide<16, 240, true>(*wide, r4, n, order, nullptr, occluded, d_status, stream, pt, work, replay)
-                       : launch_wide<16, 240, false>(*wide, r4, n, order, h4, nullptr, d_status, stream, pt, work, replay);
-    }
     const int block = 128;
     const unsigned grid = (unsigned)((n + block - 1) / block);
-    const float4* r4 = reinterpret_cast<const float4*>(rays);
-    float4* h4 = reinterpret_cast<float4*>(hits);
     int stack = trace_stack_for_depth(depth);
     bool any = occluded != nullptr;
     if (variant == kVariantPairPersistent) {
@@ -859,43 +695,10 @@ static cudaError_t launch_streamed(const DevBVH& bvh, const PbrtRay* rays, uint3
     if (!work || !trace_streams(bvh, wide, wide_bound, n) || (host_hits && occ)) return cudaErrorInvalidValue;
     const float4* r4 = reinterpret_cast<const float4*>(rays);
     float4* h4 = reinterpret_cast<float4*>(hits);
-    const bool any = occ != nullptr, inst = bvh.insts != nullptr;
-    if (host_hits) {
-        float4* hh = reinterpret_cast<float4*>(host_hits);
-        if (wide_stack_variant(wide_bound) == 64)
-            return inst ? launch_wide_persistent<16, 48, false, 0, true, true>(*wide, r4, n, nullptr, h4, nullptr,
-                                                                              d_status, stream, work, replay, in,
-                                                                              hh)
-                        : launch_wide_persistent<16, 48, false, 0, false, true>(*wide, r4, n, nullptr, h4, nullptr,
-                                                                               d_status, stream, work, replay, in,
-                                                                               hh);
-        return inst ? launch_wide_persistent<16, 240, false, 0, true, true>(*wide, r4, n, nullptr, h4, nullptr,
-                                                                           d_status, stream, work, replay, in,
-                                                                           hh)
-                    : launch_wide_persistent<16, 240, false, 0, false, true>(*wide, r4, n, nullptr, h4, nullptr,
-                                                                            d_status, stream, work, replay, in,
-                                                                            hh);
-    }
-    if (wide_stack_variant(wide_bound) == 64) {
-        if (inst)
-            return any ? launch_wide_persistent<16, 48, true, 0, true>(*wide, r4, n, nullptr, nullptr, occ, d_status,
-                                                                       stream, work, replay, in)
-                       : launch_wide_persistent<16, 48, false, 0, true>(*wide, r4, n, nullptr, h4, nullptr, d_status,
-                                                                        stream, work, replay, in);
-        return any ? launch_wide_persistent<16, 48, true, 0>(*wide, r4, n, nullptr, nullptr, occ, d_status, stream,
-                                                             work, replay, in)
-                   : launch_wide_persistent<16, 48, false, 0>(*wide, r4, n, nullptr, h4, nullptr, d_status, stream,
-                                                              work, replay, in);
-    }
-    if (inst)
-        return any ? launch_wide_persistent<16, 240, true, 0, true>(*wide, r4, n, nullptr, nullptr, occ, d_status,
-                                                                    stream, work, replay, in)
-                   : launch_wide_persistent<16, 240, false, 0, true>(*wide, r4, n, nullptr, h4, nullptr, d_status,
-                                                                     stream, work, replay, in);
-    return any ? launch_wide_persistent<16, 240, true, 0>(*wide, r4, n, nullptr, nullptr, occ, d_status, stream,
-                                                          work, replay, in)
-               : launch_wide_persistent<16, 240, false, 0>(*wide, r4, n, nullptr, h4, nullptr, d_status, stream, work,
-                                                           replay, in);
+    float4* hh = reinterpret_cast<float4*>(host_hits);
+    return wide_stack_variant(wide_bound) == 64
+               ? launch_wide<64>(*wide, r4, n, nullptr, h4, occ, d_status, stream, true, work, replay, in, hh)
+               : launch_wide<256>(*wide, r4, n, nullptr, h4, occ, d_status, stream, true, work, replay, in, hh);
 }
 
 cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays, uint32_t n, PbrtHit* hits,
@@ -903,35 +706,27 @@ cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays,
                          uint32_t wide_bound, int kernel, const uint32_t* order, uint32_t* work, uint32_t* replay,
                          StreamIn in, PbrtHit* host_hits) {
     if (n == 0) return cudaSuccess;
-    if (!occluded && !replay) return cudaErrorInvalidValue;
+    if (!replay) return cudaErrorInvalidValue;
     read_variant();
     if ((in.ready || host_hits) && order) return cudaErrorInvalidValue;
+    bool replays = true;
     cudaError_t e = in.ready || host_hits
                         ? launch_streamed(bvh, rays, n, hits, occluded, d_status, stream, wide, wide_bound, work,
                                           replay, in, host_hits)
                         : launch_main(bvh, depth, rays, n, hits, occluded, d_status, stream, wide, wide_bound, kernel,
-                                      order, work, replay);
-    if (e != cudaSuccess || occluded) return e;
-    // the replay pass of closest hits (one empty launch unless a ray was marked)
+                                      order, work, replay, &replays);
+    if (e != cudaSuccess || !replays) return e;
+    // the replay pass (one empty launch unless a ray was marked)
     const unsigned grid = (unsigned)(device_sms() * 4);
     const float4* r4 = reinterpret_cast<const float4*>(rays);
     float4* h4 = reinterpret_cast<float4*>(hits);
     const bool inst = bvh.insts != nullptr;
-    const int v = wide ? wide_stack_variant(wide_bound) : 0;
-    const size_t smem = 16 * sizeof(uint2) * 128;
     float4* hh = reinterpret_cast<float4*>(host_hits);
-    if (v == 64)
-        inst ? k_replay4<16, 48, true><<<grid, 128, smem, stream>>>(*wide, r4, n, h4, replay, d_status, hh)
-             : k_replay4<16, 48, false><<<grid, 128, smem, stream>>>(*wide, r4, n, h4, replay, d_status, hh);
-    else if (v == 256)
-        inst ? k_replay4<16, 240, true><<<grid, 128, smem, stream>>>(*wide, r4, n, h4, replay, d_status, hh)
-             : k_replay4<16, 240, false><<<grid, 128, smem, stream>>>(*wide, r4, n, h4, replay, d_status, hh);
-    else if (trace_stack_for_depth(depth) == 64)
-        inst ? k_replay2<64, true><<<grid, 128, 0, stream>>>(bvh, r4, n, h4, replay, d_status)
-             : k_replay2<64, false><<<grid, 128, 0, stream>>>(bvh, r4, n, h4, replay, d_status);
+    auto go = [&](auto kernel) { kernel<<<grid, 128, 0, stream>>>(bvh, r4, n, h4, occluded, replay, d_status, hh); };
+    if (trace_stack_for_depth(depth) == 64)
+        inst ? go(k_replay2<64, true>) : go(k_replay2<64, false>);
     else
-        inst ? k_replay2<256, true><<<grid, 128, 0, stream>>>(bvh, r4, n, h4, replay, d_status)
-             : k_replay2<256, false><<<grid, 128, 0, stream>>>(bvh, r4, n, h4, replay, d_status);
+        inst ? go(k_replay2<256, true>) : go(k_replay2<256, false>);
     return cudaGetLastError();
 }
 

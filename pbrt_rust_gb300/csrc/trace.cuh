@@ -126,11 +126,11 @@ __device__ __forceinline__ bool slab_clean(float lox, float loy, float loz, floa
     return !(t0 > t1);
 }
 
-// src/shape/mesh.rs:41-72 with e1, e2 precomputed (same f32 subtraction).
+// src/shape/mesh.rs:41-72 for the triangle (r0, r1, r2) of a PrimRec.
 __device__ __forceinline__ bool tri_test(float4 r0, float4 r1, float4 r2, const DRay& r, float maxt, float* t_out,
                                          float* b1_out, float* b2_out) {
-    float e1x = r1.x, e1y = r1.y, e1z = r1.z;
-    float e2x = r2.x, e2y = r2.y, e2z = r2.z;
+    float e1x = r1.x - r0.x, e1y = r1.y - r0.y, e1z = r1.z - r0.z;
+    float e2x = r2.x - r0.x, e2y = r2.y - r0.y, e2z = r2.z - r0.z;
     float s1x = (r.dy * e2z) - (r.dz * e2y);
     float s1y = (r.dz * e2x) - (r.dx * e2z);
     float s1z = (r.dx * e2y) - (r.dy * e2x);
@@ -311,7 +311,7 @@ struct TraceResult {
 // Returns the definition-local hit (prim = its refined index, -1 on a miss);
 // the caller's maxt becomes the hit's t, as ray.set_maxt(r.maxt()) does.
 // Kept out of line so that the outer traversal's registers do not grow;
-// defined in trace4.cuh (the definitions are walked in the 4-wide layout).
+// defined in trace4.cuh (DevBVH4 carries the definitions' binary layout).
 template <bool ANY>
 __device__ __noinline__ TraceResult instance_test(const DevBVH4* insts, const SphereRec* s, float ox, float oy,
                                                   float oz, float dx, float dy, float dz, float tmin, float maxt);
@@ -499,6 +499,8 @@ __device__ __forceinline__ bool traverse(const DevBVH& bvh, const DRay& r, Trace
 // A closest hit whose walk accepted a NaN distance is written with this
 // prim value and rewritten by the replay kernels.
 constexpr int32_t kReplayMark = -2;
+// An any-hit answer that a replay kernel has to find.
+constexpr uint8_t kReplayOcc = 2;
 
 // True when every lane of the warp that has a ray (`active`) shares the
 // three direction signs, so that every node orders its children the same

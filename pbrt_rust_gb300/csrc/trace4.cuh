@@ -1,26 +1,69 @@
-// trace4.cuh - traversal over the 4-wide layout (layout.h: Node4).
+// trace4.cuh - traversal over the 4-wide layout (layout.h: QuadNode).
 //
-// Each Node4 holds the four grandchildren of one binary node N of the
-// reference tree.  A visit tests the four child boxes against the current
-// maxt and orders the hits exactly as BVHAccelerator::intersect
-// (src/primitive/aggregates/bvh.rs:390-417) would visit them: N's children
-// in dir_is_neg[axis(N)] order, and inside each, that child's children in
-// dir_is_neg order of its own axis.  The reference also tests the boxes of
-// N's two children; skipping them changes nothing: each is the union of
-// its children's boxes, so its planes are among theirs, and because f32
-// subtraction and multiplication are monotone the child's slab interval
-// always lies inside the parent's - a child that passes implies a parent
-// that passes.  The deferred children are pushed with their entry
-// distance t0 and re-checked against maxt when popped (see trace.cuh), so
-// every box decision, every primitive test and their order are the
-// reference's, and results are bit-identical to it, ties included.
+// Each node holds the four grandchildren of one binary node N of the
+// reference tree.  A visit tests the four child boxes and takes the ones that
+// pass in the order in which BVHAccelerator::intersect
+// (src/primitive/aggregates/bvh.rs:390-417) would: N's children in
+// dir_is_neg[axis(N)] order, and inside each, that child's children in
+// dir_is_neg order of its own axis.
 //
-// The stack lives in shared memory (SMAX 8-byte entries per thread,
-// [entry][thread] so a warp's accesses hit distinct banks) with an
-// optional local-memory overflow of OVF entries; the host picks a variant
-// whose SMAX + OVF covers the tree's bound (HostBVH::stack4_bound).
-// INST: the tree may hold instance records (kernels take it only for
-// scenes that have instances).
+// Why the results are the reference's bit for bit although the boxes here are
+// rounded.  The reference tests a leaf's primitives iff the leaf's own box
+// and every box above it pass against the maxt of the moment.  A box contains
+// its children's boxes, its planes are among theirs or beyond them, and f32
+// subtraction and multiplication are monotone, so whenever a leaf's box
+// passes, the boxes above it do (they are tested earlier, against a maxt at
+// least as large): the leaf's own box alone decides.  So a walk is exact if
+// it reaches, in the reference's order, every leaf whose box passes, and
+// lets a leaf's hits count only if the leaf's exact box passes.  Testing a
+// primitive changes nothing unless it is hit, so a leaf of one primitive has
+// its exact box tested only then (with the reference's operations,
+// trace.cuh: slab).  The boxes on the way need only never be smaller than
+// the exact ones:
+//  * the stored planes are rounded outwards;
+//  * a plane's distance is one fused multiply-add, t = code * (scale / d) +
+//    (org - o) / d, where the reference computes (plane - o) * (1 / d).  With
+//    u = 2^-24, R the largest coordinate of the tree and i = |1 / d|, the
+//    rounding of the two forms adds up to at most u i (9.2 R + 5 |o|), |o| the sum of the components (code *
+//    scale is at most 2.8 R, |org| 1.7 R); the near planes are moved towards
+//    the ray's start and the far planes away from it by e = u i (10 R + 8
+//    |o|);
+//  * an axis with d = 0 has 1 / d replaced by kZeroInv, so large that e is
+//    beyond every other distance: a plane at the origin or within e / i of it
+//    never culls, one farther off does.  The exact test has +-inf there, as
+//    the reference (d = -0 rejects an origin on the boundary of
+//    a box that is not flat, where a flat box inside it passes; but what is
+//    flat there and hit by a ray that runs within it is no triangle, whose
+//    determinant is 0; instances, which are entered on their box alone, send
+//    such rays the other way below).
+// The deferred children are pushed with their entry distance and re-checked
+// against maxt when popped.
+//
+// All of this needs finite numbers of moderate size.  Trees beyond 2^40 have
+// no 4-wide layout (HostBVH::wide), and a ray that is not `clean` (NaN or
+// infinite components, |o| > 2^40, |d| or 1 / d above 2^60, tmin below
+// -2^60) is walked over the binary layout in the exact mode of trace.cuh
+// instead (exact_hit / exact_any), as is a ray that accepted a hit at
+// distance NaN, after which the reference's box tests ignore maxt.  Kernels
+// with one thread per ray do that after the walk; the persistent ones mark
+// the ray for a replay kernel queued behind them, because the call inside
+// their loop costs the walk its registers (2^22 incoherent rays into a
+// terrain of a million triangles: 586 us with the calls, 529 without).
+//
+// The stack: ROWS 8-byte entries per thread in shared memory ([entry][thread],
+// so a warp's accesses hit distinct banks), the oldest entries going to an
+// array in local memory when they run out.  The bottom entry is a word that
+// ends the walk, so a pop needs no test for an empty stack.  A visit stores
+// all four children without branches: a 128-word table in shared memory,
+// indexed by the node's visiting order for the ray's octant and the mask of
+// passing children, gives each child's place above the top (children that
+// fail go to the place above the last one), and the first child is then
+// popped like any other, so the lanes of a warp run the same instructions
+// whether they hit children or not.  Against ordering the children by
+// compare-and-swap and branching per push, a visit is about 110 instructions
+// instead of 210 (2^20 rays into 4096 random triangles: 524 -> 405 us).
+// INST: the tree may hold instance records (kernels take it only for scenes
+// that have instances).
 #pragma once
 #include <stdint.h>
 
@@ -29,385 +72,28 @@
 
 namespace pbrt {
 
+// A tree in both layouts.
 struct DevBVH4 {
-    const Node4* nodes;
-    const PrimRec* prims;
-    const SphereRec* spheres;
-    ChildRec root;
-    uint32_t empty;
-    const DevBVH4* insts;  // the instance definitions' BVHs (kQuadInstance records index it)
+    DevBVH pair;            // the binary layout, primitives and analytic records
+    const QuadNode* nodes;
+    const LeafBox* boxes;
+    uint32_t root_ref;      // the root's child word
+    float reach;            // 5/4 of the tree's largest coordinate
 };
 
-struct ChildV {
-    float lx, ly, lz, hx, hy, hz;
-    uint32_t a, b;
-};
+// Stack words that are not children (leaf words stay below: HostBVH::wide
+// bounds the primitives).
+constexpr uint32_t kWalkDone = 0xfffffffdu;  // the bottom of the stack
+constexpr uint32_t kExitInst = 0xfffffffeu;  // ends the walk of an instance definition
 
-__device__ __forceinline__ ChildV ld_child(const ChildRec* c) {
-    ChildV v;
-    float f0, f1, f2, f3, f4, f5, f6, f7;
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(f0), "=f"(f1), "=f"(f2), "=f"(f3), "=f"(f4), "=f"(f5), "=f"(f6), "=f"(f7)
-                 : "l"(c));
-    v.lx = f0;
-    v.ly = f1;
-    v.lz = f2;
-    v.a = __float_as_uint(f3);
-    v.hx = f4;
-    v.hy = f5;
-    v.hz = f6;
-    v.b = __float_as_uint(f7);
-    return v;
-}
+constexpr float kRayReach = 1.099511627776e12f;         // 2^40
+constexpr float kInvMax = 1.152921504606846976e18f;     // 2^60, for |d| too
+constexpr float kZeroInv = 1.9342813113834067e25f;      // 2^84, in place of 1 / 0
+constexpr float kMarginUnit = 4.76837158203125e-07f;    // 8 u; DevBVH4::reach is 5/4 R
 
-// The same record through two 128-bit loads.
-__device__ __forceinline__ ChildV ld_child_v4(const ChildRec* c) {
-    ChildV v;
-    const float4 a = __ldg(reinterpret_cast<const float4*>(c)), b = __ldg(reinterpret_cast<const float4*>(c) + 1);
-    v.lx = a.x;
-    v.ly = a.y;
-    v.lz = a.z;
-    v.a = __float_as_uint(a.w);
-    v.hx = b.x;
-    v.hy = b.y;
-    v.hz = b.z;
-    v.b = __float_as_uint(b.w);
-    return v;
-}
-
-// Swaps two (child word, hit, entry distance) entries when c.
-__device__ __forceinline__ void cswap(bool c, uint32_t& a, uint32_t& b, bool& ha, bool& hb, float& ta, float& tb) {
-    const uint32_t x = c ? b : a, y = c ? a : b;
-    const bool hx = c ? hb : ha, hy = c ? ha : hb;
-    const float tx = c ? tb : ta, ty = c ? ta : tb;
-    a = x;
-    b = y;
-    ha = hx;
-    hb = hy;
-    ta = tx;
-    tb = ty;
-}
-
-// Stack word that ends the walk of an instance definition (never a leaf:
-// primitive offsets stay below 0x7ffffffe).
-constexpr uint32_t kExitInst = 0xfffffffeu;
-
-// LD256: fetch child records with one 256-bit load each (else two 128-bit
-// loads; the nested instance walk of the binary kernels lives in an
-// out-of-line function, where nvcc 13.0's back end crashes on the 256-bit
-// form).
-//
-// INST: the tree may hold instance records.  An instance is walked in the
-// same loop as the scene's tree (TransformedPrimitive::intersect,
-// transformed.rs:35-56): when its leaf entry is reached and the
-// primitive-space ray w2p(ray) - o as a point, d as a vector, mint and the
-// current maxt kept - passes the definition's root box, the walk pushes the
-// rest of the leaf and an exit word (both with entry distance -inf, so they
-// are always taken) and continues in the definition's tree with that ray;
-// popping the exit word restores the world ray and the scene's tree.  The
-// definition is thus searched completely, in the reference's order, before
-// the leaf's next primitive, and the shared maxt is the reference's
-// ray.set_maxt.  Hits inside report the instance's first id + the
-// definition-local index.  The stack bound of such a tree includes the
-// largest definition's bound + 2 (HostBVH::stack4_bound).
-// INST walks' extra state: the arrays of the tree being walked, the world
-// ray while inside an instance, and the instance's first id (0 outside).
-template <bool INST>
-struct InstWalk {
-    const Node4* nodes_;
-    const PrimRec* prims_;
-    const SphereRec* spheres_;
-    DRay world_;  // the world ray while inside an instance
-    uint32_t base_;
-};
-template <>
-struct InstWalk<false> {};
-
-//
-// EXACT: the replay walk (Traversal in trace.cuh): children are pushed on
-// their box alone and checked against maxt when taken.
-template <int SMAX, int OVF, bool INST = false, bool LD256 = true, bool EXACT = false>
-struct Traversal4 : InstWalk<INST> {
-    float maxt;
-    uint32_t cur;
-    int sp;
-    bool found;
-    bool overflow;
-    bool nan_hit;  // a NaN-distance hit was accepted: the result needs an EXACT replay
-    TraceResult res;
-    uint2* sstack;  // this thread's column: entry k at sstack[k * stride]
-    uint32_t stride;
-    uint2 ov[OVF > 0 ? OVF : 1];
-
-    __device__ __forceinline__ void bind(uint2* smem, uint32_t tid, uint32_t nthreads) {
-        sstack = smem + tid;
-        stride = nthreads;
-    }
-
-    __device__ __forceinline__ const Node4* node_base(const DevBVH4& bvh) const {
-        if constexpr (INST)
-            return this->nodes_;
-        else
-            return bvh.nodes;
-    }
-    __device__ __forceinline__ const PrimRec* prim_base(const DevBVH4& bvh) const {
-        if constexpr (INST)
-            return this->prims_;
-        else
-            return bvh.prims;
-    }
-    __device__ __forceinline__ const SphereRec* sphere_base(const DevBVH4& bvh) const {
-        if constexpr (INST)
-            return this->spheres_;
-        else
-            return bvh.spheres;
-    }
-
-    __device__ __forceinline__ bool start(const DevBVH4& bvh, const DRay& r) {
-        maxt = r.tmax;
-        found = false;
-        overflow = false;
-        nan_hit = false;
-        sp = 0;
-        res.prim = -1;
-        res.t = 0.0f;
-        res.b1 = 0.0f;
-        res.b2 = 0.0f;
-        if constexpr (INST) {
-            this->nodes_ = bvh.nodes;
-            this->prims_ = bvh.prims;
-            this->spheres_ = bvh.spheres;
-            this->base_ = 0;
-        }
-        if (bvh.empty) return false;
-        float tr;
-        const ChildRec& R = bvh.root;
-        if (!slab(R.lo_x, R.lo_y, R.lo_z, R.hi_x, R.hi_y, R.hi_z, r, maxt, &tr)) return false;
-        cur = R.a;
-        return true;
-    }
-
-    // The host only launches a variant whose SMAX + OVF covers the tree's
-    // stack bound; a full stack is still caught and reported, never written.
-    __device__ __forceinline__ void push(uint32_t ref, float t0) {
-        if (sp >= SMAX + OVF) {
-            overflow = true;
-            return;
-        }
-        uint2 e = make_uint2(ref, __float_as_uint(t0));
-        if (OVF == 0 || sp < SMAX)
-            sstack[(uint32_t)sp * stride] = e;
-        else
-            ov[sp - SMAX] = e;
-        ++sp;
-    }
-
-    __device__ __forceinline__ bool pop() {
-        while (sp > 0) {
-            --sp;
-            uint2 e = (OVF == 0 || sp < SMAX) ? sstack[(uint32_t)sp * stride] : ov[sp - SMAX];
-            if (!(__uint_as_float(e.y) > maxt)) {
-                cur = e.x;
-                return true;
-            }
-        }
-        return false;
-    }
-
-    // INST: starts the walk of instance record S (first id `first`) if the
-    // primitive-space ray hits its definition's root box; `resume` is the
-    // leaf word of the rest of the current leaf (0: none).
-    template <class R>
-    __device__ __forceinline__ bool enter(const DevBVH4& bvh, R& r, const SphereRec* S, uint32_t first,
-                                          uint32_t resume) {
-        float o[3], d[3];
-        xf_point(S->w2o, r.ox, r.oy, r.oz, o);  // transform.rs:230-237
-        xf_vector(S->w2o, r.dx, r.dy, r.dz, d);
-        // (tmax is not read while walking; it keeps the world ray's for a replay)
-        const DRay ri = make_dray(make_float4(o[0], o[1], o[2], r.tmin), make_float4(d[0], d[1], d[2], r.tmax));
-        const DevBVH4& D = bvh.insts[S->instance];
-        float tr;
-        const ChildRec& Rt = D.root;
-        if (D.empty || !slab(Rt.lo_x, Rt.lo_y, Rt.lo_z, Rt.hi_x, Rt.hi_y, Rt.hi_z, ri, maxt, &tr)) return false;
-        if (resume) push(resume, __int_as_float(0xff800000));  // -inf: always taken
-        push(kExitInst, __int_as_float(0xff800000));
-        this->world_ = r;
-        r = ri;
-        this->nodes_ = D.nodes;
-        this->prims_ = D.prims;
-        this->spheres_ = D.spheres;
-        this->base_ = first;
-        cur = Rt.a;
-        return !overflow;
-    }
-
-    // INST: back to the scene's tree and the world ray.
-    template <class R>
-    __device__ __forceinline__ void leave(const DevBVH4& bvh, R& r) {
-        r = this->world_;
-        this->nodes_ = bvh.nodes;
-        this->prims_ = bvh.prims;
-        this->spheres_ = bvh.spheres;
-        this->base_ = 0;
-    }
-
-    // Tests the primitives of leaf `ref` (a kNode4Leaf child word) in
-    // order.  Returns 0 when the leaf is done, 1 when ANY and a primitive
-    // was hit, 2 when an instance walk was entered (`cur` set).
-    template <bool ANY, class R>
-    __device__ __forceinline__ int leaf(const DevBVH4& bvh, R& r, uint32_t ref) {
-        uint32_t off = ref & ~kNode4Leaf;
-        for (;;) {
-            const PrimRec* pr = prim_base(bvh) + off;
-            float4 r0 = ldg4(pr->r0);
-            float4 r1 = ldg4(pr->r1);
-            float4 r2 = ldg4(pr->r2);
-            uint32_t id = __float_as_uint(r0.w);
-            const bool last = (__float_as_uint(r2.w) & kPrimLastBit) != 0;
-            float t, b1 = 0.0f, b2 = 0.0f;
-            bool hit;
-            if (id & kSphereBit) {
-                const uint32_t si = __float_as_uint(r1.w);
-                if constexpr (INST) {
-                    const SphereRec* S = sphere_base(bvh) + si;
-                    if (S->kind == kQuadInstance) {  // only in the scene's tree: definitions hold none
-                        if (enter(bvh, r, S, id & ~kSphereBit, last ? 0u : (kNode4Leaf | (off + 1)))) return 2;
-                        if (last) return 0;
-                        ++off;
-                        continue;
-                    }
-                }
-                hit = sphere_test(sphere_base(bvh), si, r, maxt, &t);
-            } else {
-                hit = tri_test(r0, r1, r2, r, maxt, &t, &b1, &b2);
-            }
-            if (hit) {
-                maxt = t;
-                found = true;
-                nan_hit |= !(t == t);
-                if constexpr (INST)
-                    res.prim = (int32_t)(this->base_ + (id & ~kSphereBit));
-                else
-                    res.prim = (int32_t)(id & ~kSphereBit);
-                res.t = t;
-                res.b1 = b1;
-                res.b2 = b2;
-                if (ANY) return 1;
-            }
-            if (last) return 0;
-            ++off;
-        }
-    }
-
-    // One unit of work; false once the ray is finished.
-    template <bool ANY, class R>
-    __device__ __forceinline__ bool step(const DevBVH4& bvh, R& r) {
-        if constexpr (INST) {
-            if (cur == kExitInst) {
-                leave(bvh, r);
-                return pop();
-            }
-        }
-        if (cur & kNode4Leaf) {
-            const int st = leaf<ANY>(bvh, r, cur);
-            if (st == 1) return false;
-            if (INST && st == 2) return !overflow;
-            return pop();
-        }
-        return node<ANY>(bvh, r);
-    }
-
-    // Visits inner node `cur`: tests its children and moves `cur` to the
-    // next node or leaf in the reference's order (an any-hit walk: nearest
-    // entry first); false once nothing is left.
-    template <bool ANY>
-    __device__ __forceinline__ bool node(const DevBVH4& bvh, const DRay& r) {
-        const Node4* nd = node_base(bvh) + cur;
-        ChildV c0, c1, c2, c3;
-        if (LD256) {
-            c0 = ld_child(&nd->c[0]);
-            c1 = ld_child(&nd->c[1]);
-            c2 = ld_child(&nd->c[2]);
-            c3 = ld_child(&nd->c[3]);
-        } else {
-            c0 = ld_child_v4(&nd->c[0]);
-            c1 = ld_child_v4(&nd->c[1]);
-            c2 = ld_child_v4(&nd->c[2]);
-            c3 = ld_child_v4(&nd->c[3]);
-        }
-        float t0, t1, t2, t3;
-        bool h0, h1, h2, h3;
-        const float lim = EXACT ? __int_as_float(0x7f800000) : maxt;  // replay: box alone
-        if (r.neg & kRayClean) {
-            h0 = c0.a != kNode4Empty && slab_clean(c0.lx, c0.ly, c0.lz, c0.hx, c0.hy, c0.hz, r, lim, &t0);
-            h1 = c1.a != kNode4Empty && slab_clean(c1.lx, c1.ly, c1.lz, c1.hx, c1.hy, c1.hz, r, lim, &t1);
-            h2 = c2.a != kNode4Empty && slab_clean(c2.lx, c2.ly, c2.lz, c2.hx, c2.hy, c2.hz, r, lim, &t2);
-            h3 = c3.a != kNode4Empty && slab_clean(c3.lx, c3.ly, c3.lz, c3.hx, c3.hy, c3.hz, r, lim, &t3);
-        } else {
-            h0 = c0.a != kNode4Empty && slab(c0.lx, c0.ly, c0.lz, c0.hx, c0.hy, c0.hz, r, lim, &t0);
-            h1 = c1.a != kNode4Empty && slab(c1.lx, c1.ly, c1.lz, c1.hx, c1.hy, c1.hz, r, lim, &t1);
-            h2 = c2.a != kNode4Empty && slab(c2.lx, c2.ly, c2.lz, c2.hx, c2.hy, c2.hz, r, lim, &t2);
-            h3 = c3.a != kNode4Empty && slab(c3.lx, c3.ly, c3.lz, c3.hx, c3.hy, c3.hz, r, lim, &t3);
-        }
-        if (!(h0 | h1 | h2 | h3)) return pop();
-        const uint32_t meta = c0.b;
-        const bool sN = (r.neg >> (meta & 3u)) & 1u;
-        const bool sL = (r.neg >> ((meta >> 2) & 3u)) & 1u;
-        const bool sR = (r.neg >> ((meta >> 4) & 3u)) & 1u;
-        // into visit order (bvh.rs:409-415): each child's pair of children
-        // by that child's axis sign, then the two pairs by N's
-        uint32_t a0 = c0.a, a1 = c1.a, a2 = c2.a, a3 = c3.a;
-        if (ANY && !EXACT) {
-            // An any-hit walk's answer does not depend on the order it takes
-            // children in (some primitive whose boxes all pass the ray's own
-            // maxt is hit, or none is), so it takes them by entry distance:
-            // an occluder near the ray's origin is met sooner.  Children that
-            // fail sort last; a five-comparator network sorts the four.
-            const float inf = __int_as_float(0x7f800000);
-            t0 = h0 ? t0 : inf;
-            t1 = h1 ? t1 : inf;
-            t2 = h2 ? t2 : inf;
-            t3 = h3 ? t3 : inf;
-            cswap(t0 > t1, a0, a1, h0, h1, t0, t1);
-            cswap(t2 > t3, a2, a3, h2, h3, t2, t3);
-            cswap(t0 > t2, a0, a2, h0, h2, t0, t2);
-            cswap(t1 > t3, a1, a3, h1, h3, t1, t3);
-            cswap(t1 > t2, a1, a2, h1, h2, t1, t2);
-        } else {
-            cswap(sL, a0, a1, h0, h1, t0, t1);
-            cswap(sR, a2, a3, h2, h3, t2, t3);
-            cswap(sN, a0, a2, h0, h2, t0, t2);
-            cswap(sN, a1, a3, h1, h3, t1, t3);
-        }
-        if (EXACT) {
-            // replay: the reference takes the first child whose box passes
-            // maxt now, culls the ones before it now, and tests the pushed
-            // ones against maxt when it pops them
-            bool scan = true;
-            if (scan && h0) {
-                if (t0 > maxt) h0 = false; else scan = false;
-            }
-            if (scan && h1) {
-                if (t1 > maxt) h1 = false; else scan = false;
-            }
-            if (scan && h2) {
-                if (t2 > maxt) h2 = false; else scan = false;
-            }
-            if (scan && h3 && t3 > maxt) h3 = false;
-            if (!(h0 | h1 | h2 | h3)) return pop();
-        }
-        const int first = h0 ? 0 : (h1 ? 1 : (h2 ? 2 : 3));
-        if (h3 && first < 3) push(a3, t3);
-        if (h2 && first < 2) push(a2, t2);
-        if (h1 && first < 1) push(a1, t1);
-        cur = first == 0 ? a0 : (first == 1 ? a1 : (first == 2 ? a2 : a3));
-        return !overflow;
-    }
-};
-
-// An instance definition's stack bound (HostBVH::stack4_bound) is at most
-// kInstStack4 (checked at creation), so the nested stack never overflows.
-constexpr int kInstStack4 = 96;
+// An instance definition's 4-wide stack bound is at most 96 (checked at
+// creation) and a binary walk defers no more entries than the 4-wide one.
+constexpr int kInstStack = 104;
 
 template <bool ANY>
 __device__ __noinline__ TraceResult instance_test(const DevBVH4* insts, const SphereRec* s, float ox, float oy,
@@ -416,19 +102,511 @@ __device__ __noinline__ TraceResult instance_test(const DevBVH4* insts, const Sp
     xf_point(s->w2o, ox, oy, oz, o);  // transform.rs:230-237: o as a point, d as a vector
     xf_vector(s->w2o, dx, dy, dz, d);
     DRay ri = make_dray(make_float4(o[0], o[1], o[2], tmin), make_float4(d[0], d[1], d[2], maxt));
-    const DevBVH4& B = insts[s->instance];
-    Traversal4<0, kInstStack4, false, false> T;  // the whole stack in local memory
-    if (T.start(B, ri)) {
-        while (T.template step<ANY>(B, ri)) {
-        }
-    }
-    if (ANY || !T.nan_hit) return T.res;
-    Traversal4<0, kInstStack4, false, false, true> E;  // replay
-    if (E.start(B, ri)) {
-        while (E.template step<false>(B, ri)) {
-        }
-    }
-    return E.res;
+    const DevBVH& B = insts[s->instance].pair;
+    TraceResult res;
+    int st = 0;
+    bool nan_hit = false;
+    traverse<kInstStack, ANY>(B, ri, &res, &st, &nan_hit);
+    if (!ANY && nan_hit) traverse<kInstStack, false, false, true>(B, ri, &res, &st);  // replay
+    return res;
 }
+
+// One ray over the binary layout in exact mode: the closest hit's record /
+// whether anything is hit.  `ray`: its two float4.  Out of line: few rays
+// need them.
+template <int STACK, bool INST>
+static __device__ __noinline__ float4 exact_hit(const DevBVH& bvh, const float4* ray, int* status) {
+    const DRay r = make_dray(__ldg(ray), __ldg(ray + 1));
+    TraceResult res;
+    int st = 0;
+    traverse<STACK, false, INST, true>(bvh, r, &res, &st);
+    if (st) atomicMax(status, st);
+    return make_float4(__int_as_float(res.prim), res.t, res.b1, res.b2);
+}
+template <int STACK, bool INST>
+static __device__ __noinline__ bool exact_any(const DevBVH& bvh, const float4* ray, int* status) {
+    const DRay r = make_dray(__ldg(ray), __ldg(ray + 1));
+    TraceResult res;
+    int st = 0;
+    const bool found = traverse<STACK, true, INST>(bvh, r, &res, &st);
+    if (st) atomicMax(status, st);
+    return found;
+}
+
+// Two f32 values in one 64-bit register; sm_103a multiplies and adds both in
+// one instruction, each rounded on its own.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+struct Words8 {
+    uint32_t w[8];
+};
+__device__ __forceinline__ Words8 ld_words8(const void* p) {  // 32 bytes in one load
+    Words8 q;
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(q.w[0]), "=r"(q.w[1]), "=r"(q.w[2]), "=r"(q.w[3]), "=r"(q.w[4]), "=r"(q.w[5]), "=r"(q.w[6]),
+                   "=r"(q.w[7])
+                 : "l"(p));
+    return q;
+}
+
+// Byte k of a plane word as the plane's grid coordinate (layout.h).
+__device__ __forceinline__ float plane(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x43000000u, 0x7044u | ((uint32_t)k << 8)));
+}
+
+// Stack entries by 32-bit shared-memory address.
+__device__ __forceinline__ void st_entry(uint32_t addr, uint32_t ref, float t) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(ref), "f"(t) : "memory");
+}
+__device__ __forceinline__ void ld_entry(uint32_t addr, uint32_t& ref, float& t) {
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(ref), "=f"(t) : "r"(addr) : "memory");
+}
+
+// The push table: entry [code][mask], byte k = rows above the top at which
+// child k goes (the child visited first on top; children not in the mask
+// above them all).  code: bit 0 / 1 = the first / second pair's children swap
+// places, bit 2 = the pairs do.
+constexpr int kPushTable = 128;
+__device__ __forceinline__ uint32_t push_entry(uint32_t i) {
+    const uint32_t code = i >> 4, mask = i & 15u;
+    auto place = [&](uint32_t k) {  // of child k among the four
+        const uint32_t pair = k >> 1;
+        return ((pair ^ (code >> 2)) << 1) | ((k & 1u) ^ ((code >> pair) & 1u));
+    };
+    uint32_t e = 0;
+    for (uint32_t k = 0; k < 4; ++k) {
+        uint32_t row = 0;
+        for (uint32_t j = 0; j < 4; ++j)
+            if ((mask >> j) & 1u) row += ((mask >> k) & 1u) ? (place(j) > place(k) ? 1u : 0u) : 1u;
+        e |= row << (8 * k);
+    }
+    return e;
+}
+
+// Shared memory of a block of 4-wide walks: the stacks, the push table and,
+// with instances, the world rays of the lanes that are inside one.
+template <int BLOCK, int ROWS, bool INST>
+struct alignas(16) WalkShared {
+    uint2 stack[ROWS][BLOCK];
+    uint32_t push[kPushTable];
+    float world[INST ? 9 : 1][INST ? BLOCK : 1];
+    // every thread of the block; __syncthreads() inside
+    __device__ __forceinline__ void init() {
+        if (threadIdx.x < kPushTable) push[threadIdx.x] = push_entry(threadIdx.x);
+        __syncthreads();
+    }
+};
+
+// INST walks' extra state: the tree being walked (-1: the scene's, else the
+// definition) with its arrays, and the instance's first id (0 outside).
+template <bool INST>
+struct InstWalk {
+    const QuadNode* nodes_;
+    const PrimRec* prims_;
+    int32_t def_;
+    uint32_t base_;
+};
+template <>
+struct InstWalk<false> {};
+
+enum { kStartMiss = 0, kStartWalk = 1, kStartExact = 2 };
+
+// The oldest entries of a walk's stack, in local memory.  A kernel declares
+// it beside the walk: inside it, its variable indexing would keep the whole
+// walk out of registers.
+template <int OVF>
+struct Overflow {
+    uint2 e[OVF];
+};
+
+// The walk of one ray.  `cur` is the next node (non-negative as an integer),
+// the next leaf, or one of the stack words above; node() and leaf() move it
+// on.  OVF: entries of the overflow (64 or 256, as the tree's stack bound
+// asks).
+template <int BLOCK, int ROWS, int OVF, bool ANY, bool INST = false>
+struct Walk4 : InstWalk<INST> {
+    static constexpr uint32_t kRow = BLOCK * 8u;
+    static constexpr int kSpill = ROWS - 8;  // rows moved to the overflow at a time
+    using Shared = WalkShared<BLOCK, ROWS, INST>;
+    using Ovf = Overflow<OVF>;
+
+    float ox, oy, oz, tmin;
+    float dx, dy, dz, maxt;
+    float ix, iy, iz;  // 1 / d (kZeroInv for d = 0)
+    float ex, ey, ez;  // margins of a plane's distance
+    uint32_t oct3;     // 3 * the ray's octant
+    uint32_t cur;
+    uint32_t top;      // shared-memory address of the first free row
+    int spilled;       // entries in the overflow; -1: they would not fit (reported, never written)
+    int32_t prim;
+    float b1, b2;
+    bool give_up;      // a hit at distance NaN or an instance ray that is not clean: the ray needs the exact walk
+    uint32_t bottom, push_tab;
+
+    __device__ __forceinline__ void bind(Shared& sh) {
+        bottom = (uint32_t)__cvta_generic_to_shared(&sh.stack[0][threadIdx.x]);
+        push_tab = (uint32_t)__cvta_generic_to_shared(sh.push);
+        st_entry(bottom, kWalkDone, __int_as_float(0xff800000));  // -inf: always taken
+        cur = kWalkDone;
+    }
+
+    // 1 / d, octant and margins of the ray (o, d) in a tree of the given
+    // reach; false if the ray is not clean (see above).
+    __device__ __forceinline__ bool aim(float reach) {
+        const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
+        ix = 1.0f / dx;
+        iy = 1.0f / dy;
+        iz = 1.0f / dz;
+        // sums, so that a NaN component fails the comparison
+        const float so = fabsf(ox) + fabsf(oy) + fabsf(oz), sd = fabsf(dx) + fabsf(dy) + fabsf(dz);
+        bool ok = so <= kRayReach && sd <= kInvMax && sd > 0.0f && tmin >= -kInvMax && maxt == maxt &&
+                  max3f(zx ? 0.0f : fabsf(ix), zy ? 0.0f : fabsf(iy), zz ? 0.0f : fabsf(iz)) <= kInvMax;
+        if (INST)  // -0: see above
+            ok = ok && __float_as_uint(dx) != 0x80000000u && __float_as_uint(dy) != 0x80000000u &&
+                 __float_as_uint(dz) != 0x80000000u;
+        if (zx) ix = copysignf(kZeroInv, dx);
+        if (zy) iy = copysignf(kZeroInv, dy);
+        if (zz) iz = copysignf(kZeroInv, dz);
+        margins(reach);
+        return ok;
+    }
+    __device__ __forceinline__ void margins(float reach) {
+        oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) | ((__float_as_uint(iz) >> 31) << 2));
+        const float m = kMarginUnit * (reach + (fabsf(ox) + fabsf(oy) + fabsf(oz)));
+        ex = m * fabsf(ix);
+        ey = m * fabsf(iy);
+        ez = m * fabsf(iz);
+    }
+    // The ray with the reference's 1 / d, for the exact tests.
+    __device__ __forceinline__ DRay ray() const {
+        DRay r;
+        r.ox = ox;
+        r.oy = oy;
+        r.oz = oz;
+        r.tmin = tmin;
+        r.dx = dx;
+        r.dy = dy;
+        r.dz = dz;
+        r.tmax = maxt;
+        auto inv = [](float i) { return fabsf(i) == kZeroInv ? copysignf(__int_as_float(0x7f800000), i) : i; };
+        r.ix = inv(ix);
+        r.iy = inv(iy);
+        r.iz = inv(iz);
+        r.neg = 0;
+        return r;
+    }
+
+    __device__ __forceinline__ int start(const DevBVH4& bvh, float4 a, float4 b) {
+        ox = a.x;
+        oy = a.y;
+        oz = a.z;
+        tmin = a.w;
+        dx = b.x;
+        dy = b.y;
+        dz = b.z;
+        maxt = b.w;
+        prim = -1;
+        b1 = 0.0f;
+        b2 = 0.0f;
+        give_up = false;
+        spilled = 0;
+        top = bottom + kRow;
+        if constexpr (INST) {
+            this->nodes_ = bvh.nodes;
+            this->prims_ = bvh.pair.prims;
+            this->def_ = -1;
+            this->base_ = 0;
+        }
+        if (bvh.pair.empty) return kStartMiss;
+        if (!aim(bvh.reach)) return kStartExact;
+        // the root's box by the same conservative test
+        const ChildRec& R = bvh.pair.root;
+        const float ax = (R.lo_x - ox) * ix, bx = (R.hi_x - ox) * ix;
+        const float ay = (R.lo_y - oy) * iy, by = (R.hi_y - oy) * iy;
+        const float az = (R.lo_z - oz) * iz, bz = (R.hi_z - oz) * iz;
+        const float t0 = max3f(fminf(ax, bx) - ex, fminf(ay, by) - ey, fmaxf(fminf(az, bz) - ez, tmin));
+        const float t1 = min3f(fmaxf(ax, bx) + ex, fmaxf(ay, by) + ey, fminf(fmaxf(az, bz) + ez, maxt));
+        if (t0 > t1) return kStartMiss;
+        cur = bvh.root_ref;
+        return kStartWalk;
+    }
+
+    // Moves the oldest rows to the overflow when fewer than four are free.
+    __device__ __forceinline__ void make_room(Ovf& ov) {
+        if (top <= bottom + (ROWS - 4) * kRow) return;
+        if (spilled < 0 || spilled + kSpill > OVF) {
+            spilled = -1;
+            top = bottom + kRow;  // the pop that follows ends the walk
+            return;
+        }
+        for (int i = 0; i < kSpill; ++i) {
+            uint32_t ref;
+            float t;
+            ld_entry(bottom + (uint32_t)(1 + i) * kRow, ref, t);
+            ov.e[spilled + i] = make_uint2(ref, __float_as_uint(t));
+        }
+        spilled += kSpill;
+        for (uint32_t a = bottom + (1 + kSpill) * kRow; a < top; a += kRow) {
+            uint32_t ref;
+            float t;
+            ld_entry(a, ref, t);
+            st_entry(a - kSpill * kRow, ref, t);
+        }
+        top -= kSpill * kRow;
+    }
+    // An any-hit walk's maxt does not change, so its entries still pass.
+    __device__ __forceinline__ void pop() {
+        float t;
+        do {
+            top -= kRow;
+            ld_entry(top, cur, t);
+        } while (!ANY && t > maxt);
+    }
+    // cur == kWalkDone: brings spilled rows back and goes on; false when the
+    // walk is over.
+    __device__ __forceinline__ bool resume(Ovf& ov) {
+        if (spilled <= 0) return false;
+        spilled -= kSpill;
+        for (int i = 0; i < kSpill; ++i)
+            st_entry(bottom + (uint32_t)(1 + i) * kRow, ov.e[spilled + i].x, __uint_as_float(ov.e[spilled + i].y));
+        top = bottom + (1 + kSpill) * kRow;
+        pop();
+        return true;
+    }
+
+    // Visits inner node `cur`.
+    __device__ __forceinline__ void node(const DevBVH4& bvh, Ovf& ov) {
+        const QuadNode* nodes;
+        if constexpr (INST)
+            nodes = this->nodes_;
+        else
+            nodes = bvh.nodes;
+        const char* p = reinterpret_cast<const char*>(nodes + cur);
+        const Words8 q0 = ld_words8(p), q1 = ld_words8(p + 32);
+        const bool px = ix < 0.0f, py = iy < 0.0f, pz = iz < 0.0f;
+        const uint32_t nx = px ? q0.w[7] : q0.w[6], fx = px ? q0.w[6] : q0.w[7];
+        const uint32_t ny = py ? q1.w[1] : q1.w[0], fy = py ? q1.w[0] : q1.w[1];
+        const uint32_t nz = pz ? q1.w[3] : q1.w[2], fz = pz ? q1.w[2] : q1.w[3];
+        const float gx = __uint_as_float(q0.w[0]) - ox, gy = __uint_as_float(q0.w[1]) - oy,
+                    gz = __uint_as_float(q0.w[2]) - oz;
+        const float ax = __uint_as_float(q0.w[3]) * ix, ay = __uint_as_float(q0.w[3] << 16) * iy,
+                    az = __uint_as_float(q0.w[4]) * iz;
+        const uint64_t bx = pack2(__fmaf_rn(gx, ix, -ex), __fmaf_rn(gx, ix, ex));
+        const uint64_t by = pack2(__fmaf_rn(gy, iy, -ey), __fmaf_rn(gy, iy, ey));
+        const uint64_t bz = pack2(__fmaf_rn(gz, iz, -ez), __fmaf_rn(gz, iz, ez));
+        const uint64_t ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+        float t[4];
+        uint32_t mask = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float n0, f0, n1, f1, n2, f2;
+            unpack2(fma2(pack2(plane(nx, k), plane(fx, k)), ax2, bx), n0, f0);
+            unpack2(fma2(pack2(plane(ny, k), plane(fy, k)), ay2, by), n1, f1);
+            unpack2(fma2(pack2(plane(nz, k), plane(fz, k)), az2, bz), n2, f2);
+            t[k] = max3f(n0, n1, fmaxf(n2, tmin));
+            const float t1 = min3f(f0, f1, fminf(f2, maxt));
+            if (!(t[k] > t1)) mask |= 1u << k;
+        }
+        const uint32_t code = (q0.w[5] >> oct3) & 7u;
+        uint32_t e;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e) : "r"(push_tab + (code * 16u + mask) * 4u));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) st_entry(top + kRow * __byte_perm(e, 0u, 0x4440u | (uint32_t)k), q1.w[4 + k], t[k]);
+        top += kRow * (uint32_t)__popc(mask);
+        make_room(ov);
+        pop();
+    }
+
+    // Hit at t of primitive word `id`.
+    __device__ __forceinline__ void accept(uint32_t id, float t, float u, float v) {
+        maxt = t;
+        give_up |= !(t == t);
+        if constexpr (INST)
+            prim = (int32_t)(this->base_ + (id & ~kSphereBit));
+        else
+            prim = (int32_t)(id & ~kSphereBit);
+        b1 = u;
+        b2 = v;
+    }
+    // An any-hit walk is over.
+    __device__ __forceinline__ void stop() {
+        cur = kWalkDone;
+        spilled = min(spilled, 0);
+    }
+
+    // INST: the instance record S (first id `first`) of the scene's tree;
+    // `rest` is the leaf word of the rest of its leaf (0: none).  1 when its
+    // walk was entered (`cur` set), 0 when the ray misses it, 2 when the
+    // primitive-space ray is not clean: the whole ray then takes the exact
+    // walk.  TransformedPrimitive::intersect
+    // (transformed.rs:35-56): the primitive-space ray is w2p(ray) - o as a
+    // point, d as a vector, mint and the current maxt kept.  If it passes the
+    // definition's root box, the walk pushes the rest of the leaf and an exit
+    // word (both with entry distance -inf, so they are always taken) and
+    // continues in the definition's tree with that ray; popping the exit word
+    // restores the world ray and the scene's tree.  The definition is thus
+    // searched completely, in the reference's order, before the leaf's next
+    // primitive, and the shared maxt is the reference's ray.set_maxt.
+    __device__ __forceinline__ int enter(const DevBVH4& bvh, Shared& sh, const SphereRec* S, uint32_t first,
+                                         uint32_t rest) {
+        const DevBVH4& D = bvh.pair.insts[S->instance];
+        if (D.pair.empty) return 0;
+        float o[3], d[3];
+        xf_point(S->w2o, ox, oy, oz, o);  // transform.rs:230-237
+        xf_vector(S->w2o, dx, dy, dz, d);
+        float* w = &sh.world[0][threadIdx.x];
+        const float keep[9] = {ox, oy, oz, dx, dy, dz, ix, iy, iz};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) w[k * BLOCK] = keep[k];
+        ox = o[0];
+        oy = o[1];
+        oz = o[2];
+        dx = d[0];
+        dy = d[1];
+        dz = d[2];
+        const ChildRec& R = D.pair.root;
+        float tr;
+        if (!aim(D.reach)) return 2;
+        if (!slab(R.lo_x, R.lo_y, R.lo_z, R.hi_x, R.hi_y, R.hi_z, ray(), maxt, &tr)) {
+            restore(bvh, sh);
+            return 0;
+        }
+        if (rest) {
+            st_entry(top, rest, __int_as_float(0xff800000));
+            top += kRow;
+        }
+        st_entry(top, kExitInst, __int_as_float(0xff800000));
+        top += kRow;
+        if constexpr (INST) {
+            this->nodes_ = D.nodes;
+            this->prims_ = D.pair.prims;
+            this->def_ = (int32_t)S->instance;
+            this->base_ = first;
+        }
+        cur = D.root_ref;
+        return 1;
+    }
+    // Back to the scene's tree and the world ray.
+    __device__ __forceinline__ void restore(const DevBVH4& bvh, Shared& sh) {
+        const float* w = &sh.world[0][threadIdx.x];
+        ox = w[0];
+        oy = w[BLOCK];
+        oz = w[2 * BLOCK];
+        dx = w[3 * BLOCK];
+        dy = w[4 * BLOCK];
+        dz = w[5 * BLOCK];
+        ix = w[6 * BLOCK];
+        iy = w[7 * BLOCK];
+        iz = w[8 * BLOCK];
+        margins(bvh.reach);
+        if constexpr (INST) {
+            this->nodes_ = bvh.nodes;
+            this->prims_ = bvh.pair.prims;
+            this->def_ = -1;
+            this->base_ = 0;
+        }
+    }
+
+    // `cur` is a leaf (or INST: the exit word): tests its primitives in order
+    // and goes on.
+    __device__ __forceinline__ void leaf(const DevBVH4& bvh, Shared& sh, Ovf& ov) {
+        const PrimRec* prims;
+        const SphereRec* spheres;
+        const LeafBox* boxes;
+        if constexpr (INST) {
+            if (cur == kExitInst) {
+                restore(bvh, sh);
+                pop();
+                return;
+            }
+            prims = this->prims_;
+            const DevBVH4& B = this->def_ < 0 ? bvh : bvh.pair.insts[this->def_];
+            spheres = B.pair.spheres;
+            boxes = B.boxes;
+        } else {
+            prims = bvh.pair.prims;
+            spheres = bvh.pair.spheres;
+            boxes = bvh.boxes;
+        }
+        uint32_t off = cur & ~kNode4Leaf;
+        for (;;) {
+            const PrimRec* pr = prims + off;
+            const float4 r0 = ldg4(pr->r0), r1 = ldg4(pr->r1), r2 = ldg4(pr->r2);
+            const uint32_t id = __float_as_uint(r0.w), flags = __float_as_uint(r2.w);
+            auto table_box = [&]() {
+                const LeafBox* b = boxes + (flags >> kPrimBoxShift);
+                const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
+                float tr;
+                return slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr);
+            };
+            if ((flags & kPrimBoxEntry) && !table_box()) break;
+            float t, u = 0.0f, v = 0.0f;
+            bool hit;
+            if (id & kSphereBit) {
+                const uint32_t si = __float_as_uint(r1.w);
+                if constexpr (INST) {
+                    const SphereRec* S = spheres + si;
+                    if (S->kind == kQuadInstance) {  // only in the scene's tree: definitions hold none
+                        const int e = enter(bvh, sh, S, id & ~kSphereBit,
+                                            (flags & kPrimLastBit) ? 0u : (kNode4Leaf | (off + 1)));
+                        if (e == 1) return make_room(ov);
+                        if (e == 2) {
+                            give_up = true;
+                            return stop();
+                        }
+                        if (flags & kPrimLastBit) break;
+                        ++off;
+                        continue;
+                    }
+                }
+                hit = sphere_test(spheres, si, ray(), maxt, &t);
+                if (hit && (flags & kPrimHitBox)) hit = table_box();
+            } else {
+                hit = tri_test(r0, r1, r2, ray(), maxt, &t, &u, &v);
+                if (hit && (flags & kPrimOwnBox)) {
+                    float tr;
+                    hit = slab(fminf(fminf(r0.x, r1.x), r2.x), fminf(fminf(r0.y, r1.y), r2.y),
+                               fminf(fminf(r0.z, r1.z), r2.z), fmaxf(fmaxf(r0.x, r1.x), r2.x),
+                               fmaxf(fmaxf(r0.y, r1.y), r2.y), fmaxf(fmaxf(r0.z, r1.z), r2.z), ray(), maxt, &tr);
+                }
+            }
+            if (hit) {
+                accept(id, t, u, v);
+                if (ANY) return stop();
+            }
+            if (flags & kPrimLastBit) break;
+            ++off;
+        }
+        pop();
+    }
+
+    // The whole walk after start() returned kStartWalk.
+    __device__ __forceinline__ void run(const DevBVH4& bvh, Shared& sh, Ovf& ov) {
+        for (;;) {
+            if ((int32_t)cur >= 0)
+                node(bvh, ov);
+            else if (cur != kWalkDone)
+                leaf(bvh, sh, ov);
+            else if (!resume(ov))
+                return;
+        }
+    }
+    __device__ __forceinline__ bool found() const { return prim >= 0; }
+    __device__ __forceinline__ float4 hit_record() const {
+        return make_float4(__int_as_float(prim), prim >= 0 ? maxt : 0.0f, b1, b2);
+    }
+};
 
 }  // namespace pbrt
