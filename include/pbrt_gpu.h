@@ -330,7 +330,8 @@ typedef struct PbrtTraceConfig {
                                are streamed with 0 only */
     int32_t render_kernel;  /* PBRT_TRACE_*: camera rays inside pbrtgpu_render; shadow
                                rays take the 4-wide kernel with a 4-wide choice, else
-                               the binary one */
+                               the binary one.  The default, PBRT_TRACE_WIDE, takes the
+                               binary kernels for trees of fewer than 4096 primitives */
     uint32_t reorder;       /* 1: pbrtgpu_intersect / intersect_p batches of 32768 rays
                                or more are binned by direction and origin before
                                traversal (same results, more coherent warps) */

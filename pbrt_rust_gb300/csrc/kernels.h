@@ -120,8 +120,9 @@ cudaError_t launch_chacha_blocks(const uint32_t key[8], uint64_t ctr, uint64_t s
                                  uint32_t n_blocks, uint32_t* d_out, cudaStream_t s);
 cudaError_t launch_rng_words(const uint32_t key[8], uint64_t first, uint32_t n, uint32_t seg, uint32_t* d_out,
                              cudaStream_t s);
-// Kernel used for the coherent camera and shadow rays of a render.
-int render_trace_kernel();
+// Kernel used for the coherent camera and shadow rays of a render over a
+// tree of n_prims primitives.
+int render_trace_kernel(uint32_t n_prims);
 // 64 or 256 when a compiled 4-wide variant covers this stack bound, else 0.
 int wide_stack_variant(uint32_t bound);
 

@@ -180,7 +180,7 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
     if (P.n_samples) {
         // camera rays of neighbouring pixels are coherent: one thread per
         // ray keeps them together in a warp
-        const int rk = render_trace_kernel();
+        const int rk = render_trace_kernel(P.bvh.n_prims);
         e = launch_trace(P.bvh, P.depth, P.rays, (uint32_t)P.n_samples, reinterpret_cast<PbrtHit*>(P.hits), nullptr,
                          (int*)&P.counters[2], s, P.has_wide ? &P.bvh4 : nullptr, P.wide_bound, rk, nullptr, nullptr,
                          &P.counters[3]);

@@ -413,7 +413,7 @@ enum {
 static int g_kernel_variant = -1;
 static unsigned g_refill = 4;
 static unsigned g_min_blocks = 0;
-static int g_render_kernel = kVariantPairPlain;
+static int g_render_kernel = kVariantWidePlain;
 static unsigned g_reorder = 0;
 static unsigned g_chunk = 64;
 
@@ -564,9 +564,17 @@ bool trace_reorder() {
     read_variant();
     return g_reorder != 0;
 }
-int render_trace_kernel() {
+// A tree of a few thousand primitives sits in L1, where a binary visit's
+// fewer instructions win over the 4-wide walk's fewer steps.  Camera + shadow
+// rays of 512 x 512 x 4 frames, binary against 4-wide, us: terrains of 300 /
+// 2000 / 20000 triangles 84 / 134 / 251 against 95 / 144 / 221, 64 spheres
+// 100 against 117, soups of 300 / 1000 / 4000 triangles 61 / 97 / 241 against
+// 58 / 78 / 168: the line is where no scene is slower.
+constexpr uint32_t kWideRenderPrims = 4096;
+int render_trace_kernel(uint32_t n_prims) {
     read_variant();
-    return g_render_kernel;
+    return g_render_kernel == kVariantWidePlain && n_prims < kWideRenderPrims ? (int)kVariantPairPlain
+                                                                              : g_render_kernel;
 }
 
 int wide_stack_variant(uint32_t bound) {

@@ -592,15 +592,19 @@ struct Walk4 : InstWalk<INST> {
         pop();
     }
 
-    // The whole walk after start() returned kStartWalk.
+    // The whole walk after start() returned kStartWalk.  Two visits per turn
+    // before the leaves: the lanes of a warp that reach a leaf one visit apart
+    // test it together (camera / shadow rays of a 1024 x 1024 x 16 terrain
+    // frame: 2282 / 3911 us with node or leaf per turn, 2038 / 2676 with one
+    // visit, 1952 / 2631 with two, 1985 / 2831 with three; waiting for 4 or
+    // more lanes at leaves is slower, 2111 / 2757).
     __device__ __forceinline__ void run(const DevBVH4& bvh, Shared& sh, Ovf& ov) {
         for (;;) {
-            if ((int32_t)cur >= 0)
-                node(bvh, ov);
-            else if (cur != kWalkDone)
-                leaf(bvh, sh, ov);
-            else if (!resume(ov))
-                return;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                if ((int32_t)cur >= 0) node(bvh, ov);
+            if ((int32_t)cur < 0 && cur != kWalkDone) leaf(bvh, sh, ov);
+            if (cur == kWalkDone && !resume(ov)) return;
         }
     }
     __device__ __forceinline__ bool found() const { return prim >= 0; }
