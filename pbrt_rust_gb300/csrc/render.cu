@@ -24,7 +24,7 @@
 namespace pbrt {
 
 __global__ void __launch_bounds__(128) k_generate(RenderParams P) {
-    __shared__ uint32_t words[32 * 128];  // the threads' ChaCha block pairs
+    __shared__ uint32_t words[16 * 128];  // the threads' ChaCha blocks
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= P.n_pixels) return;
     generate_pixel(P, pix, words + threadIdx.x, 128u);
@@ -125,17 +125,22 @@ __global__ void __launch_bounds__(128) k_chacha_blocks(Key8 key, uint64_t ctr0, 
 }
 
 // Words [first, first + n) of one task's stream as generate_pixel reads
-// them: thread t seeks to word first + t * seg and reads its segment of seg
-// words (the last one shorter) with the WordStream reader.
+// them: thread t reads the seg words from first + t * seg (the last one
+// fewer) through its window, block by block.
 __global__ void __launch_bounds__(128) k_rng_words(Key8 key, uint64_t first, uint32_t n, uint32_t seg,
                                                    uint32_t* out) {
-    __shared__ uint32_t words[32 * 128];
+    __shared__ uint32_t words[16 * 128];
     const uint64_t lo = (uint64_t)(blockIdx.x * blockDim.x + threadIdx.x) * seg;
     if (lo >= n) return;
     const uint64_t hi = lo + seg < n ? lo + seg : n;
-    WordStream rng;
-    rng.seek(key.k, first + lo, first + hi, words + threadIdx.x, 128u);
-    for (uint64_t w = lo; w < hi; ++w) out[w] = rng.next_u32();
+    WordWindow rng(key.k, words + threadIdx.x, 128u);
+    for (uint64_t w = lo; w < hi;) {
+        rng.load(first + w);
+        do {
+            out[w] = rng.word(first + w);
+            ++w;
+        } while (w < hi && ((first + w) & 15u));
+    }
 }
 
 // ------------------------------------------------------------ launchers ---

@@ -37,38 +37,6 @@ __device__ __forceinline__ int32_t dev_f2i32(float f) {  // Rust `as i32`: satur
 }
 
 // ------------------------------------------------------------- generate ---
-// montecarlo.rs:115-128
-__device__ __forceinline__ void stratified_2d(float* s, uint32_t nx, uint32_t ny, WordStream& rng, bool jitter) {
-    float dx = 1.0f / (float)nx, dy = 1.0f / (float)ny;
-    for (uint32_t y = 0; y < ny; ++y)
-        for (uint32_t x = 0; x < nx; ++x) {
-            float jx = jitter ? rng.random_float() : 0.5f;
-            float jy = jitter ? rng.random_float() : 0.5f;
-            uint32_t off = 2 * (y * nx + x);
-            s[off] = ((float)x + jx) * dx;
-            s[off + 1] = ((float)y + jy) * dy;
-        }
-}
-// montecarlo.rs:106-113
-__device__ __forceinline__ void stratified_1d(float* s, uint32_t n, WordStream& rng, bool jitter) {
-    float inv = 1.0f / (float)n;
-    for (uint32_t i = 0; i < n; ++i) {
-        float d = jitter ? rng.random_float() : 0.5f;
-        s[i] = ((float)i + d) * inv;
-    }
-}
-// rng.rs:23-33
-__device__ __forceinline__ void shuffle(float* v, uint32_t count, uint32_t dims, WordStream& rng) {
-    for (uint32_t i = 0; i < count; ++i) {
-        uint32_t other = i + (uint32_t)(rng.random_uint() % (uint64_t)(count - i));
-        for (uint32_t j = 0; j < dims; ++j) {
-            float t = v[dims * i + j];
-            v[dims * i + j] = v[dims * other + j];
-            v[dims * other + j] = t;
-        }
-    }
-}
-
 // r2c / c2w: the camera's raster-to-camera and camera-to-world matrices
 // (a copy in registers, or the parameters themselves).
 __device__ __forceinline__ void camera_ray(const RenderParams& P, const float* r2c, const float* c2w, float ix,
@@ -141,7 +109,18 @@ struct PosWriter {
 };
 
 // One sampler pixel (k_generate's item).  `rng_col`: this thread's column
-// of 32 words in shared memory (word k at rng_col[k * stride]).
+// of 16 words in shared memory (word k at rng_col[k * stride]).
+//
+// The pixel's slice of its task's stream, in words: with jitter the image
+// strata (2 spp, montecarlo.rs:115-128), the lens strata (2 spp) and the time
+// strata (spp, :106-113); the shuffles of lens and time (one u64 = 2 words
+// per element each, rng.rs:23-33); then per sample and light a 1-D sample
+// (one float, one swap draw) and a 2-D sample (two floats, two draws), all
+// 1-D ones first (latin_hypercube of one sample, :88-104, whose draws always
+// swap the sample with itself).  Only the words that reach a ray or a light
+// sample are read: never the time strata, which no ray uses, their shuffle or
+// the swap draws, and the lens strata and shuffle only for a camera with a
+// lens.
 __device__ __forceinline__ void generate_pixel(const RenderParams& P, uint32_t pix, uint32_t* rng_col,
                                                uint32_t stride) {
     int32_t sw = P.sx1 - P.sx0;
@@ -166,98 +145,106 @@ __device__ __forceinline__ void generate_pixel(const RenderParams& P, uint32_t p
     }
     const TaskRec& T = P.tasks[t];
     uint64_t j = (uint64_t)(y - T.wy0) * (uint64_t)(T.wx1 - T.wx0) + (uint64_t)(x - T.wx0);
-    WordStream rng;
-    rng.seek(T.key, j * P.words_per_pixel, (j + 1) * P.words_per_pixel, rng_col, stride);
-    const bool jit = P.jitter != 0;
-    if (!(P.lens_radius > 0.0f)) {
-        // Pinhole camera: the ray depends on the image position alone, so
-        // the lens and time samples and their two shuffles (which permute
-        // only those arrays) are never read - their words are skipped
-        // instead of drawn, and each stratum's camera ray is made as soon
-        // as its image position is known (image samples are not shuffled).
-        // Same stream positions, same values as the general path below.
-        // the matrices go to registers once per pixel (in a batch P lives in
-        // global memory, where every use would be a load)
-        float r2c[16], c2w[16];
+    const uint64_t w0 = j * P.words_per_pixel;
+    WordWindow rng(T.key, rng_col, stride);
+    const bool jit = P.jitter != 0, has_lens = P.lens_radius > 0.0f;
+    // the matrices go to registers once per pixel (in a batch P lives in
+    // global memory, where every use would be a load)
+    float r2c[16], c2w[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            r2c[k] = P.r2c[k];
-            c2w[k] = P.c2w[k];
-        }
-        const float dx = 1.0f / (float)P.xs, dy = 1.0f / (float)P.ys;
-        float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
-        PosWriter pos(P.img + s0, spp);
-        for (uint32_t yy = 0; yy < P.ys; ++yy)
-            for (uint32_t xx = 0; xx < P.xs; ++xx) {
-                const float jx = jit ? rng.random_float() : 0.5f;
-                const float jy = jit ? rng.random_float() : 0.5f;
-                const float ix = (((float)xx + jx) * dx) + (float)x;
-                const float iy = (((float)yy + jy) * dy) + (float)y;
-                const uint32_t k = yy * P.xs + xx;
-                pos.put(k, make_float2(ix, iy));
-                bb = make_float4(fminf(bb.x, ix), fminf(bb.y, iy), fmaxf(bb.z, ix), fmaxf(bb.w, iy));
-                PbrtRay r;
-                camera_ray(P, r2c, c2w, ix, iy, 0.0f, 0.0f, &r);
-                st_ray(P.rays + s0 + k, r);
-            }
-        P.pixbox[pix] = bb;
-        // lens (2 spp) and time (spp) strata when jittered, then one u64 per
-        // element of each shuffle (2 x 2 spp words)
-        rng.skip((jit ? 3u * spp : 0u) + 4u * spp);
-        for (uint32_t i = 0; i < spp; ++i) {
-            float* ls = P.lsamp + (s0 + i) * (3 * nl);
-            for (uint32_t l = 0; l < nl; ++l) {
-                ls[l] = (0.0f + rng.random_float()) * 1.0f;
-                rng.skip(2);
-            }
-            for (uint32_t l = 0; l < nl; ++l) {
-                float u0 = (0.0f + rng.random_float()) * 1.0f;
-                float u1 = (0.0f + rng.random_float()) * 1.0f;
-                rng.skip(4);
-                ls[nl + 2 * l] = u0;
-                ls[nl + 2 * l + 1] = u1;
-            }
-        }
-        return;
+    for (int k = 0; k < 16; ++k) {
+        r2c[k] = P.r2c[k];
+        c2w[k] = P.c2w[k];
     }
-    float image[2 * kMaxSpp], lens[2 * kMaxSpp], time[kMaxSpp];
-    stratified_2d(image, P.xs, P.ys, rng, jit);
-    stratified_2d(lens, P.xs, P.ys, rng, jit);
-    stratified_1d(time, spp, rng, jit);
+    const float sdx = 1.0f / (float)P.xs, sdy = 1.0f / (float)P.ys;
     float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
-    for (uint32_t i = 0; i < spp; ++i) {
-        image[2 * i] += (float)x;
-        image[2 * i + 1] += (float)y;
-        bb = make_float4(fminf(bb.x, image[2 * i]), fminf(bb.y, image[2 * i + 1]), fmaxf(bb.z, image[2 * i]),
-                         fmaxf(bb.w, image[2 * i + 1]));
+    PosWriter pos(P.img + s0, spp);
+    uint32_t xx = 0, yy = 0;  // the next stratum
+    float2 kept[kMaxSpp], lens[kMaxSpp];  // with a lens: image positions, lens samples (local memory)
+    // Sample k's image position from its stratum's offsets (image samples
+    // are not shuffled); without a lens its ray too.
+    auto image = [&](uint32_t k, float jx, float jy) {
+        const float ix = (((float)xx + jx) * sdx) + (float)x;
+        const float iy = (((float)yy + jy) * sdy) + (float)y;
+        if (++xx == P.xs) {
+            xx = 0;
+            ++yy;
+        }
+        pos.put(k, make_float2(ix, iy));
+        bb = make_float4(fminf(bb.x, ix), fminf(bb.y, iy), fmaxf(bb.z, ix), fmaxf(bb.w, iy));
+        if (has_lens) {
+            kept[k] = make_float2(ix, iy);
+        } else {
+            PbrtRay r;
+            camera_ray(P, r2c, c2w, ix, iy, 0.0f, 0.0f, &r);
+            st_ray(P.rays + s0 + k, r);
+        }
+    };
+    auto lens_stratum = [&](uint32_t k, float jx, float jy) {
+        lens[k] = make_float2(((float)(k % P.xs) + jx) * sdx, ((float)(k / P.xs) + jy) * sdy);
+    };
+    if (!jit)
+        for (uint32_t k = 0; k < spp; ++k) {
+            image(k, 0.5f, 0.5f);
+            if (has_lens) lens_stratum(k, 0.5f, 0.5f);
+        }
+    // the ranges of words read, relative to w0
+    const uint32_t strata = jit ? (has_lens ? 4u : 2u) * spp : 0u;     // [0, strata)
+    const uint32_t swaps = jit ? 5u * spp : 0u;                        // lens shuffle: [swaps, swaps_end)
+    const uint32_t swaps_end = has_lens ? swaps + 2u * spp : swaps;
+    const uint32_t lights = swaps + 4u * spp;                          // light samples
+    const uint32_t n_light = 3u * nl * spp;                            // floats read there
+    float* ls = P.lsamp + s0 * (3u * nl);
+    uint32_t i = strata ? 0u : (has_lens ? swaps : lights);  // the next word read
+    uint32_t nq = 0, q = 0;                                  // light floats read, and of this sample
+    float held = 0.0f;
+    uint32_t held_lo = 0;
+    // words of every range are left until the light samples are all read
+    // (without lights until the last of the others)
+    const uint32_t last = nl ? 0xffffffffu : (has_lens ? swaps_end : strata);
+    while (i < last && (nl == 0 || nq < n_light)) {
+        rng.load(w0 + i);
+        const uint32_t lim = (uint32_t)((((w0 + i) >> 4) + 1u) * 16u - w0);  // first word past the block
+        for (; i < strata && i < lim; ++i) {
+            const float v = rng.unit(w0 + i);
+            if (!(i & 1u))
+                held = v;
+            else if (i < 2u * spp)
+                image(i >> 1, held, v);
+            else
+                lens_stratum((i - 2u * spp) >> 1, held, v);
+        }
+        if (i == strata && i < swaps) i = has_lens ? swaps : lights;
+        if (has_lens && i >= swaps && i < swaps_end) {
+            for (; i < swaps_end && i < lim; ++i) {
+                const uint32_t v = rng.word(w0 + i);
+                if (!((i - swaps) & 1u)) {  // low word first
+                    held_lo = v;
+                    continue;
+                }
+                const uint32_t k = (i - swaps) >> 1, o = k + random_index(held_lo, v, spp - k);
+                const float2 a = lens[k];
+                lens[k] = lens[o];
+                lens[o] = a;
+            }
+            if (i == swaps_end) {
+                for (uint32_t k = 0; k < spp; ++k) {
+                    PbrtRay r;
+                    camera_ray(P, r2c, c2w, kept[k].x, kept[k].y, lens[k].x, lens[k].y, &r);
+                    st_ray(P.rays + s0 + k, r);
+                }
+                i = lights;
+            }
+        }
+        while (i >= lights && i < lim && nq < n_light) {
+            ls[nq++] = (0.0f + rng.unit(w0 + i)) * 1.0f;
+            // the words between a sample's floats: 1-D ones lie 3 apart, the
+            // two of a 2-D sample together, 2-D ones 6 apart
+            i += q < nl ? 3u : (((q - nl) & 1u) ? 5u : 1u);
+            if (++q == 3u * nl) q = 0;
+        }
     }
     P.pixbox[pix] = bb;
-    shuffle(lens, spp, 2, rng);
-    shuffle(time, spp, 1, rng);
-    PosWriter pos(P.img + s0, spp);
-    for (uint32_t i = 0; i < spp; ++i) {
-        const uint64_t s = s0 + i;
-        pos.put(i, make_float2(image[2 * i], image[2 * i + 1]));
-        // integrator arrays: one 1-D and one 2-D sample per light, each a
-        // latin_hypercube of one sample (montecarlo.rs:88-104): the floats,
-        // then one swap draw per dimension (always with itself).
-        float* ls = P.lsamp + s * (3 * nl);
-        for (uint32_t l = 0; l < nl; ++l) {
-            ls[l] = (0.0f + rng.random_float()) * 1.0f;
-            rng.random_uint();
-        }
-        for (uint32_t l = 0; l < nl; ++l) {
-            float u0 = (0.0f + rng.random_float()) * 1.0f;
-            float u1 = (0.0f + rng.random_float()) * 1.0f;
-            rng.random_uint();
-            rng.random_uint();
-            ls[nl + 2 * l] = u0;
-            ls[nl + 2 * l + 1] = u1;
-        }
-        PbrtRay r;
-        camera_ray(P, P.r2c, P.c2w, image[2 * i], image[2 * i + 1], lens[2 * i], lens[2 * i + 1], &r);
-        st_ray(P.rays + s, r);
-    }
 }
 
 // ----------------------------------------------------------------- shade ---
