@@ -213,6 +213,10 @@ static int launch_batch(PbrtBVH* b, const PbrtRay* d_rays, uint32_t n, PbrtHit* 
     uint32_t* work = nullptr;
     void* scratch = nullptr;
     int st;
+    if (!in.ready && !host_hits && trace_is_small(wide_of(b), b->host.stack4_bound, n))
+        return cuda_status(launch_trace(b->dev, b->host.depth, d_rays, n, d_hits, d_occ, b->d_status, s, wide_of(b),
+                                        b->host.stack4_bound, kTraceSmall),
+                           "trace launch");
     const bool reorder = !in.ready && !host_hits && trace_reorder() && n >= kReorderMinRays && !b->host.nodes.empty();
     const bool chunked = in.ready || host_hits || trace_chunk() != 0;
     // [256 B: chunk counter, replay flag][permutation scratch]

@@ -74,6 +74,12 @@ struct StreamIn {
     uint32_t shift = 0;
     uint32_t wait_ms = 0;
 };
+// `kernel` = kTraceSmall (a call that trace_is_small): one thread per ray over
+// the 4-wide layout, one launch, neither `work` nor `replay` used.
+constexpr int kTraceSmall = 100;
+bool trace_is_small(const DevBVH4* wide, uint32_t wide_bound, uint32_t n);
+// Lanes per warp that get a ray of a launch of n one-thread-per-ray walks.
+uint32_t rays_per_warp(uint64_t n);
 cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays, uint32_t n, PbrtHit* hits,
                          uint8_t* occluded, int* d_status, cudaStream_t stream, const DevBVH4* wide = nullptr,
                          uint32_t wide_bound = 0, int kernel = -1, const uint32_t* order = nullptr,

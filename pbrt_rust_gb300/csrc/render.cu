@@ -71,13 +71,15 @@ __global__ void __launch_bounds__(128) k_shadow_packet(RenderParams P) {
     P.occluded[P.shadow_slot[q]] = occ ? 1 : 0;
 }
 
+// The first per_warp lanes of each warp have a ray (rays_per_warp).
 template <int OVF, bool INST>
-__global__ void __launch_bounds__(128) k_shadow4(const __grid_constant__ RenderParams P) {
+__global__ void __launch_bounds__(128) k_shadow4(const __grid_constant__ RenderParams P, uint32_t per_warp) {
     using Walk = Walk4<128, 16, OVF, true, INST>;
     __shared__ typename Walk::Shared sh;
     sh.init();
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= *(volatile uint32_t*)&P.counters[0]) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t q = (uint64_t)(blockIdx.x * 4u + (threadIdx.x >> 5)) * per_warp + lane;
+    if (lane >= per_warp || q >= *(volatile uint32_t*)&P.counters[0]) return;
     const float4* ray = reinterpret_cast<const float4*>(P.shadow_rays) + 2 * (size_t)q;
     int* status = (int*)&P.counters[2];
     Walk T;
@@ -194,6 +196,8 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         uint64_t max_shadow = P.n_samples * P.n_lights;
         if (max_shadow) {
+            const uint32_t pw = rays_per_warp(max_shadow);
+            const unsigned grid4 = blocks_for(max_shadow, 4 * (int)pw);
             // scenes with instances: the 4-wide walk with instances when a
             // variant covers its stack bound, else the binary one
             const bool inst = P.bvh.insts != nullptr;
@@ -201,9 +205,9 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             const bool wide_rk = rk == PBRT_TRACE_WIDE || rk == PBRT_TRACE_WIDE_PERSISTENT || rk == PBRT_TRACE_WIDE_SPECULATIVE;
             int wv = (P.has_wide && wide_rk && !inst) ? wide_stack_variant(P.wide_bound) : 0;
             if (iv == 64)
-                k_shadow4<64, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
+                k_shadow4<64, true><<<grid4, 128, 0, s>>>(P, pw);
             else if (iv == 256)
-                k_shadow4<256, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
+                k_shadow4<256, true><<<grid4, 128, 0, s>>>(P, pw);
             else if (inst && trace_stack_for_depth(P.depth) == 64)
                 k_shadow<64, true><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (inst)
@@ -213,9 +217,9 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             else if (rk == PBRT_TRACE_PAIR_PACKET)
                 k_shadow_packet<256><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else if (wv == 64)
-                k_shadow4<64, false><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
+                k_shadow4<64, false><<<grid4, 128, 0, s>>>(P, pw);
             else if (wv == 256)
-                k_shadow4<256, false><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
+                k_shadow4<256, false><<<grid4, 128, 0, s>>>(P, pw);
             else if (trace_stack_for_depth(P.depth) == 64)
                 k_shadow<64><<<blocks_for(max_shadow, 128), 128, 0, s>>>(P);
             else

@@ -136,17 +136,21 @@ __global__ void __launch_bounds__(128) k_trace_persistent(const __grid_constant_
 constexpr int kWalkBlock = 128;  // threads per block and stack rows of the 4-wide kernels
 constexpr int kWalkRows = 16;
 
-// 4-wide traversal, one thread per ray.
-template <int OVF, bool ANY>
+// 4-wide traversal, one thread per ray; the first per_warp lanes of each warp
+// have one (rays_per_warp).
+template <int OVF, bool ANY, bool INST>
 __global__ void __launch_bounds__(kWalkBlock) k_trace4(const __grid_constant__ DevBVH4 bvh,
                                                        const float4* __restrict__ rays, uint32_t n,
                                                        const uint32_t* __restrict__ order, float4* __restrict__ hits,
-                                                       uint8_t* __restrict__ occ, int* __restrict__ status) {
-    using Walk = Walk4<kWalkBlock, kWalkRows, OVF, ANY>;
+                                                       uint8_t* __restrict__ occ, int* __restrict__ status,
+                                                       uint32_t per_warp) {
+    using Walk = Walk4<kWalkBlock, kWalkRows, OVF, ANY, INST>;
     __shared__ typename Walk::Shared sh;
     sh.init();
-    uint32_t i = blockIdx.x * kWalkBlock + threadIdx.x;
-    if (i >= n) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t g = (uint64_t)(blockIdx.x * (kWalkBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
+    if (lane >= per_warp || g >= n) return;
+    uint32_t i = (uint32_t)g;
     if (order) i = __ldg(order + i);
     const float4* ray = rays + 2 * (size_t)i;
     Walk T;
@@ -156,9 +160,9 @@ __global__ void __launch_bounds__(kWalkBlock) k_trace4(const __grid_constant__ D
     if (st == kStartWalk) T.run(bvh, sh, ov);
     if (T.spilled < 0) atomicMax(status, 6);
     if (ANY)
-        occ[i] = (st == kStartExact ? exact_any<OVF + 8, false>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
+        occ[i] = (st == kStartExact || T.give_up ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
     else
-        hits[i] = st == kStartExact || T.give_up ? exact_hit<OVF + 8, false>(bvh.pair, ray, status) : T.hit_record();
+        hits[i] = st == kStartExact || T.give_up ? exact_hit<OVF + 8, INST>(bvh.pair, ray, status) : T.hit_record();
 }
 
 // A ray is read once: its lines go to L2 only, leaving L1 to the tree.
@@ -509,8 +513,35 @@ static cudaError_t launch_wide_persistent(const DevBVH4& bvh, const float4* r4, 
     return cudaGetLastError();
 }
 
+// A launch of few rays is as long as its longest walk.  A warp whose lanes
+// walk different rays takes the sum of their detours, so few rays are spread
+// over more warps than they would fill, up to 14 warps per SM (an SM keeps 32
+// of them, but from there on they slow each other down more than sharing a
+// warp does).  Closest hits of 64 / 1000 / 4000 / 16000 / 64000 rays into 4096
+// random triangles, us: 33 / 33 / 42 / 58 / 72 with this rule (1 / 1 / 2 / 8 /
+// 32 lanes), 59 / 58 / 58 / 62 / 72 with full warps, 121 with one lane at
+// 16000; the persistent kernel 79 / 84 / 87 / 89 / 96.
+uint32_t rays_per_warp(uint64_t n) {
+    const uint64_t warps = 14ull * (uint64_t)device_sms();
+    uint32_t r = 1;
+    while (r < 32u && n > warps * r) r *= 2;
+    return r;
+}
+
+// The most rays of a call that takes one thread per ray instead of the
+// persistent kernel: what fits the chip at once (8 blocks of 128 per SM).
+// 128000 / 256000 rays into 4096 and 200000 random triangles, us: 95 / 159 and
+// 196 / 298 one thread per ray, 110 / 150 and 204 / 242 persistent; and such a
+// call needs no work counter, no replay launch and no scratch.
+static uint64_t small_call_rays() { return 8ull * kWalkBlock * (uint64_t)device_sms(); }
+bool trace_is_small(const DevBVH4* wide, uint32_t wide_bound, uint32_t n) {
+    read_variant();
+    return wide && wide_stack_variant(wide_bound) && g_kernel_variant == kVariantWidePersistent && !g_reorder &&
+           n <= small_call_rays();
+}
+
 // The 4-wide kernel for a call: closest hits into h4 (occ null) or answers
-// into occ; persistent or one thread per ray (never with instances).
+// into occ; persistent or one thread per ray.
 template <int OVF>
 static cudaError_t launch_wide(const DevBVH4& bvh, const float4* r4, uint32_t n, const uint32_t* order, float4* h4,
                                uint8_t* occ, int* d_status, cudaStream_t stream, bool persistent, uint32_t* work,
@@ -518,18 +549,22 @@ static cudaError_t launch_wide(const DevBVH4& bvh, const float4* r4, uint32_t n,
     auto pt = [&](auto launch) {
         return launch(bvh, r4, n, order, h4, occ, d_status, stream, work, replay, in, host_hits);
     };
-    if (bvh.pair.insts)
+    const bool inst = bvh.pair.insts != nullptr;
+    if (inst && persistent)
         return host_hits ? pt(launch_wide_persistent<OVF, false, true, true>)
                : occ     ? pt(launch_wide_persistent<OVF, true, true>)
                          : pt(launch_wide_persistent<OVF, false, true>);
     if (host_hits) return pt(launch_wide_persistent<OVF, false, false, true>);
     if (persistent) return occ ? pt(launch_wide_persistent<OVF, true, false>) : pt(launch_wide_persistent<OVF, false, false>);
-    const unsigned grid = (unsigned)((n + (uint64_t)kWalkBlock - 1) / kWalkBlock);
-    if (occ)
-        k_trace4<OVF, true><<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, nullptr, occ, d_status);
-    else
-        k_trace4<OVF, false><<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, h4, nullptr, d_status);
-    return cudaGetLastError();
+    const uint32_t per_warp = rays_per_warp(n);
+    const uint64_t per_block = (uint64_t)per_warp * (kWalkBlock / 32);
+    const unsigned grid = (unsigned)((n + per_block - 1) / per_block);
+    auto plain = [&](auto kernel) {
+        kernel<<<grid, kWalkBlock, 0, stream>>>(bvh, r4, n, order, h4, occ, d_status, per_warp);
+        return cudaGetLastError();
+    };
+    if (inst) return occ ? plain(k_trace4<OVF, true, true>) : plain(k_trace4<OVF, false, true>);
+    return occ ? plain(k_trace4<OVF, true, false>) : plain(k_trace4<OVF, false, false>);
 }
 
 int set_trace_config(const PbrtTraceConfig& c) {
@@ -612,17 +647,20 @@ static cudaError_t launch_main(const DevBVH& bvh, uint32_t depth, const PbrtRay*
                                uint8_t* occluded, int* d_status, cudaStream_t stream, const DevBVH4* wide,
                                uint32_t wide_bound, int kernel, const uint32_t* order, uint32_t* work,
                                uint32_t* replay, bool* replays) {
-    const int variant = kernel >= 0 ? kernel : g_kernel_variant;
-    // a scene with instances takes the persistent walk with nested instance
-    // traversal (4-wide when a variant covers the stack bound), whatever the
-    // configured kernel
+    const int variant = kernel == kTraceSmall ? (int)kVariantWidePlain : (kernel >= 0 ? kernel : g_kernel_variant);
+    // a scene with instances takes a walk with nested instance traversal
+    // (4-wide when a variant covers the stack bound), whatever the configured
+    // kernel
     const bool inst = bvh.insts != nullptr;
     const int v = wide ? wide_stack_variant(wide_bound) : 0;
     const float4* r4 = reinterpret_cast<const float4*>(rays);
     float4* h4 = reinterpret_cast<float4*>(hits);
     if (v && (inst || variant == kVariantWidePlain || variant == kVariantWidePersistent ||
               variant == kVariantWideSpeculative)) {
-        const bool pt = inst || variant != kVariantWidePlain;
+        // with instances: one thread per ray for a render's camera rays
+        // (kernel >= 0; 390 -> 151 us for a 517 x 389 x 4 forest frame), the
+        // persistent walk for batches
+        const bool pt = kernel == kTraceSmall ? false : (inst ? kernel < 0 : variant != kVariantWidePlain);
         *replays = pt;
         return v == 64 ? launch_wide<64>(*wide, r4, n, order, h4, occluded, d_status, stream, pt, work, replay)
                        : launch_wide<256>(*wide, r4, n, order, h4, occluded, d_status, stream, pt, work, replay);
@@ -714,7 +752,7 @@ cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays,
                          uint32_t wide_bound, int kernel, const uint32_t* order, uint32_t* work, uint32_t* replay,
                          StreamIn in, PbrtHit* host_hits) {
     if (n == 0) return cudaSuccess;
-    if (!replay) return cudaErrorInvalidValue;
+    if (!replay && kernel != kTraceSmall) return cudaErrorInvalidValue;
     read_variant();
     if ((in.ready || host_hits) && order) return cudaErrorInvalidValue;
     bool replays = true;

@@ -116,11 +116,15 @@ def rays(box, n, seed, prims):
 SCENES = ["floor", "chain", "offset", "wide_range", "past_reach", "mixed", "instances"]
 
 
-def config(lib, kernel):
+def config(lib, kernel, reorder=0):
+    """Sets the traversal; reorder = 1 keeps calls of few rays on the
+    persistent kernel (and bins those of 32768 or more).  Returns the old
+    configuration."""
     cfg = abi.PbrtTraceConfig()
     abi.check(lib.pbrtgpu_get_trace_config(C.byref(cfg)), lib)
     old = abi.PbrtTraceConfig.from_buffer_copy(cfg)
     cfg.kernel = abi.TRACE_KERNELS[kernel]
+    cfg.reorder = reorder
     abi.check(lib.pbrtgpu_set_trace_config(C.byref(cfg)), lib)
     return old
 
@@ -146,10 +150,10 @@ def test_quad_walk_equals_oracle(lib, oracle, name, leaf):
             assert np.array_equal(got[f], want[f], equal_nan=True), (what, f)
         assert np.array_equal(occ.cpu().numpy(), want_p), what
 
-    for kernel in ("w4pt", "w4"):
-        old = config(lib, kernel)
+    for kernel, reorder in (("w4pt", 1), ("w4pt", 0), ("w4", 0)):
+        old = config(lib, kernel, reorder)
         try:
-            check(bvh.intersect(dev), bvh.intersect_p(dev), kernel)
+            check(bvh.intersect(dev), bvh.intersect_p(dev), (kernel, reorder))
         finally:
             abi.check(lib.pbrtgpu_set_trace_config(C.byref(old)), lib)
     for tuning in (dict(refill=32), dict(refill=8), dict(refill=8, stack=8, block=256)):
@@ -183,3 +187,27 @@ def test_shadow_rays_beside_axis_planes(oracle):
         b.set_tuning(shadow_kernel="wide", extend_kernel="wide", **tuning)
         b.add_render(sc, rn)
         assert np.array_equal(b.run()[0], want)
+
+
+@pytest.mark.parametrize("n", [1, 33, 2128, 2129, 8513, 155648, 155649])
+def test_calls_of_any_size(n, oracle):
+    """Few rays are spread over more warps than they fill, in steps of the
+    rays per warp, up to the count from which the persistent kernel takes over
+    (the edges for 152 SMs): every ray gets its own hit, none past the end is
+    written."""
+    import torch
+    from pbrt_rust_gb300.gpu import GpuBVHAccel
+    prims, box = scene("mixed")
+    bvh, ob = GpuBVHAccel(prims), oracle.OracleBVH(prims, 4, "sah")
+    r = rays(box, n, 11, prims)
+    want, want_p = ob.intersect(r), ob.intersect_p(r)
+    dev = torch.from_numpy(r.view(np.float32).reshape(-1, 8).copy()).cuda()
+    hits = torch.full((n + 64, 4), 7.0, device="cuda")
+    occ = torch.full((n + 64,), 7, device="cuda", dtype=torch.uint8)
+    bvh.intersect(dev, out=hits)
+    bvh.intersect_p(dev, out=occ)
+    got = hits[:n].cpu().numpy().view(abi.HIT_DTYPE).reshape(-1)
+    for f in ("prim", "t", "b1", "b2"):
+        assert np.array_equal(got[f], want[f], equal_nan=True), f
+    assert np.array_equal(occ[:n].cpu().numpy(), want_p)
+    assert bool((hits[n:] == 7.0).all()) and bool((occ[n:] == 7).all())
