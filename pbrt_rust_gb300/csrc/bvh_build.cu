@@ -13,10 +13,10 @@
 //      and a stable scatter writes the two sides in their original order
 //      (Iterator::partition keeps order, bvh.rs:89, 174).  The host reads the
 //      few per-range decisions back and lays out the next level.
-//   B. ranges of at most kSmall primitives: one thread runs the whole
-//      subtree with the host algorithm (including partition_by for the
-//      equal-counts split of ranges of up to four, utils/mod.rs:112-169),
-//      writing its nodes in pre-order.
+//   B. ranges of at most kSmall primitives: one warp runs the whole subtree,
+//      one primitive per lane, with the host algorithm (including
+//      partition_by for the equal-counts split of ranges of up to four,
+//      utils/mod.rs:112-169), writing its nodes in pre-order.
 //
 // Bounds are combined with a min/max that ignores NaN and orders -0 below
 // +0, in any order; f32 bucket indices and SAH costs repeat the host's
@@ -37,12 +37,7 @@ namespace pbrt {
 
 namespace {
 
-#ifndef PBRT_BUILD_SMALL
-#define PBRT_BUILD_SMALL 32
-#endif
-// ranges of at most this many primitives go to phase B (one thread each:
-// small ranges keep that serial work short and the thread count high)
-constexpr uint32_t kSmall = PBRT_BUILD_SMALL;
+constexpr uint32_t kSmall = 32;   // ranges of at most this many primitives go to phase B (a lane each)
 constexpr uint32_t kChunk = 2048; // phase A chunk
 constexpr int kNB = 12;           // SAH buckets (bvh.rs:188)
 
@@ -235,46 +230,64 @@ __global__ void __launch_bounds__(256) k_a_buckets(Prims P, const uint32_t* __re
     }
 }
 
-// One thread per range: the SAH costs in the host's order and the leaf test
-// (bvh.rs:133-185).
-__global__ void k_a_choose(const int32_t* __restrict__ acc, SegDecision* dec, const uint32_t* __restrict__ counts,
-                           uint32_t nseg, uint32_t mp) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
-    SegDecision d = dec[s];
-    if (d.action != 1) return;
-    const int32_t* a = acc + (size_t)s * kAccWords + 12;
-    size_t bc[kNB];
-    DBox bb[kNB];
-    for (int i = 0; i < kNB; ++i) {
-        const int32_t* q = a + i * 7;
-        bc[i] = (size_t)q[0];
-        bb[i] = DBox{unord(q[1]), unord(q[2]), unord(q[3]), unord(q[4]), unord(q[5]), unord(q[6])};
+// The cheapest of the eleven splits and its cost (bvh.rs:133-160): the first
+// whose cost is below every earlier one's and FLT_MAX.  The boxes of the left
+// sides grow bucket by bucket and those of the right sides come from a
+// backward pass; unions do not depend on their order (dmin / dmax), so the
+// costs are those of the host's loop over all buckets per split.
+__device__ inline int cheapest_split(const DBox* bb, const uint32_t* bc, float tsa, float* cost_out) {
+    DBox right[kNB];  // union of buckets j ..
+    uint32_t n_right[kNB];
+    DBox u = dbox_empty();
+    uint32_t n = 0;
+#pragma unroll
+    for (int j = kNB - 1; j > 0; --j) {
+        u = dunion(u, bb[j]);
+        n += bc[j];
+        right[j] = u;
+        n_right[j] = n;
     }
-    DBox total{d.lo[0], d.lo[1], d.lo[2], d.hi[0], d.hi[1], d.hi[2]};
-    const float tsa = darea(total);
     int best = 0;
     float best_cost = FLT_MAX;
+    u = dbox_empty();
+    n = 0;
+#pragma unroll
     for (int sp = 0; sp + 1 < kNB; ++sp) {
-        size_t c0 = 0, c1 = 0;
-        DBox b0 = dbox_empty(), b1 = dbox_empty();
-        for (int j = 0; j <= sp; ++j) {
-            c0 += bc[j];
-            b0 = dunion(b0, bb[j]);
-        }
-        for (int j = sp + 1; j < kNB; ++j) {
-            c1 += bc[j];
-            b1 = dunion(b1, bb[j]);
-        }
-        const float cost = 0.125f * ((float)c0 * darea(b0) + (float)c1 * darea(b1)) / tsa;
+        u = dunion(u, bb[sp]);
+        n += bc[sp];
+        const float cost =
+            0.125f * ((float)n * darea(u) + (float)n_right[sp + 1] * darea(right[sp + 1])) / tsa;
         if (cost < best_cost) {
             best_cost = cost;
             best = sp;
         }
     }
+    *cost_out = best_cost;
+    return best;
+}
+
+// One thread per range: the SAH costs in the host's order and the leaf test
+// (bvh.rs:133-185).
+__global__ void __launch_bounds__(32) k_a_choose(const int32_t* __restrict__ acc, SegDecision* dec,
+                                                 const uint32_t* __restrict__ counts, uint32_t nseg, uint32_t mp) {
+    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nseg) return;
+    SegDecision d = dec[s];
+    if (d.action != 1) return;
+    const int32_t* a = acc + (size_t)s * kAccWords + 12;
+    uint32_t bc[kNB];
+    DBox bb[kNB];
+#pragma unroll
+    for (int i = 0; i < kNB; ++i) {
+        const int32_t* q = a + i * 7;
+        bc[i] = (uint32_t)q[0];
+        bb[i] = DBox{unord(q[1]), unord(q[2]), unord(q[3]), unord(q[4]), unord(q[5]), unord(q[6])};
+    }
+    DBox total{d.lo[0], d.lo[1], d.lo[2], d.hi[0], d.hi[1], d.hi[2]};
+    float best_cost;
+    d.best = cheapest_split(bb, bc, darea(total), &best_cost);
     const size_t cnt = counts[s];
     if (!(mp < cnt || to_usize(best_cost) < cnt)) d.action = 0;  // a leaf of cnt primitives
-    d.best = best;
     dec[s] = d;
 }
 
@@ -361,21 +374,16 @@ struct PoolNode {      // a = leaf ? first prim : second child (pool index); b =
     uint32_t b;
 };
 constexpr uint32_t kLeaf = 0x80000000u;
-struct Task {
-    uint32_t lo, hi;
-    int32_t parent;
-    uint32_t depth;
-};
 struct JobOut {
     uint32_t nodes, depth, err, pad;
 };
 
 // utils/mod.rs:112-169 (as host_scene.cpp partition_by_key)
-__device__ void partition_by_key(uint32_t* v, uint32_t n, const float* key) {
+__device__ void partition_by_key(uint8_t* v, uint32_t n, const float* key) {
     while (true) {
         if (n < 3) {
             if (n == 2 && key[v[1]] < key[v[0]]) {
-                uint32_t t = v[0];
+                uint8_t t = v[0];
                 v[0] = v[1];
                 v[1] = t;
             }
@@ -387,7 +395,7 @@ __device__ void partition_by_key(uint32_t* v, uint32_t n, const float* key) {
         for (uint32_t i = 0; i < n; ++i) {
             float k = key[v[i]];
             if (k < pivot) {
-                uint32_t t = v[ls + np];
+                uint8_t t = v[ls + np];
                 v[ls + np] = v[i];
                 v[i] = t;
                 t = v[ls + np];
@@ -395,7 +403,7 @@ __device__ void partition_by_key(uint32_t* v, uint32_t n, const float* key) {
                 v[ls] = t;
                 ++ls;
             } else if (k == pivot) {
-                uint32_t t = v[ls + np];
+                uint8_t t = v[ls + np];
                 v[ls + np] = v[i];
                 v[i] = t;
                 ++np;
@@ -413,127 +421,172 @@ __device__ void partition_by_key(uint32_t* v, uint32_t n, const float* key) {
     }
 }
 
-// One thread per job: build_tree on [lo, hi) (host_scene.cpp), nodes in
-// pre-order at pool[node0 ...]; `stack` and `tmp` are scratch at the same
-// offsets as the range.
-__global__ void __launch_bounds__(128) k_b_build(Prims P, uint32_t* idx, uint32_t* tmp, Task* stack,
-                                                 const Job* __restrict__ jobs, uint32_t njobs, PoolNode* pool,
-                                                 JobOut* outs, uint32_t mp, int split) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per job: build_tree on [lo, hi) (host_scene.cpp), nodes in
+// pre-order at pool[node0 ...], the range's primitive order in idx.  The
+// range's boxes and centroids sit in shared memory, one slot per primitive;
+// a lane holds the slot at its position of the range.  A node's bounds are
+// warp reductions over the lanes of its sub-range (an inner node's box is the
+// union of its children's, bvh.rs:247, which is the union of its primitives'
+// boxes whatever the order), the twelve buckets are filled with shared-memory
+// atomics and their eleven splits costed one per lane, and a split moves
+// the slots by rank, which keeps their order.  As one thread per range, whose
+// lanes diverge at every node, 180000 terrain triangles took 2.40 ms here.
+constexpr int kBWarps = 4;
+struct BScratch {
+    float box[6][kSmall], cen[3][kSmall];  // by slot
+    uint8_t order[kSmall];                 // slot at each position of the range
+    int32_t bucket[kNB][7];                // count, bounds (ord)
+    uint4 stack[kSmall];                   // (lo, hi, parent or ~0, depth)
+};
+__global__ void __launch_bounds__(32 * kBWarps) k_b_build(Prims P, uint32_t* idx, const Job* __restrict__ jobs,
+                                                         uint32_t njobs, PoolNode* pool, JobOut* outs, uint32_t mp,
+                                                         int split) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ BScratch scratch[kBWarps];
+    BScratch& S = scratch[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t j = blockIdx.x * kBWarps + (threadIdx.x >> 5);
     if (j >= njobs) return;
     const Job J = jobs[j];
-    Task* st = stack + J.lo;
-    uint32_t sp = 0, nn = 0, maxd = 0, err = 0;
-    st[sp++] = Task{J.lo, J.hi, -1, 1};
+    const uint32_t n = J.hi - J.lo;
+    uint32_t prim = 0;  // of slot `lane`
+    if (lane < n) {
+        prim = idx[J.lo + lane];
+        const DBox b = pbox(P, prim);
+        S.box[0][lane] = b.lx, S.box[1][lane] = b.ly, S.box[2][lane] = b.lz;
+        S.box[3][lane] = b.hx, S.box[4][lane] = b.hy, S.box[5][lane] = b.hz;
+        for (int k = 0; k < 3; ++k) S.cen[k][lane] = __ldg(P.cen[k] + prim);
+    }
+    uint32_t slot = lane;  // at this lane's position
+    uint32_t sp = 1, nn = 0, maxd = 0, err = 0;  // warp-uniform
+    if (lane == 0) S.stack[0] = make_uint4(0, n, kAll, 1);
+    __syncwarp();
+    const int32_t lowest = ord(FLT_MAX), highest = ord(-FLT_MAX);  // of an empty box
+    // ord of a bound that takes part; NaNs and other lanes leave it alone
+    auto part = [](bool in, float v, int32_t none) { return in && v == v ? ord(v) : none; };
     while (sp > 0) {
-        const Task t = st[--sp];
-        const uint32_t k = nn++;
-        if (t.parent >= 0) pool[J.node0 + t.parent].a = k;
-        maxd = max(maxd, t.depth);
-        const uint32_t cnt = t.hi - t.lo;
-        DBox bbox = dbox_empty();
-        for (uint32_t i = t.lo; i < t.hi; ++i) bbox = dunion(bbox, pbox(P, idx[i]));
+        const uint4 t = S.stack[--sp];
+        const uint32_t k = nn++, cnt = t.y - t.x;
+        const bool in = lane >= t.x && lane < t.y;
+        __syncwarp();
+        if (lane == 0 && t.z != kAll) pool[J.node0 + t.z].a = k;
+        maxd = max(maxd, t.w);
+        float box[6], cen[3];
+        int32_t m[6], c[6];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            box[i] = S.box[i][slot];
+            box[3 + i] = S.box[3 + i][slot];
+            cen[i] = S.cen[i][slot];
+            m[i] = min(lowest, __reduce_min_sync(kAll, part(in, box[i], lowest)));
+            m[3 + i] = max(highest, __reduce_max_sync(kAll, part(in, box[3 + i], highest)));
+            c[i] = min(lowest, __reduce_min_sync(kAll, part(in, cen[i], lowest)));
+            c[3 + i] = max(highest, __reduce_max_sync(kAll, part(in, cen[i], highest)));
+        }
         uint32_t mid = 0;
         bool split_it = false;
         int dim = 0;
         if (cnt > 1) {
-            DBox cb = dbox_empty();
-            for (uint32_t i = t.lo; i < t.hi; ++i) {
-                const uint32_t p = idx[i];
-                const float cx = __ldg(P.cen[0] + p), cy = __ldg(P.cen[1] + p), cz = __ldg(P.cen[2] + p);
-                cb = dunion(cb, DBox{cx, cy, cz, cx, cy, cz});
-            }
-            dim = dmax_extent(cb);
-            const float cmin = dim == 0 ? cb.lx : (dim == 1 ? cb.ly : cb.lz);
-            const float cmax = dim == 0 ? cb.hx : (dim == 1 ? cb.hy : cb.hz);
-            const float* key = P.cen[dim];
+            dim = dmax_extent(DBox{unord(c[0]), unord(c[1]), unord(c[2]), unord(c[3]), unord(c[4]), unord(c[5])});
+            const float cmin = unord(dim == 0 ? c[0] : (dim == 1 ? c[1] : c[2]));
+            const float cmax = unord(dim == 0 ? c[3] : (dim == 1 ? c[4] : c[5]));
+            const float key = dim == 0 ? cen[0] : (dim == 1 ? cen[1] : cen[2]);
+            bool left = false;  // a stable split sends this lane's primitive left
+            bool stable = false;
             if (cmin != cmax) {
-                auto stable_split = [&](auto pred) {
-                    uint32_t w = t.lo, r = t.lo;
-                    for (uint32_t i = t.lo; i < t.hi; ++i) {
-                        const uint32_t p = idx[i];
-                        if (pred(p))
-                            idx[w++] = p;
-                        else
-                            tmp[r++] = p;
-                    }
-                    mid = w;
-                    for (uint32_t i = t.lo; i < r; ++i) idx[w++] = tmp[i];
-                    split_it = true;
-                };
                 if (split == PBRT_SPLIT_MIDDLE) {
-                    const float p_mid = 0.5f * (cmin + cmax);
-                    stable_split([&](uint32_t p) { return key[p] < p_mid; });
+                    left = key < 0.5f * (cmin + cmax);
+                    stable = true;
                 } else if (split == PBRT_SPLIT_EQUAL || cnt <= 4) {
-                    partition_by_key(idx + t.lo, cnt, key);
-                    mid = t.lo + cnt / 2;
+                    S.order[lane] = (uint8_t)slot;
+                    __syncwarp();
+                    if (lane == 0) partition_by_key(S.order + t.x, cnt, S.cen[dim]);
+                    __syncwarp();
+                    slot = S.order[lane];
+                    mid = t.x + cnt / 2;
                     split_it = true;
                 } else {
+                    for (uint32_t i = lane; i < kNB * 7; i += 32u)
+                        (&S.bucket[0][0])[i] = i % 7u == 0u ? 0 : (i % 7u <= 3u ? lowest : highest);
+                    __syncwarp();
                     const float dist = cmax - cmin;
-                    size_t bc[kNB];
-                    DBox bb[kNB];
-                    for (int i = 0; i < kNB; ++i) {
-                        bc[i] = 0;
-                        bb[i] = dbox_empty();
-                    }
-                    for (uint32_t i = t.lo; i < t.hi; ++i) {
-                        const uint32_t p = idx[i];
-                        const int b = bucket_of(key[p], cmin, dist);
-                        bc[b] += 1;
-                        bb[b] = dunion(bb[b], pbox(P, p));
-                    }
-                    const float tsa = darea(bbox);
-                    int best = 0;
-                    float best_cost = FLT_MAX;
-                    for (int s = 0; s + 1 < kNB; ++s) {
-                        size_t c0 = 0, c1 = 0;
-                        DBox b0 = dbox_empty(), b1 = dbox_empty();
-                        for (int q = 0; q <= s; ++q) {
-                            c0 += bc[q];
-                            b0 = dunion(b0, bb[q]);
-                        }
-                        for (int q = s + 1; q < kNB; ++q) {
-                            c1 += bc[q];
-                            b1 = dunion(b1, bb[q]);
-                        }
-                        const float cost = 0.125f * ((float)c0 * darea(b0) + (float)c1 * darea(b1)) / tsa;
-                        if (cost < best_cost) {
-                            best_cost = cost;
-                            best = s;
+                    int b = 0;
+                    if (in) {
+                        b = bucket_of(key, cmin, dist);
+                        int32_t* q = S.bucket[b];
+                        atomicAdd(q, 1);
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            atomicMin(q + 1 + i, part(true, box[i], lowest));
+                            atomicMax(q + 4 + i, part(true, box[3 + i], highest));
                         }
                     }
-                    if (mp < cnt || to_usize(best_cost) < cnt)
-                        stable_split([&](uint32_t p) { return bucket_of(key[p], cmin, dist) <= best; });
+                    __syncwarp();
+                    // lane s < 11: the cost of the split after bucket s
+                    float cost = FLT_MAX;
+                    if (lane + 1u < (uint32_t)kNB) {
+                        DBox u0 = dbox_empty(), u1 = dbox_empty();
+                        uint32_t n0 = 0;
+                        for (uint32_t q = 0; q < (uint32_t)kNB; ++q) {
+                            const int32_t* e = S.bucket[q];
+                            const DBox bq{unord(e[1]), unord(e[2]), unord(e[3]), unord(e[4]), unord(e[5]), unord(e[6])};
+                            if (q <= lane) {
+                                n0 += (uint32_t)e[0];
+                                u0 = dunion(u0, bq);
+                            } else {
+                                u1 = dunion(u1, bq);
+                            }
+                        }
+                        const float tsa = darea(DBox{unord(m[0]), unord(m[1]), unord(m[2]), unord(m[3]), unord(m[4]),
+                                                     unord(m[5])});
+                        cost = 0.125f * ((float)n0 * darea(u0) + (float)(cnt - n0) * darea(u1)) / tsa;
+                        if (!(cost < FLT_MAX)) cost = FLT_MAX;  // also NaN: never below the best
+                    }
+                    const int32_t lo_cost = __reduce_min_sync(kAll, ord(cost));
+                    const float best_cost = unord(lo_cost);
+                    const int best = best_cost < FLT_MAX ? __ffs(__ballot_sync(kAll, ord(cost) == lo_cost)) - 1 : 0;
+                    if (mp < cnt || to_usize(best_cost) < cnt) {
+                        left = b <= best;
+                        stable = true;
+                    }
                 }
             }
+            if (stable) {
+                const unsigned ml = __ballot_sync(kAll, in && left), below = (1u << lane) - 1u;
+                const uint32_t nl = (uint32_t)__popc(ml);
+                if (in) {
+                    const uint32_t rank = (uint32_t)__popc(ml & below);
+                    S.order[left ? t.x + rank : t.x + nl + (lane - t.x - rank)] = (uint8_t)slot;
+                }
+                __syncwarp();
+                if (in) slot = S.order[lane];
+                mid = t.x + nl;
+                split_it = true;
+            }
         }
-        PoolNode& N = pool[J.node0 + k];
-        N.lo[0] = bbox.lx, N.lo[1] = bbox.ly, N.lo[2] = bbox.lz;
-        N.hi[0] = bbox.hx, N.hi[1] = bbox.hy, N.hi[2] = bbox.hz;
-        if (split_it) {
-            if (mid == t.lo || mid == t.hi) err = 1;
-            N.a = 0;
-            N.b = (uint32_t)dim;
-            st[sp++] = Task{mid, t.hi, (int32_t)k, t.depth + 1};
-            st[sp++] = Task{t.lo, mid, -1, t.depth + 1};
-            if (err) break;
-        } else {
-            N.a = t.lo;
-            N.b = kLeaf | cnt;
+        if (split_it && (mid == t.x || mid == t.y)) err = 1;
+        __syncwarp();
+        if (lane == 0) {
+            PoolNode& N = pool[J.node0 + k];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                N.lo[i] = unord(m[i]);
+                N.hi[i] = unord(m[3 + i]);
+            }
+            N.a = split_it ? 0u : J.lo + t.x;
+            N.b = split_it ? (uint32_t)dim : (kLeaf | cnt);
+            if (split_it) {
+                S.stack[sp] = make_uint4(mid, t.y, k, t.w + 1);
+                S.stack[sp + 1] = make_uint4(t.x, mid, kAll, t.w + 1);
+            }
         }
+        __syncwarp();
+        if (err) break;
+        if (split_it) sp += 2;
     }
-    // inner bounds are the union of the two children (bvh.rs:247)
-    for (uint32_t k = nn; k-- > 0;) {
-        PoolNode& N = pool[J.node0 + k];
-        if (N.b & kLeaf) continue;
-        const PoolNode& L = pool[J.node0 + k + 1];
-        const PoolNode& R = pool[J.node0 + N.a];
-        for (int c = 0; c < 3; ++c) {
-            N.lo[c] = dmin(L.lo[c], R.lo[c]);
-            N.hi[c] = dmax(L.hi[c], R.hi[c]);
-        }
-    }
-    outs[j] = JobOut{nn, maxd, err, 0};
+    const uint32_t p = __shfl_sync(kAll, prim, (int)(slot & 31u));
+    if (lane < n) idx[J.lo + lane] = p;
+    if (lane == 0) outs[j] = JobOut{nn, maxd, err, 0};
 }
 
 // ---- host ------------------------------------------------------------------
@@ -590,7 +643,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         lo[i] = make_float4(bounds[i].lo.x, bounds[i].lo.y, bounds[i].lo.z, 0.0f);
         hi[i] = make_float4(bounds[i].hi.x, bounds[i].hi.y, bounds[i].hi.z, 0.0f);
     }
-    Buf d_lo, d_hi, d_c[3], d_idx, d_tmp, d_stack, d_pool;
+    Buf d_lo, d_hi, d_c[3], d_idx, d_tmp, d_pool;
     CK(cudaMalloc(&d_lo.p, n * sizeof(float4)));
     CK(cudaMalloc(&d_hi.p, n * sizeof(float4)));
     for (int k = 0; k < 3; ++k) CK(cudaMalloc(&d_c[k].p, n * sizeof(float)));
@@ -657,7 +710,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         if (split == PBRT_SPLIT_SAH) {
             k_a_buckets<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_chunks.as<Chunk>(), d_dec.as<SegDecision>(),
                                      d_acc.as<int32_t>());
-            k_a_choose<<<(S + 127) / 128, 128>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_cnt.as<uint32_t>(),
+            k_a_choose<<<(S + 31) / 32, 32>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_cnt.as<uint32_t>(),
                                                  S, mp);
         }
         k_a_count<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_chunks.as<Chunk>(), d_dec.as<SegDecision>(),
@@ -721,7 +774,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         level.swap(next);
     }
 
-    // ---- phase B: every small range, one thread each
+    // ---- phase B: every small range, one warp each
     const uint32_t NJ = (uint32_t)jobs.size();
     uint64_t pool_nodes = 0;
     for (Job& j : jobs) {
@@ -729,13 +782,12 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         pool_nodes += 2ull * (j.hi - j.lo) - 1;
     }
     Buf d_jobs, d_outs;
-    CK(cudaMalloc(&d_stack.p, n * sizeof(Task)));
     CK(cudaMalloc(&d_pool.p, pool_nodes * sizeof(PoolNode)));
     CK(cudaMalloc(&d_jobs.p, (size_t)NJ * sizeof(Job)));
     CK(cudaMalloc(&d_outs.p, (size_t)NJ * sizeof(JobOut)));
     CK(cudaMemcpy(d_jobs.p, jobs.data(), (size_t)NJ * sizeof(Job), cudaMemcpyHostToDevice));
-    k_b_build<<<(NJ + 127) / 128, 128>>>(P, d_idx.as<uint32_t>(), d_tmp.as<uint32_t>(), d_stack.as<Task>(),
-                                         d_jobs.as<Job>(), NJ, d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp, split);
+    k_b_build<<<(NJ + kBWarps - 1) / kBWarps, 32 * kBWarps>>>(P, d_idx.as<uint32_t>(), d_jobs.as<Job>(), NJ,
+                                                              d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp, split);
     CK(cudaGetLastError());
     std::vector<JobOut> outs(NJ);
     std::vector<PoolNode> pool(pool_nodes);
