@@ -592,6 +592,7 @@ __global__ void __launch_bounds__(32 * kBWarps) k_b_build(Prims P, uint32_t* idx
 // ---- host ------------------------------------------------------------------
 struct Buf {  // a device allocation owned by the build
     void* p = nullptr;
+    size_t cap = 0;
     Buf() = default;
     Buf(const Buf&) = delete;
     Buf& operator=(const Buf&) = delete;
@@ -599,6 +600,24 @@ struct Buf {  // a device allocation owned by the build
     void reset() {
         if (p) cudaFree(p);
         p = nullptr;
+        cap = 0;
+    }
+    // At least `bytes`, contents not kept.  Grown ahead of the need: the
+    // levels' buffers double from level to level, and an allocation and its
+    // release synchronise the device.
+    cudaError_t reserve(size_t bytes) {
+        if (bytes <= cap) return cudaSuccess;
+        reset();
+        const size_t want = std::max<size_t>(4 * bytes, 1u << 16);
+        cudaError_t e = cudaMalloc(&p, want);
+        cap = want;
+        if (e != cudaSuccess) {  // not that much room: what is needed
+            (void)cudaGetLastError();
+            p = nullptr;
+            e = cudaMalloc(&p, bytes);
+            cap = e == cudaSuccess ? bytes : 0;
+        }
+        return e;
     }
     template <class T>
     T* as() {
@@ -635,14 +654,20 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         *err = "device BVH build: more than 2^31 primitives";
         return PBRT_ERR_UNSUPPORTED;
     }
-    std::vector<Box> bounds;
-    std::vector<float> cx, cy, cz;
-    prim_bounds(H, &bounds, &cx, &cy, &cz);
-    std::vector<float4> lo(n), hi(n);
-    for (size_t i = 0; i < n; ++i) {
-        lo[i] = make_float4(bounds[i].lo.x, bounds[i].lo.y, bounds[i].lo.z, 0.0f);
-        hi[i] = make_float4(bounds[i].hi.x, bounds[i].hi.y, bounds[i].hi.z, 0.0f);
-    }
+    RawVec<float4> lo(n), hi(n);
+    RawVec<float> cx(n), cy(n), cz(n);
+    host_parallel(n, [&](size_t, size_t from, size_t to) {
+        for (size_t i = from; i < to; ++i) {
+            V3 c;
+            const Box b = prim_bounds(H, i, &c);
+            lo[i] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
+            hi[i] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
+            cx[i] = c.x;
+            cy[i] = c.y;
+            cz[i] = c.z;
+            H.ordered[i] = (uint32_t)i;
+        }
+    });
     Buf d_lo, d_hi, d_c[3], d_idx, d_tmp, d_pool;
     CK(cudaMalloc(&d_lo.p, n * sizeof(float4)));
     CK(cudaMalloc(&d_hi.p, n * sizeof(float4)));
@@ -654,11 +679,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
     CK(cudaMemcpy(d_c[0].p, cx.data(), n * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_c[1].p, cy.data(), n * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_c[2].p, cz.data(), n * 4, cudaMemcpyHostToDevice));
-    {
-        std::vector<uint32_t> iota(n);
-        for (size_t i = 0; i < n; ++i) iota[i] = (uint32_t)i;
-        CK(cudaMemcpy(d_idx.p, iota.data(), n * 4, cudaMemcpyHostToDevice));
-    }
+    CK(cudaMemcpy(d_idx.p, H.ordered.data(), n * 4, cudaMemcpyHostToDevice));
     Prims P;
     P.lo = d_lo.as<float4>();
     P.hi = d_hi.as<float4>();
@@ -692,14 +713,12 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
                 chunks.push_back(Chunk{s, a.lo + o, a.lo + std::min(a.cnt, o + kChunk), 0});
         }
         const uint32_t NC = (uint32_t)chunks.size();
-        // per-level buffers (freed by the next assignment)
-        for (Buf* b : {&d_acc, &d_dec, &d_cnt, &d_chunks, &d_left, &d_base}) b->reset();
-        CK(cudaMalloc(&d_acc.p, (size_t)S * kAccWords * 4));
-        CK(cudaMalloc(&d_dec.p, (size_t)S * sizeof(SegDecision)));
-        CK(cudaMalloc(&d_cnt.p, (size_t)S * 4));
-        CK(cudaMalloc(&d_chunks.p, (size_t)NC * sizeof(Chunk)));
-        CK(cudaMalloc(&d_left.p, (size_t)NC * 4));
-        CK(cudaMalloc(&d_base.p, (size_t)NC * sizeof(uint2)));
+        CK(d_acc.reserve((size_t)S * kAccWords * 4));
+        CK(d_dec.reserve((size_t)S * sizeof(SegDecision)));
+        CK(d_cnt.reserve((size_t)S * 4));
+        CK(d_chunks.reserve((size_t)NC * sizeof(Chunk)));
+        CK(d_left.reserve((size_t)NC * 4));
+        CK(d_base.reserve((size_t)NC * sizeof(uint2)));
         CK(cudaMemcpy(d_cnt.p, counts.data(), (size_t)S * 4, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_chunks.p, chunks.data(), (size_t)NC * sizeof(Chunk), cudaMemcpyHostToDevice));
         const uint32_t acc_words = S * kAccWords;
@@ -790,7 +809,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
                                                               d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp, split);
     CK(cudaGetLastError());
     std::vector<JobOut> outs(NJ);
-    std::vector<PoolNode> pool(pool_nodes);
+    RawVec<PoolNode> pool(pool_nodes);
     CK(cudaMemcpy(outs.data(), d_outs.p, (size_t)NJ * sizeof(JobOut), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(pool.data(), d_pool.p, pool_nodes * sizeof(PoolNode), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(H.ordered.data(), d_idx.p, n * 4, cudaMemcpyDeviceToHost));
@@ -823,23 +842,15 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         uint32_t a;
         uint64_t at;
     };
+    std::vector<uint64_t> job_at(NJ);  // first node of each small range
     std::vector<Item> todo{{0, 0}};
     while (!todo.empty()) {
         const Item it = todo.back();
         todo.pop_back();
         const ANode& a = A[it.a];
         if (a.small) {
-            const Job& J = jobs[a.job];
-            const JobOut& o = outs[a.job];
-            for (uint32_t k = 0; k < o.nodes; ++k) {
-                const PoolNode& p = pool[J.node0 + k];
-                FlatNode& f = H.nodes[it.at + k];
-                f.box = Box{v3(p.lo[0], p.lo[1], p.lo[2]), v3(p.hi[0], p.hi[1], p.hi[2])};
-                f.leaf = (p.b & kLeaf) != 0;
-                f.offset = f.leaf ? p.a : (uint32_t)(it.at + p.a);
-                f.count = f.leaf ? (p.b & ~kLeaf) : p.b;
-            }
-            H.depth = std::max(H.depth, a.depth + o.depth - 1);
+            job_at[a.job] = it.at;
+            H.depth = std::max(H.depth, a.depth + outs[a.job].depth - 1);
             continue;
         }
         FlatNode& f = H.nodes[it.at];
@@ -858,6 +869,28 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         todo.push_back(Item{(uint32_t)a.right, right_at});
         todo.push_back(Item{(uint32_t)a.left, it.at + 1});
     }
+    // the ranges' nodes, cut at equal numbers of primitives
+    std::vector<uint32_t> order(NJ);
+    for (uint32_t j = 0; j < NJ; ++j) order[j] = j;
+    std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return jobs[x].lo < jobs[y].lo; });
+    host_parallel(n, [&](size_t, size_t from, size_t to) {
+        auto first = [&](size_t prim) {
+            return std::lower_bound(order.begin(), order.end(), prim,
+                                    [&](uint32_t j, size_t p) { return jobs[j].lo < p; });
+        };
+        for (auto i = first(from), e = first(to); i != e; ++i) {
+            const Job& J = jobs[*i];
+            const uint64_t at = job_at[*i];
+            for (uint32_t k = 0; k < outs[*i].nodes; ++k) {
+                const PoolNode& p = pool[J.node0 + k];
+                FlatNode& f = H.nodes[at + k];
+                f.box = Box{v3(p.lo[0], p.lo[1], p.lo[2]), v3(p.hi[0], p.hi[1], p.hi[2])};
+                f.leaf = (p.b & kLeaf) != 0;
+                f.offset = f.leaf ? p.a : (uint32_t)(at + p.a);
+                f.count = f.leaf ? (p.b & ~kLeaf) : p.b;
+            }
+        }
+    });
     return PBRT_OK;
 }
 

@@ -82,8 +82,8 @@ DeviceGuard::~DeviceGuard() {
     if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
 }
 
-template <class T>
-static int upload(T** dst, const std::vector<T>& src) {
+template <class T, class A>
+static int upload(T** dst, const std::vector<T, A>& src) {
     *dst = nullptr;
     if (src.empty()) return PBRT_OK;
     int st = cuda_status(cudaMalloc((void**)dst, src.size() * sizeof(T)), "cudaMalloc");

@@ -5,6 +5,7 @@
 #include "host_scene.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -235,36 +236,25 @@ struct Task {
 
 }  // namespace
 
-void prim_bounds(const HostBVH& H, std::vector<Box>* bounds, std::vector<float>* cx, std::vector<float>* cy,
-                 std::vector<float>* cz) {
-    const size_t n = H.prims.size();
-    bounds->resize(n);
-    cx->resize(n);
-    cy->resize(n);
-    cz->resize(n);
-    for (size_t i = 0; i < n; ++i) {
-        const HostPrim& p = H.prims[i];
-        Box b;
-        if (p.kind == PBRT_SHAPE_TRIANGLE_MESH) {
-            b = box_union(box_union(box_union(box_empty(), p.p1), p.p2), p.p3);  // mesh.rs:196-205
+Box prim_bounds(const HostBVH& H, size_t i, V3* centroid) {
+    const HostPrim& p = H.prims[i];
+    Box b;
+    if (p.kind == PBRT_SHAPE_TRIANGLE_MESH) {
+        b = box_union(box_union(box_union(box_empty(), p.p1), p.p2), p.p3);  // mesh.rs:196-205
+    } else {
+        const SphereRec& s = H.spheres[p.sphere];
+        M4 o2w;
+        std::memcpy(o2w.m, s.o2w, sizeof(o2w.m));
+        if (s.kind == kQuadInstance) {
+            // transformed.rs:62-65: motion_bounds of a static transform =
+            // the definition's bound through primitive-to-world
+            b = xf_box(o2w, H.insts[s.instance].nodes[0].box);  // definitions are not empty
         } else {
-            const SphereRec& s = H.spheres[p.sphere];
-            M4 o2w;
-            std::memcpy(o2w.m, s.o2w, sizeof(o2w.m));
-            if (s.kind == kQuadInstance) {
-                // transformed.rs:62-65: motion_bounds of a static transform =
-                // the definition's bound through primitive-to-world
-                b = xf_box(o2w, H.insts[s.instance].nodes[0].box);  // definitions are not empty
-            } else {
-                b = xf_box(o2w, Box{v3(-s.radius, -s.radius, s.z_min), v3(s.radius, s.radius, s.z_max)});
-            }
+            b = xf_box(o2w, Box{v3(-s.radius, -s.radius, s.z_min), v3(s.radius, s.radius, s.z_max)});
         }
-        (*bounds)[i] = b;
-        V3 c = (b.lo + b.hi) * 0.5f;  // bvh.rs:77
-        (*cx)[i] = c.x;
-        (*cy)[i] = c.y;
-        (*cz)[i] = c.z;
     }
+    *centroid = (b.lo + b.hi) * 0.5f;  // bvh.rs:77
+    return b;
 }
 
 static int build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
@@ -272,10 +262,18 @@ static int build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
     H.nodes.clear();
     H.ordered.resize(n);
     if (n == 0) return PBRT_OK;
-    std::vector<Box> bounds;
-    std::vector<float> cx, cy, cz;
-    prim_bounds(H, &bounds, &cx, &cy, &cz);
-    for (size_t i = 0; i < n; ++i) H.ordered[i] = (uint32_t)i;
+    RawVec<Box> bounds(n);
+    RawVec<float> cx(n), cy(n), cz(n);
+    host_parallel(n, [&](size_t, size_t lo, size_t hi) {
+        for (size_t i = lo; i < hi; ++i) {
+            V3 c;
+            bounds[i] = prim_bounds(H, i, &c);
+            cx[i] = c.x;
+            cy[i] = c.y;
+            cz[i] = c.z;
+            H.ordered[i] = (uint32_t)i;
+        }
+    });
     const float* cent[3] = {cx.data(), cy.data(), cz.data()};
     uint32_t* idx = H.ordered.data();
     H.nodes.reserve(2 * n);
@@ -392,12 +390,29 @@ static int build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
     return PBRT_OK;
 }
 
+static void set_flags(PrimRec& r, uint32_t f) {
+    uint32_t v;
+    std::memcpy(&v, &r.r2[3], 4);
+    v |= f;
+    std::memcpy(&r.r2[3], &v, 4);
+}
+
+// The binary layout, and with it the primitive flags of the 4-wide walk, the
+// leaf boxes they refer to, and whether the tree can have the 4-wide layout
+// at all.
 static void fill_device_layout(HostBVH& H) {
     const size_t m = H.nodes.size();
-    std::vector<uint32_t> pair_of(m, 0xffffffffu);
-    uint32_t np = 0;
-    for (size_t k = 0; k < m; ++k)
-        if (!H.nodes[k].leaf) pair_of[k] = np++;
+    // pairs are numbered in the pre-order of their parents
+    RawVec<uint32_t> pair_of(m);
+    std::vector<size_t> inner(host_parts(m) + 1, 0);  // inner nodes before each part
+    host_parallel(m, [&](size_t part, size_t lo, size_t hi) {
+        for (size_t k = lo; k < hi; ++k) inner[part + 1] += !H.nodes[k].leaf;
+    });
+    for (size_t p = 1; p < inner.size(); ++p) inner[p] += inner[p - 1];
+    host_parallel(m, [&](size_t part, size_t lo, size_t hi) {
+        uint32_t np = (uint32_t)inner[part];
+        for (size_t k = lo; k < hi; ++k) pair_of[k] = H.nodes[k].leaf ? 0xffffffffu : np++;
+    });
     auto rec = [&](size_t k) {
         const FlatNode& nd = H.nodes[k];
         ChildRec c;
@@ -416,87 +431,96 @@ static void fill_device_layout(HostBVH& H) {
         }
         return c;
     };
-    H.pairs.assign(np, NodePair{});
-    for (size_t k = 0; k < m; ++k) {
-        const FlatNode& nd = H.nodes[k];
-        if (nd.leaf) continue;
-        NodePair& p = H.pairs[pair_of[k]];
-        p.c[0] = rec(k + 1);
-        p.c[1] = rec(nd.offset);
-    }
+    H.pairs.resize(inner.back());
     if (m) H.root = rec(0);
     H.recs.resize(H.ordered.size() + 1);  // and the null record
     std::memset(&H.recs.back(), 0, sizeof(PrimRec));
-    for (size_t i = 0; i < H.ordered.size(); ++i) {
-        const HostPrim& p = H.prims[H.ordered[i]];
-        PrimRec& r = H.recs[i];
-        std::memset(&r, 0, sizeof(r));
-        uint32_t id = H.flat_id.empty() ? H.ordered[i] : H.flat_id[H.ordered[i]];
-        if (p.kind == PBRT_SHAPE_TRIANGLE_MESH) {
-            r.r0[0] = p.p1.x;
-            r.r0[1] = p.p1.y;
-            r.r0[2] = p.p1.z;
-            std::memcpy(&r.r0[3], &id, 4);
-            r.r1[0] = p.p2.x;
-            r.r1[1] = p.p2.y;
-            r.r1[2] = p.p2.z;
-            r.r2[0] = p.p3.x;
-            r.r2[1] = p.p3.y;
-            r.r2[2] = p.p3.z;
-        } else {
-            uint32_t tagged = id | kSphereBit;
-            uint32_t si = (uint32_t)p.sphere;
-            std::memcpy(&r.r0[3], &tagged, 4);
-            std::memcpy(&r.r1[3], &si, 4);
+    set_flags(H.recs.back(), kPrimLastBit);
+    auto usable = [](float v) { return std::fabs(v) <= kWideReach; };  // false for NaN
+    auto usable3 = [&](V3 v) { return usable(v.x) && usable(v.y) && usable(v.z); };
+    struct Part {
+        bool wide = true;
+        bool boxed = false;  // some leaf's box goes to the table
+    };
+    std::vector<Part> parts(host_parts(m));
+    host_parallel(m, [&](size_t part, size_t lo, size_t hi) {
+        Part& A = parts[part];
+        for (size_t k = lo; k < hi; ++k) {
+            const FlatNode& nd = H.nodes[k];
+            if (!nd.leaf) {
+                NodePair& p = H.pairs[pair_of[k]];
+                p.c[0] = rec(k + 1);
+                p.c[1] = rec(nd.offset);
+                continue;
+            }
+            A.wide = A.wide && usable3(nd.box.lo) && usable3(nd.box.hi);
+            bool tri = false;
+            for (uint32_t i = 0; i < nd.count; ++i) {
+                const uint32_t ref = H.ordered[nd.offset + i];
+                const HostPrim& p = H.prims[ref];
+                PrimRec& r = H.recs[nd.offset + i];
+                std::memset(&r, 0, sizeof(r));
+                uint32_t id = H.flat_id.empty() ? ref : H.flat_id[ref];
+                tri = p.kind == PBRT_SHAPE_TRIANGLE_MESH;
+                if (tri) {
+                    r.r0[0] = p.p1.x;
+                    r.r0[1] = p.p1.y;
+                    r.r0[2] = p.p1.z;
+                    r.r1[0] = p.p2.x;
+                    r.r1[1] = p.p2.y;
+                    r.r1[2] = p.p2.z;
+                    r.r2[0] = p.p3.x;
+                    r.r2[1] = p.p3.y;
+                    r.r2[2] = p.p3.z;
+                    A.wide = A.wide && usable3(p.p1) && usable3(p.p2) && usable3(p.p3);
+                } else {
+                    const uint32_t si = (uint32_t)p.sphere;
+                    id |= kSphereBit;
+                    std::memcpy(&r.r1[3], &si, 4);
+                }
+                std::memcpy(&r.r0[3], &id, 4);
+            }
+            if (nd.count == 0) continue;
+            set_flags(H.recs[nd.offset + nd.count - 1], kPrimLastBit);
+            if (nd.count == 1 && tri)
+                set_flags(H.recs[nd.offset], kPrimOwnBox);
+            else
+                A.boxed = true;
         }
+    });
+    H.wide = H.ordered.size() < 0x7ffffff0u && H.pairs.size() < (1u << kQuadAxisShift);
+    H.leaf_boxes.clear();
+    bool boxed = false;
+    for (const Part& A : parts) {
+        H.wide = H.wide && A.wide;
+        boxed = boxed || A.boxed;
+    }
+    for (size_t k = 0; boxed && k < m; ++k) {
+        const FlatNode& nd = H.nodes[k];
+        if (!nd.leaf || nd.count == 0) continue;
+        const HostPrim& first = H.prims[H.ordered[nd.offset]];
+        if (nd.count == 1 && first.kind == PBRT_SHAPE_TRIANGLE_MESH) continue;
+        const bool entry = nd.count > 1 || H.spheres[first.sphere].kind == kQuadInstance;
+        if (H.leaf_boxes.size() >= (1u << (32u - kPrimBoxShift))) {
+            H.wide = false;
+            break;
+        }
+        set_flags(H.recs[nd.offset],
+                  (entry ? kPrimBoxEntry : kPrimHitBox) | ((uint32_t)H.leaf_boxes.size() << kPrimBoxShift));
+        const Box& b = nd.box;
+        H.leaf_boxes.push_back(LeafBox{{b.lo.x, b.lo.y, b.lo.z, 0.0f}, {b.hi.x, b.hi.y, b.hi.z, 0.0f}});
     }
 }
 
 // Where the 4-wide nodes start (two binary levels each, see layout.h:
-// QuadNode), the primitive flags of the 4-wide walk with the leaf boxes they
-// refer to, and whether the tree can have that layout at all.
+// QuadNode).
 static void fill_quad_layout(HostBVH& H) {
     const size_t m = H.nodes.size();
-    H.quad_of.assign(H.pairs.size(), kNoQuad);
-    H.leaf_boxes.clear();
+    H.quad_of.resize(H.pairs.size());
     H.n_quads = 0;
     H.quad_root = 0;
     H.stack4_bound = 0;
     H.reach = 0.0f;
-    auto set_flags = [&](size_t i, uint32_t f) {
-        uint32_t v;
-        std::memcpy(&v, &H.recs[i].r2[3], 4);
-        v |= f;
-        std::memcpy(&H.recs[i].r2[3], &v, 4);
-    };
-    set_flags(H.recs.size() - 1, kPrimLastBit);
-    H.wide = H.ordered.size() < 0x7ffffff0u && H.pairs.size() < (1u << kQuadAxisShift);
-    auto usable = [](float v) { return std::fabs(v) <= kWideReach; };  // false for NaN
-    auto usable3 = [&](V3 v) { return usable(v.x) && usable(v.y) && usable(v.z); };
-    for (size_t k = 0; k < m; ++k) {
-        const FlatNode& nd = H.nodes[k];
-        if (!nd.leaf || nd.count == 0) continue;
-        H.wide = H.wide && usable3(nd.box.lo) && usable3(nd.box.hi);
-        for (uint32_t i = 0; i < nd.count; ++i) {
-            const HostPrim& p = H.prims[H.ordered[nd.offset + i]];
-            if (p.kind == PBRT_SHAPE_TRIANGLE_MESH)
-                H.wide = H.wide && usable3(p.p1) && usable3(p.p2) && usable3(p.p3);
-        }
-        set_flags(nd.offset + nd.count - 1, kPrimLastBit);
-        const HostPrim& first = H.prims[H.ordered[nd.offset]];
-        if (nd.count == 1 && first.kind == PBRT_SHAPE_TRIANGLE_MESH) {
-            set_flags(nd.offset, kPrimOwnBox);
-            continue;
-        }
-        const bool entry = nd.count > 1 || H.spheres[first.sphere].kind == kQuadInstance;
-        if (H.leaf_boxes.size() >= (1u << (32u - kPrimBoxShift))) {
-            H.wide = false;
-            continue;
-        }
-        set_flags(nd.offset, (entry ? kPrimBoxEntry : kPrimHitBox) | ((uint32_t)H.leaf_boxes.size() << kPrimBoxShift));
-        const Box& b = nd.box;
-        H.leaf_boxes.push_back(LeafBox{{b.lo.x, b.lo.y, b.lo.z, 0.0f}, {b.hi.x, b.hi.y, b.hi.z, 0.0f}});
-    }
     for (const HostBVH& I : H.insts) H.wide = H.wide && I.wide;
     if (m == 0) return;
     const Box& rb = H.nodes[0].box;
@@ -505,11 +529,15 @@ static void fill_quad_layout(HostBVH& H) {
     if (H.nodes[0].leaf) return;
     // pairs are numbered in pre-order, so a node's 4-wide start is decided
     // before its grandchildren's
-    std::vector<uint32_t> deferred(H.pairs.size(), 0);  // entries the walk may hold above a start
-    std::vector<uint8_t> starts(H.pairs.size(), 0);      // split axis + 1 of a start
+    RawVec<uint32_t> deferred(H.pairs.size());       // entries the walk may hold above a start
+    std::vector<uint8_t> starts(H.pairs.size(), 0);  // split axis + 1 of a start
     starts[0] = (uint8_t)(H.nodes[0].count + 1);
+    deferred[0] = 0;
     for (size_t p = 0; p < H.pairs.size(); ++p) {
-        if (!starts[p]) continue;
+        if (!starts[p]) {
+            H.quad_of[p] = kNoQuad;
+            continue;
+        }
         H.quad_of[p] = H.n_quads++ | ((uint32_t)(starts[p] - 1) << kQuadAxisShift);
         uint32_t slots = 0;
         for (const ChildRec& c : H.pairs[p].c) slots += (c.b & kLeafBit) ? 1u : 2u;
@@ -561,26 +589,37 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
                 *err = "triangle mesh: index count must be a multiple of 3 with points and indices given";
                 return PBRT_ERR_INVALID_ARGUMENT;
             }
-            std::vector<V3> wp(d.n_points);
-            for (uint32_t i = 0; i < d.n_points; ++i)
-                wp[i] = m4_point(o2w.m, v3(d.points[3 * i], d.points[3 * i + 1], d.points[3 * i + 2]));
-            for (uint32_t k = 0; k < d.n_indices / 3; ++k) {
-                uint32_t i0 = d.indices[3 * k], i1 = d.indices[3 * k + 1], i2 = d.indices[3 * k + 2];
-                if (i0 >= d.n_points || i1 >= d.n_points || i2 >= d.n_points) {
-                    *err = "triangle mesh: vertex index out of range";
-                    return PBRT_ERR_INVALID_ARGUMENT;
+            RawVec<V3> wp(d.n_points);
+            host_parallel(d.n_points, [&](size_t, size_t lo, size_t hi) {
+                for (size_t i = lo; i < hi; ++i)
+                    wp[i] = m4_point(o2w.m, v3(d.points[3 * i], d.points[3 * i + 1], d.points[3 * i + 2]));
+            });
+            const size_t first = H.prims.size(), nt = d.n_indices / 3;
+            H.prims.resize(first + nt);
+            std::atomic<bool> bad{false};
+            host_parallel(nt, [&](size_t, size_t lo, size_t hi) {
+                for (size_t k = lo; k < hi; ++k) {
+                    uint32_t i0 = d.indices[3 * k], i1 = d.indices[3 * k + 1], i2 = d.indices[3 * k + 2];
+                    if (i0 >= d.n_points || i1 >= d.n_points || i2 >= d.n_points) {
+                        bad = true;
+                        return;
+                    }
+                    HostPrim p{};
+                    p.kind = PBRT_SHAPE_TRIANGLE_MESH;
+                    p.shape = (int)si;
+                    p.material = d.material;
+                    p.area_light = d.area_light;
+                    p.p1 = wp[i2];  // refine pops indices: v = (i2, i1, i0)
+                    p.p2 = wp[i1];
+                    p.p3 = wp[i0];
+                    p.flip = flip;
+                    p.sphere = -1;
+                    H.prims[first + k] = p;
                 }
-                HostPrim p{};
-                p.kind = PBRT_SHAPE_TRIANGLE_MESH;
-                p.shape = (int)si;
-                p.material = d.material;
-                p.area_light = d.area_light;
-                p.p1 = wp[i2];  // refine pops indices: v = (i2, i1, i0)
-                p.p2 = wp[i1];
-                p.p3 = wp[i0];
-                p.flip = flip;
-                p.sphere = -1;
-                H.prims.push_back(p);
+            });
+            if (bad) {
+                *err = "triangle mesh: vertex index out of range";
+                return PBRT_ERR_INVALID_ARGUMENT;
             }
         } else if (d.kind == PBRT_SHAPE_SPHERE) {
             if (!(d.radius > 0.0f)) {

@@ -5,15 +5,69 @@
 // SAH/middle/equal BVH build, its depth-first flattening, and the
 // conversion to the device pair layout of layout.h.
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <memory>
 #include <string>
+#include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/pbrt_gpu.h"
 #include "layout.h"
 
 namespace pbrt {
+
+// A vector whose resize leaves new elements uninitialised: the arrays of a
+// scene are written element by element right after, by several threads
+// (zeroing them first costs one thread's pass and all their page faults).
+template <class T>
+struct RawAlloc : std::allocator<T> {
+    template <class U>
+    struct rebind {
+        using other = RawAlloc<U>;
+    };
+    RawAlloc() = default;
+    template <class U>
+    RawAlloc(const RawAlloc<U>&) {}
+    template <class U>
+    void construct(U* p) noexcept {
+        ::new (static_cast<void*>(p)) U;
+    }
+    template <class U, class... A>
+    void construct(U* p, A&&... a) {
+        ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+    }
+};
+template <class T>
+using RawVec = std::vector<T, RawAlloc<T>>;
+
+// f(part, lo, hi) over [0, n) cut into host_parts(n) equal parts, each on its
+// own thread; f must not throw.  A part has at least 16384 items, so small
+// scenes stay on the caller's thread.  Creating a terrain of 180000 triangles
+// with the device build took 18.2 ms with these loops on one thread and 11.9 ms
+// with eight.
+inline size_t host_parts(size_t n) {
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    return std::max<size_t>(1, std::min(std::min<size_t>(8, cores), n / 16384));
+}
+template <class F>
+void host_parallel(size_t n, F f) {
+    const size_t parts = host_parts(n);
+    auto at = [&](size_t p) { return n / parts * p + std::min(p, n % parts); };
+    std::vector<std::thread> others;
+    size_t next = 1;
+    try {
+        others.reserve(parts - 1);
+        for (; next < parts; ++next)
+            others.emplace_back([&f, &at, next] { f(next, at(next), at(next + 1)); });
+    } catch (...) {  // no thread to be had: the caller takes the remaining parts
+    }
+    f((size_t)0, (size_t)0, at(1));
+    for (size_t p = next; p < parts; ++p) f(p, at(p), at(p + 1));
+    for (std::thread& t : others) t.join();
+}
 
 struct V3 {
     float x, y, z;
@@ -79,21 +133,21 @@ struct FlatNode {
 };
 
 struct HostBVH {
-    std::vector<HostPrim> prims;
+    RawVec<HostPrim> prims;
     std::vector<SphereRec> spheres;
-    std::vector<FlatNode> nodes;
-    std::vector<uint32_t> ordered;  // ordered_prims: refined input index
+    RawVec<FlatNode> nodes;
+    RawVec<uint32_t> ordered;  // ordered_prims: refined input index
     uint32_t depth = 0;
     // device layout
     ChildRec root{};
-    std::vector<NodePair> pairs;
-    std::vector<PrimRec> recs;
+    RawVec<NodePair> pairs;
+    RawVec<PrimRec> recs;
     bool has_spheres = false;
     // 4-wide layout (layout.h: QuadNode; same tree, two binary levels per
     // node), encoded on the device from the pairs: quad_of[pair] = index of
     // the 4-wide node that starts at the pair's node | its split axis <<
     // kQuadAxisShift, kNoQuad for the pairs in between
-    std::vector<uint32_t> quad_of;
+    RawVec<uint32_t> quad_of;
     uint32_t n_quads = 0;
     uint32_t quad_root = 0;           // the root's child word
     std::vector<LeafBox> leaf_boxes;  // leaf boxes the records' flags refer to
@@ -123,10 +177,9 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
                    HostBVH* out, std::string* err, bool on_device = false, const PbrtInstanceDesc* defs = nullptr,
                    uint32_t n_defs = 0);
 
-// Bounds (mesh.rs:196-205, sphere.rs:111-126) and centroids (bvh.rs:77) of
-// the refined primitives.
-void prim_bounds(const HostBVH& H, std::vector<Box>* bounds, std::vector<float>* cx, std::vector<float>* cy,
-                 std::vector<float>* cz);
+// Bounds (mesh.rs:196-205, sphere.rs:111-126) and centroid (bvh.rs:77) of
+// refined primitive i.
+Box prim_bounds(const HostBVH& H, size_t i, V3* centroid);
 
 // The tree of build_tree (H.nodes, H.ordered, H.depth) built on the current
 // CUDA device (bvh_build.cu): identical nodes and primitive order.
