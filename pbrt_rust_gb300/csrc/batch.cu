@@ -21,7 +21,7 @@
 namespace pbrt {
 
 cudaError_t launch_batch_trace(const BatchArgs& A, const BatchTuning& T, bool shadow, bool mixed, bool inst,
-                               uint32_t cover_pair, uint32_t cover_wide, int sms, cudaStream_t s);
+                               bool queries, uint32_t cover_pair, uint32_t cover_wide, int sms, cudaStream_t s);
 cudaError_t launch_batch_replay(const BatchArgs& A, const BatchTuning& T, bool shadow, int sms, cudaStream_t s);
 
 namespace {
@@ -99,8 +99,9 @@ __global__ void __launch_bounds__(BLOCK) kb_film(BatchArgs A) {
 
 }  // namespace
 
-cudaError_t launch_batch_stages(const BatchArgs& A, const BatchTuning& T, bool mixed, bool inst, uint32_t cover_pair,
-                                uint32_t cover_wide, int sms, size_t counter_bytes, cudaStream_t s, int* launches) {
+cudaError_t launch_batch_stages(const BatchArgs& A, const BatchTuning& T, bool mixed, bool inst, bool queries,
+                                uint32_t cover_pair, uint32_t cover_wide, int sms, size_t counter_bytes, cudaStream_t s,
+                                int* launches) {
     *launches = 0;
     cudaError_t e = cudaMemsetAsync(A.counters, 0, counter_bytes, s);
     if (e != cudaSuccess) return e;
@@ -113,12 +114,12 @@ cudaError_t launch_batch_stages(const BatchArgs& A, const BatchTuning& T, bool m
     };
     const bool b256 = T.block == 256;
     if ((e = b256 ? stage(kb_generate<256>) : stage(kb_generate<128>)) != cudaSuccess) return e;
-    if ((e = launch_batch_trace(A, T, false, mixed, inst, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
+    if ((e = launch_batch_trace(A, T, false, mixed, inst, queries, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
     ++*launches;
     if ((e = launch_batch_replay(A, T, false, sms, s)) != cudaSuccess) return e;
     ++*launches;
     if ((e = b256 ? stage(kb_shade<256>) : stage(kb_shade<128>)) != cudaSuccess) return e;
-    if ((e = launch_batch_trace(A, T, true, false, inst, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
+    if ((e = launch_batch_trace(A, T, true, false, inst, false, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
     ++*launches;
     if (T.shadow_wide && !inst && T.refill_shadow < 32) {  // the shadow walk that marks rays
         if ((e = launch_batch_replay(A, T, true, sms, s)) != cudaSuccess) return e;

@@ -120,18 +120,22 @@ struct PbrtBatch {
     // (serving mix of 32 soups: 5280 against 5100 requests/s with 32 / 32)
     BatchTuning tune{1, 1, 128, 16, 64, 32, 8};
     bool use_graph = true;
-    cudaGraphExec_t graph = nullptr;
-    BatchTuning graph_tune{};
-    bool graph_mixed = false;
-    bool graph_inst = false;
-    uint32_t graph_cover_pair = 0, graph_cover_wide = 0;
-    int graph_kernels = 0;
+    // the captured sequences, one for batches with and one for batches
+    // without many query rays (requests of both kinds alternate in a server)
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        BatchTuning tune{};
+        bool mixed = false, inst = false;
+        uint32_t cover_pair = 0, cover_wide = 0;
+        int kernels = 0;
+    } graphs[2];
     int last_kernels = 0;
     bool last_graph = false;
 
     explicit PbrtBatch(const PbrtBatchLimits& L) : lim(L), lay(L) {}
     ~PbrtBatch() {
-        if (graph) cudaGraphExecDestroy(graph);
+        for (Graph& g : graphs)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
         if (done) cudaEventDestroy(done);
         if (t0) cudaEventDestroy(t0);
         if (t1) cudaEventDestroy(t1);
@@ -192,6 +196,9 @@ struct PbrtBatch {
         ++n_jobs;
     }
 
+    // query rays make up at least 1/8 of the batch's rays
+    bool queries() const { return 8 * (n_ray - n_smp) >= n_ray && n_ray > n_smp; }
+
     size_t counter_bytes() const { return (size_t)(n_jobs + 1) * kCtrWords * 4; }
 };
 
@@ -199,19 +206,19 @@ namespace {
 
 int enqueue_stages(PbrtBatch* b, cudaStream_t s) {
     BatchArgs A = b->args();
-    const bool key_match = b->graph && !std::memcmp(&b->graph_tune, &b->tune, sizeof(BatchTuning)) &&
-                           b->graph_mixed == b->mixed && b->graph_inst == b->inst &&
-                           b->graph_cover_pair == b->cover_pair &&
-                           b->graph_cover_wide == b->cover_wide;
+    PbrtBatch::Graph& G = b->graphs[b->queries() ? 1 : 0];
+    const bool key_match = G.exec && !std::memcmp(&G.tune, &b->tune, sizeof(BatchTuning)) && G.mixed == b->mixed &&
+                           G.inst == b->inst && G.cover_pair == b->cover_pair && G.cover_wide == b->cover_wide;
     // the graph zeroes every job slot's counters, so it serves any job count
     const size_t cbytes = (size_t)(b->lim.max_jobs + 1) * kCtrWords * 4;
     if (b->use_graph && key_match) {
         b->last_graph = true;
-        b->last_kernels = b->graph_kernels;
-        return cuda_status(cudaGraphLaunch(b->graph, s), "cudaGraphLaunch");
+        b->last_kernels = G.kernels;
+        return cuda_status(cudaGraphLaunch(G.exec, s), "cudaGraphLaunch");
     }
     int n = 0;
-    int st = cuda_status(launch_batch_stages(A, b->tune, b->mixed, b->inst, b->cover_pair, b->cover_wide, b->sms, cbytes, s, &n),
+    int st = cuda_status(launch_batch_stages(A, b->tune, b->mixed, b->inst, b->queries(), b->cover_pair, b->cover_wide,
+                                             b->sms, cbytes, s, &n),
                          "batch stages");
     if (st) return st;
     b->last_graph = false;
@@ -219,30 +226,30 @@ int enqueue_stages(PbrtBatch* b, cudaStream_t s) {
     if (b->use_graph) {
         // capture the same sequence for the next launches with this key (the
         // direct launch above has fixed every kernel's occupancy first)
-        if (b->graph) cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
+        if (G.exec) cudaGraphExecDestroy(G.exec);
+        G.exec = nullptr;
         cudaGraph_t g = nullptr;
         if ((st = cuda_status(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal),
                               "cudaStreamBeginCapture")))
             return st;
         int m = 0;
         cudaError_t e =
-            launch_batch_stages(A, b->tune, b->mixed, b->inst, b->cover_pair, b->cover_wide, b->sms, cbytes,
+            launch_batch_stages(A, b->tune, b->mixed, b->inst, b->queries(), b->cover_pair, b->cover_wide, b->sms, cbytes,
                                 b->cap_stream, &m);
         cudaError_t e2 = cudaStreamEndCapture(b->cap_stream, &g);
         if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, g, 0);
         if (g) cudaGraphDestroy(g);
         if ((st = cuda_status(e, "batch graph capture"))) {
-            b->graph = nullptr;
+            G.exec = nullptr;
             return st;
         }
-        b->graph_tune = b->tune;
-        b->graph_mixed = b->mixed;
-        b->graph_inst = b->inst;
-        b->graph_cover_pair = b->cover_pair;
-        b->graph_cover_wide = b->cover_wide;
-        b->graph_kernels = m;
+        G.tune = b->tune;
+        G.mixed = b->mixed;
+        G.inst = b->inst;
+        G.cover_pair = b->cover_pair;
+        G.cover_wide = b->cover_wide;
+        G.kernels = m;
     }
     return PBRT_OK;
 }
