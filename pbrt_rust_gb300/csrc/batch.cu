@@ -59,8 +59,10 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) kb_generate(BatchArgs A) {
     }
 }
 
+// 1024 resident threads per SM: 0.80 ms for 24 scenes' samples, 1.14 ms as the
+// compiler chose, 0.83 / 1.19 with 1152 / 1280.
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) kb_shade(BatchArgs A) {
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) kb_shade(BatchArgs A) {
     const uint64_t total = A.hdr->samples;
     const uint32_t nj = A.hdr->n_jobs;
     const ShadowSink Q{A.q_rays, A.q_slot, A.q_job, A.counters + kCtrShadowCount};

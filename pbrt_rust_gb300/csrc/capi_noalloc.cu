@@ -172,6 +172,7 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     P.fy1 = fe[3];
     P.filter_xw = cam->filter_x_width;
     P.filter_yw = cam->filter_y_width;
+    P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
     P.filter_inv_xw = 1.0f / cam->filter_x_width;
     P.filter_inv_yw = 1.0f / cam->filter_y_width;
     gather_offsets(cam->filter_x_width, P.sx0, P.sx1, &P.gx0, &P.gx1);
@@ -255,7 +256,6 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     P.pixbox = (float4*)p_pixbox;
     P.lsamp = (float*)p_lsamp;
     P.contrib = (float4*)p_contrib;
-    P.le = (float4*)p_le;
     P.L = (float4*)p_L;
     P.shadow_rays = (PbrtRay*)p_srays;
     P.shadow_slot = (uint32_t*)p_sslot;

@@ -477,6 +477,7 @@ int prepare_render(PbrtScene* S, const PbrtCameraDesc* cam, const PbrtSamplerDes
     P.fy1 = fe[3];
     P.filter_xw = cam->filter_x_width;
     P.filter_yw = cam->filter_y_width;
+    P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
     P.filter_inv_xw = 1.0f / cam->filter_x_width;
     P.filter_inv_yw = 1.0f / cam->filter_y_width;
     gather_offsets(cam->filter_x_width, P.sx0, P.sx1, &P.gx0, &P.gx1);
@@ -591,7 +592,7 @@ int pbrtgpu_render_tasks(const PbrtScene* cS, const PbrtCameraDesc* cam, const P
     if ((st = S->rays.reserve(S_ * sizeof(PbrtRay))) || (st = S->hits.reserve(S_ * 16)) ||
         (st = S->img.reserve(S_ * 8)) || (st = S->pixbox.reserve((uint64_t)P.n_pixels * 16)) ||
         (st = S->lsamp.reserve(S_ * 3 * nl * 4 + 4)) ||
-        (st = S->contrib.reserve(SL * 16 + 16)) || (st = S->le.reserve(S_ * 16)) || (st = S->L.reserve(S_ * 16)) ||
+        (st = S->contrib.reserve(SL * 16 + 16)) || (st = S->L.reserve(S_ * 16)) ||
         (st = S->srays.reserve(SL * sizeof(PbrtRay) + 32)) || (st = S->sslot.reserve(SL * 4 + 4)) ||
         (st = S->occ.reserve(SL + 1)) || (st = S->counters.reserve(64)) ||
         (st = S->tasks.reserve(tasks.size() * sizeof(TaskRec))) || (st = S->table.reserve(256 * 4)))
@@ -613,7 +614,6 @@ int pbrtgpu_render_tasks(const PbrtScene* cS, const PbrtCameraDesc* cam, const P
     P.pixbox = (float4*)S->pixbox.p;
     P.lsamp = (float*)S->lsamp.p;
     P.contrib = (float4*)S->contrib.p;
-    P.le = (float4*)S->le.p;
     P.L = (float4*)S->L.p;
     P.shadow_rays = (PbrtRay*)S->srays.p;
     P.shadow_slot = (uint32_t*)S->sslot.p;

@@ -30,7 +30,9 @@ __global__ void __launch_bounds__(128) k_generate(RenderParams P) {
     generate_pixel(P, pix, words + threadIdx.x, 128u);
 }
 
-__global__ void __launch_bounds__(128) k_shade(RenderParams P) {
+// 9 blocks per SM: 363 us for 1024 x 1024 x 16 samples and one light, 386 with
+// 8, 509 with 10 (spills).
+__global__ void __launch_bounds__(128, 9) k_shade(RenderParams P) {
     const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const ShadowSink Q{P.shadow_rays, P.shadow_slot, nullptr, &P.counters[0]};
     shade_sample(P, s, s < P.n_samples, Q, 0u);

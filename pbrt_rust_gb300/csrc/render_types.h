@@ -70,6 +70,7 @@ struct RenderParams {
     // (gather_offsets in capi_render.cu)
     int32_t gx0, gx1, gy0, gy1;
     const float* filter_table;   // 16 x 16
+    uint32_t filter_flat;        // every entry is 1 (a box filter)
     // tasks
     const TaskRec* tasks;
     uint32_t n_tasks;
@@ -98,13 +99,12 @@ struct RenderParams {
     float2* img;
     float4* pixbox;     // per sampler pixel: (min x, min y, max x, max y) of its sample positions
     float* lsamp;       // 3 * n_lights floats per sample: components then positions
-    float4* contrib;    // per (sample, light): rgb, w = 1 if a shadow ray decides it
-    float4* le;         // per sample emitted radiance
+    float4* contrib;    // per (sample, light) with a shadow ray: rgb
     float4* L;          // per sample radiance
     PbrtRay* shadow_rays;
     uint32_t* shadow_slot;
     uint32_t* counters;  // [0] shadow rays, [1] NaN samples, [2] status, [3] replay flag (zero at launch)
-    uint8_t* occluded;   // per (sample, light)
+    uint8_t* occluded;   // per (sample, light): 0 unoccluded, 1 occluded, kNoContribution
     float* rgb;          // film output
 };
 

@@ -10,7 +10,8 @@
 //                    unoccluded contribution of one camera sample; shadow
 //                    rays go to a compacted queue (integrator/whitted.rs:30-65,
 //                    light/point.rs:28-35)
-//   combine_sample : L = Le + the unoccluded contributions in light order
+//   combine_sample : L += the unoccluded contributions in light order (the
+//                    shading left Le there)
 //   film_pixel     : one film pixel gathers the samples that land on it, from
 //                    its own task only, in the task's sample order
 //                    (camera/film.rs:192-249, 175-186, 316-354)
@@ -387,6 +388,10 @@ __device__ __forceinline__ float oren_nayar_term(float a, float b, V wo, V wi) {
     return a + b * maxcos * sinalpha * tanbeta;
 }
 
+// RenderParams::occluded of a (sample, light) without a shadow ray (others
+// get 0 or 1 from the shadow stage, kReplayOcc in between).
+constexpr uint8_t kNoContribution = 3;
+
 // Where shade_sample appends its shadow rays: the ray, the (sample, light)
 // slot it decides and, in a batch, the job it belongs to.
 struct ShadowSink {
@@ -406,7 +411,14 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
     const uint32_t nl = live ? P.n_lights : 0u;
     const unsigned lane = threadIdx.x & 31;
     const uint32_t nl_warp = __reduce_max_sync(0xffffffffu, nl);
-    float4 h = live ? P.hits[s] : make_float4(__int_as_float(-1), 0, 0, 0);
+    // the ray does not wait for the hit: both loads are in flight together
+    float4 h = make_float4(__int_as_float(-1), 0, 0, 0), ra = h, rb = h;
+    if (live) {
+        const float4* ray = reinterpret_cast<const float4*>(P.rays) + 2 * s;
+        h = P.hits[s];
+        ra = ray[0];
+        rb = ray[1];
+    }
     int32_t prim = __float_as_int(h.x);
     bool hit = live && prim >= 0;
     V p = mkv(0, 0, 0), nn = mkv(0, 0, 1), wo = mkv(0, 0, 1), dpdu = mkv(1, 0, 0);
@@ -416,9 +428,8 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
     bool oren = false;
     float le[3] = {0, 0, 0};
     if (hit) {
-        const PbrtRay r = P.rays[s];
         float t = h.y;
-        V o = mkv(r.ox, r.oy, r.oz), d = mkv(r.dx, r.dy, r.dz);
+        V o = mkv(ra.x, ra.y, ra.z), d = mkv(rb.x, rb.y, rb.z);
         const ShadePrim* shade = P.shade;
         const SphereRec* spheres = P.spheres;
         const SphereRec* inst = nullptr;
@@ -468,7 +479,7 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
                            m[2] * nn.x + m[6] * nn.y + m[10] * nn.z));
         }
         eps = t * 5e-4f;  // mesh.rs:262, sphere.rs:174
-        wo = mkv(-r.dx, -r.dy, -r.dz);
+        wo = mkv(-rb.x, -rb.y, -rb.z);
         uint32_t al = __float_as_uint(sp.b[3]);
         if (al != 0u) {  // Le of an emitter (pbrt-v2 semantics; intersection.rs:58 is 0)
             const LightRec& L = P.lights[al - 1];
@@ -495,7 +506,10 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
         sn = vcross(nn, tn);
         wo_l = mkv(vdot(wo, sn), vdot(wo, tn), vdot(wo, nn));
     }
-    if (live) P.le[s] = make_float4(le[0], le[1], le[2], 0.0f);
+    if (live) {
+        P.L[s] = make_float4(le[0], le[1], le[2], 0.0f);
+        if (le[0] != le[0] || le[1] != le[1] || le[2] != le[2]) atomicAdd(&P.counters[1], 1u);
+    }
     const float invpi = 1.0f / 3.14159265358979323846f;  // lambertian.rs:21
     for (uint32_t l = 0; l < nl_warp; ++l) {
         bool want = false;
@@ -561,12 +575,14 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
                     c.x = ((f[0] * Li[0]) * ad) / pdf;
                     c.y = ((f[1] * Li[1]) * ad) / pdf;
                     c.z = ((f[2] * Li[2]) * ad) / pdf;
-                    c.w = 1.0f;
                     want = true;
                 }
             }
         }
-        if (live && l < nl) P.contrib[s * nl + l] = c;
+        if (want)
+            P.contrib[s * nl + l] = c;
+        else if (live && l < nl)
+            P.occluded[s * nl + l] = kNoContribution;
         // warp-aggregated append to the shadow-ray queue
         unsigned mask = __ballot_sync(0xffffffffu, want);
         if (mask) {
@@ -584,20 +600,26 @@ __device__ __forceinline__ void shade_sample(const RenderParams& P, uint64_t s, 
     }
 }
 
-// One sample (k_combine's item).
+// One sample (k_combine's item): its emitted radiance, which the shading left
+// in L, plus the contributions whose shadow ray found nothing, in light order.
+// Samples without such contributions are neither read nor written.
 __device__ __forceinline__ void combine_sample(const RenderParams& P, uint64_t s) {
-    float4 e = P.le[s];
-    float L0 = e.x, L1 = e.y, L2 = e.z;
-    for (uint32_t l = 0; l < P.n_lights; ++l) {
-        float4 c = P.contrib[s * P.n_lights + l];
-        if (c.w != 0.0f && !P.occluded[s * P.n_lights + l]) {
-            L0 = L0 + c.x;
-            L1 = L1 + c.y;
-            L2 = L2 + c.z;
-        }
+    const uint32_t nl = P.n_lights;
+    const uint8_t* occ = P.occluded + s * nl;
+    uint32_t l = 0;
+    while (l < nl && occ[l] != 0) ++l;
+    if (l == nl) return;
+    float4 L = P.L[s];
+    const bool was_nan = L.x != L.x || L.y != L.y || L.z != L.z;
+    for (; l < nl; ++l) {
+        if (occ[l] != 0) continue;
+        const float4 c = P.contrib[s * nl + l];
+        L.x = L.x + c.x;
+        L.y = L.y + c.y;
+        L.z = L.z + c.z;
     }
-    if (L0 != L0 || L1 != L1 || L2 != L2) atomicAdd(&P.counters[1], 1u);
-    P.L[s] = make_float4(L0, L1, L2, 0.0f);
+    if (!was_nan && (L.x != L.x || L.y != L.y || L.z != L.z)) atomicAdd(&P.counters[1], 1u);
+    P.L[s] = L;
 }
 
 // ------------------------------------------------------------------ film ---
@@ -613,6 +635,14 @@ __device__ __forceinline__ void xyz_to_rgb(const float* x, float* r) {  // spect
 }
 
 // One film pixel, idx in [0, film width * height) (k_film's item).
+//
+// A sample at image position v lands on pixel p, along one axis, iff
+// ceil(v - 0.5 - w) <= p <= floor(v - 0.5 + w) (film.rs:198-210); p is an
+// integer, so the bounds need no rounding: p >= ceil(a) iff p >= a.  Film
+// coordinates below 2^22 are compared as floats (four comparisons instead of
+// eight conversions to integers, which run at a quarter of their rate), larger
+// ones as the reference does.  p lies in its task's film already, so the clamp
+// to the task's extent decides nothing more.
 __device__ __forceinline__ void film_pixel(const RenderParams& P, uint32_t idx) {
     const int32_t fw = P.fx1 - P.fx0;
     const int32_t px = P.fx0 + (int32_t)(idx % (uint32_t)fw);
@@ -629,37 +659,41 @@ __device__ __forceinline__ void film_pixel(const RenderParams& P, uint32_t idx) 
         const int32_t ylo = max(py + P.gy0, T.wy0), yhi = min(py + P.gy1, T.wy1 - 1);
         const int32_t xlo = max(px + P.gx0, T.wx0), xhi = min(px + P.gx1, T.wx1 - 1);
         const int32_t sw = P.sx1 - P.sx0;
+        const float xw = P.filter_xw, yw = P.filter_yw, ixw = P.filter_inv_xw, iyw = P.filter_inv_yw;
+        const uint32_t spp = P.spp;
+        const bool flat = P.filter_flat != 0;  // a box filter: every weight is 1
+        const float fpx = (float)px, fpy = (float)py;
+        const bool small = max(abs(px), abs(py)) < (1 << 22);
+        // p in [ceil(a), floor(b)]
+        auto lands = [&](int32_t p, float fp, float a, float b) {
+            return small ? fp >= a && fp <= b : p >= dev_f2i32(ceilf(a)) && p <= dev_f2i32(floorf(b));
+        };
         for (int32_t sy = ylo; sy <= yhi; ++sy)
             for (int32_t sx = xlo; sx <= xhi; ++sx) {
                 const uint64_t sp = (uint64_t)(sy - P.sy0) * (uint64_t)sw + (uint64_t)(sx - P.sx0);
-                // The landing bounds below are non-decreasing in the sample
+                // The landing bounds are non-decreasing in the sample
                 // position, so if the source pixel's extreme samples cannot
                 // land on (px, py), none of its samples can.
                 const float4 bb = P.pixbox[sp];
-                if (dev_f2i32(floorf((bb.z - 0.5f) + P.filter_xw)) < px ||
-                    dev_f2i32(ceilf((bb.x - 0.5f) - P.filter_xw)) > px ||
-                    dev_f2i32(floorf((bb.w - 0.5f) + P.filter_yw)) < py ||
-                    dev_f2i32(ceilf((bb.y - 0.5f) - P.filter_yw)) > py)
+                if (!lands(px, fpx, (bb.x - 0.5f) - xw, (bb.z - 0.5f) + xw) ||
+                    !lands(py, fpy, (bb.y - 0.5f) - yw, (bb.w - 0.5f) + yw))
                     continue;
-                const uint64_t base = sp * P.spp;
-                for (uint32_t i = 0; i < P.spp; ++i) {
+                const uint64_t base = sp * spp;
+                for (uint32_t i = 0; i < spp; ++i) {
                     const float2 im = P.img[base + i];
-                    // film.rs:198-210 against the task film's extent
-                    float dix = im.x - 0.5f, diy = im.y - 0.5f;
-                    int32_t x0 = max(T.fx0, dev_f2i32(ceilf(dix - P.filter_xw)));
-                    int32_t x1 = min(T.fx1 - 1, dev_f2i32(floorf(dix + P.filter_xw)));
-                    int32_t y0 = max(T.fy0, dev_f2i32(ceilf(diy - P.filter_yw)));
-                    int32_t y1 = min(T.fy1 - 1, dev_f2i32(floorf(diy + P.filter_yw)));
-                    if ((x1 - x0) < 0 || (y1 - y0) < 0) continue;
-                    if (px < x0 || px > x1 || py < y0 || py > y1) continue;
+                    const float dix = im.x - 0.5f, diy = im.y - 0.5f;
+                    if (!lands(px, fpx, dix - xw, dix + xw) || !lands(py, fpy, diy - yw, diy + yw)) continue;
                     const float4 Ls = P.L[base + i];
                     float sx3[3];
                     rgb_to_xyz(Ls.x, Ls.y, Ls.z, sx3);
-                    float fx = ((float)px - dix) * P.filter_inv_xw * 16.0f;
-                    float fy = ((float)py - diy) * P.filter_inv_yw * 16.0f;
-                    int ix = min(dev_f2i32(floorf(fabsf(fx))), 15);
-                    int iy = min(dev_f2i32(floorf(fabsf(fy))), 15);
-                    float w = P.filter_table[iy * 16 + ix];
+                    float w = 1.0f;
+                    if (!flat) {
+                        float fx = (fpx - dix) * ixw * 16.0f;
+                        float fy = (fpy - diy) * iyw * 16.0f;
+                        int ix = min(dev_f2i32(floorf(fabsf(fx))), 15);
+                        int iy = min(dev_f2i32(floorf(fabsf(fy))), 15);
+                        w = P.filter_table[iy * 16 + ix];
+                    }
                     xyz[0] += w * sx3[0];
                     xyz[1] += w * sx3[1];
                     xyz[2] += w * sx3[2];
