@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 1024 / BLOCK : 1) kb_trace_flat(
                     const int st = T.start(bv, __ldg(src), __ldg(src + 1));
                     if (st == kStartWalk) T.run(bv, sh, ov);
                     if (T.spilled < 0) atomicMax(status, 6);
-                    *exact = st == kStartExact || T.give_up;
+                    *exact = st == kStartExact || T.gave_up();
                 };
                 bool exact;
                 if (any) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) kb_trace4_refill(BatchArg
                 T.leaf(bv, sh, ov);
                 if (MODE == kPerJob && any && T.found()) T.stop();
             }
-            if (T.cur == kWalkDone && !T.resume(ov)) finish(!any && T.give_up);
+            if (T.cur == kWalkDone && !T.resume(ov)) finish(T.gave_up());
         }
     }
 }

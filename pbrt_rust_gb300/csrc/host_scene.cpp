@@ -520,7 +520,7 @@ static void fill_quad_layout(HostBVH& H) {
     H.n_quads = 0;
     H.quad_root = 0;
     H.stack4_bound = 0;
-    H.reach = 0.0f;
+    H.reach = 8.8817842e-16f;  // 2^-50: the margins stay normal numbers (trace4.cuh)
     for (const HostBVH& I : H.insts) H.wide = H.wide && I.wide;
     if (m == 0) return;
     const Box& rb = H.nodes[0].box;

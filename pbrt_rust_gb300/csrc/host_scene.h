@@ -154,7 +154,7 @@ struct HostBVH {
     // the tree has the 4-wide layout: every coordinate is finite and at most
     // kWideReach away from the origin
     bool wide = false;
-    float reach = 0.0f;          // 5/4 of the largest coordinate of the root's box
+    float reach = 0.0f;          // 5/4 of the largest coordinate of the root's box, 2^-50 at least
     uint32_t stack4_bound = 0;  // most entries a 4-wide traversal can defer
     // instance definitions: one BVH each, shared by all their instances
     std::vector<HostBVH> insts;

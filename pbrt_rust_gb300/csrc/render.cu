@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) k_shadow_packet(RenderParams P) {
 
 // The first per_warp lanes of each warp have a ray (rays_per_warp).
 template <int OVF, bool INST>
-__global__ void __launch_bounds__(128) k_shadow4(const __grid_constant__ RenderParams P, uint32_t per_warp) {
+__global__ void __launch_bounds__(128, INST ? 6 : 9) k_shadow4(const __grid_constant__ RenderParams P, uint32_t per_warp) {
     using Walk = Walk4<128, 16, OVF, true, INST>;
     __shared__ typename Walk::Shared sh;
     sh.init();
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(128) k_shadow4(const __grid_constant__ RenderP
     const int st = T.start(P.bvh4, ray[0], ray[1]);
     if (st == kStartWalk) T.run(P.bvh4, sh, ov);
     if (T.spilled < 0) atomicMax(status, 6);
-    P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.give_up ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
+    P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
 }
 
 // --------------------------------------------------------------- combine ---

@@ -137,9 +137,12 @@ constexpr int kWalkBlock = 128;  // threads per block and stack rows of the 4-wi
 constexpr int kWalkRows = 16;
 
 // 4-wide traversal, one thread per ray; the first per_warp lanes of each warp
-// have one (rays_per_warp).
+// have one (rays_per_warp).  Blocks per SM: what the registers allow without
+// spills (any hit, 8 / 9 / 10 blocks on a terrain frame's shadow rays: 2594 /
+// 2553 / 2844 us; closest hit, 7 / 8 / 9 on its camera rays: 1916 / 1899 /
+// 1935).
 template <int OVF, bool ANY, bool INST>
-__global__ void __launch_bounds__(kWalkBlock) k_trace4(const __grid_constant__ DevBVH4 bvh,
+__global__ void __launch_bounds__(kWalkBlock, INST ? 6 : (ANY ? 9 : 8)) k_trace4(const __grid_constant__ DevBVH4 bvh,
                                                        const float4* __restrict__ rays, uint32_t n,
                                                        const uint32_t* __restrict__ order, float4* __restrict__ hits,
                                                        uint8_t* __restrict__ occ, int* __restrict__ status,
@@ -160,9 +163,9 @@ __global__ void __launch_bounds__(kWalkBlock) k_trace4(const __grid_constant__ D
     if (st == kStartWalk) T.run(bvh, sh, ov);
     if (T.spilled < 0) atomicMax(status, 6);
     if (ANY)
-        occ[i] = (st == kStartExact || T.give_up ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
+        occ[i] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
     else
-        hits[i] = st == kStartExact || T.give_up ? exact_hit<OVF + 8, INST>(bvh.pair, ray, status) : T.hit_record();
+        hits[i] = st == kStartExact || T.gave_up() ? exact_hit<OVF + 8, INST>(bvh.pair, ray, status) : T.hit_record();
 }
 
 // A ray is read once: its lines go to L2 only, leaving L1 to the tree.
@@ -272,7 +275,6 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : 8)
     bool more = work != nullptr;  // the shared counter may still hold rays
     const uint32_t kNone = 0xffffffffu;
     uint32_t ray = kNone;
-    bool overflow = false;
     Walk T;
     typename Walk::Ovf ov;
     T.bind(sh);
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : 8)
     };
     // The lane's ray ends with what T found, or marked for the replay.
     auto finish = [&](bool exact) {
-        if (T.spilled < 0) overflow = true;
+        if (T.spilled < 0) atomicMax(status, 6);
         if (exact) *replay = 1u;
         if (ANY) {
             occ[ray] = exact ? kReplayOcc : (T.found() ? 1 : 0);
@@ -400,10 +402,9 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : 8)
         for (int k = 0; k < kNodeSteps; ++k)
             if ((int32_t)T.cur >= 0) T.node(bvh, ov);
         if ((int32_t)T.cur < 0 && T.cur != kWalkDone) T.leaf(bvh, sh, ov);
-        if (T.cur == kWalkDone && ray != kNone && !T.resume(ov)) finish(T.give_up);
+        if (T.cur == kWalkDone && ray != kNone && !T.resume(ov)) finish(T.gave_up());
     }
     write_out();
-    if (overflow) atomicMax(status, 6);
 }
 
 enum {

@@ -62,6 +62,9 @@
 // whether they hit children or not.  Against ordering the children by
 // compare-and-swap and branching per push, a visit is about 110 instructions
 // instead of 210 (2^20 rays into 4096 random triangles: 524 -> 405 us).
+// Registers are what the walk is short of (64 at 8 blocks per SM): a thread's
+// rows follow from the top's address, and a ray that has to give up is one
+// whose maxt is NaN.
 // INST: the tree may hold instance records (kernels take it only for scenes
 // that have instances).
 #pragma once
@@ -78,7 +81,7 @@ struct DevBVH4 {
     const QuadNode* nodes;
     const LeafBox* boxes;
     uint32_t root_ref;      // the root's child word
-    float reach;            // 5/4 of the tree's largest coordinate
+    float reach;            // 5/4 of the tree's largest coordinate, 2^-50 at least
 };
 
 // Stack words that are not children (leaf words stay below: HostBVH::wide
@@ -174,13 +177,13 @@ __device__ __forceinline__ void ld_entry(uint32_t addr, uint32_t& ref, float& t)
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(ref), "=f"(t) : "r"(addr) : "memory");
 }
 
-// The push table: entry [code][mask], byte k = rows above the top at which
-// child k goes (the child visited first on top; children not in the mask
-// above them all).  code: bit 0 / 1 = the first / second pair's children swap
-// places, bit 2 = the pairs do.
+// The push table: entry [code][fails], byte k = rows above the top at which
+// child k goes (the child visited first on top; children whose box failed,
+// bit 3 - k of `fails`, above them all).  code: bit 0 / 1 = the first / second
+// pair's children swap places, bit 2 = the pairs do.
 constexpr int kPushTable = 128;
 __device__ __forceinline__ uint32_t push_entry(uint32_t i) {
-    const uint32_t code = i >> 4, mask = i & 15u;
+    const uint32_t code = i >> 4, mask = (__brev(i) >> 28) ^ 15u;  // bit k: child k passed
     auto place = [&](uint32_t k) {  // of child k among the four
         const uint32_t pair = k >> 1;
         return ((pair ^ (code >> 2)) << 1) | ((k & 1u) ^ ((code >> pair) & 1u));
@@ -194,17 +197,20 @@ __device__ __forceinline__ uint32_t push_entry(uint32_t i) {
     }
     return e;
 }
+// The rows that stay on the stack.
+__device__ __forceinline__ uint32_t push_rows(uint32_t i) { return 4u - (uint32_t)__popc(i & 15u); }
 
 // Shared memory of a block of 4-wide walks: the stacks, the push table and,
 // with instances, the world rays of the lanes that are inside one.
 template <int BLOCK, int ROWS, bool INST>
 struct alignas(16) WalkShared {
     uint2 stack[ROWS][BLOCK];
-    uint32_t push[kPushTable];
+    uint2 push[kPushTable];  // the places; by how much the top moves
     float world[INST ? 9 : 1][INST ? BLOCK : 1];
     // every thread of the block; __syncthreads() inside
     __device__ __forceinline__ void init() {
-        if (threadIdx.x < kPushTable) push[threadIdx.x] = push_entry(threadIdx.x);
+        if (threadIdx.x < kPushTable)
+            push[threadIdx.x] = make_uint2(push_entry(threadIdx.x), push_rows(threadIdx.x) * (BLOCK * 8u));
         __syncthreads();
     }
 };
@@ -250,16 +256,21 @@ struct Walk4 : InstWalk<INST> {
     uint32_t cur;
     uint32_t top;      // shared-memory address of the first free row
     int spilled;       // entries in the overflow; -1: they would not fit (reported, never written)
-    int32_t prim;
+    int32_t prim;      // -1: none yet
     float b1, b2;
-    bool give_up;      // a hit at distance NaN or an instance ray that is not clean: the ray needs the exact walk
-    uint32_t bottom, push_tab;
+    uint32_t base, push_tab;  // shared-memory addresses, the same for all threads
 
     __device__ __forceinline__ void bind(Shared& sh) {
-        bottom = (uint32_t)__cvta_generic_to_shared(&sh.stack[0][threadIdx.x]);
+        base = (uint32_t)__cvta_generic_to_shared(sh.stack);
         push_tab = (uint32_t)__cvta_generic_to_shared(sh.push);
-        st_entry(bottom, kWalkDone, __int_as_float(0xff800000));  // -inf: always taken
+        top = base + threadIdx.x * 8u;
+        st_entry(top, kWalkDone, __int_as_float(0xff800000));  // -inf: always taken
         cur = kWalkDone;
+    }
+
+    // Row i of this thread, from the top's address, which is in one of its rows.
+    __device__ __forceinline__ uint32_t row(int i) const {
+        return base + ((top - base) & (kRow - 1u)) + (uint32_t)i * kRow;
     }
 
     // 1 / d, octant and margins of the ray (o, d) in a tree of the given
@@ -312,7 +323,7 @@ struct Walk4 : InstWalk<INST> {
         ox = a.x;
         oy = a.y;
         oz = a.z;
-        tmin = a.w;
+        tmin = a.w == 0.0f ? -0.0f : a.w;  // node(): an entry at +0 would fail against an exit at -0
         dx = b.x;
         dy = b.y;
         dz = b.z;
@@ -320,9 +331,8 @@ struct Walk4 : InstWalk<INST> {
         prim = -1;
         b1 = 0.0f;
         b2 = 0.0f;
-        give_up = false;
         spilled = 0;
-        top = bottom + kRow;
+        top = row(1);
         if constexpr (INST) {
             this->nodes_ = bvh.nodes;
             this->prims_ = bvh.pair.prims;
@@ -345,20 +355,20 @@ struct Walk4 : InstWalk<INST> {
 
     // Moves the oldest rows to the overflow when fewer than four are free.
     __device__ __forceinline__ void make_room(Ovf& ov) {
-        if (top <= bottom + (ROWS - 4) * kRow) return;
+        if (top < base + (ROWS - 3) * kRow) return;
         if (spilled < 0 || spilled + kSpill > OVF) {
             spilled = -1;
-            top = bottom + kRow;  // the pop that follows ends the walk
+            top = row(1);  // the pop that follows ends the walk
             return;
         }
         for (int i = 0; i < kSpill; ++i) {
             uint32_t ref;
             float t;
-            ld_entry(bottom + (uint32_t)(1 + i) * kRow, ref, t);
+            ld_entry(row(1 + i), ref, t);
             ov.e[spilled + i] = make_uint2(ref, __float_as_uint(t));
         }
         spilled += kSpill;
-        for (uint32_t a = bottom + (1 + kSpill) * kRow; a < top; a += kRow) {
+        for (uint32_t a = row(1 + kSpill); a < top; a += kRow) {
             uint32_t ref;
             float t;
             ld_entry(a, ref, t);
@@ -380,13 +390,24 @@ struct Walk4 : InstWalk<INST> {
         if (spilled <= 0) return false;
         spilled -= kSpill;
         for (int i = 0; i < kSpill; ++i)
-            st_entry(bottom + (uint32_t)(1 + i) * kRow, ov.e[spilled + i].x, __uint_as_float(ov.e[spilled + i].y));
-        top = bottom + (1 + kSpill) * kRow;
+            st_entry(row(1 + i), ov.e[spilled + i].x, __uint_as_float(ov.e[spilled + i].y));
+        top = row(1 + kSpill);
         pop();
         return true;
     }
 
-    // Visits inner node `cur`.
+    // Visits inner node `cur`.  The integer pipe is the busiest (69 % with
+    // issue at 77 % on camera rays of a terrain frame; the byte permutes,
+    // minima and selects run there), so a child's failing is the sign bit of
+    // exit - entry, shifted into the table index (the sign is wrong only for
+    // an exit at -0, a hit's or the ray's maxt, and an entry at +0, which
+    // cannot be: tmin is not +0 and a near plane at +0 less the margin is
+    // beyond -0 without it), and its row's address one
+    // 16-bit dot product, which the multiply pipe does; the table also holds
+    // how far the top moves (a population count otherwise).  Against
+    // compares, a mask, permutes and multiplies: terrain frame's camera /
+    // shadow rays 1945 / 2692 -> 1899 / 2594 us, shadow rays at 56 registers
+    // (9 blocks per SM) 2553.
     __device__ __forceinline__ void node(const DevBVH4& bvh, Ovf& ov) {
         const QuadNode* nodes;
         if constexpr (INST)
@@ -408,7 +429,7 @@ struct Walk4 : InstWalk<INST> {
         const uint64_t bz = pack2(__fmaf_rn(gz, iz, -ez), __fmaf_rn(gz, iz, ez));
         const uint64_t ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
         float t[4];
-        uint32_t mask = 0;
+        uint32_t index = q0.w[5] >> oct3;  // the visiting order, then a bit per child: not passed
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             float n0, f0, n1, f1, n2, f2;
@@ -417,22 +438,22 @@ struct Walk4 : InstWalk<INST> {
             unpack2(fma2(pack2(plane(nz, k), plane(fz, k)), az2, bz), n2, f2);
             t[k] = max3f(n0, n1, fmaxf(n2, tmin));
             const float t1 = min3f(f0, f1, fminf(f2, maxt));
-            if (!(t[k] > t1)) mask |= 1u << k;
+            index = __funnelshift_l(__float_as_uint(t1 - t[k]), index, 1);
         }
-        const uint32_t code = (q0.w[5] >> oct3) & 7u;
-        uint32_t e;
-        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e) : "r"(push_tab + (code * 16u + mask) * 4u));
-#pragma unroll
-        for (int k = 0; k < 4; ++k) st_entry(top + kRow * __byte_perm(e, 0u, 0x4440u | (uint32_t)k), q1.w[4 + k], t[k]);
-        top += kRow * (uint32_t)__popc(mask);
+        uint32_t e, up;
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(e), "=r"(up) : "r"(push_tab + (index & 127u) * 8u));
+        st_entry(__dp2a_lo(kRow, e, top), q1.w[4], t[0]);
+        st_entry(__dp2a_lo(kRow << 16, e, top), q1.w[5], t[1]);
+        st_entry(__dp2a_hi(kRow, e, top), q1.w[6], t[2]);
+        st_entry(__dp2a_hi(kRow << 16, e, top), q1.w[7], t[3]);
+        top += up;
         make_room(ov);
         pop();
     }
 
     // Hit at t of primitive word `id`.
     __device__ __forceinline__ void accept(uint32_t id, float t, float u, float v) {
-        maxt = t;
-        give_up |= !(t == t);
+        maxt = ANY || maxt == maxt ? t : maxt;  // NaN stays: gave_up()
         if constexpr (INST)
             prim = (int32_t)(this->base_ + (id & ~kSphereBit));
         else
@@ -563,7 +584,7 @@ struct Walk4 : InstWalk<INST> {
                                             (flags & kPrimLastBit) ? 0u : (kNode4Leaf | (off + 1)));
                         if (e == 1) return make_room(ov);
                         if (e == 2) {
-                            give_up = true;
+                            maxt = __int_as_float(0x7fc00000);  // gave_up()
                             return stop();
                         }
                         if (flags & kPrimLastBit) break;
@@ -607,6 +628,9 @@ struct Walk4 : InstWalk<INST> {
             if (cur == kWalkDone && !resume(ov)) return;
         }
     }
+    // A closest hit at distance NaN, or an instance ray that was not clean:
+    // the ray needs the exact walk.
+    __device__ __forceinline__ bool gave_up() const { return !(maxt == maxt); }
     __device__ __forceinline__ bool found() const { return prim >= 0; }
     __device__ __forceinline__ float4 hit_record() const {
         return make_float4(__int_as_float(prim), prim >= 0 ? maxt : 0.0f, b1, b2);
