@@ -642,6 +642,48 @@ struct ANode {
     Box box{};
 };
 
+// A phase-A node, at its place in the tree.
+struct TopNode {
+    uint32_t at;
+    FlatNode node;
+};
+
+// The small ranges' roots.
+__global__ void __launch_bounds__(128) k_b_roots(const PoolNode* __restrict__ pool, const Job* __restrict__ jobs,
+                                                 uint32_t njobs, PoolNode* __restrict__ roots) {
+    const uint32_t j = blockIdx.x * 128u + threadIdx.x;
+    if (j < njobs) roots[j] = pool[jobs[j].node0];
+}
+
+// Every node in the reference's depth-first order: a small range's nodes
+// start at at[job], one warp each (on the host, from the downloaded pool,
+// this took 1.4 ms for 180000 triangles).
+__global__ void __launch_bounds__(128) k_number(const PoolNode* __restrict__ pool, const Job* __restrict__ jobs,
+                                                const JobOut* __restrict__ outs, const uint32_t* __restrict__ at,
+                                                uint32_t njobs, const TopNode* __restrict__ top, uint32_t ntop,
+                                                FlatNode* __restrict__ nodes) {
+    const uint64_t t = (uint64_t)blockIdx.x * 128u + threadIdx.x;
+    if (t < ntop) nodes[top[t].at] = top[t].node;
+    const uint64_t j = t >> 5;
+    if (j >= njobs) return;
+    const uint32_t base = at[j], count = outs[j].nodes;
+    const PoolNode* p = pool + jobs[j].node0;
+    for (uint32_t k = threadIdx.x & 31u; k < count; k += 32u) {
+        const PoolNode q = p[k];
+        FlatNode f;
+        f.box = Box{V3{q.lo[0], q.lo[1], q.lo[2]}, V3{q.hi[0], q.hi[1], q.hi[2]}};
+        f.leaf = (q.b & kLeaf) != 0;
+        f.offset = f.leaf ? q.a : base + q.a;
+        f.count = f.leaf ? q.b & ~kLeaf : q.b;
+        nodes[base + k] = f;
+    }
+}
+
+// Trees of at least this many primitives get their layout on the device,
+// unless a range beyond kSmall primitives could not be split: one thread
+// writes a leaf.
+constexpr size_t kDeviceLayoutMin = 16384;
+
 }  // namespace
 
 int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
@@ -800,18 +842,20 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         j.node0 = (uint32_t)pool_nodes;
         pool_nodes += 2ull * (j.hi - j.lo) - 1;
     }
-    Buf d_jobs, d_outs;
+    Buf d_jobs, d_outs, d_roots;
     CK(cudaMalloc(&d_pool.p, pool_nodes * sizeof(PoolNode)));
     CK(cudaMalloc(&d_jobs.p, (size_t)NJ * sizeof(Job)));
     CK(cudaMalloc(&d_outs.p, (size_t)NJ * sizeof(JobOut)));
+    CK(cudaMalloc(&d_roots.p, (size_t)NJ * sizeof(PoolNode)));
     CK(cudaMemcpy(d_jobs.p, jobs.data(), (size_t)NJ * sizeof(Job), cudaMemcpyHostToDevice));
     k_b_build<<<(NJ + kBWarps - 1) / kBWarps, 32 * kBWarps>>>(P, d_idx.as<uint32_t>(), d_jobs.as<Job>(), NJ,
                                                               d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp, split);
+    k_b_roots<<<(NJ + 127) / 128, 128>>>(d_pool.as<PoolNode>(), d_jobs.as<Job>(), NJ, d_roots.as<PoolNode>());
     CK(cudaGetLastError());
     std::vector<JobOut> outs(NJ);
-    RawVec<PoolNode> pool(pool_nodes);
+    std::vector<PoolNode> roots(NJ);
     CK(cudaMemcpy(outs.data(), d_outs.p, (size_t)NJ * sizeof(JobOut), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(pool.data(), d_pool.p, pool_nodes * sizeof(PoolNode), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(roots.data(), d_roots.p, (size_t)NJ * sizeof(PoolNode), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(H.ordered.data(), d_idx.p, n * 4, cudaMemcpyDeviceToHost));
     for (const JobOut& o : outs)
         if (o.err) {
@@ -827,7 +871,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         const ANode& a = A[i];
         if (a.small) {
             size[i] = outs[a.job].nodes;
-            const PoolNode& r = pool[jobs[a.job].node0];
+            const PoolNode& r = roots[a.job];
             abox[i] = Box{v3(r.lo[0], r.lo[1], r.lo[2]), v3(r.hi[0], r.hi[1], r.hi[2])};
         } else if (a.leaf) {
             size[i] = 1;
@@ -837,23 +881,24 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
             abox[i] = box_union(abox[a.left], abox[a.right]);  // bvh.rs:247
         }
     }
-    H.nodes.resize(size[0]);
     struct Item {
         uint32_t a;
         uint64_t at;
     };
-    std::vector<uint64_t> job_at(NJ);  // first node of each small range
+    std::vector<uint32_t> job_at(NJ);  // first node of each small range
+    std::vector<TopNode> top;
     std::vector<Item> todo{{0, 0}};
     while (!todo.empty()) {
         const Item it = todo.back();
         todo.pop_back();
         const ANode& a = A[it.a];
         if (a.small) {
-            job_at[a.job] = it.at;
+            job_at[a.job] = (uint32_t)it.at;
             H.depth = std::max(H.depth, a.depth + outs[a.job].depth - 1);
             continue;
         }
-        FlatNode& f = H.nodes[it.at];
+        top.push_back(TopNode{(uint32_t)it.at, FlatNode{}});
+        FlatNode& f = top.back().node;
         f.box = abox[it.a];
         H.depth = std::max(H.depth, a.depth);
         if (a.leaf) {
@@ -869,28 +914,26 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         todo.push_back(Item{(uint32_t)a.right, right_at});
         todo.push_back(Item{(uint32_t)a.left, it.at + 1});
     }
-    // the ranges' nodes, cut at equal numbers of primitives
-    std::vector<uint32_t> order(NJ);
-    for (uint32_t j = 0; j < NJ; ++j) order[j] = j;
-    std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return jobs[x].lo < jobs[y].lo; });
-    host_parallel(n, [&](size_t, size_t from, size_t to) {
-        auto first = [&](size_t prim) {
-            return std::lower_bound(order.begin(), order.end(), prim,
-                                    [&](uint32_t j, size_t p) { return jobs[j].lo < p; });
-        };
-        for (auto i = first(from), e = first(to); i != e; ++i) {
-            const Job& J = jobs[*i];
-            const uint64_t at = job_at[*i];
-            for (uint32_t k = 0; k < outs[*i].nodes; ++k) {
-                const PoolNode& p = pool[J.node0 + k];
-                FlatNode& f = H.nodes[at + k];
-                f.box = Box{v3(p.lo[0], p.lo[1], p.lo[2]), v3(p.hi[0], p.hi[1], p.hi[2])};
-                f.leaf = (p.b & kLeaf) != 0;
-                f.offset = f.leaf ? p.a : (uint32_t)(at + p.a);
-                f.count = f.leaf ? (p.b & ~kLeaf) : p.b;
-            }
-        }
-    });
+    const uint32_t m = (uint32_t)size[0];
+    for (Buf* b : {&d_lo, &d_hi, &d_c[0], &d_c[1], &d_c[2], &d_tmp}) b->reset();  // room for the nodes
+    Buf d_nodes, d_at, d_top;
+    CK(cudaMalloc(&d_nodes.p, (size_t)m * sizeof(FlatNode)));
+    CK(cudaMalloc(&d_at.p, (size_t)NJ * 4));
+    CK(cudaMemcpy(d_at.p, job_at.data(), (size_t)NJ * 4, cudaMemcpyHostToDevice));
+    if (!top.empty()) {
+        CK(cudaMalloc(&d_top.p, top.size() * sizeof(TopNode)));
+        CK(cudaMemcpy(d_top.p, top.data(), top.size() * sizeof(TopNode), cudaMemcpyHostToDevice));
+    }
+    const size_t threads = std::max<size_t>(32 * (size_t)NJ, top.size());
+    k_number<<<(unsigned)((threads + 127) / 128), 128>>>(d_pool.as<PoolNode>(), d_jobs.as<Job>(), d_outs.as<JobOut>(),
+                                                         d_at.as<uint32_t>(), NJ, d_top.as<TopNode>(),
+                                                         (uint32_t)top.size(), d_nodes.as<FlatNode>());
+    CK(cudaGetLastError());
+    H.nodes.resize(m);
+    CK(cudaMemcpy(H.nodes.data(), d_nodes.p, (size_t)m * sizeof(FlatNode), cudaMemcpyDeviceToHost));
+    const bool big_leaf = std::any_of(top.begin(), top.end(), [](const TopNode& t) { return t.node.leaf; });
+    d_pool.reset();
+    if (n >= kDeviceLayoutMin && !big_leaf) device_fill_layout(H, d_nodes.as<FlatNode>(), m, d_idx.as<uint32_t>());
     return PBRT_OK;
 }
 

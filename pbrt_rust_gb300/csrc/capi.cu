@@ -127,38 +127,62 @@ static DevBVH4 device_tree(const HostBVH& H, const NodePair* pairs, const QuadNo
     return d;
 }
 
+// A tree's layout arrays on `device`: those it was built with, or uploaded
+// from the host's.
+struct TreeArrays {
+    NodePair* pairs = nullptr;
+    PrimRec* prims = nullptr;
+    LeafBox* boxes = nullptr;
+    QuadNode* quads = nullptr;
+};
+static int tree_arrays(HostBVH& H, int device, TreeArrays* out) {
+    if (H.layout && H.layout->device == device) {
+        *out = TreeArrays{H.layout->pairs, H.layout->prims, H.layout->boxes, H.layout->quads};
+        return PBRT_OK;
+    }
+    if (H.layout) {
+        try {
+            fill_host_layout(H);
+        } catch (const std::bad_alloc&) {
+            return set_error(PBRT_ERR_OUT_OF_MEMORY, "host memory for the tree's layout");
+        }
+        H.layout.reset();
+    }
+    int st;
+    if ((st = upload(&out->pairs, H.pairs)) || (st = upload(&out->prims, H.recs)) ||
+        (st = upload(&out->boxes, H.leaf_boxes)))
+        return st;
+    return make_quads(H, out->pairs, &out->quads);
+}
+
 int bvh_upload(PbrtBVH* b) {
     std::lock_guard<std::mutex> lk(b->upload_mu);
     if (b->uploaded) return PBRT_OK;
     int st;
     if ((st = cuda_status(cudaGetDevice(&b->device), "cudaGetDevice"))) return st;
-    if ((st = upload(&b->d_pairs, b->host.pairs))) return st;
-    if ((st = upload(&b->d_prims, b->host.recs))) return st;
+    TreeArrays tree;
+    st = tree_arrays(b->host, b->device, &tree);
+    b->d_pairs = tree.pairs;
+    b->d_prims = tree.prims;
+    b->d_leaf_boxes = tree.boxes;
+    b->d_quads = tree.quads;
+    if (st) return st;
     if ((st = upload(&b->d_spheres, b->host.spheres))) return st;
-    if ((st = upload(&b->d_leaf_boxes, b->host.leaf_boxes))) return st;
-    if ((st = make_quads(b->host, b->d_pairs, &b->d_quads))) return st;
     if ((st = cuda_status(cudaMalloc(&b->d_status, sizeof(int)), "cudaMalloc"))) return st;
     if ((st = cuda_status(cudaMemset(b->d_status, 0, sizeof(int)), "cudaMemset"))) return st;
     // instance definitions
     std::vector<DevBVH4> defs;
-    for (const HostBVH& I : b->host.insts) {
-        NodePair* pairs = nullptr;
-        QuadNode* quads = nullptr;
-        LeafBox* boxes = nullptr;
-        PrimRec* prims = nullptr;
+    for (HostBVH& I : b->host.insts) {
+        TreeArrays t;
         SphereRec* spheres = nullptr;
-        st = upload(&pairs, I.pairs);
-        if (pairs) b->d_inst_bufs.push_back(pairs);
-        if (!st) st = make_quads(I, pairs, &quads);
-        if (quads) b->d_inst_bufs.push_back(quads);
-        if (!st) st = upload(&boxes, I.leaf_boxes);
-        if (boxes) b->d_inst_bufs.push_back(boxes);
-        if (!st) st = upload(&prims, I.recs);
-        if (prims) b->d_inst_bufs.push_back(prims);
+        st = tree_arrays(I, b->device, &t);
+        if (!I.layout)  // its own arrays otherwise
+            for (void* p : {(void*)t.pairs, (void*)t.quads, (void*)t.boxes, (void*)t.prims})
+                if (p) b->d_inst_bufs.push_back(p);
         if (!st) st = upload(&spheres, I.spheres);
         if (spheres) b->d_inst_bufs.push_back(spheres);
         if (st) return st;
-        defs.push_back(device_tree(I, pairs, quads, boxes, prims, spheres, nullptr));
+        defs.push_back(device_tree(I, t.pairs, t.quads, t.boxes, t.prims, spheres, nullptr));
     }
     b->inst_dev = defs;
     if ((st = upload(&b->d_insts, defs))) return st;
@@ -580,11 +604,13 @@ PbrtBVH::~PbrtBVH() {
     if (h_one) cudaFreeHost(h_one);
     for (void* p : d_inst_bufs) cudaFree(p);
     if (d_insts) cudaFree(d_insts);
-    if (d_pairs) cudaFree(d_pairs);
-    if (d_prims) cudaFree(d_prims);
+    if (!host.layout) {  // which has its own
+        if (d_pairs) cudaFree(d_pairs);
+        if (d_prims) cudaFree(d_prims);
+        if (d_quads) cudaFree(d_quads);
+        if (d_leaf_boxes) cudaFree(d_leaf_boxes);
+    }
     if (d_spheres) cudaFree(d_spheres);
-    if (d_quads) cudaFree(d_quads);
-    if (d_leaf_boxes) cudaFree(d_leaf_boxes);
     if (d_status) cudaFree(d_status);
     stage_in.release();
     stage_out.release();
@@ -690,8 +716,10 @@ int pbrtgpu_bvh_device_bytes(const PbrtBVH* b, uint64_t* bytes) {
     if (!b || !bytes) return set_error(PBRT_ERR_INVALID_ARGUMENT, "NULL argument");
     const HostBVH& H = b->host;
     auto tree = [](const HostBVH& T) -> uint64_t {
-        return T.pairs.size() * sizeof(NodePair) + (T.wide ? (uint64_t)T.n_quads * sizeof(QuadNode) : 0) +
-               T.leaf_boxes.size() * sizeof(LeafBox) + T.recs.size() * sizeof(PrimRec) +
+        const size_t pairs = T.layout ? T.layout->n_pairs : T.pairs.size();
+        const size_t boxes = T.layout ? T.layout->n_boxes : T.leaf_boxes.size();
+        return pairs * sizeof(NodePair) + (T.wide ? (uint64_t)T.n_quads * sizeof(QuadNode) : 0) +
+               boxes * sizeof(LeafBox) + (T.ordered.size() + 1) * sizeof(PrimRec) +
                T.spheres.size() * sizeof(SphereRec);
     };
     uint64_t n = tree(H) + sizeof(int);

@@ -512,21 +512,24 @@ static void fill_device_layout(HostBVH& H) {
     }
 }
 
+void tree_reach(HostBVH& H) {
+    H.reach = 8.8817842e-16f;  // 2^-50: the margins stay normal numbers (trace4.cuh)
+    H.quad_root = 0;
+    if (H.nodes.empty()) return;
+    const Box& rb = H.nodes[0].box;
+    for (float v : {rb.lo.x, rb.lo.y, rb.lo.z, rb.hi.x, rb.hi.y, rb.hi.z}) H.reach = std::max(H.reach, 1.25f * std::fabs(v));
+    if (H.nodes[0].leaf) H.quad_root = kNode4Leaf | H.nodes[0].offset;
+}
+
 // Where the 4-wide nodes start (two binary levels each, see layout.h:
 // QuadNode).
 static void fill_quad_layout(HostBVH& H) {
     const size_t m = H.nodes.size();
     H.quad_of.resize(H.pairs.size());
     H.n_quads = 0;
-    H.quad_root = 0;
     H.stack4_bound = 0;
-    H.reach = 8.8817842e-16f;  // 2^-50: the margins stay normal numbers (trace4.cuh)
-    for (const HostBVH& I : H.insts) H.wide = H.wide && I.wide;
-    if (m == 0) return;
-    const Box& rb = H.nodes[0].box;
-    for (float v : {rb.lo.x, rb.lo.y, rb.lo.z, rb.hi.x, rb.hi.y, rb.hi.z}) H.reach = std::max(H.reach, 1.25f * std::fabs(v));
-    H.quad_root = H.nodes[0].leaf ? (kNode4Leaf | H.nodes[0].offset) : 0u;
-    if (H.nodes[0].leaf) return;
+    tree_reach(H);
+    if (m == 0 || H.nodes[0].leaf) return;
     // pairs are numbered in pre-order, so a node's 4-wide start is decided
     // before its grandchildren's
     RawVec<uint32_t> deferred(H.pairs.size());       // entries the walk may hold above a start
@@ -552,6 +555,15 @@ static void fill_quad_layout(HostBVH& H) {
             }
         }
     }
+}
+
+void fill_host_layout(HostBVH& H) {
+    const bool wide = H.wide;  // as created: the definitions' limits are in them
+    const uint32_t bound = H.stack4_bound;
+    fill_device_layout(H);
+    fill_quad_layout(H);
+    H.wide = wide;
+    H.stack4_bound = bound;
 }
 
 int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_prims, const char* split_method,
@@ -733,8 +745,11 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
     int st = (on_device && split != PBRT_SPLIT_EQUAL) ? device_build_tree(H, max_prims, split, err)
                                                       : build_tree(H, max_prims, split, err);
     if (st) return st;
-    fill_device_layout(H);
-    fill_quad_layout(H);
+    if (!H.layout) {
+        fill_device_layout(H);
+        fill_quad_layout(H);
+    }
+    for (const HostBVH& I : H.insts) H.wide = H.wide && I.wide;
     if (!H.insts.empty()) {
         // the 4-wide walk enters a definition with two more entries (the
         // rest of the leaf, the exit word) on top of the scene's stack

@@ -132,13 +132,28 @@ struct FlatNode {
     uint32_t count;   // leaf: prim count; inner: axis
 };
 
+// A tree's arrays on the device where it was built (device_fill_layout).
+struct DeviceLayout {
+    int device = 0;
+    NodePair* pairs = nullptr;
+    PrimRec* prims = nullptr;
+    LeafBox* boxes = nullptr;
+    QuadNode* quads = nullptr;
+    size_t n_pairs = 0, n_boxes = 0;
+    DeviceLayout() = default;
+    DeviceLayout(const DeviceLayout&) = delete;
+    DeviceLayout& operator=(const DeviceLayout&) = delete;
+    ~DeviceLayout();
+};
+
 struct HostBVH {
     RawVec<HostPrim> prims;
     std::vector<SphereRec> spheres;
     RawVec<FlatNode> nodes;
     RawVec<uint32_t> ordered;  // ordered_prims: refined input index
     uint32_t depth = 0;
-    // device layout
+    // device layout: the arrays below, or `layout`, which has them on the device
+    std::shared_ptr<DeviceLayout> layout;
     ChildRec root{};
     RawVec<NodePair> pairs;
     RawVec<PrimRec> recs;
@@ -177,13 +192,25 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
                    HostBVH* out, std::string* err, bool on_device = false, const PbrtInstanceDesc* defs = nullptr,
                    uint32_t n_defs = 0);
 
+// H.reach and H.quad_root of the nodes.
+void tree_reach(HostBVH& H);
+
+// The layout arrays on the host (after build_host_bvh left them on a device).
+void fill_host_layout(HostBVH& H);
+
 // Bounds (mesh.rs:196-205, sphere.rs:111-126) and centroid (bvh.rs:77) of
 // refined primitive i.
 Box prim_bounds(const HostBVH& H, size_t i, V3* centroid);
 
 // The tree of build_tree (H.nodes, H.ordered, H.depth) built on the current
-// CUDA device (bvh_build.cu): identical nodes and primitive order.
+// CUDA device (bvh_build.cu): identical nodes and primitive order.  Larger
+// trees get their layout there too (H.layout).
 int device_build_tree(HostBVH& H, uint32_t max_prims, int split, std::string* err);
+
+// The layout of a tree whose nodes (m) and primitive order are on the current
+// device too, made there (quads.cu): the same arrays as fill_host_layout's.
+// Leaves H.layout null if the device's memory does not suffice.
+void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const uint32_t* d_ordered);
 
 int parse_split_method(const char* s);
 
