@@ -86,7 +86,7 @@ struct PbrtScene {
     float* d_area_cdf = nullptr;
     std::atomic<bool> uploaded{false};
     std::mutex mu;  // serialises renders: they share the scratch buffers below
-    pbrt::DeviceBuf rays, hits, img, pixbox, lsamp, contrib, L, srays, sslot, occ, counters, tasks, table, rgb;
+    pbrt::DeviceBuf rays, hits, img, pixbox, lsamp, contrib, L, srays, sslot, occ, counters, tasks, rgb;
     ~PbrtScene() {
         if (bvh) delete bvh;
         for (void* p : {(void*)d_shade, (void*)d_materials, (void*)d_lights, (void*)d_area_tris, (void*)d_area_cdf,
@@ -94,7 +94,7 @@ struct PbrtScene {
             if (p) cudaFree(p);
         for (void* p : d_inst_bufs) cudaFree(p);
         for (pbrt::DeviceBuf* b : {&rays, &hits, &img, &pixbox, &lsamp, &contrib, &L, &srays, &sslot, &occ, &counters,
-                                   &tasks, &table, &rgb})
+                                   &tasks, &rgb})
             b->release();
     }
 };

@@ -173,6 +173,7 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     P.filter_xw = cam->filter_x_width;
     P.filter_yw = cam->filter_y_width;
     P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
+    P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
     P.filter_inv_xw = 1.0f / cam->filter_x_width;
     P.filter_inv_yw = 1.0f / cam->filter_y_width;
     gather_offsets(cam->filter_x_width, P.sx0, P.sx1, &P.gx0, &P.gx1);
@@ -239,12 +240,12 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     Carve real{base, 0};
     layout(real);
 
-    // The scratch keeps the previous call's contents: the counters must
-    // start at zero; every other buffer is written before it is read.
-    if ((st = cuda_status(cudaMemsetAsync(p_cnt, 0, 64, s), "counters")) ||
-        (st = cuda_status(cudaMemcpyAsync(p_tasks, tasks, smp->num_tasks * sizeof(TaskRec), cudaMemcpyHostToDevice, s),
+    // The scratch keeps the previous call's contents: every buffer is written
+    // (the counters by the first kernel) before it is read.
+    if ((st = cuda_status(cudaMemcpyAsync(p_tasks, tasks, smp->num_tasks * sizeof(TaskRec), cudaMemcpyHostToDevice, s),
                           "tasks H2D")) ||
-        (st = cuda_status(cudaMemcpyAsync(p_table, table, sizeof(table), cudaMemcpyHostToDevice, s), "table H2D")))
+        (!P.filter_flat &&
+         (st = cuda_status(cudaMemcpyAsync(p_table, table, sizeof(table), cudaMemcpyHostToDevice, s), "table H2D"))))
         return st;
     P.filter_table = (const float*)p_table;
     P.tasks = (const TaskRec*)p_tasks;

@@ -584,8 +584,14 @@ int pbrtgpu_render_tasks(const PbrtScene* cS, const PbrtCameraDesc* cam, const P
     std::lock_guard<std::mutex> lk(S->mu);
     cudaStream_t s = (cudaStream_t)stream_v;
     const uint32_t nl = P.n_lights;
-    std::vector<float> table(256);
-    filter_table(*cam, table.data());  // kind checked by prepare_render
+    // the filter's table goes up behind the tasks, in one copy (a box filter's
+    // is not read)
+    const size_t task_bytes = smp->num_tasks * sizeof(TaskRec);
+    const size_t upload_bytes = task_bytes + (P.filter_flat ? 0 : 256 * 4);
+    if (!P.filter_flat) {
+        tasks.resize((upload_bytes + sizeof(TaskRec) - 1) / sizeof(TaskRec));
+        filter_table(*cam, reinterpret_cast<float*>(tasks.data() + smp->num_tasks));  // kind checked by prepare_render
+    }
 
     const uint64_t S_ = P.n_samples, SL = P.n_samples * (uint64_t)nl;
     const uint64_t npx = (uint64_t)(P.fx1 - P.fx0) * (uint64_t)(P.fy1 - P.fy0);
@@ -595,17 +601,14 @@ int pbrtgpu_render_tasks(const PbrtScene* cS, const PbrtCameraDesc* cam, const P
         (st = S->contrib.reserve(SL * 16 + 16)) || (st = S->L.reserve(S_ * 16)) ||
         (st = S->srays.reserve(SL * sizeof(PbrtRay) + 32)) || (st = S->sslot.reserve(SL * 4 + 4)) ||
         (st = S->occ.reserve(SL + 1)) || (st = S->counters.reserve(64)) ||
-        (st = S->tasks.reserve(tasks.size() * sizeof(TaskRec))) || (st = S->table.reserve(256 * 4)))
+        (st = S->tasks.reserve(upload_bytes)))
         return st;
     bool dev_out = is_device_pointer(rgb_out);
     if (!dev_out && (st = S->rgb.reserve(npx * 3 * 4))) return st;
-    if ((st = cuda_status(cudaMemcpyAsync(S->tasks.p, tasks.data(), tasks.size() * sizeof(TaskRec),
-                                          cudaMemcpyHostToDevice, s),
-                          "tasks H2D")) ||
-        (st = cuda_status(cudaMemcpyAsync(S->table.p, table.data(), 256 * 4, cudaMemcpyHostToDevice, s), "table H2D")) ||
-        (st = cuda_status(cudaMemsetAsync(S->counters.p, 0, 64, s), "counters")))
+    if ((st = cuda_status(cudaMemcpyAsync(S->tasks.p, tasks.data(), upload_bytes, cudaMemcpyHostToDevice, s),
+                          "tasks H2D")))
         return st;
-    P.filter_table = (const float*)S->table.p;
+    P.filter_table = reinterpret_cast<const float*>(static_cast<const char*>(S->tasks.p) + task_bytes);
     P.tasks = (const TaskRec*)S->tasks.p;
     P.n_tasks = smp->num_tasks;
     P.rays = (PbrtRay*)S->rays.p;

@@ -23,9 +23,11 @@
 
 namespace pbrt {
 
+constexpr uint32_t kCounterWords = 16;  // 64 bytes
 __global__ void __launch_bounds__(128) k_generate(RenderParams P) {
     __shared__ uint32_t words[16 * 128];  // the threads' ChaCha blocks
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pix < kCounterWords) P.counters[pix] = 0u;  // the later kernels' (a memset of its own is 4 us of stream time)
     if (pix >= P.n_pixels) return;
     generate_pixel(P, pix, words + threadIdx.x, 128u);
 }
@@ -185,6 +187,8 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
     if (P.n_pixels) {
         k_generate<<<blocks_for(P.n_pixels, 128), 128, 0, s>>>(P);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    } else if ((e = cudaMemsetAsync(P.counters, 0, 4 * kCounterWords, s)) != cudaSuccess) {
+        return e;
     }
     if (P.n_samples) {
         // camera rays of neighbouring pixels are coherent: one thread per
