@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(BLOCK) kb_trace(BatchArgs A) {
 // WIDE: the 4-wide layout, S1 stack rows in shared memory, S2 overflow
 // entries; else the binary layout, S1 stack entries, S2 = 1 with instances.
 template <int BLOCK, bool SHADOW, bool WIDE, int S1, int S2, int MODE>
-__global__ void __launch_bounds__(BLOCK, WIDE ? 1024 / BLOCK : 1) kb_trace_flat(BatchArgs A) {
+__global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1) kb_trace_flat(BatchArgs A) {
     using Closest = Walk4<BLOCK, WIDE ? S1 : 16, WIDE ? S2 : 64, false>;
     using Any = Walk4<BLOCK, WIDE ? S1 : 16, WIDE ? S2 : 64, true>;
     __shared__ typename std::conditional<WIDE, typename Closest::Shared, int>::type sh;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 1024 / BLOCK : 1) kb_trace_flat(
 // same as in the other stage kernels, so are the results.
 constexpr uint32_t kQueryRefill = 8;
 template <int BLOCK, bool SHADOW, int S1, int S2, int MODE>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) kb_trace4_refill(BatchArgs A) {
+__global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs A) {
     // per job: every ray takes a closest-hit walk, which an any-hit job's
     // rays leave at their first hit
     using Walk = Walk4<BLOCK, S1, S2, MODE == kAny>;
