@@ -679,6 +679,54 @@ __global__ void __launch_bounds__(128) k_number(const PoolNode* __restrict__ poo
     }
 }
 
+// The bounds and centroids of triangles (as prim_bounds: mesh.rs:196-205,
+// bvh.rs:77), and every primitive's index.  From the refined primitives, which
+// the layout reads again, instead of arrays that the host computes first.
+__global__ void __launch_bounds__(256) k_bounds(const HostPrim* __restrict__ prims, uint32_t n, float4* __restrict__ lo,
+                                                float4* __restrict__ hi, float* __restrict__ cx,
+                                                float* __restrict__ cy, float* __restrict__ cz,
+                                                uint32_t* __restrict__ idx) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n) return;
+    idx[i] = i;
+    const HostPrim& p = prims[i];
+    if (p.kind != PBRT_SHAPE_TRIANGLE_MESH) return;  // k_set_bounds
+    auto low = [](float a, float b, float c) { return fminf(fminf(fminf(FLT_MAX, a), b), c); };
+    auto high = [](float a, float b, float c) { return fmaxf(fmaxf(fmaxf(-FLT_MAX, a), b), c); };
+    const V3 a = p.p1, b = p.p2, c = p.p3;
+    const float4 l = make_float4(low(a.x, b.x, c.x), low(a.y, b.y, c.y), low(a.z, b.z, c.z), 0.0f);
+    const float4 h = make_float4(high(a.x, b.x, c.x), high(a.y, b.y, c.y), high(a.z, b.z, c.z), 0.0f);
+    lo[i] = l;
+    hi[i] = h;
+    cx[i] = (l.x + h.x) * 0.5f;
+    cy[i] = (l.y + h.y) * 0.5f;
+    cz[i] = (l.z + h.z) * 0.5f;
+}
+
+// The same of the other primitives, from the host.
+struct PrimBounds {
+    uint32_t prim;
+    Box box;
+    V3 centroid;
+};
+__global__ void __launch_bounds__(256) k_set_bounds(const PrimBounds* __restrict__ b, uint32_t n,
+                                                    float4* __restrict__ lo, float4* __restrict__ hi,
+                                                    float* __restrict__ cx, float* __restrict__ cy,
+                                                    float* __restrict__ cz) {
+    const uint32_t k = blockIdx.x * 256u + threadIdx.x;
+    if (k >= n) return;
+    const PrimBounds q = b[k];
+    lo[q.prim] = make_float4(q.box.lo.x, q.box.lo.y, q.box.lo.z, 0.0f);
+    hi[q.prim] = make_float4(q.box.hi.x, q.box.hi.y, q.box.hi.z, 0.0f);
+    cx[q.prim] = q.centroid.x;
+    cy[q.prim] = q.centroid.y;
+    cz[q.prim] = q.centroid.z;
+}
+
+// Up to this many the primitives stay on the device for the layout; beyond it
+// (240 MB) they make room and are uploaded again.
+constexpr size_t kKeepPrims = 1u << 22;
+
 // Trees of at least this many primitives get their layout on the device,
 // unless a range beyond kSmall primitives could not be split: one thread
 // writes a leaf.
@@ -696,36 +744,38 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         *err = "device BVH build: more than 2^31 primitives";
         return PBRT_ERR_UNSUPPORTED;
     }
-    RawVec<float4> lo(n), hi(n);
-    RawVec<float> cx(n), cy(n), cz(n);
-    host_parallel(n, [&](size_t, size_t from, size_t to) {
-        for (size_t i = from; i < to; ++i) {
-            V3 c;
-            const Box b = prim_bounds(H, i, &c);
-            lo[i] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
-            hi[i] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
-            cx[i] = c.x;
-            cy[i] = c.y;
-            cz[i] = c.z;
-            H.ordered[i] = (uint32_t)i;
-        }
-    });
-    Buf d_lo, d_hi, d_c[3], d_idx, d_tmp, d_pool;
+    std::vector<PrimBounds> analytic;
+    for (size_t i = 0; !H.spheres.empty() && i < n; ++i) {
+        if (H.prims[i].kind == PBRT_SHAPE_TRIANGLE_MESH) continue;
+        PrimBounds b;
+        b.prim = (uint32_t)i;
+        b.box = prim_bounds(H, i, &b.centroid);
+        analytic.push_back(b);
+    }
+    Buf d_prims, d_analytic, d_lo, d_hi, d_c[3], d_idx, d_tmp, d_pool;
+    CK(cudaMalloc(&d_prims.p, n * sizeof(HostPrim)));
     CK(cudaMalloc(&d_lo.p, n * sizeof(float4)));
     CK(cudaMalloc(&d_hi.p, n * sizeof(float4)));
     for (int k = 0; k < 3; ++k) CK(cudaMalloc(&d_c[k].p, n * sizeof(float)));
     CK(cudaMalloc(&d_idx.p, n * 4));
     CK(cudaMalloc(&d_tmp.p, n * 4));
-    CK(cudaMemcpy(d_lo.p, lo.data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_hi.p, hi.data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_c[0].p, cx.data(), n * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_c[1].p, cy.data(), n * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_c[2].p, cz.data(), n * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_idx.p, H.ordered.data(), n * 4, cudaMemcpyHostToDevice));
     Prims P;
     P.lo = d_lo.as<float4>();
     P.hi = d_hi.as<float4>();
     for (int k = 0; k < 3; ++k) P.cen[k] = d_c[k].as<float>();
+    CK(cudaMemcpy(d_prims.p, H.prims.data(), n * sizeof(HostPrim), cudaMemcpyHostToDevice));
+    k_bounds<<<(unsigned)((n + 255) / 256), 256>>>(d_prims.as<HostPrim>(), (uint32_t)n, d_lo.as<float4>(),
+                                                   d_hi.as<float4>(), d_c[0].as<float>(), d_c[1].as<float>(),
+                                                   d_c[2].as<float>(), d_idx.as<uint32_t>());
+    if (!analytic.empty()) {
+        const uint32_t na = (uint32_t)analytic.size();
+        CK(cudaMalloc(&d_analytic.p, na * sizeof(PrimBounds)));
+        CK(cudaMemcpy(d_analytic.p, analytic.data(), na * sizeof(PrimBounds), cudaMemcpyHostToDevice));
+        k_set_bounds<<<(na + 255) / 256, 256>>>(d_analytic.as<PrimBounds>(), na, d_lo.as<float4>(), d_hi.as<float4>(),
+                                                d_c[0].as<float>(), d_c[1].as<float>(), d_c[2].as<float>());
+    }
+    CK(cudaGetLastError());
+    if (n > kKeepPrims) d_prims.reset();
 
     // ---- phase A: one level per round
     std::vector<ANode> A;
@@ -933,7 +983,8 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
     CK(cudaMemcpy(H.nodes.data(), d_nodes.p, (size_t)m * sizeof(FlatNode), cudaMemcpyDeviceToHost));
     const bool big_leaf = std::any_of(top.begin(), top.end(), [](const TopNode& t) { return t.node.leaf; });
     d_pool.reset();
-    if (n >= kDeviceLayoutMin && !big_leaf) device_fill_layout(H, d_nodes.as<FlatNode>(), m, d_idx.as<uint32_t>());
+    if (n >= kDeviceLayoutMin && !big_leaf)
+        device_fill_layout(H, d_nodes.as<FlatNode>(), m, d_idx.as<uint32_t>(), d_prims.as<HostPrim>());
     return PBRT_OK;
 }
 

@@ -209,8 +209,10 @@ int device_build_tree(HostBVH& H, uint32_t max_prims, int split, std::string* er
 
 // The layout of a tree whose nodes (m) and primitive order are on the current
 // device too, made there (quads.cu): the same arrays as fill_host_layout's.
-// Leaves H.layout null if the device's memory does not suffice.
-void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const uint32_t* d_ordered);
+// d_prims: H.prims on the device, or null.  Leaves H.layout null if the
+// device's memory does not suffice.
+void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const uint32_t* d_ordered,
+                        const HostPrim* d_prims);
 
 int parse_split_method(const char* s);
 

@@ -353,7 +353,8 @@ DeviceLayout::~DeviceLayout() {
         if (p) cudaFree(p);
 }
 
-void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const uint32_t* d_ordered) {
+void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const uint32_t* d_ordered,
+                        const HostPrim* d_prims) {
     const size_t n = H.ordered.size();
     const uint32_t nb = (m + kLayoutBlock - 1) / kLayoutBlock;
     const size_t n_pairs = (m - 1) / 2;
@@ -365,7 +366,7 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
         bytes += (b + 255) & ~(size_t)255;
         return at;
     };
-    const size_t o_tot = take(sizeof(LayoutTotals)), o_prims = take(n * sizeof(HostPrim)),
+    const size_t o_tot = take(sizeof(LayoutTotals)), o_prims = take(d_prims ? 0 : n * sizeof(HostPrim)),
                  o_sph = take(H.spheres.size() * sizeof(SphereRec)), o_flat = take(H.flat_id.size() * 4),
                  o_parent = take((size_t)m * 4), o_rank = take((size_t)m * 4), o_cls = take(m), o_start = take(m),
                  o_part = take((size_t)nb * 12), o_quad = take(n_pairs * 4);
@@ -386,7 +387,7 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
         (n_pairs && !fits(cudaMalloc((void**)&L->pairs, n_pairs * sizeof(NodePair)))))
         return;
     auto* totals = reinterpret_cast<LayoutTotals*>(ws + o_tot);
-    auto* prims = reinterpret_cast<HostPrim*>(ws + o_prims);
+    const HostPrim* prims = d_prims ? d_prims : reinterpret_cast<HostPrim*>(ws + o_prims);
     auto* spheres = reinterpret_cast<SphereRec*>(ws + o_sph);
     auto* flat = H.flat_id.empty() ? nullptr : reinterpret_cast<uint32_t*>(ws + o_flat);
     auto* parent = reinterpret_cast<uint32_t*>(ws + o_parent);
@@ -396,7 +397,7 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
     auto* part = reinterpret_cast<uint32_t*>(ws + o_part);
     auto* quad_of = reinterpret_cast<uint32_t*>(ws + o_quad);
     if (!fits(cudaMemsetAsync(totals, 0, sizeof(LayoutTotals), 0)) ||
-        !fits(cudaMemcpy(prims, H.prims.data(), n * sizeof(HostPrim), cudaMemcpyHostToDevice)) ||
+        (!d_prims && !fits(cudaMemcpy(ws + o_prims, H.prims.data(), n * sizeof(HostPrim), cudaMemcpyHostToDevice))) ||
         (!H.spheres.empty() && !fits(cudaMemcpy(spheres, H.spheres.data(), H.spheres.size() * sizeof(SphereRec),
                                                 cudaMemcpyHostToDevice))) ||
         (flat && !fits(cudaMemcpy(flat, H.flat_id.data(), H.flat_id.size() * 4, cudaMemcpyHostToDevice))))
