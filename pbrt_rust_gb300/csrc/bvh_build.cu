@@ -12,7 +12,7 @@
 //      split) and count the left side, one thread per range picks the split,
 //      and a stable scatter writes the two sides in their original order
 //      (Iterator::partition keeps order, bvh.rs:89, 174).  The host reads the
-//      few per-range decisions back and lays out the next level.
+//      per-range decisions back, once per level, and lays out the next.
 //   B. ranges of at most kSmall primitives: one warp runs the whole subtree,
 //      one primitive per lane, with the host algorithm (including
 //      partition_by for the equal-counts split of ranges of up to four,
@@ -20,8 +20,9 @@
 //
 // Bounds are combined with a min/max that ignores NaN and orders -0 below
 // +0, in any order; f32 bucket indices and SAH costs repeat the host's
-// operations (--fmad=false).  The host then numbers all nodes in the
-// reference's depth-first order.
+// operations (--fmad=false).  The nodes are then numbered in the reference's
+// depth-first order (k_number), and larger trees get their layout from there
+// (quads.cu: device_fill_layout).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -105,7 +106,7 @@ __device__ inline DBox pbox(const Prims& P, uint32_t p) {
 }
 
 // ---- phase A ---------------------------------------------------------------
-struct Chunk {
+struct Chunk {  // a range's piece; as a range's record: first chunk, lo, count, chunks
     uint32_t seg, lo, hi, pad;
 };
 // Per range: [0..5] bounds, [6..11] centroid bounds (ord ints, min fields
@@ -118,6 +119,7 @@ struct SegDecision {   // filled by k_decide / k_choose
     int32_t action;    // 0 leaf, 1 split by bucket <= best, 2 split by key < pmid
     int32_t best;
     float lo[3], hi[3];  // range bounds
+    uint32_t n_left;   // k_a_base: primitives that go left
 };
 
 __global__ void k_acc_init(int32_t* acc, uint32_t nseg) {
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(256) k_a_bounds(Prims P, const uint32_t* __res
 }
 
 // One thread per range: split axis and centroid extent (bvh.rs:208-217).
-__global__ void k_a_decide(const int32_t* __restrict__ acc, SegDecision* dec, const uint32_t* __restrict__ counts,
+__global__ void k_a_decide(const int32_t* __restrict__ acc, SegDecision* dec, const Chunk* __restrict__ ranges,
                            uint32_t nseg, int split) {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nseg) return;
@@ -187,7 +189,7 @@ __global__ void k_a_decide(const int32_t* __restrict__ acc, SegDecision* dec, co
     d.dist = cmax - cmin;
     d.pmid = 0.5f * (cmin + cmax);
     d.best = 0;
-    if (counts[s] <= 1 || cmin == cmax)
+    if (ranges[s].hi <= 1 || cmin == cmax)
         d.action = 0;
     else
         d.action = split == PBRT_SPLIT_MIDDLE ? 2 : 1;
@@ -269,7 +271,7 @@ __device__ inline int cheapest_split(const DBox* bb, const uint32_t* bc, float t
 // One thread per range: the SAH costs in the host's order and the leaf test
 // (bvh.rs:133-185).
 __global__ void __launch_bounds__(32) k_a_choose(const int32_t* __restrict__ acc, SegDecision* dec,
-                                                 const uint32_t* __restrict__ counts, uint32_t nseg, uint32_t mp) {
+                                                 const Chunk* __restrict__ ranges, uint32_t nseg, uint32_t mp) {
     uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nseg) return;
     SegDecision d = dec[s];
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(32) k_a_choose(const int32_t* __restrict__ acc
     DBox total{d.lo[0], d.lo[1], d.lo[2], d.hi[0], d.hi[1], d.hi[2]};
     float best_cost;
     d.best = cheapest_split(bb, bc, darea(total), &best_cost);
-    const size_t cnt = counts[s];
+    const size_t cnt = ranges[s].hi;
     if (!(mp < cnt || to_usize(best_cost) < cnt)) d.action = 0;  // a leaf of cnt primitives
     dec[s] = d;
 }
@@ -318,9 +320,40 @@ __global__ void __launch_bounds__(256) k_a_count(Prims P, const uint32_t* __rest
     }
 }
 
+// A range's left total and where each of its chunks' sides go (a leaf's
+// chunks stay), one warp per range.  On the host this was a download, a pass
+// and an upload in the middle of every level.
+__global__ void __launch_bounds__(128) k_a_base(const Chunk* __restrict__ chunks, const Chunk* __restrict__ ranges,
+                                                uint32_t nseg, const uint32_t* __restrict__ left, SegDecision* dec,
+                                                uint2* __restrict__ base) {
+    const uint32_t s = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (s >= nseg) return;  // the whole warp
+    const Chunk r = ranges[s];
+    const uint32_t first = r.seg, lo = r.lo, cnt = r.hi, nc = r.pad;
+    const bool split = dec[s].action != 0;
+    uint32_t total = 0;
+    for (uint32_t c = lane; c < nc; c += 32u) total += left[first + c];
+    total = __reduce_add_sync(0xffffffffu, total);
+    const uint32_t mid = split ? lo + total : lo + cnt;
+    uint32_t run = 0;  // left ones before these chunks
+    for (uint32_t c0 = 0; c0 < nc; c0 += 32u) {
+        const uint32_t c = c0 + lane;
+        const Chunk k = c < nc ? chunks[first + c] : Chunk{0, 0, 0, 0};
+        const uint32_t nl = c < nc ? (split ? left[first + c] : k.hi - k.lo) : 0u;
+        uint32_t sum = nl;
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += o;
+        }
+        const uint32_t before = run + sum - nl;
+        if (c < nc) base[first + c] = make_uint2(lo + before, mid + (k.lo - lo) - before);
+        run += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) dec[s].n_left = total;
+}
+
 // Stable two-way scatter of every chunk: left side to base_left + rank,
-// right side to base_right + rank, in index order.  base_* per chunk come
-// from the host.
+// right side to base_right + rank, in index order.
 __global__ void __launch_bounds__(256) k_a_scatter(Prims P, const uint32_t* __restrict__ idx, uint32_t* out,
                                                    const Chunk* __restrict__ chunks,
                                                    const SegDecision* __restrict__ dec,
@@ -691,8 +724,8 @@ __global__ void __launch_bounds__(256) k_bounds(const HostPrim* __restrict__ pri
     idx[i] = i;
     const HostPrim& p = prims[i];
     if (p.kind != PBRT_SHAPE_TRIANGLE_MESH) return;  // k_set_bounds
-    auto low = [](float a, float b, float c) { return fminf(fminf(fminf(FLT_MAX, a), b), c); };
-    auto high = [](float a, float b, float c) { return fmaxf(fmaxf(fmaxf(-FLT_MAX, a), b), c); };
+    auto low = [](float a, float b, float c) { return dmin(dmin(dmin(FLT_MAX, a), b), c); };
+    auto high = [](float a, float b, float c) { return dmax(dmax(dmax(-FLT_MAX, a), b), c); };
     const V3 a = p.p1, b = p.p2, c = p.p3;
     const float4 l = make_float4(low(a.x, b.x, c.x), low(a.y, b.y, c.y), low(a.z, b.z, c.z), 0.0f);
     const float4 h = make_float4(high(a.x, b.x, c.x), high(a.y, b.y, c.y), high(a.z, b.z, c.z), 0.0f);
@@ -793,61 +826,46 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         to_small(0);
     else
         level.push_back(0);
-    Buf d_acc, d_dec, d_cnt, d_chunks, d_left, d_base;
+    std::vector<Chunk> chunks, ranges;
+    std::vector<SegDecision> dec;
+    Buf d_acc, d_dec, d_chunks, d_left, d_base;
     while (!level.empty()) {
         const uint32_t S = (uint32_t)level.size();
-        std::vector<Chunk> chunks;
-        std::vector<uint32_t> counts(S);
+        // the level's chunks, then its ranges, in one upload
+        chunks.clear();
+        ranges.clear();
         for (uint32_t s = 0; s < S; ++s) {
             const ANode& a = A[level[s]];
-            counts[s] = a.cnt;
+            const uint32_t first = (uint32_t)chunks.size();
             for (uint32_t o = 0; o < a.cnt; o += kChunk)
                 chunks.push_back(Chunk{s, a.lo + o, a.lo + std::min(a.cnt, o + kChunk), 0});
+            ranges.push_back(Chunk{first, a.lo, a.cnt, (uint32_t)chunks.size() - first});
         }
         const uint32_t NC = (uint32_t)chunks.size();
+        chunks.insert(chunks.end(), ranges.begin(), ranges.end());
         CK(d_acc.reserve((size_t)S * kAccWords * 4));
         CK(d_dec.reserve((size_t)S * sizeof(SegDecision)));
-        CK(d_cnt.reserve((size_t)S * 4));
-        CK(d_chunks.reserve((size_t)NC * sizeof(Chunk)));
+        CK(d_chunks.reserve(chunks.size() * sizeof(Chunk)));
         CK(d_left.reserve((size_t)NC * 4));
         CK(d_base.reserve((size_t)NC * sizeof(uint2)));
-        CK(cudaMemcpy(d_cnt.p, counts.data(), (size_t)S * 4, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(d_chunks.p, chunks.data(), (size_t)NC * sizeof(Chunk), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(d_chunks.p, chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+        const Chunk* d_ranges = d_chunks.as<Chunk>() + NC;
         const uint32_t acc_words = S * kAccWords;
         k_acc_init<<<(acc_words + 255) / 256, 256>>>(d_acc.as<int32_t>(), S);
         k_a_bounds<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_chunks.as<Chunk>(), d_acc.as<int32_t>());
-        k_a_decide<<<(S + 127) / 128, 128>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_cnt.as<uint32_t>(), S,
-                                             split);
+        k_a_decide<<<(S + 127) / 128, 128>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_ranges, S, split);
         if (split == PBRT_SPLIT_SAH) {
             k_a_buckets<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_chunks.as<Chunk>(), d_dec.as<SegDecision>(),
                                      d_acc.as<int32_t>());
-            k_a_choose<<<(S + 31) / 32, 32>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_cnt.as<uint32_t>(),
-                                                 S, mp);
+            k_a_choose<<<(S + 31) / 32, 32>>>(d_acc.as<int32_t>(), d_dec.as<SegDecision>(), d_ranges, S, mp);
         }
         k_a_count<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_chunks.as<Chunk>(), d_dec.as<SegDecision>(),
                                d_left.as<uint32_t>());
+        k_a_base<<<(S + 3) / 4, 128>>>(d_chunks.as<Chunk>(), d_ranges, S, d_left.as<uint32_t>(),
+                                       d_dec.as<SegDecision>(), d_base.as<uint2>());
         CK(cudaGetLastError());
-        std::vector<SegDecision> dec(S);
-        std::vector<uint32_t> left(NC);
+        dec.resize(S);
         CK(cudaMemcpy(dec.data(), d_dec.p, (size_t)S * sizeof(SegDecision), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(left.data(), d_left.p, (size_t)NC * 4, cudaMemcpyDeviceToHost));
-        // per-range left totals, then each chunk's destinations
-        std::vector<uint32_t> total_left(S, 0);
-        for (uint32_t c = 0; c < NC; ++c) total_left[chunks[c].seg] += left[c];
-        std::vector<uint2> base(NC);
-        std::vector<uint32_t> run_l(S, 0), run_r(S, 0);
-        for (uint32_t c = 0; c < NC; ++c) {
-            const uint32_t s = chunks[c].seg;
-            const ANode& a = A[level[s]];
-            const bool split_it = dec[s].action != 0;
-            const uint32_t mid = split_it ? a.lo + total_left[s] : a.lo + a.cnt;
-            base[c] = make_uint2(a.lo + run_l[s], mid + run_r[s]);
-            const uint32_t nc = chunks[c].hi - chunks[c].lo;
-            const uint32_t nl = split_it ? left[c] : nc;
-            run_l[s] += nl;
-            run_r[s] += nc - nl;
-        }
-        CK(cudaMemcpy(d_base.p, base.data(), (size_t)NC * sizeof(uint2), cudaMemcpyHostToDevice));
         k_a_scatter<<<NC, 256>>>(P, d_idx.as<uint32_t>(), d_tmp.as<uint32_t>(), d_chunks.as<Chunk>(),
                                  d_dec.as<SegDecision>(), d_base.as<uint2>());
         k_copy_ranges<<<NC, 256>>>(d_tmp.as<uint32_t>(), d_idx.as<uint32_t>(), d_chunks.as<Chunk>());
@@ -861,7 +879,7 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
                 A[ai].leaf = true;
                 continue;
             }
-            const uint32_t lo_ = A[ai].lo, cnt = A[ai].cnt, nl = total_left[s];
+            const uint32_t lo_ = A[ai].lo, cnt = A[ai].cnt, nl = d.n_left;
             if (nl == 0 || nl == cnt) {
                 *err = "BVH build: empty partition (the reference asserts at bvh.rs:237-238)";
                 return PBRT_ERR_BUILD;
