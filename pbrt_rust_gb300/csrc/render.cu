@@ -18,12 +18,15 @@
 // step repeats the reference's f32 operations.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "kernels.h"
 #include "wavefront.cuh"
 
 namespace pbrt {
 
 constexpr uint32_t kCounterWords = 16;  // 64 bytes
+constexpr uint32_t kCounterWork = 4, kCounterReplay = 5;  // k_shadow4_refill's
 __global__ void __launch_bounds__(128) k_generate(RenderParams P) {
     __shared__ uint32_t words[16 * 128];  // the threads' ChaCha blocks
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,6 +96,103 @@ __global__ void __launch_bounds__(128, INST ? 6 : 9) k_shadow4(const __grid_cons
     if (st == kStartWalk) T.run(P.bvh4, sh, ov);
     if (T.spilled < 0) atomicMax(status, 6);
     P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
+}
+
+// k_shadow4 with persistent warps that take kShadowChunk rays of the queue at a
+// time and refill their idle lanes once kShadowRefill are idle (see
+// k_trace4_persistent): the rays of a warp go to points all over an area light
+// and end where they hit, so 14 of 32 lanes were active.  1024 x 1024 x 16
+// terrain frame 4816 -> 4553 us, 700 x 700 x 16 into 200000 random triangles
+// 3098 -> 2828 (refill at 4 / 8 / 16 lanes: 4573 / 4553 / 4649).  A ray that
+// needs the exact walk is marked for k_shadow_replay.
+constexpr uint32_t kShadowChunk = 64, kShadowRefill = 8;
+template <int OVF, bool INST>
+__global__ void __launch_bounds__(128, INST ? 6 : 8) k_shadow4_refill(const __grid_constant__ RenderParams P) {
+    using Walk = Walk4<128, 16, OVF, true, INST>;
+    __shared__ typename Walk::Shared sh;
+    sh.init();
+    const uint32_t lane = threadIdx.x & 31u, n = *(volatile uint32_t*)&P.counters[0];
+    constexpr uint32_t kNone = 0xffffffffu;
+    uint32_t next = 0, end = 0, ray = kNone;
+    bool more = true;
+    Walk T;
+    typename Walk::Ovf ov;
+    T.bind(sh);
+    auto finish = [&](bool exact) {
+        if (T.spilled < 0) atomicMax((int*)&P.counters[2], 6);
+        if (exact) P.counters[kCounterReplay] = 1u;
+        P.occluded[P.shadow_slot[ray]] = exact ? kReplayOcc : (T.found() ? 1 : 0);
+        ray = kNone;
+        T.cur = kWalkDone;
+    };
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, ray == kNone), nidle = (uint32_t)__popc(idle);
+        if (more && next >= end && nidle >= kShadowRefill) {  // warp-uniform
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&P.counters[kCounterWork], kShadowChunk);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base < n) {
+                next = base;
+                end = n - base > kShadowChunk ? base + kShadowChunk : n;
+            } else {
+                more = false;
+            }
+        }
+        const bool tail = !more && end - next <= nidle;
+        if (next < end && nidle >= (tail ? 1u : kShadowRefill)) {
+            if (ray == kNone) {
+                const uint32_t k = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+                if (k < end - next) {
+                    ray = next + k;
+                    const float4* r = reinterpret_cast<const float4*>(P.shadow_rays) + 2 * (size_t)ray;
+                    const int st = T.start(P.bvh4, __ldg(r), __ldg(r + 1));
+                    if (st != kStartWalk) finish(st == kStartExact);
+                }
+            }
+            next += min(nidle, end - next);
+        }
+        if (!__any_sync(0xffffffffu, ray != kNone)) {
+            if (next >= end && !more) break;
+            continue;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if ((int32_t)T.cur >= 0) T.node(P.bvh4, ov);
+        if ((int32_t)T.cur < 0 && T.cur != kWalkDone) T.leaf(P.bvh4, sh, ov);
+        if (T.cur == kWalkDone && ray != kNone && !T.resume(ov)) finish(T.gave_up());
+    }
+}
+template <int STACK, bool INST>
+__global__ void __launch_bounds__(128) k_shadow_replay(const __grid_constant__ RenderParams P) {
+    if (*(volatile uint32_t*)&P.counters[kCounterReplay] == 0u) return;
+    const uint32_t n = *(volatile uint32_t*)&P.counters[0];
+    for (uint32_t q = blockIdx.x * 128u + threadIdx.x; q < n; q += gridDim.x * 128u) {
+        uint8_t* occ = P.occluded + P.shadow_slot[q];
+        if (*occ == kReplayOcc)
+            *occ = exact_any<STACK, INST>(P.bvh, reinterpret_cast<const float4*>(P.shadow_rays) + 2 * (size_t)q,
+                                          (int*)&P.counters[2]) ? 1 : 0;
+    }
+}
+// Where that pays: frames and trees so large that the walks, not their start
+// and the tail of the last warps, take the time.  Frame time without / with it, us, at
+// n = samples x lights: 17000 random triangles n = 4.3M 916 / 886, 5000 n = 6.5M
+// 843 / 853, 20000 n = 2.2M 573 / 573, 200000 n = 1.6M 599 / 610; terrains of 10000
+// n = 7.8M 1610 / 1667, 50000 n = 7.8M 1864 / 1866, 300000 n = 2.4M 853 / 864 and
+// 3.9M 1395 / 1382.  With instances, by n alone (the definitions' sizes are not
+// the scene's): n = 0.7M 421 / 435, 1.3M 569 / 560, 1.6M 678 / 633, 11.5M 3466 /
+// 3158.
+static bool shadow_refills(const RenderParams& P, uint64_t max_shadow) {
+    const uint64_t from = P.bvh.insts ? 3ull << 19 : 1ull << 22;
+    return max_shadow >= from && max_shadow < 0xF0000000ull && (P.bvh.insts || P.bvh.n_prims >= 16384u);
+}
+template <int OVF, bool INST>
+static cudaError_t launch_shadow_refill(const RenderParams& P, uint64_t max_shadow, cudaStream_t s) {
+    static ShapeCache bps_cache;
+    const uint64_t resident = (uint64_t)device_sms() * resident_blocks(bps_cache, k_shadow4_refill<OVF, INST>, 128, 0);
+    const uint64_t chunks = (max_shadow + 4 * kShadowChunk - 1) / (4 * kShadowChunk);
+    k_shadow4_refill<OVF, INST><<<(unsigned)std::min(resident, chunks), 128, 0, s>>>(P);
+    k_shadow_replay<OVF + 8, INST><<<(unsigned)device_sms(), 128, 0, s>>>(P);
+    return cudaGetLastError();
 }
 
 // --------------------------------------------------------------- combine ---
@@ -210,7 +310,12 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             const int iv = (inst && P.has_wide) ? wide_stack_variant(P.wide_bound) : 0;
             const bool wide_rk = rk == PBRT_TRACE_WIDE || rk == PBRT_TRACE_WIDE_PERSISTENT || rk == PBRT_TRACE_WIDE_SPECULATIVE;
             int wv = (P.has_wide && wide_rk && !inst) ? wide_stack_variant(P.wide_bound) : 0;
-            if (iv == 64)
+            const bool refill = shadow_refills(P, max_shadow);
+            if (refill && (iv == 64 || wv == 64))
+                e = iv ? launch_shadow_refill<64, true>(P, max_shadow, s) : launch_shadow_refill<64, false>(P, max_shadow, s);
+            else if (refill && (iv == 256 || wv == 256))
+                e = iv ? launch_shadow_refill<256, true>(P, max_shadow, s) : launch_shadow_refill<256, false>(P, max_shadow, s);
+            else if (iv == 64)
                 k_shadow4<64, true><<<grid4, 128, 0, s>>>(P, pw);
             else if (iv == 256)
                 k_shadow4<256, true><<<grid4, 128, 0, s>>>(P, pw);

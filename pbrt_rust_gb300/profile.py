@@ -11,8 +11,9 @@ closest hits go to pinned host memory: the walk that writes them out chunk
 by chunk), `render` R frames of
 the direct-lighting wavefront.  `batch` renders the multi-scene workload
 (N scenes of 1k-256k triangles + 0-32 spheres, 128-512 squared, 1/4/16 spp)
-as one batch R times, with the tuning the autotuner picks for it (binary
-walks, 256 threads, refill 32: the flat traversal stages).  Each pass is
+as one batch R times, with the tuning the autotuner picks for it (4-wide
+walks, 128 threads, the flat extend stage, shadow rays refilled at 8 idle
+lanes).  Each pass is
 timed with CUDA events on its stream.  `served` builds the serving workload
 (N resident scenes of 10k-1M triangles, Q requests: renders 128-512 squared
 at 1/4 spp and ray batches of 2^14-2^18 rays), runs every request once
@@ -177,8 +178,8 @@ def main(argv=None) -> int:
         samples = sum(n * r.sampler.x_samples * r.sampler.y_samples for n, (_, r) in zip(px, items))
         b = GpuBatch(max_jobs=a.scenes, max_tasks=64 * a.scenes, max_samples=samples,
                      max_light_samples=2 * samples, max_film_pixels=sum(px))
-        b.set_tuning(extend_kernel="pair", shadow_kernel="pair", block=256, chunk=64, refill=32, refill_shadow=32,
-                     use_graph=1)
+        b.set_tuning(extend_kernel="wide", shadow_kernel="wide", block=128, stack=16, chunk=64, refill=32,
+                     refill_shadow=8, use_graph=1)
         outs = [torch.empty((r.camera.film.y_res, r.camera.film.x_res, 3), device="cuda") for _, r in items]
         for _ in range(a.repeat):
             for (sc, r), o in zip(items, outs):
