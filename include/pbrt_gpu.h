@@ -440,10 +440,12 @@ typedef struct PbrtBatchTuning {
     int32_t extend_kernel;  /* PBRT_TRACE_PAIR or PBRT_TRACE_WIDE: camera and query rays */
     int32_t shadow_kernel;  /* PBRT_TRACE_PAIR or PBRT_TRACE_WIDE: shadow rays */
     uint32_t block;         /* threads per block: 128 or 256 */
-    uint32_t stack;         /* 4-wide kernels: shared-memory stack entries per ray, 8 or 16 */
+    uint32_t stack;         /* 4-wide kernels: shared-memory stack entries per ray, 8 (kept as 12 rows) or 16 */
     uint32_t chunk;         /* rays a warp takes from the work counter at a time: 32..4096, multiple of 32 */
     uint32_t refill;        /* extend: refill a warp when this many lanes are idle, 1..32;
-                               32: each lane walks its ray to the end, no per-step vote */
+                               32: each lane walks its ray to the end, no per-step vote
+                               (warps of query rays refill from 8 on in a batch whose rays are
+                               to an eighth or more queries) */
     uint32_t refill_shadow; /* shadow: same, 1..32 */
     uint32_t use_graph;     /* 1: replay the stage sequence as one CUDA graph */
 } PbrtBatchTuning;
