@@ -203,8 +203,8 @@ void fill_host_layout(HostBVH& H);
 Box prim_bounds(const HostBVH& H, size_t i, V3* centroid);
 
 // The tree of build_tree (H.nodes, H.ordered, H.depth) built on the current
-// CUDA device (bvh_build.cu): identical nodes and primitive order.  Larger
-// trees get their layout there too (H.layout).
+// CUDA device (bvh_build.cu): identical nodes and primitive order.  The
+// layout is made there too (H.layout) unless a leaf is too large for a thread.
 int device_build_tree(HostBVH& H, uint32_t max_prims, int split, std::string* err);
 
 // The layout of a tree whose nodes (m) and primitive order are on the current

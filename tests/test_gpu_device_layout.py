@@ -1,5 +1,5 @@
-"""Trees whose layout is made on the device (device_fill_layout), around the
-size where that begins and at sizes that leave blocks part full: the same hits
+"""Trees whose layout is made on the device (device_fill_layout), from single
+leaves to sizes that leave the last of many blocks part full: the same hits
 and sizes as the tree that the host lays out, so no tolerance is involved."""
 import numpy as np
 import pytest
@@ -46,6 +46,8 @@ def scene(kind, n):
 
 
 @pytest.mark.parametrize("kind,n,max_prims", [
+    ("triangles", 1, 4), ("triangles", 2, 1), ("triangles", 3, 4), ("triangles", 5, 1), ("triangles", 129, 4),
+    ("triangles", 130, 1), ("mixed", 40, 4), ("coincident", 200, 4), ("clusters", 257, 4),
     ("triangles", 16383, 4), ("triangles", 16384, 4), ("triangles", 16385, 1), ("triangles", 70001, 4),
     ("triangles", 300007, 2), ("clusters", 20011, 4), ("coincident", 16400, 4), ("past_reach", 16500, 4),
     ("nan", 16500, 4), ("mixed", 33333, 4), ("mixed", 16500, 1), ("instances", 16900, 4)])
