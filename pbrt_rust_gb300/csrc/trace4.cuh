@@ -31,11 +31,12 @@
 //  * an axis with d = 0 has 1 / d replaced by kZeroInv, so large that e is
 //    beyond every other distance: a plane at the origin or within e / i of it
 //    never culls, one farther off does.  The exact test has +-inf there, as
-//    the reference (d = -0 rejects an origin on the boundary of
-//    a box that is not flat, where a flat box inside it passes; but what is
-//    flat there and hit by a ray that runs within it is no triangle, whose
-//    determinant is 0; instances, which are entered on their box alone, send
-//    such rays the other way below).
+//    the reference.
+// One box may pass where a box above it does not: with d = -0 the reference
+// rejects an origin on the boundary of a box, unless the box is flat there.  A
+// triangle of such a flat leaf is not hit (its determinant is 0); an analytic
+// shape or an instance in one may be, so a walk that comes to them there gives
+// up and the ray takes the exact walk described below.
 // The deferred children are pushed with their entry distance and re-checked
 // against maxt when popped.
 //
@@ -466,6 +467,11 @@ struct Walk4 : InstWalk<INST> {
         cur = kWalkDone;
         spilled = min(spilled, 0);
     }
+    // The ray takes the exact walk.
+    __device__ __forceinline__ void give_up() {
+        maxt = __int_as_float(0x7fc00000);  // gave_up()
+        stop();
+    }
 
     // INST: the instance record S (first id `first`) of the scene's tree;
     // `rest` is the leaf word of the rest of its leaf (0: none).  1 when its
@@ -566,13 +572,18 @@ struct Walk4 : InstWalk<INST> {
             const PrimRec* pr = prims + off;
             const float4 r0 = ldg4(pr->r0), r1 = ldg4(pr->r1), r2 = ldg4(pr->r2);
             const uint32_t id = __float_as_uint(r0.w), flags = __float_as_uint(r2.w);
+            bool beside = false;  // the box passed, but one above it need not
             auto table_box = [&]() {
                 const LeafBox* b = boxes + (flags >> kPrimBoxShift);
                 const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
                 float tr;
-                return slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr);
+                if (!slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr)) return false;
+                beside = (ix == -kZeroInv && lo.x == hi.x) || (iy == -kZeroInv && lo.y == hi.y) ||
+                         (iz == -kZeroInv && lo.z == hi.z);
+                return true;
             };
             if ((flags & kPrimBoxEntry) && !table_box()) break;
+            if (beside) return give_up();
             float t, u = 0.0f, v = 0.0f;
             bool hit;
             if (id & kSphereBit) {
@@ -583,10 +594,7 @@ struct Walk4 : InstWalk<INST> {
                         const int e = enter(bvh, sh, S, id & ~kSphereBit,
                                             (flags & kPrimLastBit) ? 0u : (kNode4Leaf | (off + 1)));
                         if (e == 1) return make_room(ov);
-                        if (e == 2) {
-                            maxt = __int_as_float(0x7fc00000);  // gave_up()
-                            return stop();
-                        }
+                        if (e == 2) return give_up();
                         if (flags & kPrimLastBit) break;
                         ++off;
                         continue;
@@ -594,6 +602,7 @@ struct Walk4 : InstWalk<INST> {
                 }
                 hit = sphere_test(spheres, si, ray(), maxt, &t);
                 if (hit && (flags & kPrimHitBox)) hit = table_box();
+                if (beside) return give_up();
             } else {
                 hit = tri_test(r0, r1, r2, ray(), maxt, &t, &u, &v);
                 if (hit && (flags & kPrimOwnBox)) {
@@ -628,8 +637,8 @@ struct Walk4 : InstWalk<INST> {
             if (cur == kWalkDone && !resume(ov)) return;
         }
     }
-    // A closest hit at distance NaN, or an instance ray that was not clean:
-    // the ray needs the exact walk.
+    // A hit at distance NaN, a flat box beside the ray or an instance ray that
+    // was not clean: the ray needs the exact walk.
     __device__ __forceinline__ bool gave_up() const { return !(maxt == maxt); }
     __device__ __forceinline__ bool found() const { return prim >= 0; }
     __device__ __forceinline__ float4 hit_record() const {

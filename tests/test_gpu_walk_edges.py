@@ -1,0 +1,86 @@
+"""Rays and trees at the edges of what the 4-wide walk (trace4.cuh) takes: the
+hits are the oracle's bit for bit whichever walk a ray ends up in, so no
+tolerance is involved."""
+import numpy as np
+import pytest
+
+from pbrt_rust_gb300 import abi
+from pbrt_rust_gb300.scene import InstanceDefinition, Primitive, Shape
+from pbrt_rust_gb300.transform import Transform
+from test_gpu_quads import mesh, soup
+
+pytestmark = pytest.mark.gpu
+
+
+def check(oracle, prims, r, max_prims=4, method="sah", on_device=False):
+    """Every form of a query against the oracle: a call of few rays, the
+    persistent kernel, and a batch of closest and any-hit jobs with and
+    without refilling."""
+    import torch
+
+    from pbrt_rust_gb300.batch import GpuBatch
+    from pbrt_rust_gb300.gpu import GpuBVHAccel
+    bvh = GpuBVHAccel(prims, max_prims, method, build_on_device=on_device)
+    ob = oracle.OracleBVH(prims, max_prims, method)
+    want, want_p = ob.intersect(r), ob.intersect_p(r)
+    dev = torch.from_numpy(r.view(np.float32).reshape(-1, 8).copy()).cuda()
+
+    def same(hits, occ, what):
+        got = hits.cpu().numpy().view(abi.HIT_DTYPE).reshape(-1)
+        for f in ("prim", "t", "b1", "b2"):
+            assert np.array_equal(got[f], want[f], equal_nan=True), (what, f, got[:3], want[:3])
+        assert np.array_equal(occ.cpu().numpy(), want_p), what
+
+    def called(what):
+        hits, occ = bvh.intersect(dev), bvh.intersect_p(dev)
+        torch.cuda.synchronize()
+        same(hits, occ, what)
+
+    called("few rays")
+    before = abi.get_trace_config()
+    abi.set_trace_config(reorder=True)  # keeps calls of few rays on the persistent kernel
+    try:
+        called("persistent")
+    finally:
+        abi.set_trace_config(**before)
+    for tuning in (dict(refill=32), dict(refill=8)):
+        b = GpuBatch(max_jobs=3, max_query_rays=0)
+        b.set_tuning(extend_kernel="wide", **tuning)
+        b.add_query(bvh, dev)
+        b.add_query(bvh, dev, any_hit=True)
+        same(*b.run(), tuning)
+    return bvh, want
+
+
+def flat_shape(kind):
+    """A shape whose box has no thickness in y, at y = 1."""
+    at = Transform.translate((0.0, 1.0, 0.0)) * Transform.scale(1.0, 1.0e-12, 1.0)
+    if kind == "sphere":
+        return Shape.sphere(at, None, False, 0.5, -0.5, 0.5, 360.0)
+    if kind == "cylinder":
+        return Shape.cylinder(at, None, False, 0.5, -0.5, 0.5, 360.0)
+    lump = InstanceDefinition([Primitive.simple(mesh(soup(np.random.default_rng(3), 20, 0.4, 0.3)))])
+    return Primitive.transformed(lump, at.inverse())
+
+
+@pytest.mark.parametrize("max_prims", [1, 4])
+@pytest.mark.parametrize("kind", ["sphere", "cylinder", "instance"])
+@pytest.mark.parametrize("below", [False, True])
+def test_rays_within_a_flat_box_on_the_boundary_of_the_boxes_around_it(oracle, kind, below, max_prims):
+    """With a direction of -0 the reference rejects the boxes around, so that
+    it never comes to the flat shape; with +0 it does."""
+    s = -1.0 if below else 1.0
+    rest = [mesh([[(3, 1 + s, 0), (4, 1 + s, 0), (3, 1 + 2 * s, 1)], [(3, 1, 4), (4, 1 + s / 2, 4), (3, 1 + 2 * s, 5)],
+                  [(-3, 1 + s, 4), (-4, 1 + s / 2, 4), (-3, 1 + 2 * s, 5)]])]
+    r = np.zeros(96, abi.RAY_DTYPE)
+    r["o"] = (-2.0, 1.0, 0.0)
+    r["o"][:, 2] = np.linspace(-0.45, 0.45, 96)
+    r["d"] = (1.0, 0.0, 0.0)
+    r["d"][::2, 1] = -0.0
+    r["d"][::3, 2] = 0.05
+    r["d"][1::3, 2] = -0.0
+    r["tmax"] = np.inf
+    _, want = check(oracle, [Primitive.simple(p) if not isinstance(p, Primitive) else p
+                             for p in [flat_shape(kind)] + rest], r, max_prims)
+    hit = want["prim"] >= 0
+    assert hit[1::2].any() and not hit[::2].any()  # -0 finds nothing where +0 does
