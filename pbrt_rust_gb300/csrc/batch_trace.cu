@@ -214,7 +214,6 @@ __global__ void __launch_bounds__(BLOCK, WIDE ? 896 / BLOCK : 1) kb_trace_flat(B
                     T.bind(sh);
                     const int st = T.start(bv, __ldg(src), __ldg(src + 1));
                     if (st == kStartWalk) T.run(bv, sh, ov);
-                    if (T.spilled < 0) atomicMax(status, 6);
                     *exact = st == kStartExact || T.gave_up();
                 };
                 bool exact;
@@ -289,7 +288,6 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) kb_trace4_refill(BatchArgs
     T.bind(sh);
     auto finish = [&](bool exact) {
         const JobRec& J = A.jobs[job];
-        if (T.spilled < 0) atomicMax((int*)(J.P.counters + 2), 6);
         if (exact) A.counters[SHADOW ? kCtrReplayShadow : kCtrReplay] = 1u;  // rewritten by the replay stage
         const uint8_t found = exact ? kReplayOcc : (T.found() ? 1 : 0);
         if (SHADOW)

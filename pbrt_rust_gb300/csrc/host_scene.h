@@ -170,7 +170,7 @@ struct HostBVH {
     // kWideReach away from the origin
     bool wide = false;
     float reach = 0.0f;          // 5/4 of the largest coordinate of the root's box, 2^-50 at least
-    uint32_t stack4_bound = 0;  // most entries a 4-wide traversal can defer
+    uint32_t stack4_bound = 0;  // most children a 4-wide traversal can defer (trace4.cuh: the stack)
     // instance definitions: one BVH each, shared by all their instances
     std::vector<HostBVH> insts;
     // With instances, the id a hit reports: refined primitives numbered in

@@ -94,7 +94,6 @@ __global__ void __launch_bounds__(128, INST ? 6 : 9) k_shadow4(const __grid_cons
     T.bind(sh);
     const int st = T.start(P.bvh4, ray[0], ray[1]);
     if (st == kStartWalk) T.run(P.bvh4, sh, ov);
-    if (T.spilled < 0) atomicMax(status, 6);
     P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
 }
 
@@ -119,7 +118,6 @@ __global__ void __launch_bounds__(128, INST ? 6 : 8) k_shadow4_refill(const __gr
     typename Walk::Ovf ov;
     T.bind(sh);
     auto finish = [&](bool exact) {
-        if (T.spilled < 0) atomicMax((int*)&P.counters[2], 6);
         if (exact) P.counters[kCounterReplay] = 1u;
         P.occluded[P.shadow_slot[ray]] = exact ? kReplayOcc : (T.found() ? 1 : 0);
         ray = kNone;

@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : (ANY ? 9 : 8)) k_trace4
     T.bind(sh);
     const int st = T.start(bvh, __ldg(ray), __ldg(ray + 1));
     if (st == kStartWalk) T.run(bvh, sh, ov);
-    if (T.spilled < 0) atomicMax(status, 6);
     if (ANY)
         occ[i] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
     else
@@ -304,7 +303,6 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : 8)
     };
     // The lane's ray ends with what T found, or marked for the replay.
     auto finish = [&](bool exact) {
-        if (T.spilled < 0) atomicMax(status, 6);
         if (exact) *replay = 1u;
         if (ANY) {
             occ[ray] = exact ? kReplayOcc : (T.found() ? 1 : 0);

@@ -53,7 +53,12 @@
 //
 // The stack: ROWS 8-byte entries per thread in shared memory ([entry][thread],
 // so a warp's accesses hit distinct banks), the oldest entries going to an
-// array in local memory when they run out.  The bottom entry is a word that
+// array in local memory when they run out.  The tree's bound
+// (HostBVH::stack4_bound) counts the children that exist.  An empty slot's
+// planes lie the wrong way round, but in a node smaller than the margins it
+// passes all the same and takes entries beyond the bound, so a walk may find
+// its stack full; it then gives up and the ray takes the exact walk, whose
+// entries (one per level at most) the bound does cover.  The bottom entry is a word that
 // ends the walk, so a pop needs no test for an empty stack.  A visit stores
 // all four children without branches: a 128-word table in shared memory,
 // indexed by the node's visiting order for the ray's octant and the mask of
@@ -256,7 +261,7 @@ struct Walk4 : InstWalk<INST> {
     uint32_t oct3;     // 3 * the ray's octant
     uint32_t cur;
     uint32_t top;      // shared-memory address of the first free row
-    int spilled;       // entries in the overflow; -1: they would not fit (reported, never written)
+    int spilled;       // entries in the overflow
     int32_t prim;      // -1: none yet
     float b1, b2;
     uint32_t base, push_tab;  // shared-memory addresses, the same for all threads
@@ -354,13 +359,14 @@ struct Walk4 : InstWalk<INST> {
         return kStartWalk;
     }
 
-    // Moves the oldest rows to the overflow when fewer than four are free.
+    // Moves the oldest rows to the overflow when fewer than four are free; a
+    // walk whose overflow is full gives up (`cur` ends it, with or without a
+    // pop that follows).
     __device__ __forceinline__ void make_room(Ovf& ov) {
         if (top < base + (ROWS - 3) * kRow) return;
-        if (spilled < 0 || spilled + kSpill > OVF) {
-            spilled = -1;
-            top = row(1);  // the pop that follows ends the walk
-            return;
+        if (spilled + kSpill > OVF) {
+            top = row(1);
+            return give_up();
         }
         for (int i = 0; i < kSpill; ++i) {
             uint32_t ref;
@@ -388,7 +394,7 @@ struct Walk4 : InstWalk<INST> {
     // cur == kWalkDone: brings spilled rows back and goes on; false when the
     // walk is over.
     __device__ __forceinline__ bool resume(Ovf& ov) {
-        if (spilled <= 0) return false;
+        if (spilled == 0) return false;
         spilled -= kSpill;
         for (int i = 0; i < kSpill; ++i)
             st_entry(row(1 + i), ov.e[spilled + i].x, __uint_as_float(ov.e[spilled + i].y));
@@ -465,7 +471,7 @@ struct Walk4 : InstWalk<INST> {
     // An any-hit walk is over.
     __device__ __forceinline__ void stop() {
         cur = kWalkDone;
-        spilled = min(spilled, 0);
+        spilled = 0;
     }
     // The ray takes the exact walk.
     __device__ __forceinline__ void give_up() {
@@ -637,8 +643,8 @@ struct Walk4 : InstWalk<INST> {
             if (cur == kWalkDone && !resume(ov)) return;
         }
     }
-    // A hit at distance NaN, a flat box beside the ray or an instance ray that
-    // was not clean: the ray needs the exact walk.
+    // A hit at distance NaN, a flat box beside the ray, an instance ray that
+    // was not clean or a full stack: the ray needs the exact walk.
     __device__ __forceinline__ bool gave_up() const { return !(maxt == maxt); }
     __device__ __forceinline__ bool found() const { return prim >= 0; }
     __device__ __forceinline__ float4 hit_record() const {

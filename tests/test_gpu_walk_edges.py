@@ -84,3 +84,32 @@ def test_rays_within_a_flat_box_on_the_boundary_of_the_boxes_around_it(oracle, k
                              for p in [flat_shape(kind)] + rest], r, max_prims)
     hit = want["prim"] >= 0
     assert hit[1::2].any() and not hit[::2].any()  # -0 finds nothing where +0 does
+
+
+def funnel(n, ratio):
+    """Triangles that shrink towards the origin, each `ratio` of the last: a
+    tree that is one chain of nodes, the innermost far smaller than the walk's
+    margins, where slots without a child pass too."""
+    t = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0]], np.float64) + 1.0
+    return np.array([t * float(ratio) ** -k for k in range(n)])
+
+
+@pytest.mark.parametrize("where", ["alone", "instanced"])
+@pytest.mark.parametrize("n,ratio", [(40, 3.0), (44, 3.0), (61, 3.0), (61, 2.0), (90, 2.0)])
+def test_walks_whose_stack_runs_out(oracle, n, ratio, where):
+    """Rays from the funnel's tip through every node of it, and from so far
+    away that the margins exceed the whole tree."""
+    rng = np.random.default_rng(n)
+    r = np.zeros(300, abi.RAY_DTYPE)
+    r["d"] = 1.0 + rng.uniform(-0.2, 0.2, (300, 3))
+    far = np.arange(300) % 3 == 2
+    r["o"][far] = -r["d"][far] * 10.0 ** rng.uniform(5, 7, (far.sum(), 1))
+    r["tmax"] = np.inf
+    prims = [Primitive.simple(mesh(funnel(n, ratio)))]
+    if where == "instanced":
+        lump = InstanceDefinition(prims)
+        at = Transform.translate((0.0, 0.0, 2.0))
+        prims = [Primitive.simple(mesh(funnel(n // 2, ratio))), Primitive.transformed(lump, Transform()),
+                 Primitive.transformed(lump, at.inverse())]
+    _, want = check(oracle, prims, r, 1, "middle")
+    assert (want["prim"] >= 0).any()
