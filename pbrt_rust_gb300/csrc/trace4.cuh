@@ -290,9 +290,6 @@ struct Walk4 : InstWalk<INST> {
         const float so = fabsf(ox) + fabsf(oy) + fabsf(oz), sd = fabsf(dx) + fabsf(dy) + fabsf(dz);
         bool ok = so <= kRayReach && sd <= kInvMax && sd > 0.0f && tmin >= -kInvMax && maxt == maxt &&
                   max3f(zx ? 0.0f : fabsf(ix), zy ? 0.0f : fabsf(iy), zz ? 0.0f : fabsf(iz)) <= kInvMax;
-        if (INST)  // -0: see above
-            ok = ok && __float_as_uint(dx) != 0x80000000u && __float_as_uint(dy) != 0x80000000u &&
-                 __float_as_uint(dz) != 0x80000000u;
         if (zx) ix = copysignf(kZeroInv, dx);
         if (zy) iy = copysignf(kZeroInv, dy);
         if (zz) iz = copysignf(kZeroInv, dz);
@@ -360,14 +357,10 @@ struct Walk4 : InstWalk<INST> {
     }
 
     // Moves the oldest rows to the overflow when fewer than four are free; a
-    // walk whose overflow is full gives up (`cur` ends it, with or without a
-    // pop that follows).
+    // walk whose overflow is full gives up.
     __device__ __forceinline__ void make_room(Ovf& ov) {
         if (top < base + (ROWS - 3) * kRow) return;
-        if (spilled + kSpill > OVF) {
-            top = row(1);
-            return give_up();
-        }
+        if (spilled + kSpill > OVF) return give_up();
         for (int i = 0; i < kSpill; ++i) {
             uint32_t ref;
             float t;
@@ -473,9 +466,10 @@ struct Walk4 : InstWalk<INST> {
         cur = kWalkDone;
         spilled = 0;
     }
-    // The ray takes the exact walk.
+    // The ray takes the exact walk; this one is over, also after a pop.
     __device__ __forceinline__ void give_up() {
         maxt = __int_as_float(0x7fc00000);  // gave_up()
+        top = row(1);
         stop();
     }
 
@@ -578,18 +572,18 @@ struct Walk4 : InstWalk<INST> {
             const PrimRec* pr = prims + off;
             const float4 r0 = ldg4(pr->r0), r1 = ldg4(pr->r1), r2 = ldg4(pr->r2);
             const uint32_t id = __float_as_uint(r0.w), flags = __float_as_uint(r2.w);
-            bool beside = false;  // the box passed, but one above it need not
             auto table_box = [&]() {
                 const LeafBox* b = boxes + (flags >> kPrimBoxShift);
                 const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
                 float tr;
                 if (!slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr)) return false;
-                beside = (ix == -kZeroInv && lo.x == hi.x) || (iy == -kZeroInv && lo.y == hi.y) ||
-                         (iz == -kZeroInv && lo.z == hi.z);
-                return true;
+                if ((ix != -kZeroInv || lo.x != hi.x) && (iy != -kZeroInv || lo.y != hi.y) &&
+                    (iz != -kZeroInv || lo.z != hi.z))
+                    return true;
+                give_up();  // one above it need not pass; the pop ends the walk
+                return false;
             };
             if ((flags & kPrimBoxEntry) && !table_box()) break;
-            if (beside) return give_up();
             float t, u = 0.0f, v = 0.0f;
             bool hit;
             if (id & kSphereBit) {
@@ -608,7 +602,6 @@ struct Walk4 : InstWalk<INST> {
                 }
                 hit = sphere_test(spheres, si, ray(), maxt, &t);
                 if (hit && (flags & kPrimHitBox)) hit = table_box();
-                if (beside) return give_up();
             } else {
                 hit = tri_test(r0, r1, r2, ray(), maxt, &t, &u, &v);
                 if (hit && (flags & kPrimOwnBox)) {
