@@ -169,7 +169,11 @@ struct HostBVH {
     // the tree has the 4-wide layout: every coordinate is finite and at most
     // kWideReach away from the origin
     bool wide = false;
-    float reach = 0.0f;          // 5/4 of the largest coordinate of the root's box, 2^-50 at least
+    // its margins (tree_margins): the middle of the root's box, half its
+    // extent and 2^-22 of its coordinates, kTreeMargin times that, and the sum
+    // of the axes' margins up to which the 4-wide walk is the one to take
+    V3 middle{}, half{}, spread{};
+    float far = 0.0f;
     uint32_t stack4_bound = 0;  // most children a 4-wide traversal can defer (trace4.cuh: the stack)
     // instance definitions: one BVH each, shared by all their instances
     std::vector<HostBVH> insts;
@@ -184,7 +188,7 @@ struct HostBVH {
 
 constexpr uint32_t kNoQuad = 0xffffffffu;
 constexpr uint32_t kQuadAxisShift = 30u;
-constexpr float kWideReach = 1.099511627776e12f;  // 2^40 (kRayReach in trace4.cuh)
+constexpr float kWideReach = 1.099511627776e12f;  // 2^40
 
 // Fully refine shapes, build and flatten the BVH, and fill the device
 // layout.  Returns a PbrtStatus; *err gets a message on failure.
@@ -192,8 +196,9 @@ int build_host_bvh(const PbrtShapeDesc* shapes, uint32_t n_shapes, uint32_t max_
                    HostBVH* out, std::string* err, bool on_device = false, const PbrtInstanceDesc* defs = nullptr,
                    uint32_t n_defs = 0);
 
-// H.reach and H.quad_root of the nodes.
-void tree_reach(HostBVH& H);
+// H.middle, H.half, H.spread, H.far and H.quad_root of the nodes, whose boxes' half
+// areas and edge lengths add up to `area` and `length`.
+void tree_margins(HostBVH& H, double area, double length);
 
 // The layout arrays on the host (after build_host_bvh left them on a device).
 void fill_host_layout(HostBVH& H);

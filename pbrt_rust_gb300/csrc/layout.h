@@ -106,6 +106,11 @@ constexpr uint32_t kPrimOwnBox = 4u;
 constexpr uint32_t kPrimHitBox = 8u;
 constexpr uint32_t kPrimBoxShift = 4u;
 
+// The 4-wide walk's margins (trace4.cuh), u = 2^-24: kFarMargin (6 u) per
+// distance of the origin, kTreeMargin (32 u) per half extent of the tree.
+constexpr float kFarMargin = 3.57627868652343750e-07f;
+constexpr float kTreeMargin = 1.90734863281250e-06f;
+
 // A leaf's exact box in the table of leaf boxes.
 struct alignas(32) LeafBox {
     float lo[4], hi[4];

@@ -150,6 +150,7 @@ constexpr uint32_t kClassBoxed = 0x10u;  // a leaf whose box goes to the table
 
 struct LayoutTotals {
     uint32_t inner, boxed, starts, stack, bad;
+    double area, length;  // of the boxes (tree_margins)
 };
 
 __device__ __forceinline__ bool usable(const V3& v) {  // false for NaN
@@ -157,17 +158,23 @@ __device__ __forceinline__ bool usable(const V3& v) {  // false for NaN
 }
 
 // Blocks' numbers of inner nodes and boxed leaves (part[0..nb), part[nb..2 nb)),
-// every node's class and parent, and whether a coordinate is out of reach.
+// their boxes' half areas and edges (sums[0..nb)), every node's class and
+// parent, and whether a coordinate is out of reach.
 __global__ void __launch_bounds__(kLayoutBlock) k_layout_mark(const FlatNode* __restrict__ nodes, uint32_t m,
                                                               const HostPrim* __restrict__ prims,
                                                               const uint32_t* __restrict__ ordered,
                                                               uint32_t* __restrict__ parent, uint8_t* __restrict__ cls,
                                                               uint32_t* __restrict__ part, uint32_t nb,
-                                                              LayoutTotals* totals) {
+                                                              float2* __restrict__ sums, LayoutTotals* totals) {
+    __shared__ float2 warps[kLayoutBlock / 32];
     const uint32_t k = blockIdx.x * kLayoutBlock + threadIdx.x;
     bool inner = false, boxed = false, ok = true;
+    float area = 0.0f, length = 0.0f;
     if (k < m) {
         const FlatNode& nd = nodes[k];
+        const float ex = nd.box.hi.x - nd.box.lo.x, ey = nd.box.hi.y - nd.box.lo.y, ez = nd.box.hi.z - nd.box.lo.z;
+        area = ex * ey + ey * ez + ez * ex;
+        length = ex + ey + ez;
         if (k == 0) parent[0] = kNone;
         uint32_t c = 0;
         if (!nd.leaf) {
@@ -188,8 +195,16 @@ __global__ void __launch_bounds__(kLayoutBlock) k_layout_mark(const FlatNode* __
         }
         cls[k] = (uint8_t)c;
     }
+    for (uint32_t d = 16; d; d >>= 1) {
+        area += __shfl_down_sync(0xffffffffu, area, d);
+        length += __shfl_down_sync(0xffffffffu, length, d);
+    }
+    if ((threadIdx.x & 31u) == 0) warps[threadIdx.x >> 5] = make_float2(area, length);
     const int ni = __syncthreads_count(inner), nx = __syncthreads_count(boxed), nbad = __syncthreads_count(!ok);
     if (threadIdx.x == 0) {
+        float2 s = warps[0];
+        for (uint32_t w = 1; w < kLayoutBlock / 32; ++w) s = make_float2(s.x + warps[w].x, s.y + warps[w].y);
+        sums[blockIdx.x] = s;
         part[blockIdx.x] = (uint32_t)ni;
         part[nb + blockIdx.x] = (uint32_t)nx;
         if (nbad) atomicOr(&totals->bad, 1u);
@@ -226,9 +241,12 @@ __global__ void __launch_bounds__(kLayoutBlock) k_layout_starts(const uint32_t* 
     if (threadIdx.x == 0) part[2u * nb + blockIdx.x] = (uint32_t)ns;
 }
 
-// The exclusive sums of the three arrays of nb counts, and their totals.
-__global__ void __launch_bounds__(1024) k_layout_scan(uint32_t* __restrict__ part, uint32_t nb, LayoutTotals* totals) {
+// The exclusive sums of the three arrays of nb counts, their totals and those
+// of the boxes (in a fixed order).
+__global__ void __launch_bounds__(1024) k_layout_scan(uint32_t* __restrict__ part, uint32_t nb,
+                                                      const float2* __restrict__ sums, LayoutTotals* totals) {
     __shared__ uint32_t warps[32];
+    __shared__ double2 box_sums[32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t a = 0; a < 3; ++a) {
         uint32_t carry = 0;
@@ -252,6 +270,25 @@ __global__ void __launch_bounds__(1024) k_layout_scan(uint32_t* __restrict__ par
             __syncthreads();
         }
         if (threadIdx.x == 0) (a == 0 ? totals->inner : a == 1 ? totals->boxed : totals->starts) = carry;
+    }
+    double area = 0.0, length = 0.0;
+    for (uint32_t i = threadIdx.x; i < nb; i += 1024u) {
+        area += (double)sums[i].x;
+        length += (double)sums[i].y;
+    }
+    for (uint32_t d = 16; d; d >>= 1) {
+        area += __shfl_down_sync(0xffffffffu, area, d);
+        length += __shfl_down_sync(0xffffffffu, length, d);
+    }
+    if (lane == 0) box_sums[warp] = make_double2(area, length);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (uint32_t w = 1; w < 32; ++w) {
+            area += box_sums[w].x;
+            length += box_sums[w].y;
+        }
+        totals->area = area;
+        totals->length = length;
     }
 }
 
@@ -369,7 +406,7 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
     const size_t o_tot = take(sizeof(LayoutTotals)), o_prims = take(d_prims ? 0 : n * sizeof(HostPrim)),
                  o_sph = take(H.spheres.size() * sizeof(SphereRec)), o_flat = take(H.flat_id.size() * 4),
                  o_parent = take((size_t)m * 4), o_rank = take((size_t)m * 4), o_cls = take(m), o_start = take(m),
-                 o_part = take((size_t)nb * 12), o_quad = take(n_pairs * 4);
+                 o_part = take((size_t)nb * 12), o_quad = take(n_pairs * 4), o_sums = take((size_t)nb * sizeof(float2));
     char* ws = nullptr;
     struct Free {
         char*& p;
@@ -396,15 +433,16 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
     auto* start = reinterpret_cast<uint8_t*>(ws + o_start);
     auto* part = reinterpret_cast<uint32_t*>(ws + o_part);
     auto* quad_of = reinterpret_cast<uint32_t*>(ws + o_quad);
+    auto* sums = reinterpret_cast<float2*>(ws + o_sums);
     if (!fits(cudaMemsetAsync(totals, 0, sizeof(LayoutTotals), 0)) ||
         (!d_prims && !fits(cudaMemcpy(ws + o_prims, H.prims.data(), n * sizeof(HostPrim), cudaMemcpyHostToDevice))) ||
         (!H.spheres.empty() && !fits(cudaMemcpy(spheres, H.spheres.data(), H.spheres.size() * sizeof(SphereRec),
                                                 cudaMemcpyHostToDevice))) ||
         (flat && !fits(cudaMemcpy(flat, H.flat_id.data(), H.flat_id.size() * 4, cudaMemcpyHostToDevice))))
         return;
-    k_layout_mark<<<nb, kLayoutBlock>>>(d_nodes, m, prims, d_ordered, parent, cls, part, nb, totals);
+    k_layout_mark<<<nb, kLayoutBlock>>>(d_nodes, m, prims, d_ordered, parent, cls, part, nb, sums, totals);
     k_layout_starts<<<nb, kLayoutBlock>>>(parent, m, cls, start, part, nb, totals);
-    k_layout_scan<<<1, 1024>>>(part, nb, totals);
+    k_layout_scan<<<1, 1024>>>(part, nb, sums, totals);
     k_layout_rank<<<nb, kLayoutBlock>>>(d_nodes, m, cls, start, part, nb, rank, quad_of);
     LayoutTotals T;
     if (!fits(cudaGetLastError()) || !fits(cudaMemcpy(&T, totals, sizeof(T), cudaMemcpyDeviceToHost))) return;
@@ -427,7 +465,7 @@ void device_fill_layout(HostBVH& H, const FlatNode* d_nodes, uint32_t m, const u
     H.wide = wide;
     H.n_quads = T.starts;
     H.stack4_bound = T.stack;
-    tree_reach(H);
+    tree_margins(H, T.area, T.length);
     H.layout = std::move(L);
 }
 

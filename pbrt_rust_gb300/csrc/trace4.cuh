@@ -22,14 +22,18 @@
 // the exact ones:
 //  * the stored planes are rounded outwards;
 //  * a plane's distance is one fused multiply-add, t = code * (scale / d) +
-//    (org - o) / d, where the reference computes (plane - o) * (1 / d).  With
-//    u = 2^-24, R the largest coordinate of the tree and i = |1 / d|, the
-//    rounding of the two forms adds up to at most u i (9.2 R + 5 |o|), |o| the sum of the components (code *
-//    scale is at most 2.8 R, |org| 1.7 R); the near planes are moved towards
-//    the ray's start and the far planes away from it by e = u i (10 R + 8
-//    |o|);
-//  * an axis with d = 0 has 1 / d replaced by kZeroInv, so large that e is
-//    beyond every other distance: a plane at the origin or within e / i of it
+//    (org - o) / d, where the reference computes (plane - o) * (1 / d).  Both
+//    subtractions are exact but for one rounding of their result, so what
+//    matters is how far the tree is from the ray's origin, not how far either
+//    is from the coordinates' zero.  With u = 2^-24, i = |1 / d|, c the middle
+//    of the tree's box on the axis, h half its extent and a few units in the
+//    last place of its coordinates (tree_margins), a node has |org - o| <=
+//    |c - o| + 2.1 h and code * scale <= 4.1 h, and the rounding of the two
+//    forms adds up to at most u i (5 |c - o| + 27 h); the near planes are
+//    moved towards the ray's start and the far planes away from it by
+//    e = u i (6 |c - o| + 32 h);
+//  * an axis with d = 0 has 1 / d replaced by kZeroInv, so large that e, here
+//    of all three axes' sums, is beyond every other distance: a plane at the origin or within e / i of it
 //    never culls, one farther off does.  The exact test has +-inf there, as
 //    the reference.
 // One box may pass where a box above it does not: with d = -0 the reference
@@ -42,10 +46,12 @@
 //
 // All of this needs finite numbers of moderate size.  Trees beyond 2^40 have
 // no 4-wide layout (HostBVH::wide), and a ray that is not `clean` (NaN or
-// infinite components, |o| > 2^40, |d| or 1 / d above 2^60, tmin below
+// infinite components, |c - o| above 2^41, |d| or 1 / d above 2^60, tmin below
 // -2^60) is walked over the binary layout in the exact mode of trace.cuh
 // instead (exact_hit / exact_any), as is a ray that accepted a hit at
-// distance NaN, after which the reference's box tests ignore maxt.  Kernels
+// distance NaN, after which the reference's box tests ignore maxt, and a ray
+// from so far away (DevBVH4::mid.w) that its margins would have it visit most
+// of the tree.  Kernels
 // with one thread per ray do that after the walk; the persistent ones mark
 // the ray for a replay kernel queued behind them, because the call inside
 // their loop costs the walk its registers (2^22 incoherent rays into a
@@ -87,7 +93,7 @@ struct DevBVH4 {
     const QuadNode* nodes;
     const LeafBox* boxes;
     uint32_t root_ref;      // the root's child word
-    float reach;            // 5/4 of the tree's largest coordinate, 2^-50 at least
+    float4 mid, half, spread;  // HostBVH::middle (w: far), ::half, ::spread
 };
 
 // Stack words that are not children (leaf words stay below: HostBVH::wide
@@ -95,10 +101,8 @@ struct DevBVH4 {
 constexpr uint32_t kWalkDone = 0xfffffffdu;  // the bottom of the stack
 constexpr uint32_t kExitInst = 0xfffffffeu;  // ends the walk of an instance definition
 
-constexpr float kRayReach = 1.099511627776e12f;         // 2^40
 constexpr float kInvMax = 1.152921504606846976e18f;     // 2^60, for |d| too
 constexpr float kZeroInv = 1.9342813113834067e25f;      // 2^84, in place of 1 / 0
-constexpr float kMarginUnit = 4.76837158203125e-07f;    // 8 u; DevBVH4::reach is 5/4 R
 
 // An instance definition's 4-wide stack bound is at most 96 (checked at
 // creation) and a binary walk defers no more entries than the 4-wide one.
@@ -212,7 +216,7 @@ template <int BLOCK, int ROWS, bool INST>
 struct alignas(16) WalkShared {
     uint2 stack[ROWS][BLOCK];
     uint2 push[kPushTable];  // the places; by how much the top moves
-    float world[INST ? 9 : 1][INST ? BLOCK : 1];
+    float world[INST ? 12 : 1][INST ? BLOCK : 1];
     // every thread of the block; __syncthreads() inside
     __device__ __forceinline__ void init() {
         if (threadIdx.x < kPushTable)
@@ -279,29 +283,36 @@ struct Walk4 : InstWalk<INST> {
         return base + ((top - base) & (kRow - 1u)) + (uint32_t)i * kRow;
     }
 
-    // 1 / d, octant and margins of the ray (o, d) in a tree of the given
-    // reach; false if the ray is not clean (see above).
-    __device__ __forceinline__ bool aim(float reach) {
+    // 1 / d, octant and margins of the ray (o, d) in a tree; false if the ray
+    // is not clean or too far away (see above).
+    __device__ __forceinline__ bool aim(const DevBVH4& tree) {
         const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
         ix = 1.0f / dx;
         iy = 1.0f / dy;
         iz = 1.0f / dz;
-        // sums, so that a NaN component fails the comparison
-        const float so = fabsf(ox) + fabsf(oy) + fabsf(oz), sd = fabsf(dx) + fabsf(dy) + fabsf(dz);
-        bool ok = so <= kRayReach && sd <= kInvMax && sd > 0.0f && tmin >= -kInvMax && maxt == maxt &&
+        // a sum, so that a NaN component fails the comparison
+        const float sd = fabsf(dx) + fabsf(dy) + fabsf(dz);
+        bool ok = sd <= kInvMax && sd > 0.0f && tmin >= -kInvMax && maxt == maxt &&
                   max3f(zx ? 0.0f : fabsf(ix), zy ? 0.0f : fabsf(iy), zz ? 0.0f : fabsf(iz)) <= kInvMax;
         if (zx) ix = copysignf(kZeroInv, dx);
         if (zy) iy = copysignf(kZeroInv, dy);
         if (zz) iz = copysignf(kZeroInv, dz);
-        margins(reach);
-        return ok;
+        octant();
+        return margins(tree, zx, zy, zz) && ok;
     }
-    __device__ __forceinline__ void margins(float reach) {
+    __device__ __forceinline__ void octant() {
         oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) | ((__float_as_uint(iz) >> 31) << 2));
-        const float m = kMarginUnit * (reach + (fabsf(ox) + fabsf(oy) + fabsf(oz)));
-        ex = m * fabsf(ix);
-        ey = m * fabsf(iy);
-        ez = m * fabsf(iz);
+    }
+    // false: too far away, or a NaN in the origin.
+    __device__ __forceinline__ bool margins(const DevBVH4& tree, bool zx, bool zy, bool zz) {
+        const float4 mid = tree.mid, spread = tree.spread;
+        const float mx = __fmaf_rn(kFarMargin, fabsf(mid.x - ox), spread.x),
+                    my = __fmaf_rn(kFarMargin, fabsf(mid.y - oy), spread.y),
+                    mz = __fmaf_rn(kFarMargin, fabsf(mid.z - oz), spread.z), all = mx + my + mz;
+        ex = (zx ? all : mx) * fabsf(ix);
+        ey = (zy ? all : my) * fabsf(iy);
+        ez = (zz ? all : mz) * fabsf(iz);
+        return all <= mid.w;
     }
     // The ray with the reference's 1 / d, for the exact tests.
     __device__ __forceinline__ DRay ray() const {
@@ -343,14 +354,14 @@ struct Walk4 : InstWalk<INST> {
             this->base_ = 0;
         }
         if (bvh.pair.empty) return kStartMiss;
-        if (!aim(bvh.reach)) return kStartExact;
-        // the root's box by the same conservative test
-        const ChildRec& R = bvh.pair.root;
-        const float ax = (R.lo_x - ox) * ix, bx = (R.hi_x - ox) * ix;
-        const float ay = (R.lo_y - oy) * iy, by = (R.hi_y - oy) * iy;
-        const float az = (R.lo_z - oz) * iz, bz = (R.hi_z - oz) * iz;
-        const float t0 = max3f(fminf(ax, bx) - ex, fminf(ay, by) - ey, fmaxf(fminf(az, bz) - ez, tmin));
-        const float t1 = min3f(fmaxf(ax, bx) + ex, fmaxf(ay, by) + ey, fminf(fmaxf(az, bz) + ez, maxt));
+        if (!aim(bvh)) return kStartExact;
+        // the root's box, from its middle, with the same margins (this form's
+        // rounding: u i (5 |c - o| + 4 h) against the reference's)
+        const float tx = (bvh.mid.x - ox) * ix, rx = __fmaf_rn(bvh.half.x, fabsf(ix), ex);
+        const float ty = (bvh.mid.y - oy) * iy, ry = __fmaf_rn(bvh.half.y, fabsf(iy), ey);
+        const float tz = (bvh.mid.z - oz) * iz, rz = __fmaf_rn(bvh.half.z, fabsf(iz), ez);
+        const float t0 = max3f(tx - rx, ty - ry, fmaxf(tz - rz, tmin));
+        const float t1 = min3f(tx + rx, ty + ry, fminf(tz + rz, maxt));
         if (t0 > t1) return kStartMiss;
         cur = bvh.root_ref;
         return kStartWalk;
@@ -494,9 +505,9 @@ struct Walk4 : InstWalk<INST> {
         xf_point(S->w2o, ox, oy, oz, o);  // transform.rs:230-237
         xf_vector(S->w2o, dx, dy, dz, d);
         float* w = &sh.world[0][threadIdx.x];
-        const float keep[9] = {ox, oy, oz, dx, dy, dz, ix, iy, iz};
+        const float keep[12] = {ox, oy, oz, dx, dy, dz, ix, iy, iz, ex, ey, ez};
 #pragma unroll
-        for (int k = 0; k < 9; ++k) w[k * BLOCK] = keep[k];
+        for (int k = 0; k < 12; ++k) w[k * BLOCK] = keep[k];
         ox = o[0];
         oy = o[1];
         oz = o[2];
@@ -505,7 +516,7 @@ struct Walk4 : InstWalk<INST> {
         dz = d[2];
         const ChildRec& R = D.pair.root;
         float tr;
-        if (!aim(D.reach)) return 2;
+        if (!aim(D)) return 2;
         if (!slab(R.lo_x, R.lo_y, R.lo_z, R.hi_x, R.hi_y, R.hi_z, ray(), maxt, &tr)) {
             restore(bvh, sh);
             return 0;
@@ -537,7 +548,10 @@ struct Walk4 : InstWalk<INST> {
         ix = w[6 * BLOCK];
         iy = w[7 * BLOCK];
         iz = w[8 * BLOCK];
-        margins(bvh.reach);
+        ex = w[9 * BLOCK];
+        ey = w[10 * BLOCK];
+        ez = w[11 * BLOCK];
+        octant();
         if constexpr (INST) {
             this->nodes_ = bvh.nodes;
             this->prims_ = bvh.pair.prims;
@@ -576,14 +590,23 @@ struct Walk4 : InstWalk<INST> {
                 const LeafBox* b = boxes + (flags >> kPrimBoxShift);
                 const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
                 float tr;
-                if (!slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr)) return false;
-                if ((ix != -kZeroInv || lo.x != hi.x) && (iy != -kZeroInv || lo.y != hi.y) &&
-                    (iz != -kZeroInv || lo.z != hi.z))
-                    return true;
-                give_up();  // one above it need not pass; the pop ends the walk
-                return false;
+                return slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr);
+            };
+            // Gives up if the leaf's box, the one of flag word f, is flat where
+            // the direction is -0: a box above it need not pass.  Asked for
+            // when an analytic shape is hit, or an instance's leaf entered.
+            auto beside = [&](uint32_t f) {
+                if (min3f(ix, iy, iz) != -kZeroInv) return false;
+                const LeafBox* b = boxes + (f >> kPrimBoxShift);
+                const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
+                if (!((ix == -kZeroInv && lo.x == hi.x) || (iy == -kZeroInv && lo.y == hi.y) ||
+                      (iz == -kZeroInv && lo.z == hi.z)))
+                    return false;
+                give_up();
+                return true;
             };
             if ((flags & kPrimBoxEntry) && !table_box()) break;
+            if (INST && (flags & kPrimBoxEntry) && beside(flags)) break;
             float t, u = 0.0f, v = 0.0f;
             bool hit;
             if (id & kSphereBit) {
@@ -602,6 +625,10 @@ struct Walk4 : InstWalk<INST> {
                 }
                 hit = sphere_test(spheres, si, ray(), maxt, &t);
                 if (hit && (flags & kPrimHitBox)) hit = table_box();
+                if (hit && (flags & kPrimHitBox) && beside(flags)) break;
+                if (!INST && hit && !(flags & kPrimHitBox) &&
+                    beside(__float_as_uint(__ldg(&prims[cur & ~kNode4Leaf].r2[3]))))
+                    break;
             } else {
                 hit = tri_test(r0, r1, r2, ray(), maxt, &t, &u, &v);
                 if (hit && (flags & kPrimOwnBox)) {

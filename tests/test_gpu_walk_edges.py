@@ -113,3 +113,32 @@ def test_walks_whose_stack_runs_out(oracle, n, ratio, where):
                  Primitive.transformed(lump, at.inverse())]
     _, want = check(oracle, prims, r, 1, "middle")
     assert (want["prim"] >= 0).any()
+
+
+@pytest.mark.parametrize("on_device", [False, True])
+@pytest.mark.parametrize("kind", ["soup", "instanced"])
+@pytest.mark.parametrize("offset", [0.0, 3.0e3, 2.0e5])
+def test_rays_from_afar_and_trees_off_the_origin(oracle, offset, kind, on_device):
+    """Margins from a small part of the boxes to many times the whole tree,
+    beyond which rays take the exact walk, some of them axis-parallel."""
+    rng = np.random.default_rng(8)
+    at = np.array([offset, -0.5 * offset, 2.0 * offset])
+    prims = [Primitive.simple(mesh(soup(rng, 400, 1.0, 0.15, at)))]
+    if kind == "instanced":
+        lump = InstanceDefinition([Primitive.simple(mesh(soup(rng, 200, 1.0, 0.15)))])
+        for k in range(6):
+            place = Transform.translate(tuple(float(v) for v in at + rng.uniform(-2, 2, 3))) * Transform.rotate(
+                30.0 * k, (0.0, 1.0, 0.0))
+            prims.append(Primitive.transformed(lump, place.inverse()))
+    n = 3000
+    u = rng.standard_normal((n, 3))
+    u[::5] = np.eye(3)[rng.integers(0, 3, len(u[::5]))]
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    far = 10.0 ** rng.uniform(0, 7, (n, 1))
+    r = np.zeros(n, abi.RAY_DTYPE)
+    r["o"] = at + rng.uniform(-1, 1, (n, 3)) + u * far
+    r["d"] = -u * 10.0 ** rng.uniform(-3, 3, (n, 1))
+    r["tmax"] = np.inf
+    _, want = check(oracle, prims, r, on_device=on_device)
+    hit = want["prim"] >= 0
+    assert hit[far[:, 0] < 100].any() and hit[far[:, 0] > 1.0e5].any()
