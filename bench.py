@@ -293,7 +293,9 @@ def bench_served(torch, dev, stream, n_scenes: int = 32, n_requests: int = 2000,
         plain_lat[rk] = run_plain(reqs, stream)
         plain_s[rk] = time.perf_counter() - t0
     abi.set_trace_config(**before)
-    default_rk = before["render_kernel"] if before["render_kernel"] in plain_s else "plain"
+    # "auto" takes the 4-wide walk for scenes of this size
+    default_rk = {"auto": "w4"}.get(before["render_kernel"], before["render_kernel"])
+    default_rk = default_rk if default_rk in plain_s else "plain"
 
     def pct(lat, q):  # milliseconds
         return float(np.percentile(np.asarray(lat) * 1e3, q))

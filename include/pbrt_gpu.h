@@ -310,7 +310,7 @@ int pbrtgpu_intersect_streamed(const PbrtBVH* bvh, const PbrtRay* rays,
  * do not depend on the choice.  The first value is also read from the
  * environment (PBRT_TRACE_KERNEL = plain | pt | w4 | w4pt | w4spec | packet,
  * PBRT_TRACE_REFILL = 1..32, PBRT_TRACE_MINB = 0 | 8 | 9,
- * PBRT_RENDER_KERNEL = plain | w4 | packet, PBRT_TRACE_REORDER = 0 | 1,
+ * PBRT_RENDER_KERNEL = auto | plain | w4 | packet, PBRT_TRACE_REORDER = 0 | 1,
  * PBRT_TRACE_CHUNK = 0 | 32..4096) when no call has set it. */
 enum {
     PBRT_TRACE_PAIR = 0,            /* binary pairs, one thread per ray */
@@ -318,9 +318,11 @@ enum {
     PBRT_TRACE_WIDE = 2,            /* 4-wide nodes, one thread per ray */
     PBRT_TRACE_WIDE_PERSISTENT = 3, /* 4-wide nodes, persistent warps */
     PBRT_TRACE_WIDE_SPECULATIVE = 4, /* the same walk as PBRT_TRACE_WIDE_PERSISTENT */
-    PBRT_TRACE_PAIR_PACKET = 5       /* binary pairs, one thread per ray; a warp whose rays share their
+    PBRT_TRACE_PAIR_PACKET = 5,      /* binary pairs, one thread per ray; a warp whose rays share their
                                         direction signs walks them together, node by node, each lane
                                         testing what its own walk tests (coherent rays) */
+    PBRT_TRACE_AUTO = 6              /* render_kernel only: PBRT_TRACE_PAIR for trees of fewer than
+                                        4096 primitives, PBRT_TRACE_WIDE for larger ones */
 };
 typedef struct PbrtTraceConfig {
     int32_t kernel;         /* PBRT_TRACE_*: pbrtgpu_intersect / intersect_p batches */
@@ -330,8 +332,7 @@ typedef struct PbrtTraceConfig {
                                are streamed with 0 only */
     int32_t render_kernel;  /* PBRT_TRACE_*: camera rays inside pbrtgpu_render; shadow
                                rays take the 4-wide kernel with a 4-wide choice, else
-                               the binary one.  The default, PBRT_TRACE_WIDE, takes the
-                               binary kernels for trees of fewer than 4096 primitives */
+                               the binary one.  Default: PBRT_TRACE_AUTO */
     uint32_t reorder;       /* 1: pbrtgpu_intersect / intersect_p batches of 32768 rays
                                or more are binned by direction and origin before
                                traversal (same results, more coherent warps) */

@@ -121,7 +121,7 @@ class PbrtTraceConfig(C.Structure):
                 ("render_kernel", C.c_int32), ("reorder", C.c_uint32), ("chunk", C.c_uint32)]
 
 
-TRACE_KERNELS = {"plain": 0, "pt": 1, "w4": 2, "w4pt": 3, "w4spec": 4, "packet": 5}
+TRACE_KERNELS = {"plain": 0, "pt": 1, "w4": 2, "w4pt": 3, "w4spec": 4, "packet": 5, "auto": 6}
 FILTERS = {"box": 0, "triangle": 1, "gaussian": 2, "mitchell": 3, "lanczos": 4}
 
 
@@ -271,8 +271,9 @@ def get_trace_config() -> dict:
 def set_trace_config(kernel: str | None = None, refill: int | None = None, min_blocks: int | None = None,
                      render_kernel: str | None = None, reorder: bool | None = None,
                      chunk: int | None = None) -> None:
-    """Choose the traversal kernels ('plain', 'pt', 'w4', 'w4pt') and their
-    options; unset fields keep their current value."""
+    """Choose the traversal kernels ('plain', 'pt', 'w4', 'w4pt', 'packet';
+    for renders also 'auto', by the tree's size) and their options; unset
+    fields keep their current value."""
     lib = load()
     cur = get_trace_config()
     cfg = PbrtTraceConfig(TRACE_KERNELS[kernel or cur["kernel"]], refill or cur["refill"],

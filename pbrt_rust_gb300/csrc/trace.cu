@@ -411,12 +411,13 @@ enum {
     kVariantWidePlain = 2,
     kVariantWidePersistent = 3,
     kVariantWideSpeculative = 4,
-    kVariantPairPacket = 5
+    kVariantPairPacket = 5,
+    kVariantAuto = PBRT_TRACE_AUTO  // renders: by the tree's size
 };
 static int g_kernel_variant = -1;
 static unsigned g_refill = 4;
 static unsigned g_min_blocks = 0;
-static int g_render_kernel = kVariantWidePlain;
+static int g_render_kernel = kVariantAuto;
 static unsigned g_reorder = 0;
 static unsigned g_chunk = 64;
 
@@ -450,8 +451,7 @@ static void read_variant() {
         if (!strcmp(v, "0") || !strcmp(v, "1")) g_reorder = (unsigned)(v[0] - '0');
     }
     if (const char* v = getenv("PBRT_RENDER_KERNEL")) {
-        int k = variant_from_name(v, g_render_kernel);
-        if (k >= kVariantPairPlain && k <= kVariantPairPacket) g_render_kernel = k;
+        g_render_kernel = strcmp(v, "auto") ? variant_from_name(v, g_render_kernel) : (int)kVariantAuto;
     }
 }
 
@@ -573,7 +573,7 @@ static cudaError_t launch_wide(const DevBVH4& bvh, const float4* r4, uint32_t n,
 int set_trace_config(const PbrtTraceConfig& c) {
     if (c.kernel < kVariantPairPlain || c.kernel > kVariantPairPacket || c.refill < 1 || c.refill > 32) return 1;
     if (!(c.min_blocks == 0 || c.min_blocks == 7 || c.min_blocks == 8 || c.min_blocks == 9)) return 1;
-    if (c.render_kernel < kVariantPairPlain || c.render_kernel > kVariantPairPacket) return 1;
+    if (c.render_kernel < kVariantPairPlain || c.render_kernel > kVariantAuto) return 1;
     if (c.reorder > 1) return 1;
     if (!(c.chunk == 0 || (c.chunk >= 32 && c.chunk <= 4096 && c.chunk % 32 == 0))) return 1;
     read_variant();
@@ -602,17 +602,18 @@ bool trace_reorder() {
     read_variant();
     return g_reorder != 0;
 }
-// A tree of a few thousand primitives sits in L1, where a binary visit's
-// fewer instructions win over the 4-wide walk's fewer steps.  Camera + shadow
-// rays of 512 x 512 x 4 frames, binary against 4-wide, us: terrains of 300 /
-// 2000 / 20000 triangles 84 / 134 / 251 against 95 / 144 / 221, 64 spheres
-// 100 against 117, soups of 300 / 1000 / 4000 triangles 61 / 97 / 241 against
-// 58 / 78 / 168: the line is where no scene is slower.
+// The choice of kVariantAuto.  Which walk a small tree's frame is faster with
+// depends on the visits per ray, not on the tree's size alone.  Camera + shadow rays of
+// 512 x 512 x 4 frames, binary against 4-wide, us: terrains of 300 / 2000 /
+// 20000 triangles 84 / 134 / 251 against 95 / 144 / 221, 64 spheres 100 against
+// 117, soups of 300 / 1000 / 4000 triangles 61 / 97 / 241 against 58 / 78 / 168.
+// The line is where none of them is slower than with the binary walk; soups
+// below it would be faster with PBRT_TRACE_WIDE.
 constexpr uint32_t kWideRenderPrims = 4096;
 int render_trace_kernel(uint32_t n_prims) {
     read_variant();
-    return g_render_kernel == kVariantWidePlain && n_prims < kWideRenderPrims ? (int)kVariantPairPlain
-                                                                              : g_render_kernel;
+    if (g_render_kernel != kVariantAuto) return g_render_kernel;
+    return n_prims < kWideRenderPrims ? kVariantPairPlain : kVariantWidePlain;
 }
 
 int wide_stack_variant(uint32_t bound) {
