@@ -907,19 +907,22 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
         pool_nodes += 2ull * (j.hi - j.lo) - 1;
     }
     Buf d_jobs, d_outs, d_roots;
-    CK(cudaMalloc(&d_pool.p, pool_nodes * sizeof(PoolNode)));
-    CK(cudaMalloc(&d_jobs.p, (size_t)NJ * sizeof(Job)));
-    CK(cudaMalloc(&d_outs.p, (size_t)NJ * sizeof(JobOut)));
-    CK(cudaMalloc(&d_roots.p, (size_t)NJ * sizeof(PoolNode)));
-    CK(cudaMemcpy(d_jobs.p, jobs.data(), (size_t)NJ * sizeof(Job), cudaMemcpyHostToDevice));
-    k_b_build<<<(NJ + kBWarps - 1) / kBWarps, 32 * kBWarps>>>(P, d_idx.as<uint32_t>(), d_jobs.as<Job>(), NJ,
-                                                              d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp, split);
-    k_b_roots<<<(NJ + 127) / 128, 128>>>(d_pool.as<PoolNode>(), d_jobs.as<Job>(), NJ, d_roots.as<PoolNode>());
-    CK(cudaGetLastError());
     std::vector<JobOut> outs(NJ);
     std::vector<PoolNode> roots(NJ);
-    CK(cudaMemcpy(outs.data(), d_outs.p, (size_t)NJ * sizeof(JobOut), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(roots.data(), d_roots.p, (size_t)NJ * sizeof(PoolNode), cudaMemcpyDeviceToHost));
+    if (NJ) {  // none if no range beyond kSmall primitives could be split
+        CK(cudaMalloc(&d_pool.p, pool_nodes * sizeof(PoolNode)));
+        CK(cudaMalloc(&d_jobs.p, (size_t)NJ * sizeof(Job)));
+        CK(cudaMalloc(&d_outs.p, (size_t)NJ * sizeof(JobOut)));
+        CK(cudaMalloc(&d_roots.p, (size_t)NJ * sizeof(PoolNode)));
+        CK(cudaMemcpy(d_jobs.p, jobs.data(), (size_t)NJ * sizeof(Job), cudaMemcpyHostToDevice));
+        k_b_build<<<(NJ + kBWarps - 1) / kBWarps, 32 * kBWarps>>>(P, d_idx.as<uint32_t>(), d_jobs.as<Job>(), NJ,
+                                                                  d_pool.as<PoolNode>(), d_outs.as<JobOut>(), mp,
+                                                                  split);
+        k_b_roots<<<(NJ + 127) / 128, 128>>>(d_pool.as<PoolNode>(), d_jobs.as<Job>(), NJ, d_roots.as<PoolNode>());
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(outs.data(), d_outs.p, (size_t)NJ * sizeof(JobOut), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(roots.data(), d_roots.p, (size_t)NJ * sizeof(PoolNode), cudaMemcpyDeviceToHost));
+    }
     CK(cudaMemcpy(H.ordered.data(), d_idx.p, n * 4, cudaMemcpyDeviceToHost));
     for (const JobOut& o : outs)
         if (o.err) {
@@ -982,8 +985,10 @@ int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {
     for (Buf* b : {&d_lo, &d_hi, &d_c[0], &d_c[1], &d_c[2], &d_tmp}) b->reset();  // room for the nodes
     Buf d_nodes, d_at, d_top;
     CK(cudaMalloc(&d_nodes.p, (size_t)m * sizeof(FlatNode)));
-    CK(cudaMalloc(&d_at.p, (size_t)NJ * 4));
-    CK(cudaMemcpy(d_at.p, job_at.data(), (size_t)NJ * 4, cudaMemcpyHostToDevice));
+    if (NJ) {
+        CK(cudaMalloc(&d_at.p, (size_t)NJ * 4));
+        CK(cudaMemcpy(d_at.p, job_at.data(), (size_t)NJ * 4, cudaMemcpyHostToDevice));
+    }
     if (!top.empty()) {
         CK(cudaMalloc(&d_top.p, top.size() * sizeof(TopNode)));
         CK(cudaMemcpy(d_top.p, top.data(), top.size() * sizeof(TopNode), cudaMemcpyHostToDevice));

@@ -142,3 +142,22 @@ def test_rays_from_afar_and_trees_off_the_origin(oracle, offset, kind, on_device
     _, want = check(oracle, prims, r, on_device=on_device)
     hit = want["prim"] >= 0
     assert hit[far[:, 0] < 100].any() and hit[far[:, 0] > 1.0e5].any()
+
+
+@pytest.mark.parametrize("method", ["sah", "middle"])
+@pytest.mark.parametrize("n", [32, 33, 64, 2048, 2049, 5000])
+def test_a_device_build_of_coincident_primitives_is_one_leaf(oracle, n, method):
+    """Nothing to split at any size, so no small ranges either."""
+    from pbrt_rust_gb300.gpu import GpuBVHAccel
+    t = np.array([[-1, -1, 0], [1, -1, 0], [0, 1, 0]], np.float32)
+    prims = [mesh(np.tile(t, (n, 1, 1)))]
+    r = np.zeros(64, abi.RAY_DTYPE)
+    r["o"] = np.random.default_rng(n).uniform(-0.7, 0.7, (64, 3)) + np.array([0, 0, 3])
+    r["d"] = (0.0, 0.0, -1.0)
+    r["tmax"] = np.inf
+    dev, want = check(oracle, prims, r, 4, method, on_device=True)
+    host = GpuBVHAccel(prims, 4, method)
+    assert host.nodes().tobytes() == dev.nodes().tobytes() and len(host.nodes()) == 1
+    assert np.array_equal(host.primitive_order(), dev.primitive_order())
+    assert host.device_bytes() == dev.device_bytes()
+    assert (want["prim"] >= 0).any()
