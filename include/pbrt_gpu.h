@@ -327,9 +327,8 @@ enum {
 typedef struct PbrtTraceConfig {
     int32_t kernel;         /* PBRT_TRACE_*: pbrtgpu_intersect / intersect_p batches */
     uint32_t refill;        /* persistent kernels: refill a warp when this many lanes idle */
-    uint32_t min_blocks;    /* 0, 7, 8 or 9: no effect on the walk, whose 64 registers per thread
-                               keep 8 128-thread blocks per SM resident; host-buffer calls
-                               are streamed with 0 only */
+    uint32_t min_blocks;    /* 0, 7, 8 or 9: no effect (the walk's 64 registers per thread
+                               keep 8 128-thread blocks per SM resident) */
     int32_t render_kernel;  /* PBRT_TRACE_*: camera rays inside pbrtgpu_render; shadow
                                rays take the 4-wide kernel with a 4-wide choice, else
                                the binary one.  Default: PBRT_TRACE_AUTO */

@@ -421,6 +421,11 @@ static int g_render_kernel = kVariantAuto;
 static unsigned g_reorder = 0;
 static unsigned g_chunk = 64;
 
+// Queries take the 4-wide persistent walk (under either of its names).
+static bool wide_persistent() {
+    return g_kernel_variant == kVariantWidePersistent || g_kernel_variant == kVariantWideSpeculative;
+}
+
 static int variant_from_name(const char* v, int dflt) {
     if (!strcmp(v, "plain")) return kVariantPairPlain;
     if (!strcmp(v, "pt")) return kVariantPairPersistent;
@@ -539,7 +544,7 @@ uint32_t rays_per_warp(uint64_t n) {
 static uint64_t small_call_rays() { return 8ull * kWalkBlock * (uint64_t)device_sms(); }
 bool trace_is_small(const DevBVH4* wide, uint32_t wide_bound, uint32_t n) {
     read_variant();
-    return wide && wide_stack_variant(wide_bound) && g_kernel_variant == kVariantWidePersistent && !g_reorder &&
+    return wide && wide_stack_variant(wide_bound) && wide_persistent() && !g_reorder &&
            n <= small_call_rays();
 }
 
@@ -733,7 +738,7 @@ bool trace_streams(const DevBVH& bvh, const DevBVH4* wide, uint32_t wide_bound, 
     read_variant();
     if (!wide || !wide_stack_variant(wide_bound) || !g_chunk || g_reorder || n > 0xF0000000u) return false;
     // scenes with instances always take the 4-wide persistent walk
-    return bvh.insts != nullptr || (g_kernel_variant == kVariantWidePersistent && g_min_blocks == 0);
+    return bvh.insts != nullptr || wide_persistent();
 }
 
 // The launch of a streamed-input or write-out call: the 4-wide persistent

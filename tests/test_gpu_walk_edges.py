@@ -1,6 +1,8 @@
 """Rays and trees at the edges of what the 4-wide walk (trace4.cuh) takes: the
 hits are the oracle's bit for bit whichever walk a ray ends up in, so no
 tolerance is involved."""
+import re
+
 import numpy as np
 import pytest
 
@@ -161,3 +163,34 @@ def test_a_device_build_of_coincident_primitives_is_one_leaf(oracle, n, method):
     assert np.array_equal(host.primitive_order(), dev.primitive_order())
     assert host.device_bytes() == dev.device_bytes()
     assert (want["prim"] >= 0).any()
+
+
+@pytest.mark.parametrize("setting", [dict(kernel="w4spec"), dict(min_blocks=8)])
+def test_settings_that_name_the_default_walk_take_its_kernels(setting):
+    """The same kernels as by default, for calls of few rays and for pinned
+    host buffers, and the same hits bit for bit."""
+    import torch
+
+    from pbrt_rust_gb300.gpu import GpuBVHAccel
+    from test_gpu_render_choice import kernels_of
+    bvh = GpuBVHAccel([mesh(soup(np.random.default_rng(5), 4000, 1.0, 0.1))])
+    rng = np.random.default_rng(6)
+    r = np.zeros(1 << 18, abi.RAY_DTYPE)
+    r["o"], r["tmax"] = rng.uniform(-2, 2, (len(r), 3)), np.inf
+    r["d"] = rng.uniform(-1, 1, (len(r), 3)) - r["o"]
+    host = torch.from_numpy(r.view(np.float32).reshape(-1, 8)).pin_memory()
+    few, out = host[:500].cuda(), torch.empty((len(r), 4)).pin_memory()
+
+    def both():
+        names = [set(re.findall(r"k_\w+(?:<[^>]*>)?", kernels_of(f)))
+                 for f in (lambda: bvh.intersect(few), lambda: bvh.intersect(host, out=out))]
+        return names, bvh.intersect(few).cpu().numpy().tobytes(), out.numpy().tobytes()
+    want = both()
+    before = abi.get_trace_config()
+    abi.set_trace_config(**setting)
+    try:
+        got = both()
+    finally:
+        abi.set_trace_config(**before)
+    assert got[1:] == want[1:]
+    assert got[0] == want[0], (got[0], want[0])
