@@ -383,8 +383,8 @@ int pbrtgpu_render_tasks(const PbrtScene* scene, const PbrtCameraDesc* camera, c
  * loop that cannot afford the device-wide synchronisation cudaMalloc and
  * cudaFree may cause.  Its scratch is one static array of 64 MiB of device
  * memory, present on every GPU where the library's code is loaded until the
- * process exits; a frame needing more (about 220 bytes per sample with two
- * lights, e.g. 256x256 at 4 spp) is refused with PBRT_ERR_BUDGET, and
+ * process exits; a frame needing more (about 206 bytes per sample with two
+ * lights: 280x280 at 4 spp fits) is refused with PBRT_ERR_BUDGET, and
  * num_tasks is limited to 256; windows beyond 2^32 - 1 pixels or
  * samples x lights are refused with PBRT_ERR_INVALID_ARGUMENT.  The scene
  * must have its device copy (pbrtgpu_scene_create makes it when a device is

@@ -173,7 +173,6 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     P.filter_xw = cam->filter_x_width;
     P.filter_yw = cam->filter_y_width;
     P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
-    P.filter_flat = cam->filter_kind == PBRT_FILTER_BOX ? 1u : 0u;
     P.filter_inv_xw = 1.0f / cam->filter_x_width;
     P.filter_inv_yw = 1.0f / cam->filter_y_width;
     gather_offsets(cam->filter_x_width, P.sx0, P.sx1, &P.gx0, &P.gx1);
@@ -211,8 +210,8 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
     const uint64_t S_ = P.n_samples, SL = P.n_samples * (uint64_t)nl;
     const uint64_t npx = (uint64_t)(P.fx1 - P.fx0) * (uint64_t)(P.fy1 - P.fy0);
     const bool dev_out = is_device_pointer(rgb_out);
-    void *p_rays, *p_hits, *p_img, *p_pixbox, *p_lsamp, *p_contrib, *p_le, *p_L, *p_srays, *p_sslot, *p_occ, *p_cnt, *p_tasks,
-        *p_table, *p_rgb = nullptr;
+    void *p_rays, *p_hits, *p_img, *p_pixbox, *p_lsamp, *p_contrib, *p_L, *p_srays, *p_sslot, *p_occ, *p_cnt, *p_tasks,
+        *p_table = nullptr, *p_rgb = nullptr;
     auto layout = [&](Carve& c) {
         p_rays = c.take(S_ * sizeof(PbrtRay));
         p_hits = c.take(S_ * 16);
@@ -220,14 +219,13 @@ extern "C" int pbrtgpu_render_noalloc(const PbrtScene* cS, const PbrtCameraDesc*
         p_pixbox = c.take((uint64_t)P.n_pixels * 16);
         p_lsamp = c.take(S_ * 3 * nl * 4 + 4);
         p_contrib = c.take(SL * 16 + 16);
-        p_le = c.take(S_ * 16);
         p_L = c.take(S_ * 16);
         p_srays = c.take(SL * sizeof(PbrtRay) + 32);
         p_sslot = c.take(SL * 4 + 4);
         p_occ = c.take(SL + 1);
         p_cnt = c.take(64);
         p_tasks = c.take(smp->num_tasks * sizeof(TaskRec));
-        p_table = c.take(sizeof(table));
+        if (!P.filter_flat) p_table = c.take(sizeof(table));  // a box filter's is not read
         if (!dev_out) p_rgb = c.take(npx * 3 * 4);
     };
     Carve probe{nullptr, 0};
