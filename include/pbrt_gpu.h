@@ -570,7 +570,7 @@ int pbrtgpu_server_reset_stats(PbrtServer* server);
  * counter + n_blocks - 1 of the ChaCha state (the four constants, key[8],
  * the 64-bit block counter in words 12-13, the 64-bit stream id in words
  * 14-15) after `rounds` rounds (8, 12 or 20), by the device routine the
- * sampler uses (paired = 1: the two-block routine, n_blocks even); 16
+ * sampler uses, one block at a time (paired = 1: the same, n_blocks even); 16
  * words per block into host memory `out`.  StdRng is rounds = 12,
  * stream_id = 0.  pbrtgpu_rng_words: words [first_word, first_word +
  * n_words) of RNG::new(seed)'s u32 stream (rng.rs:11-13) as the render

@@ -540,13 +540,13 @@ int pbrtgpu_chacha_blocks(const uint32_t key[8], uint64_t counter, uint64_t stre
     if (rounds != 8 && rounds != 12 && rounds != 20)
         return set_error(PBRT_ERR_INVALID_ARGUMENT, "rounds must be 8, 12 or 20");
     if (n_blocks > (1u << 20)) return set_error(PBRT_ERR_INVALID_ARGUMENT, "at most 2^20 blocks per call");
-    if (paired && (n_blocks & 1u)) return set_error(PBRT_ERR_INVALID_ARGUMENT, "the paired routine needs an even count");
+    if (paired && (n_blocks & 1u)) return set_error(PBRT_ERR_INVALID_ARGUMENT, "paired blocks need an even count");
     if (!n_blocks) return PBRT_OK;
     if (!cuda_device_present()) return set_error(PBRT_ERR_NO_DEVICE, "no CUDA device");
     const size_t bytes = (size_t)n_blocks * 64;
     uint32_t* d = nullptr;
     int st = cuda_status(cudaMalloc((void**)&d, bytes), "cudaMalloc");
-    if (!st) st = cuda_status(launch_chacha_blocks(key, counter, stream_id, rounds, paired != 0, n_blocks, d, 0),
+    if (!st) st = cuda_status(launch_chacha_blocks(key, counter, stream_id, rounds, n_blocks, d, 0),
                               "chacha launch");
     if (!st) st = cuda_status(cudaMemcpy(out, d, bytes, cudaMemcpyDeviceToHost), "D2H");
     if (d) cudaFree(d);
