@@ -116,12 +116,14 @@ cudaError_t launch_batch_stages(const BatchArgs& A, const BatchTuning& T, bool m
     };
     const bool b256 = T.block == 256;
     if ((e = b256 ? stage(kb_generate<256>) : stage(kb_generate<128>)) != cudaSuccess) return e;
-    if ((e = launch_batch_trace(A, T, false, mixed, inst, queries, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
+    if ((e = launch_batch_trace(A, T, false, mixed, inst, queries, cover_pair, cover_wide, sms, s)) != cudaSuccess)
+        return e;
     ++*launches;
     if ((e = launch_batch_replay(A, T, false, sms, s)) != cudaSuccess) return e;
     ++*launches;
     if ((e = b256 ? stage(kb_shade<256>) : stage(kb_shade<128>)) != cudaSuccess) return e;
-    if ((e = launch_batch_trace(A, T, true, false, inst, false, cover_pair, cover_wide, sms, s)) != cudaSuccess) return e;
+    if ((e = launch_batch_trace(A, T, true, false, inst, false, cover_pair, cover_wide, sms, s)) != cudaSuccess)
+        return e;
     ++*launches;
     if (T.shadow_wide && !inst && T.refill_shadow < 32) {  // the shadow walk that marks rays
         if ((e = launch_batch_replay(A, T, true, sms, s)) != cudaSuccess) return e;

@@ -760,7 +760,6 @@ __global__ void __launch_bounds__(256) k_set_bounds(const PrimBounds* __restrict
 // (240 MB) they make room and are uploaded again.
 constexpr size_t kKeepPrims = 1u << 22;
 
-
 }  // namespace
 
 int device_build_tree(HostBVH& H, uint32_t mp, int split, std::string* err) {

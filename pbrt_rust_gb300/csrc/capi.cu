@@ -287,10 +287,10 @@ static int launch_batch(PbrtBVH* b, const PbrtRay* d_rays, uint32_t n, PbrtHit* 
 // at every call) the traversal reads the rays and writes the results there
 // directly, with no staging copies; by default pinned buffers take the
 // streamed form (trace_streamed) and other host buffers the copy pipeline
-// below.  Measured with 2^22 heightfield rays in pinned buffers on GB300
-// boxes: in place 1.57-1.99 ms per call depending on the box (its scattered
-// 16-byte stores run at 37 GB/s across the link on some boxes), the copy
-// pipeline 1.68-1.76 ms, the streamed form 1.48 ms.  Identical results.
+// below.  2^22 heightfield rays in pinned buffers, closest / any hit (walk
+// alone 0.69 / 0.60 ms): in place 1.67 / 1.52 ms per call (its scattered
+// 16-byte stores cross the link at a fifth of its bandwidth), the copy pipeline
+// 1.21 / 1.01, the streamed form 1.01 / 0.90.  Identical results.
 static bool host_mapped_enabled() {
     const char* v = getenv("PBRT_HOST_MAPPED");
     return v && v[0] == '1';
@@ -309,9 +309,9 @@ static void* mapped_host_pointer(const void* p) {
 // pipe_chunks() chunks (PBRT_PIPE_CHUNKS: 1 = one piece, at most
 // kPipeChunks; default 4) whose copies overlap the other chunks' traversal;
 // consecutive chunks trace on two streams so that one kernel's tail overlaps
-// the next one's start.  Measured on GB300 with 2^22 heightfield rays and
-// pinned buffers: 2.32 ms in one piece; 1.84 / 1.76 / 1.77 ms in 3 / 4 / 6
-// chunks (one compute stream: 1.82 / 1.87 / 2.04 ms).
+// the next one's start.  2^22 / 2^21 heightfield rays in pinned buffers, ms:
+// 1.70 / 0.92 in one piece; 1.34 / 0.72, 1.21 / 0.66, 1.09 / 0.69, 1.11 / 0.71
+// in 3, 4, 6, 8 chunks.
 constexpr uint32_t kPipeChunkMin = 1u << 18;
 constexpr uint32_t kPipeChunks = 8;
 constexpr uint32_t kStreamPieces = 16;  // streamed input (trace_streamed): pieces per call at most
@@ -369,11 +369,12 @@ static int pipe_streams(PbrtBVH* b) {
 // rays in coalesced rows once its last ray is done (HOSTOUT in trace.cu);
 // any-hit answers for host memory go through the staging buffer and one
 // copy of n bytes.  PBRT_STREAM_IN=0 (read at every call) takes the copy
-// pipeline instead.  Measured on GB300 with 2^22 heightfield rays (the walk
-// alone: 1.30 ms): closest hits 1.48 ms per call (pipeline 1.68 ms), any hit
-// 1.22 ms (1.40 ms); with device outputs 1.39 ms.  Over the pipeline's
-// per-piece launches it saves the tails each launch leaves (a 2^22-ray pass
-// in four launches spent 1.50 ms in kernels against 1.30 ms in one).
+// pipeline instead.  2^22 heightfield rays: closest hits 1.01 ms per call
+// (pipeline 1.21, the walk alone 0.69), any hit 0.90 (1.01, 0.60); with device
+// outputs 0.88.  With 8 / 16 / 32 / 64 pieces of 2^22 rays 0.94 / 1.01 / 1.00 /
+// 1.13 ms, of 2^21 0.58 / 0.58 / 0.65 / 0.65; pieces of 2^14 instead of 2^16 rays
+// at least take 2^18 rays from 0.18 to 0.23 ms.  Over the pipeline's launches it
+// saves the tails that each leaves.
 constexpr uint32_t kStreamShiftMin = 16;
 static bool stream_in_enabled() {
     const char* v = getenv("PBRT_STREAM_IN");

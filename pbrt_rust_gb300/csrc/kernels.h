@@ -55,11 +55,15 @@ int trace_stack_for_depth(uint32_t depth);
 // `kernel` >= 0 overrides the process-wide choice (PBRT_TRACE_*).  With
 // `order` (a permutation of [0, n)) the kernels take ray order[j] as their
 // j-th ray; hits still land at each ray's own index.  `work` is the 4-wide
-// persistent kernel's chunk counter (see trace_chunk).  `replay` (closest
-// hit: required; a device word, zero at launch) flags that some ray's binary
-// walk accepted a NaN distance; a replay kernel queued after such a traversal
-// then rewrites those rays' hits by the exact walk (see Traversal in
-// trace.cuh; the 4-wide kernels do so by themselves).
+// persistent kernel's chunk counter (see trace_chunk).  `replay` (required but
+// for kTraceSmall; a device word, zero at launch): a kernel that cannot finish
+// a ray marks it (kReplayMark as a hit's primitive, kReplayOcc as an any-hit
+// answer) and raises this flag; a replay kernel queued behind the traversal
+// rewrites the marked rays by the exact walk.  The binary kernels mark closest
+// hits at distance NaN (Traversal in trace.cuh), the persistent 4-wide ones,
+// for closest and any hit alike, every ray that is not theirs or that they
+// gave up (trace4.cuh); only the one-thread-per-ray 4-wide kernel walks such
+// rays itself.
 // `in.ready` (streamed input; needs `work` and trace_streams()): the rays
 // arrive in pieces of 2^in.shift rays while the walk runs, in.ready[k] (zero
 // at launch) turning non-zero once piece k has landed; a piece that has not

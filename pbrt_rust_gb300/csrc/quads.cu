@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(128) k_make_quads(const NodePair* __restrict__
                            : (kid[k]->b & kLeafBit ? (kNode4Leaf | kid[k]->a) : (quad_of[kid[k]->a] & kIndex));
     q.order = 0;
     for (uint32_t oct = 0; oct < 8; ++oct)
-        q.order |= (((oct >> axis[0]) & 1u) | (((oct >> axis[1]) & 1u) << 1) | (((oct >> axis_n) & 1u) << 2)) << (3 * oct);
+        q.order |= (((oct >> axis[0]) & 1u) | (((oct >> axis[1]) & 1u) << 1) | (((oct >> axis_n) & 1u) << 2))
+                   << (3 * oct);
     uint32_t low = 0, lo_w[3], hi_w[3];
     float org[3], scale[3];
     for (int i = 0; i < 3; ++i) {

@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(128) k_shadow_packet(RenderParams P) {
 
 // The first per_warp lanes of each warp have a ray (rays_per_warp).
 template <int OVF, bool INST>
-__global__ void __launch_bounds__(128, INST ? 6 : 9) k_shadow4(const __grid_constant__ RenderParams P, uint32_t per_warp) {
+__global__ void __launch_bounds__(128, INST ? 6 : 9)
+    k_shadow4(const __grid_constant__ RenderParams P, uint32_t per_warp) {
     using Walk = Walk4<128, 16, OVF, true, INST>;
     __shared__ typename Walk::Shared sh;
     sh.init();
@@ -94,7 +95,8 @@ __global__ void __launch_bounds__(128, INST ? 6 : 9) k_shadow4(const __grid_cons
     T.bind(sh);
     const int st = T.start(P.bvh4, ray[0], ray[1]);
     if (st == kStartWalk) T.run(P.bvh4, sh, ov);
-    P.occluded[P.shadow_slot[q]] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
+    const bool exact = st == kStartExact || T.gave_up();
+    P.occluded[P.shadow_slot[q]] = (exact ? exact_any<OVF + 8, INST>(P.bvh, ray, status) : T.found()) ? 1 : 0;
 }
 
 // k_shadow4 with persistent warps that take kShadowChunk rays of the queue at a
@@ -297,13 +299,16 @@ cudaError_t launch_render(const RenderParams& P, cudaStream_t s) {
             // variant covers its stack bound, else the binary one
             const bool inst = P.bvh.insts != nullptr;
             const int iv = (inst && P.has_wide) ? wide_stack_variant(P.wide_bound) : 0;
-            const bool wide_rk = rk == PBRT_TRACE_WIDE || rk == PBRT_TRACE_WIDE_PERSISTENT || rk == PBRT_TRACE_WIDE_SPECULATIVE;
+            const bool wide_rk =
+                rk == PBRT_TRACE_WIDE || rk == PBRT_TRACE_WIDE_PERSISTENT || rk == PBRT_TRACE_WIDE_SPECULATIVE;
             int wv = (P.has_wide && wide_rk && !inst) ? wide_stack_variant(P.wide_bound) : 0;
             const bool refill = shadow_refills(P, max_shadow);
             if (refill && (iv == 64 || wv == 64))
-                e = iv ? launch_shadow_refill<64, true>(P, max_shadow, s) : launch_shadow_refill<64, false>(P, max_shadow, s);
+                e = iv ? launch_shadow_refill<64, true>(P, max_shadow, s)
+                       : launch_shadow_refill<64, false>(P, max_shadow, s);
             else if (refill && (iv == 256 || wv == 256))
-                e = iv ? launch_shadow_refill<256, true>(P, max_shadow, s) : launch_shadow_refill<256, false>(P, max_shadow, s);
+                e = iv ? launch_shadow_refill<256, true>(P, max_shadow, s)
+                       : launch_shadow_refill<256, false>(P, max_shadow, s);
             else if (iv == 64)
                 k_shadow4<64, true><<<grid4, 128, 0, s>>>(P, pw);
             else if (iv == 256)

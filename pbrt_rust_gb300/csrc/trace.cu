@@ -161,10 +161,11 @@ __global__ void __launch_bounds__(kWalkBlock, INST ? 6 : (ANY ? 9 : 8)) k_trace4
     T.bind(sh);
     const int st = T.start(bvh, __ldg(ray), __ldg(ray + 1));
     if (st == kStartWalk) T.run(bvh, sh, ov);
+    const bool exact = st == kStartExact || T.gave_up();
     if (ANY)
-        occ[i] = (st == kStartExact || T.gave_up() ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
+        occ[i] = (exact ? exact_any<OVF + 8, INST>(bvh.pair, ray, status) : T.found()) ? 1 : 0;
     else
-        hits[i] = st == kStartExact || T.gave_up() ? exact_hit<OVF + 8, INST>(bvh.pair, ray, status) : T.hit_record();
+        hits[i] = exact ? exact_hit<OVF + 8, INST>(bvh.pair, ray, status) : T.hit_record();
 }
 
 // A ray is read once: its lines go to L2 only, leaving L1 to the tree.
@@ -472,10 +473,10 @@ static void read_variant() {
 // 128 3 to 5 us.
 constexpr int kReplayBlock = 512;
 template <int STACK, bool INST>
-__global__ void __launch_bounds__(kReplayBlock) k_replay2(const __grid_constant__ DevBVH bvh, const float4* __restrict__ rays,
-                                                 uint32_t n, float4* __restrict__ hits, uint8_t* __restrict__ occ,
-                                                 const uint32_t* __restrict__ replay, int* __restrict__ status,
-                                                 float4* __restrict__ host_hits) {
+__global__ void __launch_bounds__(kReplayBlock)
+    k_replay2(const __grid_constant__ DevBVH bvh, const float4* __restrict__ rays, uint32_t n,
+              float4* __restrict__ hits, uint8_t* __restrict__ occ, const uint32_t* __restrict__ replay,
+              int* __restrict__ status, float4* __restrict__ host_hits) {
     if (*(const volatile uint32_t*)replay == 0u) return;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         if (occ) {
@@ -563,7 +564,8 @@ static cudaError_t launch_wide(const DevBVH4& bvh, const float4* r4, uint32_t n,
                : occ     ? pt(launch_wide_persistent<OVF, true, true>)
                          : pt(launch_wide_persistent<OVF, false, true>);
     if (host_hits) return pt(launch_wide_persistent<OVF, false, false, true>);
-    if (persistent) return occ ? pt(launch_wide_persistent<OVF, true, false>) : pt(launch_wide_persistent<OVF, false, false>);
+    if (persistent)
+        return occ ? pt(launch_wide_persistent<OVF, true, false>) : pt(launch_wide_persistent<OVF, false, false>);
     const uint32_t per_warp = rays_per_warp(n);
     const uint64_t per_block = (uint64_t)per_warp * (kWalkBlock / 32);
     const unsigned grid = (unsigned)((n + per_block - 1) / per_block);
@@ -651,7 +653,7 @@ int trace_stack_for_depth(uint32_t depth) {
     return 0;
 }
 
-// *replays: the launch marks rays for the replay kernel (the binary kernels).
+// *replays: the launch marks rays for the replay kernel.
 static cudaError_t launch_main(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays, uint32_t n, PbrtHit* hits,
                                uint8_t* occluded, int* d_status, cudaStream_t stream, const DevBVH4* wide,
                                uint32_t wide_bound, int kernel, const uint32_t* order, uint32_t* work,
@@ -777,7 +779,9 @@ cudaError_t launch_trace(const DevBVH& bvh, uint32_t depth, const PbrtRay* rays,
     float4* h4 = reinterpret_cast<float4*>(hits);
     const bool inst = bvh.insts != nullptr;
     float4* hh = reinterpret_cast<float4*>(host_hits);
-    auto go = [&](auto kernel) { kernel<<<grid, kReplayBlock, 0, stream>>>(bvh, r4, n, h4, occluded, replay, d_status, hh); };
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kReplayBlock, 0, stream>>>(bvh, r4, n, h4, occluded, replay, d_status, hh);
+    };
     if (trace_stack_for_depth(depth) == 64)
         inst ? go(k_replay2<64, true>) : go(k_replay2<64, false>);
     else

@@ -33,9 +33,9 @@
 //    moved towards the ray's start and the far planes away from it by
 //    e = u i (6 |c - o| + 32 h);
 //  * an axis with d = 0 has 1 / d replaced by kZeroInv, so large that e, here
-//    of all three axes' sums, is beyond every other distance: a plane at the origin or within e / i of it
-//    never culls, one farther off does.  The exact test has +-inf there, as
-//    the reference.
+//    of all three axes' sums, is beyond every other distance: a plane at the
+//    origin or within e / i of it never culls, one farther off does.  The
+//    exact test has +-inf there, as the reference.
 // One box may pass where a box above it does not: with d = -0 the reference
 // rejects an origin on the boundary of a box, unless the box is flat there.  A
 // triangle of such a flat leaf is not hit (its determinant is 0); an analytic
@@ -64,8 +64,9 @@
 // planes lie the wrong way round, but in a node smaller than the margins it
 // passes all the same and takes entries beyond the bound, so a walk may find
 // its stack full; it then gives up and the ray takes the exact walk, whose
-// entries (one per level at most) the bound does cover.  The bottom entry is a word that
-// ends the walk, so a pop needs no test for an empty stack.  A visit stores
+// entries (one per level at most) the bound does cover.  The bottom entry is a
+// word that ends the walk, so a pop needs no test for an empty stack.  A visit
+// stores
 // all four children without branches: a 128-word table in shared memory,
 // indexed by the node's visiting order for the ray's octant and the mask of
 // passing children, gives each child's place above the top (children that
@@ -301,7 +302,8 @@ struct Walk4 : InstWalk<INST> {
         return margins(tree, zx, zy, zz) && ok;
     }
     __device__ __forceinline__ void octant() {
-        oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) | ((__float_as_uint(iz) >> 31) << 2));
+        oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) |
+                     ((__float_as_uint(iz) >> 31) << 2));
     }
     // false: too far away, or a NaN in the origin.
     __device__ __forceinline__ bool margins(const DevBVH4& tree, bool zx, bool zy, bool zz) {
