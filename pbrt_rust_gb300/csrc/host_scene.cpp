@@ -513,8 +513,9 @@ static void fill_device_layout(HostBVH& H) {
             H.wide = false;
             break;
         }
-        set_flags(H.recs[nd.offset],
-                  (entry ? kPrimBoxEntry : kPrimHitBox) | ((uint32_t)H.leaf_boxes.size() << kPrimBoxShift));
+        set_flags(H.recs[nd.offset], entry ? kPrimBoxEntry : kPrimHitBox);
+        for (uint32_t i = 0; i < nd.count; ++i)
+            set_flags(H.recs[nd.offset + i], (uint32_t)H.leaf_boxes.size() << kPrimBoxShift);
         const Box& b = nd.box;
         H.leaf_boxes.push_back(LeafBox{{b.lo.x, b.lo.y, b.lo.z, 0.0f}, {b.hi.x, b.hi.y, b.hi.z, 0.0f}});
     }

@@ -93,6 +93,7 @@ constexpr uint32_t kNode4Leaf = 0x80000000u;
 //                  when the triangle is hit
 //   kPrimHitBox    a leaf of one analytic shape: the box in the table, tested
 //                  when the shape is hit
+// Every record of a leaf with a box in the table carries the box's index.
 struct alignas(16) PrimRec {
     float r0[4];
     float r1[4];

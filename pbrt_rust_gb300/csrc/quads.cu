@@ -364,9 +364,10 @@ __global__ void __launch_bounds__(kLayoutBlock) k_layout_fill(const FlatNode* __
         const HostPrim& p = prims[ref];
         uint32_t id = flat_id ? flat_id[ref] : ref, flags = i + 1 == nd.count ? kPrimLastBit : 0u;
         const bool tri = p.kind == PBRT_SHAPE_TRIANGLE_MESH;
+        if (cls[k] & kClassBoxed) flags |= rank[k] << kPrimBoxShift;
         if (i == 0 && (cls[k] & kClassBoxed)) {
             const bool entry = nd.count > 1 || spheres[p.sphere].kind == kQuadInstance;
-            flags |= (entry ? kPrimBoxEntry : kPrimHitBox) | (rank[k] << kPrimBoxShift);
+            flags |= entry ? kPrimBoxEntry : kPrimHitBox;
             float4* out = reinterpret_cast<float4*>(boxes + rank[k]);
             out[0] = make_float4(nd.box.lo.x, nd.box.lo.y, nd.box.lo.z, 0.0f);
             out[1] = make_float4(nd.box.hi.x, nd.box.hi.y, nd.box.hi.z, 0.0f);

@@ -94,7 +94,7 @@ struct DevBVH4 {
     const QuadNode* nodes;
     const LeafBox* boxes;
     uint32_t root_ref;      // the root's child word
-    float4 mid, half, spread;  // HostBVH::middle (w: far), ::half, ::spread
+    float4 mid, half, spread;  // HostBVH::middle (w: far), ::half, ::spread (w: its sum)
 };
 
 // Stack words that are not children (leaf words stay below: HostBVH::wide
@@ -285,7 +285,10 @@ struct Walk4 : InstWalk<INST> {
     }
 
     // 1 / d, octant and margins of the ray (o, d) in a tree; false if the ray
-    // is not clean or too far away (see above).
+    // is not clean or too far away (see above).  Inside an instance (DEF) all
+    // axes get the sum's margin: the definition's record is read afresh at
+    // every entry, and this needs less of it.
+    template <bool DEF>
     __device__ __forceinline__ bool aim(const DevBVH4& tree) {
         const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
         ix = 1.0f / dx;
@@ -299,14 +302,24 @@ struct Walk4 : InstWalk<INST> {
         if (zy) iy = copysignf(kZeroInv, dy);
         if (zz) iz = copysignf(kZeroInv, dz);
         octant();
-        return margins(tree, zx, zy, zz) && ok;
+        return margins<DEF>(tree, zx, zy, zz) && ok;
     }
     __device__ __forceinline__ void octant() {
         oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) |
                      ((__float_as_uint(iz) >> 31) << 2));
     }
     // false: too far away, or a NaN in the origin.
+    template <bool DEF>
     __device__ __forceinline__ bool margins(const DevBVH4& tree, bool zx, bool zy, bool zz) {
+        if constexpr (DEF) {
+            const float4 mid = tree.mid;
+            const float all = __fmaf_rn(kFarMargin, fabsf(mid.x - ox) + fabsf(mid.y - oy) + fabsf(mid.z - oz),
+                                        tree.spread.w);
+            ex = all * fabsf(ix);
+            ey = all * fabsf(iy);
+            ez = all * fabsf(iz);
+            return all <= mid.w;
+        }
         const float4 mid = tree.mid, spread = tree.spread;
         const float mx = __fmaf_rn(kFarMargin, fabsf(mid.x - ox), spread.x),
                     my = __fmaf_rn(kFarMargin, fabsf(mid.y - oy), spread.y),
@@ -356,7 +369,7 @@ struct Walk4 : InstWalk<INST> {
             this->base_ = 0;
         }
         if (bvh.pair.empty) return kStartMiss;
-        if (!aim(bvh)) return kStartExact;
+        if (!aim<false>(bvh)) return kStartExact;
         // the root's box, from its middle, with the same margins (this form's
         // rounding: u i (5 |c - o| + 4 h) against the reference's)
         const float tx = (bvh.mid.x - ox) * ix, rx = __fmaf_rn(bvh.half.x, fabsf(ix), ex);
@@ -486,11 +499,20 @@ struct Walk4 : InstWalk<INST> {
         stop();
     }
 
+    // Whether a leaf's box, which the ray passes, is flat where the ray's
+    // direction (of reciprocals i) is -0: a box above it need not pass then.
+    __device__ __forceinline__ static bool beside(const LeafBox* box, float i_x, float i_y, float i_z) {
+        if (min3f(i_x, i_y, i_z) != -kZeroInv) return false;
+        const float4 lo = ldg4(box->lo), hi = ldg4(box->hi);
+        return (i_x == -kZeroInv && lo.x == hi.x) || (i_y == -kZeroInv && lo.y == hi.y) ||
+               (i_z == -kZeroInv && lo.z == hi.z);
+    }
+
     // INST: the instance record S (first id `first`) of the scene's tree;
-    // `rest` is the leaf word of the rest of its leaf (0: none).  1 when its
-    // walk was entered (`cur` set), 0 when the ray misses it, 2 when the
-    // primitive-space ray is not clean: the whole ray then takes the exact
-    // walk.  TransformedPrimitive::intersect
+    // `rest` is the leaf word of the rest of its leaf (0: none), `box` the
+    // leaf's.  1 when its walk was entered (`cur` set), 0 when the ray misses
+    // it, 2 when the primitive-space ray is not clean or the leaf's box flat
+    // beside it: the whole ray then takes the exact walk.  TransformedPrimitive::intersect
     // (transformed.rs:35-56): the primitive-space ray is w2p(ray) - o as a
     // point, d as a vector, mint and the current maxt kept.  If it passes the
     // definition's root box, the walk pushes the rest of the leaf and an exit
@@ -500,7 +522,7 @@ struct Walk4 : InstWalk<INST> {
     // searched completely, in the reference's order, before the leaf's next
     // primitive, and the shared maxt is the reference's ray.set_maxt.
     __device__ __forceinline__ int enter(const DevBVH4& bvh, Shared& sh, const SphereRec* S, uint32_t first,
-                                         uint32_t rest) {
+                                         uint32_t rest, const LeafBox* box) {
         const DevBVH4& D = bvh.pair.insts[S->instance];
         if (D.pair.empty) return 0;
         float o[3], d[3];
@@ -518,11 +540,12 @@ struct Walk4 : InstWalk<INST> {
         dz = d[2];
         const ChildRec& R = D.pair.root;
         float tr;
-        if (!aim(D)) return 2;
+        if (!aim<true>(D)) return 2;
         if (!slab(R.lo_x, R.lo_y, R.lo_z, R.hi_x, R.hi_y, R.hi_z, ray(), maxt, &tr)) {
             restore(bvh, sh);
             return 0;
         }
+        if (beside(box, w[6 * BLOCK], w[7 * BLOCK], w[8 * BLOCK])) return 2;
         if (rest) {
             st_entry(top, rest, __int_as_float(0xff800000));
             top += kRow;
@@ -594,21 +617,7 @@ struct Walk4 : InstWalk<INST> {
                 float tr;
                 return slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, ray(), maxt, &tr);
             };
-            // Gives up if the leaf's box, the one of flag word f, is flat where
-            // the direction is -0: a box above it need not pass.  Asked for
-            // when an analytic shape is hit, or an instance's leaf entered.
-            auto beside = [&](uint32_t f) {
-                if (min3f(ix, iy, iz) != -kZeroInv) return false;
-                const LeafBox* b = boxes + (f >> kPrimBoxShift);
-                const float4 lo = ldg4(b->lo), hi = ldg4(b->hi);
-                if (!((ix == -kZeroInv && lo.x == hi.x) || (iy == -kZeroInv && lo.y == hi.y) ||
-                      (iz == -kZeroInv && lo.z == hi.z)))
-                    return false;
-                give_up();
-                return true;
-            };
             if ((flags & kPrimBoxEntry) && !table_box()) break;
-            if (INST && (flags & kPrimBoxEntry) && beside(flags)) break;
             float t, u = 0.0f, v = 0.0f;
             bool hit;
             if (id & kSphereBit) {
@@ -617,7 +626,8 @@ struct Walk4 : InstWalk<INST> {
                     const SphereRec* S = spheres + si;
                     if (S->kind == kQuadInstance) {  // only in the scene's tree: definitions hold none
                         const int e = enter(bvh, sh, S, id & ~kSphereBit,
-                                            (flags & kPrimLastBit) ? 0u : (kNode4Leaf | (off + 1)));
+                                            (flags & kPrimLastBit) ? 0u : (kNode4Leaf | (off + 1)),
+                                            boxes + (flags >> kPrimBoxShift));
                         if (e == 1) return make_room(ov);
                         if (e == 2) return give_up();
                         if (flags & kPrimLastBit) break;
@@ -627,10 +637,10 @@ struct Walk4 : InstWalk<INST> {
                 }
                 hit = sphere_test(spheres, si, ray(), maxt, &t);
                 if (hit && (flags & kPrimHitBox)) hit = table_box();
-                if (hit && (flags & kPrimHitBox) && beside(flags)) break;
-                if (!INST && hit && !(flags & kPrimHitBox) &&
-                    beside(__float_as_uint(__ldg(&prims[cur & ~kNode4Leaf].r2[3]))))
+                if (hit && beside(boxes + (flags >> kPrimBoxShift), ix, iy, iz)) {
+                    give_up();
                     break;
+                }
             } else {
                 hit = tri_test(r0, r1, r2, ray(), maxt, &t, &u, &v);
                 if (hit && (flags & kPrimOwnBox)) {
