@@ -648,6 +648,13 @@ struct Walk4 : InstWalk<INST> {
                     hit = slab(fminf(fminf(r0.x, r1.x), r2.x), fminf(fminf(r0.y, r1.y), r2.y),
                                fminf(fminf(r0.z, r1.z), r2.z), fmaxf(fmaxf(r0.x, r1.x), r2.x),
                                fmaxf(fmaxf(r0.y, r1.y), r2.y), fmaxf(fmaxf(r0.z, r1.z), r2.z), ray(), maxt, &tr);
+                    // A hit whose box a direction of -0 rejects (the origin is
+                    // on its boundary): the boxes above are likely rejected
+                    // too, and without hits nothing here would be culled.
+                    if (!hit && min3f(ix, iy, iz) == -kZeroInv) {
+                        give_up();
+                        break;
+                    }
                 }
             }
             if (hit) {
