@@ -125,7 +125,7 @@ static DevBVH4 device_tree(const HostBVH& H, const NodePair* pairs, const QuadNo
     d.root_ref = H.quad_root;
     d.mid = make_float4(H.middle.x, H.middle.y, H.middle.z, H.far);
     d.half = make_float4(H.half.x, H.half.y, H.half.z, 0.0f);
-    d.spread = make_float4(H.spread.x, H.spread.y, H.spread.z, H.spread.x + H.spread.y + H.spread.z);
+    d.spread = make_float4(H.spread.x, H.spread.y, H.spread.z, 0.0f);
     return d;
 }
 

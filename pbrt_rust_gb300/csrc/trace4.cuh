@@ -94,7 +94,7 @@ struct DevBVH4 {
     const QuadNode* nodes;
     const LeafBox* boxes;
     uint32_t root_ref;      // the root's child word
-    float4 mid, half, spread;  // HostBVH::middle (w: far), ::half, ::spread (w: its sum)
+    float4 mid, half, spread;  // HostBVH::middle (w: far), ::half, ::spread
 };
 
 // Stack words that are not children (leaf words stay below: HostBVH::wide
@@ -285,10 +285,10 @@ struct Walk4 : InstWalk<INST> {
     }
 
     // 1 / d, octant and margins of the ray (o, d) in a tree; false if the ray
-    // is not clean or too far away (see above).  Inside an instance (DEF) all
-    // axes get the sum's margin: the definition's record is read afresh at
-    // every entry, and this needs less of it.
-    template <bool DEF>
+    // is not clean or too far away (see above).  (One margin for all axes
+    // inside instances, which reads less of the definition's record, makes
+    // entries 1 % cheaper and lets far rays visit up to three times as much: 2^20
+    // rays from 3000 extents into 64 instances 570 -> 726 us.)
     __device__ __forceinline__ bool aim(const DevBVH4& tree) {
         const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
         ix = 1.0f / dx;
@@ -302,24 +302,14 @@ struct Walk4 : InstWalk<INST> {
         if (zy) iy = copysignf(kZeroInv, dy);
         if (zz) iz = copysignf(kZeroInv, dz);
         octant();
-        return margins<DEF>(tree, zx, zy, zz) && ok;
+        return margins(tree, zx, zy, zz) && ok;
     }
     __device__ __forceinline__ void octant() {
         oct3 = 3u * ((__float_as_uint(ix) >> 31) | ((__float_as_uint(iy) >> 31) << 1) |
                      ((__float_as_uint(iz) >> 31) << 2));
     }
     // false: too far away, or a NaN in the origin.
-    template <bool DEF>
     __device__ __forceinline__ bool margins(const DevBVH4& tree, bool zx, bool zy, bool zz) {
-        if constexpr (DEF) {
-            const float4 mid = tree.mid;
-            const float all = __fmaf_rn(kFarMargin, fabsf(mid.x - ox) + fabsf(mid.y - oy) + fabsf(mid.z - oz),
-                                        tree.spread.w);
-            ex = all * fabsf(ix);
-            ey = all * fabsf(iy);
-            ez = all * fabsf(iz);
-            return all <= mid.w;
-        }
         const float4 mid = tree.mid, spread = tree.spread;
         const float mx = __fmaf_rn(kFarMargin, fabsf(mid.x - ox), spread.x),
                     my = __fmaf_rn(kFarMargin, fabsf(mid.y - oy), spread.y),
@@ -369,7 +359,7 @@ struct Walk4 : InstWalk<INST> {
             this->base_ = 0;
         }
         if (bvh.pair.empty) return kStartMiss;
-        if (!aim<false>(bvh)) return kStartExact;
+        if (!aim(bvh)) return kStartExact;
         // the root's box, from its middle, with the same margins (this form's
         // rounding: u i (5 |c - o| + 4 h) against the reference's)
         const float tx = (bvh.mid.x - ox) * ix, rx = __fmaf_rn(bvh.half.x, fabsf(ix), ex);
@@ -540,7 +530,7 @@ struct Walk4 : InstWalk<INST> {
         dz = d[2];
         const ChildRec& R = D.pair.root;
         float tr;
-        if (!aim<true>(D)) return 2;
+        if (!aim(D)) return 2;
         if (!slab(R.lo_x, R.lo_y, R.lo_z, R.hi_x, R.hi_y, R.hi_z, ray(), maxt, &tr)) {
             restore(bvh, sh);
             return 0;
